@@ -950,6 +950,24 @@ inline int make_plane_map(EncodeTiledFn enc, CUtensorMap* map, const void* base,
     return r == CUDA_SUCCESS ? 0 : -1;
 }
 
+// Blocks per macro tile of k2 (at most `most`).  A taller macro tile re-primes its march less often (nb + 1 blocks of work
+// for nb tiles) but gives fewer, coarser units to spread over the SMs: take the height with the best product of the two.
+// -> macro tiles of the launch.
+inline long long k2_macro_tiles(const Geom& g, int strips, int most, int num_sms, int& nbmax, int& mt_per_grid) {
+    long long total_mt = 0;
+    double best = -1.0;
+    const int rows4 = (g.H + k2m::BR - 1) / k2m::BR;
+    for (int nb = most; nb >= 1; --nb) {
+        const int mt_rows = (rows4 + nb - 1) / nb;
+        const long long total = (long long)strips * mt_rows * g.B;
+        const double per_mt = (double)rows4 / mt_rows;                         // tiles per macro tile on average
+        const long long waves = (total + num_sms - 1) / num_sms;
+        const double eff = per_mt / (per_mt + 1.0) * (double)total / (double)(waves * num_sms);
+        if (eff > best) { best = eff; nbmax = nb; mt_per_grid = strips * mt_rows; total_mt = total; }
+    }
+    return total_mt;
+}
+
 // Tensor maps over the weight arrays and the E/V planes, and the kernels' shared-memory opt-in.  0 on success.
 inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16* wo, int sets, const __nv_bfloat16* E,
                       const __nv_bfloat16* V, const __nv_bfloat16* X, const Geom& g, int num_sms) {
@@ -1001,19 +1019,7 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
     }
     const long long total1 = (long long)p.k1_tiles * g.B;
     p.k1_grid = (int)(total1 < num_sms ? total1 : num_sms);
-    // k2: blocks per macro tile.  A taller macro tile re-primes its march less often (nb + 1 blocks of work for nb
-    // tiles) but gives fewer, coarser units to spread over the SMs: take the height with the best product of the two.
-    long long total_mt = 0;
-    double best = -1.0;
-    const int rows4 = (g.H + k2m::BR - 1) / k2m::BR;
-    for (int nb = k2m::NB; nb >= 1; nb >>= 1) {
-        const int mt_rows = (rows4 + nb - 1) / nb;
-        const long long total = (long long)p.strips * mt_rows * g.B;
-        const double per_mt = (double)rows4 / mt_rows;                         // tiles per macro tile on average
-        const long long waves = (total + num_sms - 1) / num_sms;
-        const double eff = per_mt / (per_mt + 1.0) * (double)total / (double)(waves * num_sms);
-        if (eff > best) { best = eff; p.nbmax = nb; p.mt_per_grid = p.strips * mt_rows; total_mt = total; }
-    }
+    const long long total_mt = k2_macro_tiles(g, p.strips, k2m::NB, num_sms, p.nbmax, p.mt_per_grid);
     p.k2_grid = (int)(total_mt < num_sms ? total_mt : num_sms);
     return 0;
 }

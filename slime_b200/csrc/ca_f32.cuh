@@ -1,257 +1,809 @@
-// fp32 path of the CA step: two SIMT kernels per step, exact expf and division, fp32 FMA accumulation.
-// This is the path held to 1e-5 relative L2 against the CPU oracle.
+// fp32 path of the CA step: fp32 storage of state and intermediates, exact expf and division, fp32 sums.  This is the
+// path held to 1e-5 relative L2 against the CPU oracle.  The same two-kernel split as the bf16 path (ca_bf16.cuh), and
+// like there the projections run on the 5th-generation tensor cores:
 //
-//   k1_f32  reads the state with a 1-cell halo, applies the pending per-channel scale, forms for every head
-//           the 3x3-convolved input (the stencil commutes with the linear perception projection, so
-//           conv_h(X) Wp_h = conv_h(X Wp_h)), projects to U | I | V (64 -> 3x64 per head), applies the growth
-//           bell and writes E = exp(G*I) and V, per-head planar [B][8][rows][W][64].
-//   k2_f32  reads E with a 2-cell halo and V with a 1-cell halo, Z = box3(E), R = V/Z, V' = E*box3(R)
-//           (the closed form of the per-source softmax redistribution), projects concat_h(V') with Wo,
-//           writes X+ = scale*X + dt*Y in place and one per-channel partial sum per tile.
+//   every fp32 operand is the exact sum of three bf16 values, x = hi + mid + lo (8 + 8 + 8 bits of mantissa, split3
+//   below), so a product of two operands is the sum of nine bf16 products, each exact in the fp32 accumulator.  Six of
+//   them are formed: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  The three left out (mid lo, lo mid, lo lo) are
+//   together below 2^-26 of the product, i.e. below a quarter of the rounding error of one fp32 product.
+//   The tensor core rounds its accumulator towards zero after every instruction (measured: 25 fraction bits are kept
+//   inside one K = 16 step, then the sum is truncated to fp32), so the products are issued smallest first and a sum
+//   stays on the tensor core for K = 64 (k1) or K = 32 (k2) at most - only the last two to four instructions then
+//   truncate at the sum's own magnitude - and longer sums are continued in registers, rounded to nearest.
+//   Against the fp64 oracle this is as accurate as the fp32 fused multiply-add loops it replaced.
+//
+//   k1_f32  reads the state with a 1-cell halo, applies the pending per-channel scale, forms for every head the
+//           3x3-convolved input (the stencil commutes with the linear perception projection), projects to U | I | V
+//           (64 -> 3x64 per head), applies the growth bell and writes E = exp(G*I) and V.
+//   k2_f32  Z = box3(E), R = V/Z, V' = E*box3(R) (the closed form of the per-source softmax redistribution), projects
+//           concat_h(V') with Wo, writes X+ = scale*X + dt*Y in place and one per-channel partial sum per tile.
+//
+// E/V planes are [B][8][H+4][W+4][64] fp32 with the same 2-cell apron of wrapped copies as the bf16 planes.
 // The per-channel renormalisation is lazy: the stored state is un-normalised and the next k1 applies
 // scale[b][c] = mass / sum when it loads.
 #pragma once
+#include <cuda.h>
+
+#include "ca_bf16.cuh"
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace slime {
 
-constexpr int T32 = 8;                 // tile edge of the fp32 kernels (64 cells)
-constexpr int XS32 = 68;               // padded cell stride in floats (keeps float4 alignment, breaks bank ties)
-constexpr int K1F32_SMEM = (100 * XS32 + 64 * XS32 + 64 * 192 + 16) * 4;
-constexpr int K2F32_SMEM = (144 * 64 + 100 * 64 + 64 * XS32 + 64 * 64 + 2 * 16 * 64) * 4;   // the last term: [16][64] doubles
+struct F32Plan {
+    int tiles_x = 1, k1_tiles = 1, k2_tiles = 1, k1_grid = 1, k2_grid = 1;
+    CUtensorMap map_w1;       // [sets*8*3*192][64] bf16 (parts of Wp | Wi | Wv), box 64 x 64, 128B swizzle
+    CUtensorMap map_wo;       // [sets*16*3*64][32] bf16 (parts of Wo), box 32 x 192, 64B swizzle
+    CUtensorMap map_e;        // E planes, box 32 x 36 x 4 x 1 (a block of k2: half a head's dims)
+    CUtensorMap map_v;        // V planes, box 32 x 34 x 4 x 1
+    CUtensorMap map_x;        // the state, box 32 x 32 x 4 x 1, 128B swizzle
+    CUtensorMap map_es, map_vs;   // stores of k1: box 16 x 16 x 2 x 1, 64B swizzle
+    int strips = 1, mt_per_grid = 1, nbmax = 6;
+};
 
-__global__ void __launch_bounds__(256)
-k1_f32(const float* __restrict__ X, const float* __restrict__ scale, const float* __restrict__ Wpiv,
-       const float* __restrict__ prm, float* __restrict__ E, float* __restrict__ V, Geom g) {
-    extern __shared__ __align__(16) float sm[];
-    float* xh = sm;                    // [10*10][XS32]  state halo tile, scale applied
-    float* ac = xh + 100 * XS32;       // [64][XS32]     convolved input of the current head
-    float* ws = ac + 64 * XS32;        // [64][192]      Wp | Wi | Wv rows of the current head
-    float* ps = ws + 64 * 192;         // [PRM]
-
-    const int tid = threadIdx.x;
-    const int b = blockIdx.y;
-    const int tx0 = (blockIdx.x % g.tiles_x) * T32;
-    const int ty0 = (blockIdx.x / g.tiles_x) * T32 - g.he;
-    const int set = b / g.per_set;
-    const size_t xplane = (size_t)g.state_rows() * g.W * NC;
-    const size_t eplane = (size_t)g.ev_rows() * g.W * HD;
-
-    for (int i = tid; i < 100 * 16; i += 256) {
-        const int cell = i >> 4, q = i & 15;
-        const int r = ty0 + cell / 10 - 1, x = g.wrap_x(tx0 + cell % 10 - 1);
-        float4 v = *reinterpret_cast<const float4*>(X + (size_t)b * xplane + ((size_t)g.xrow(r) * g.W + x) * NC + q * 4);
-        const float4 s = *reinterpret_cast<const float4*>(scale + b * NC + q * 4);
-        v.x *= s.x; v.y *= s.y; v.z *= s.z; v.w *= s.w;
-        *reinterpret_cast<float4*>(xh + cell * XS32 + q * 4) = v;
-    }
-
-    const int cg = tid >> 4;           // 16 groups of 4 cells (half a tile row each)
-    const int d0 = (tid & 15) * 4;     // 4 output dims
-
-    for (int h = 0; h < NH; ++h) {
-        __syncthreads();               // previous head done with ac / ws; first pass: xh complete
-        const float* wsrc = Wpiv + ((size_t)set * NH + h) * NC * 192;
-        for (int i = tid; i < 64 * 192 / 4; i += 256)
-            reinterpret_cast<float4*>(ws)[i] = reinterpret_cast<const float4*>(wsrc)[i];
-        if (tid < PRM) ps[tid] = prm[((size_t)set * NH + h) * PRM + tid];
-        __syncthreads();
-        for (int i = tid; i < 64 * 64; i += 256) {
-            const int c = i & 63, cell = i >> 6;
-            const int cy = cell >> 3, cx = cell & 7;
-            float a = 0.f;
-#pragma unroll
-            for (int t = 0; t < 9; ++t)
-                a = fmaf(ps[t], xh[((cy + t / 3) * 10 + cx + t % 3) * XS32 + c], a);
-            ac[cell * XS32 + c] = a;
-        }
-        __syncthreads();
-
-        float u[4][4], iv[4][4], vv[4][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) u[j][k] = iv[j][k] = vv[j][k] = 0.f;
-
-        for (int k4 = 0; k4 < 16; ++k4) {
-            float4 a4[4], x4[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int cell = cg * 4 + j;
-                a4[j] = *reinterpret_cast<const float4*>(ac + cell * XS32 + k4 * 4);
-                x4[j] = *reinterpret_cast<const float4*>(xh + (((cell >> 3) + 1) * 10 + (cell & 7) + 1) * XS32 + k4 * 4);
-            }
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                const float* wr = ws + (k4 * 4 + kk) * 192 + d0;
-                const float4 wp = *reinterpret_cast<const float4*>(wr);
-                const float4 wi = *reinterpret_cast<const float4*>(wr + 64);
-                const float4 wv = *reinterpret_cast<const float4*>(wr + 128);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float a = kk == 0 ? a4[j].x : kk == 1 ? a4[j].y : kk == 2 ? a4[j].z : a4[j].w;
-                    const float x = kk == 0 ? x4[j].x : kk == 1 ? x4[j].y : kk == 2 ? x4[j].z : x4[j].w;
-                    u[j][0] = fmaf(a, wp.x, u[j][0]); u[j][1] = fmaf(a, wp.y, u[j][1]);
-                    u[j][2] = fmaf(a, wp.z, u[j][2]); u[j][3] = fmaf(a, wp.w, u[j][3]);
-                    iv[j][0] = fmaf(x, wi.x, iv[j][0]); iv[j][1] = fmaf(x, wi.y, iv[j][1]);
-                    iv[j][2] = fmaf(x, wi.z, iv[j][2]); iv[j][3] = fmaf(x, wi.w, iv[j][3]);
-                    vv[j][0] = fmaf(x, wv.x, vv[j][0]); vv[j][1] = fmaf(x, wv.y, vv[j][1]);
-                    vv[j][2] = fmaf(x, wv.z, vv[j][2]); vv[j][3] = fmaf(x, wv.w, vv[j][3]);
-                }
-            }
-        }
-
-        const float mu = ps[9], nis = ps[10];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int cell = cg * 4 + j;
-            const int r = ty0 + (cell >> 3), x = tx0 + (cell & 7);
-            if (r >= g.H + g.he || x >= g.W) continue;
-            float4 e, vo;
-            float* ep = &e.x;
-            float* vp = &vo.x;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float z = u[j][k] - mu;
-                const float gr = 2.f * expf(z * z * nis) - 1.f;
-                ep[k] = expf(fminf(fmaxf(gr * iv[j][k], -ACT_CLAMP), ACT_CLAMP));
-                vp[k] = vv[j][k];
-            }
-            const size_t o = ((size_t)b * NH + h) * eplane + ((size_t)g.erow(r) * g.W + x) * HD + d0;
-            *reinterpret_cast<float4*>(E + o) = e;
-            *reinterpret_cast<float4*>(V + o) = vo;
-        }
-    }
+// x = hi + mid + lo, exactly: hi is x rounded to bf16, mid the rest rounded to bf16, lo what is left (at most 7 bits).
+// Two values at a time; each result is a packed bf16 pair.
+__device__ __forceinline__ void split3(ptx::f2 x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    const ptx::f2 m1 = ptx::make_f2(-1.f, -1.f);
+    hi = ptx::f2_to_bf16x2(x);
+    const ptx::f2 r = ptx::fma2(ptx::bf16x2_to_f2(hi), m1, x);
+    mid = ptx::f2_to_bf16x2(r);
+    lo = ptx::f2_to_bf16x2(ptx::fma2(ptx::bf16x2_to_f2(mid), m1, r));
 }
 
-__global__ void __launch_bounds__(256)
-k2_f32(float* __restrict__ X, const float* __restrict__ scale, const float* __restrict__ Wo,
-       const float* __restrict__ E, const float* __restrict__ V, float* __restrict__ partial, size_t lo_offset,
-       float* __restrict__ vprime, Geom g) {
-    extern __shared__ __align__(16) float sm[];
-    float* es = sm;                    // [12*12][64]  E with a 2-cell halo
-    float* vs = es + 144 * 64;         // [10*10][64]  V, then R = V / box3(E), with a 1-cell halo
-    float* vp = vs + 100 * 64;         // [64][XS32]   V' of the tile
-    float* wo = vp + 64 * XS32;        // [64][64]     Wo rows of the current head
-    double* red = reinterpret_cast<double*>(wo + 64 * 64);   // [16][64] fp64 (the offset is a multiple of 8 bytes)
+__device__ __forceinline__ uint32_t swz64(int m, int q) { return (uint32_t)(m * 64 + ((q ^ ((m >> 1) & 3)) << 4)); }
 
-    const int tid = threadIdx.x;
-    const int b = blockIdx.y;
-    const int tx0 = (blockIdx.x % g.tiles_x) * T32;
-    const int ty0 = (blockIdx.x / g.tiles_x) * T32;
-    const int set = b / g.per_set;
+// The six products of a split contraction, smallest first, by part of the second operand: for part 2 (lo) of W only
+// hi of A, for part 1 mid and hi, for part 0 lo, mid and hi.  Part pw of W meets parts 2 - pw .. 0 of A.
+
+namespace k1f {
+constexpr int PART = 16384;                              // one part of the stencil operand: [128 cells][64] bf16
+constexpr int A_CONV = 0, A_BYTES = 3 * PART;            // two stencil operands of 3 parts
+constexpr int WIV = A_CONV + 2 * A_BYTES, WIV_SLOT = 16384;          // two slots: one part of Wi | Wv
+constexpr int WP = WIV + 2 * WIV_SLOT, WP_SLOT = 8192;               // two slots: one part of Wp
+constexpr int STG = WP + 2 * WP_SLOT;                    // 2 KB staging tiles [32 cells][16 dims]: one per E warp, two per V warp
+constexpr int XH = STG + 16 * 2048, XH_BYTES = 10 * 18 * 256;         // state halo tile, plain [10][18] cells x 64 fp32
+constexpr int PRM_ST = XH + XH_BYTES;                    // head parameters of the tile's weight set
+constexpr int BARS = PRM_ST + NH * PRM * 4, N_BARS = 18, TMEM_PTR = BARS + N_BARS * 8;
+constexpr int BYTES = TMEM_PTR + 16;
+constexpr int SMEM = BYTES + 1024;                       // slack for manual 1024-byte alignment
+constexpr uint32_t TMEM_COLS = 512, AX = 384;            // two accumulator buffers of 192 columns, the X operand behind them
+constexpr int THREADS = 768;
+static_assert(SMEM <= 227 * 1024, "k1 (fp32) shared memory");
+}  // namespace k1f
+
+// k1: one CTA per SM, warp-specialised.  The work is the list of (tile of 8 x 16 cells, head) items in order; a CTA
+// takes one contiguous stretch of it, so that the stretches differ by one item at most whatever the size of the grid.
+//   warps 0-7   stencil group: at a new tile loads the state halo (scale applied) and writes the parts of the X operand
+//               into TMEM; per item the 3x3 stencil, two columns x four channels x four rows per thread, written as the
+//               three parts of one of two operand tiles
+//   warps 8-15  E group: TMEM -> growth bell, E = exp(G*I); warps 16-19 V group: TMEM -> V.  Each warp has its own staging
+//               tiles (its 32 cells x 16 dims) and its own TMA stores: no barrier among them
+//   warps 20,21 TMA producers of the weight chunks, parts lo, mid, hi of Wi | Wv and of Wp
+//   warps 22,23 UMMA issuers, one for I | V (N = 128, the X operand in TMEM: with both operands in shared memory the
+//               products, the stencil's loads and the stores of this kernel contend for its 128 bytes per cycle), one for U
+//               (N = 64).  One issuer for both was the longest chain of the kernel.
+__global__ void __launch_bounds__(k1f::THREADS, 1)
+k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_es,
+       const __grid_constant__ CUtensorMap map_vs, const float* __restrict__ X, const float* __restrict__ scale,
+       const float* __restrict__ prm, float* __restrict__ E, float* __restrict__ V, int* __restrict__ status, int n_items,
+       int tiles_per_grid, Geom g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = align1024(smem_raw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + k1f::BARS);
+    // one waiting party per barrier, observing every phase in turn
+    uint64_t* w_full = bars;                       // [2 of Wi|Wv][2 of Wp] weight chunk landed   (waits: its UMMA issuer)
+    uint64_t* w_empty = bars + 4;                  // ... and was consumed                        (waits: its TMA producer)
+    uint64_t* ac_full = bars + 8;                  // [2] stencil operand of an item written      (waits: issuer of U)
+    uint64_t* ac_empty = bars + 10;                // [2] ... and consumed                        (waits: stencil group)
+    uint64_t* ax_full = bars + 12;                 // X operand of a tile written                 (waits: issuer of I|V)
+    uint64_t* ax_empty = bars + 13;                // ... and consumed by the tile's last item    (waits: stencil group)
+    uint64_t* tm_full = bars + 14;                 // [2] accumulator buffer holds an item (both issuers arrive) (waits: E and V groups)
+    uint64_t* tm_empty = bars + 16;                // [2] ... and was drained (384 arrivals)      (waits: both issuers)
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k1f::TMEM_PTR);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < 14; ++i) ptx::mbar_init(&bars[i], 1);
+        for (int i = 0; i < 2; ++i) { ptx::mbar_init(&tm_full[i], 2); ptx::mbar_init(&tm_empty[i], 384); }
+        ptx::fence_barrier_init();
+        ptx::prefetch_tmap(&map_w1); ptx::prefetch_tmap(&map_es); ptx::prefetch_tmap(&map_vs);
+    }
+    if (warp == 0) ptx::tmem_alloc(tmem_ptr, k1f::TMEM_COLS);
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_ptr;
+    const int i0 = (int)((long long)n_items * blockIdx.x / gridDim.x);
+    const int i1 = (int)((long long)n_items * (blockIdx.x + 1) / gridDim.x);
     const size_t xplane = (size_t)g.state_rows() * g.W * NC;
-    const size_t eplane = (size_t)g.ev_rows() * g.W * HD;
-    const size_t vplane = (size_t)g.H * g.W * HD;
-    const int cg = tid >> 4;
-    const int c0 = (tid & 15) * 4;
+    const size_t eplane = (size_t)g.ev_h * g.ev_w * HD;
 
-    float acc[4][4];
+    if (warp == 20 || warp == 21) {
+        // ================= TMA producers of the weight chunks =================================================
+        const int u = warp - 20;                               // 0: Wi | Wv, 1: Wp
+        if (lane == 0) {
+            uint32_t c = 0;
+            for (int i = i0; i < i1; ++i) {
+                const int h = i & 7, b = (i >> 3) / tiles_per_grid, set = b / g.per_set;
+                for (int pw = 2; pw >= 0; --pw, ++c) {
+                    const int s = c & 1, row = ((set * NH + h) * 3 + pw) * 192;
+                    uint64_t* full = &w_full[2 * u + s];
+                    ptx::mbar_wait(&w_empty[2 * u + s], ((c >> 1) & 1) ^ 1, status, 310 + u);
+                    ptx::mbar_expect_tx(full, u ? k1f::WP_SLOT : k1f::WIV_SLOT);
+                    if (u) {
+                        ptx::tma_load_2d(sm + k1f::WP + s * k1f::WP_SLOT, &map_w1, 0, row, full);
+                    } else {
+                        ptx::tma_load_2d(sm + k1f::WIV + s * k1f::WIV_SLOT, &map_w1, 0, row + 64, full);
+                        ptx::tma_load_2d(sm + k1f::WIV + s * k1f::WIV_SLOT + 8192, &map_w1, 0, row + 128, full);
+                    }
+                }
+            }
+        }
+    } else if (warp == 22) {
+        // ================= UMMA issuer of I | V (the whole warp, its leader executes) =================================
+        const uint32_t leader = ptx::elect_one();
+        const uint32_t wiv = ptx::smem_u32(sm + k1f::WIV) >> 4;
+        uint32_t c = 0, n = 0, tiles = 0;
+        for (int i = i0; i < i1; ++i, ++n) {
+            const int h = i & 7, tb = n & 1;
+            if (h == 0 || i == i0) { ptx::mbar_wait(ax_full, tiles & 1, status, 320); ++tiles; }
+            ptx::mbar_wait(&tm_empty[tb], ((n >> 1) & 1) ^ 1, status, 321);
+            ptx::tc_fence_after();
+            const uint32_t acc = tmem + tb * 192 + 64;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+            for (int pw = 2; pw >= 0; --pw) {
+                const int s = c & 1;
+                ptx::mbar_wait(&w_full[s], (c >> 1) & 1, status, 322);
+                ptx::tc_fence_after();
+                ++c;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) acc[j][k] = 0.f;
+                for (int pa = 2 - pw; pa >= 0; --pa)
+                    ptx::umma4_ts<ptx::umma_idesc_bf16(128, 128)>(leader, acc, tmem + k1f::AX + pa * 32, wiv + s * (k1f::WIV_SLOT >> 4), pw < 2 || pa < 2 - pw);
+                ptx::umma_commit_by(leader, &w_empty[s]);
+            }
+            if (h == NH - 1 || i == i1 - 1) ptx::umma_commit_by(leader, ax_empty);
+            ptx::umma_commit_by(leader, &tm_full[tb]);
+        }
+    } else if (warp == 23) {
+        // ================= UMMA issuer of U =======================================================================
+        const uint32_t leader = ptx::elect_one();
+        const uint32_t wp = ptx::smem_u32(sm + k1f::WP) >> 4, a0 = ptx::smem_u32(sm + k1f::A_CONV) >> 4;
+        uint32_t c = 0, n = 0;
+        for (int i = i0; i < i1; ++i, ++n) {
+            const int tb = n & 1;
+            ptx::mbar_wait(&tm_empty[tb], ((n >> 1) & 1) ^ 1, status, 323);
+            ptx::mbar_wait(&ac_full[tb], (n >> 1) & 1, status, 324);
+            ptx::tc_fence_after();
+            const uint32_t acc = tmem + tb * 192, a = a0 + tb * (k1f::A_BYTES >> 4);
+#pragma unroll
+            for (int pw = 2; pw >= 0; --pw) {
+                const int s = c & 1;
+                ptx::mbar_wait(&w_full[2 + s], (c >> 1) & 1, status, 325);
+                ptx::tc_fence_after();
+                ++c;
+#pragma unroll
+                for (int pa = 2 - pw; pa >= 0; --pa)
+                    ptx::umma4_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW128_HI>(leader, acc, a + pa * (k1f::PART >> 4), wp + s * (k1f::WP_SLOT >> 4), pw < 2 || pa < 2 - pw);
+                ptx::umma_commit_by(leader, &w_empty[2 + s]);
+            }
+            ptx::umma_commit_by(leader, &ac_empty[tb]);
+            ptx::umma_commit_by(leader, &tm_full[tb]);
+        }
+    } else if (warp < 8) {
+        // ================= stencil group ======================================================================
+        uint8_t* xh = sm + k1f::XH;
+        float* prm_s = reinterpret_cast<float*>(sm + k1f::PRM_ST);
+        const int c4 = tid & 15, p2 = (tid >> 4) & 7, y0 = (tid >> 7) * 4;
+        uint32_t n = 0, tiles = 0;
+        for (int i = i0; i < i1; ++i, ++n) {
+            const int h = i & 7, tb = n & 1;
+            if (h == 0 || i == i0) {
+                const CaTile t = ca_tile(i >> 3, tiles_per_grid, g.tiles_x, -g.he);
+                const int set = t.b / g.per_set;
+                ptx::bar_sync(1, 256);                                    // everybody is done with the last halo
+                if (tid < NH * PRM) prm_s[tid] = __ldg(prm + (size_t)set * NH * PRM + tid);
+                // 180 cells x 16 chunks of 4 channels over 256 threads, every load issued before the first is used
+                const float* Xb = X + (size_t)t.b * xplane + c4 * 4;
+                const float4 s4 = __ldg(reinterpret_cast<const float4*>(scale + t.b * NC + c4 * 4));
+                float4 raw[12];
+#pragma unroll
+                for (int j = 0; j < 12; ++j) {
+                    const int cell = (tid >> 4) + j * 16, hy = cell / 18;
+                    if (cell < 180)
+                        raw[j] = *reinterpret_cast<const float4*>(Xb + ((size_t)g.xrow_near(t.ty0 + hy - 1) * g.W + g.wrap_x_near(t.tx0 + cell - hy * 18 - 1)) * NC);
+                }
+#pragma unroll
+                for (int j = 0; j < 12; ++j) {
+                    const int cell = (tid >> 4) + j * 16;
+                    if (cell < 180)
+                        *reinterpret_cast<float4*>(xh + cell * 256 + c4 * 16) =
+                            make_float4(raw[j].x * s4.x, raw[j].y * s4.y, raw[j].z * s4.z, raw[j].w * s4.w);
+                }
+                if ((i >> 3) + 1 <= (i1 - 1) >> 3) {                      // next tile's halo: two 128-byte lines a cell, into L2
+                    const CaTile tn = ca_tile((i >> 3) + 1, tiles_per_grid, g.tiles_x, -g.he);
+                    for (int j = tid; j < 360; j += 256) {
+                        const int cell = j >> 1, hy = cell / 18;
+                        ptx::prefetch_l2(X + (size_t)tn.b * xplane + (j & 1) * 32 +
+                                         ((size_t)g.xrow_near(tn.ty0 + hy - 1) * g.W + g.wrap_x_near(tn.tx0 + cell - hy * 18 - 1)) * NC);
+                    }
+                }
+                ptx::mbar_wait(ax_empty, (tiles & 1) ^ 1, status, 330);
+                ptx::bar_sync(1, 256);
+                // X operand: this thread's cell is TMEM lane m, half of its channels
+                {
+                    const int m = (warp & 3) * 32 + lane, half = warp >> 2;
+                    const uint8_t* src = xh + ((m >> 4) * 18 + 19 + (m & 15)) * 256 + half * 128;
+                    const uint32_t dst = tmem + ((uint32_t)((warp & 3) * 32) << 16) + k1f::AX + half * 16;
+                    uint32_t a[3][16];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float4 v = *reinterpret_cast<const float4*>(src + q * 16);
+                        split3(ptx::make_f2(v.x, v.y), a[0][2 * q], a[1][2 * q], a[2][2 * q]);
+                        split3(ptx::make_f2(v.z, v.w), a[0][2 * q + 1], a[1][2 * q + 1], a[2][2 * q + 1]);
+                    }
+#pragma unroll
+                    for (int pa = 0; pa < 3; ++pa) ptx::tmem_st16(dst + pa * 32, a[pa]);
+                    ptx::tmem_st_wait();
+                    ptx::tc_fence_before();
+                }
+                ++tiles;
+                ptx::bar_sync(1, 256);
+                if (tid == 0) { ptx::tc_fence_after(); ptx::tc_fence_before(); ptx::mbar_arrive(ax_full); }
+            }
+            // two adjacent columns x 4 channels x 4 rows per thread; input row j feeds output rows j (tap row 0), j-1 (tap
+            // row 1) and j-2 (tap row 2)
+            ptx::f2 kt[9], s1[2][2], s2[2][2];
+#pragma unroll
+            for (int tt = 0; tt < 9; ++tt) { const float kv = prm_s[h * PRM + tt]; kt[tt] = ptx::make_f2(kv, kv); }
+            ptx::mbar_wait(&ac_empty[tb], ((n >> 1) & 1) ^ 1, status, 331);
+            uint8_t* a_conv = sm + k1f::A_CONV + tb * k1f::A_BYTES + (c4 & 1) * 8;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const uint8_t* row = xh + ((y0 + j) * 18 + 2 * p2) * 256 + c4 * 16;
+                ptx::f2 c[4][2];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 w = *reinterpret_cast<const float4*>(row + q * 256);
+                    c[q][0] = ptx::make_f2(w.x, w.y);
+                    c[q][1] = ptx::make_f2(w.z, w.w);
+                }
+#pragma unroll
+                for (int col = 0; col < 2; ++col) {
+                    ptx::f2 nw[2], md[2];
+                    if (j >= 2) {
+                        uint32_t a[3], b[3];
+                        ptx::f2 o[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                            o[e] = ptx::fma2(kt[6], c[col][e], ptx::fma2(kt[7], c[col + 1][e], ptx::fma2(kt[8], c[col + 2][e], s2[col][e])));
+                        split3(o[0], a[0], a[1], a[2]);
+                        split3(o[1], b[0], b[1], b[2]);
+                        uint8_t* dst = a_conv + swz((y0 + j - 2) * TBW + 2 * p2 + col, c4 >> 1);
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dst + p * k1f::PART) = make_uint2(a[p], b[p]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if (j >= 1 && j <= 4) md[e] = ptx::fma2(kt[3], c[col][e], ptx::fma2(kt[4], c[col + 1][e], ptx::fma2(kt[5], c[col + 2][e], s1[col][e])));
+                        if (j <= 3) nw[e] = ptx::fma2(kt[0], c[col][e], ptx::fma2(kt[1], c[col + 1][e], ptx::mul2(kt[2], c[col + 2][e])));
+                        s2[col][e] = md[e]; s1[col][e] = nw[e];
+                    }
+                }
+            }
+            ptx::fence_proxy_async();
+            ptx::bar_sync(2, 256);
+            if (tid == 0) ptx::mbar_arrive(&ac_full[tb]);
+        }
+    } else {
+        // ================= E group (warps 8..15: a quarter of the cells, half of the dims) and V group (16..19: a quarter
+        // of the cells, all dims), sixteen dims at a time ===========================================================
+        const bool is_e = warp < 16;
+        const int quad = warp & 3, m_ep = quad * 32 + lane;          // TMEM lane = cell of the tile this thread finishes
+        const int d_first = is_e ? ((warp - 8) >> 2) * 32 : 0, d_last = is_e ? d_first + 16 : 48;
+        uint8_t* stg = sm + k1f::STG + (is_e ? warp - 8 : 8 + quad * 2) * 2048;
+        const bool tiny = g.W < 2 * APRON || (g.wrap_y && g.H < 2 * APRON);
+        const ptx::f2 two2 = ptx::make_f2(2.f, 2.f), minus_one2 = ptx::make_f2(-1.f, -1.f);
+        uint32_t n = 0;
+        CaTile t;
+        // Apron positions that wrap onto this thread's cell (the TMA store covers the cell itself and whatever hangs over
+        // the far edge), as cell offsets in the plane, -1 for none.  Grids narrower or shorter than twice the apron can
+        // wrap more than once and take the general loop.
+        int dup_x = -1, dup_y = -1, dup_xy = -1;
+        bool edge_x = false, edge_y = false, edge = false;           // does any cell of the warp have one
+        for (int i = i0; i < i1; ++i, ++n) {
+            const int h = i & 7, tb = n & 1;
+            if (h == 0 || i == i0) {
+                t = ca_tile(i >> 3, tiles_per_grid, g.tiles_x, -g.he);
+                const int r = t.ty0 + (m_ep >> 4), x = t.tx0 + (m_ep & 15);
+                const bool valid = r < g.H + g.he && x < g.W;
+                const int xd = x < APRON ? x + g.W : x >= g.W - APRON ? x - g.W : -100;
+                const int rd = !g.wrap_y ? -100 : r < APRON ? r + g.H : r >= g.H - APRON ? r - g.H : -100;
+                dup_x = valid && xd != -100 ? (r + APRON) * g.ev_w + xd + APRON : -1;
+                dup_y = valid && rd != -100 ? (rd + APRON) * g.ev_w + x + APRON : -1;
+                dup_xy = dup_x >= 0 && dup_y >= 0 ? (rd + APRON) * g.ev_w + xd + APRON : -1;
+                edge_x = __any_sync(0xffffffffu, dup_x >= 0);
+                edge_y = __any_sync(0xffffffffu, dup_y >= 0);
+                edge = tiny || edge_x || edge_y;
+            }
+            const float mus = __ldg(prm + ((size_t)(t.b / g.per_set) * NH + h) * PRM + 9);   // mu * s; Wp carries s and Wi carries log2(e)
+            const ptx::f2 neg_mus2 = ptx::make_f2(-mus, -mus);
+            const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16) + tb * 192;
+            ptx::mbar_wait(&tm_full[tb], (n >> 1) & 1, status, is_e ? 340 : 341);
+            ptx::tc_fence_after();
+#pragma unroll 1
+            for (int d0 = d_first; d0 <= d_last; d0 += 16) {
+                float f[16];
+                if (is_e) {
+                    // G = 2 ex2(-(s (U - mu))^2) - 1, E = ex2(clamp(G I log2 e)): the constants sit in the weights, whose
+                    // three parts hold the products to 24 bits, so each exponential's argument is rounded once
+                    uint32_t ru[16], ri[16];
+                    ptx::tmem_ld16(t_lane + d0, ru);
+                    ptx::tmem_ld16(t_lane + 64 + d0, ri);
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int k = 0; k < 16; k += 2) {
+                        const ptx::f2 z = ptx::add2(ptx::make_f2(__uint_as_float(ru[k]), __uint_as_float(ru[k + 1])), neg_mus2);
+                        float q0, q1, a0, a1;
+                        ptx::split_f2(ptx::mul2(z, z), q0, q1);
+                        const ptx::f2 gr = ptx::fma2(ptx::make_f2(ptx::ex2(-q0), ptx::ex2(-q1)), two2, minus_one2);
+                        ptx::split_f2(ptx::mul2(gr, ptx::make_f2(__uint_as_float(ri[k]), __uint_as_float(ri[k + 1]))), a0, a1);
+                        f[k] = ptx::ex2(fminf(fmaxf(a0, -ACT_CLAMP * LOG2E), ACT_CLAMP * LOG2E));
+                        f[k + 1] = ptx::ex2(fminf(fmaxf(a1, -ACT_CLAMP * LOG2E), ACT_CLAMP * LOG2E));
+                    }
+                    if (lane == 0) ptx::bulk_wait_read0();          // the last store has read the staging tile
+                } else {
+                    uint32_t rv[16];
+                    ptx::tmem_ld16(t_lane + 128 + d0, rv);
+                    if (lane == 0) ptx::bulk_wait_read1();          // the store before the last one has read its tile
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) f[k] = __uint_as_float(rv[k]);
+                }
+                if (d0 == d_last) { ptx::tc_fence_before(); ptx::mbar_arrive(&tm_empty[tb]); }      // done with the accumulator buffer
+                uint8_t* tile = is_e ? stg : stg + (d0 & 16) * 128;
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    *reinterpret_cast<float4*>(tile + swz64(lane, q)) = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+                ptx::fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {             // the warp's 32 cells are two rows of the tile
+                    ptx::tma_store_4d(is_e ? &map_es : &map_vs, tile, d0, t.tx0 + APRON, t.ty0 + quad * 2 + APRON, t.b * NH + h);
+                    ptx::bulk_commit();
+                }
+                if (edge) {
+                    float* plane = (is_e ? E : V) + ((size_t)t.b * NH + h) * eplane + d0;
+                    auto copy = [&](int cell) {
+                        float4* p = reinterpret_cast<float4*>(plane + (size_t)cell * HD);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) p[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+                    };
+                    if (!tiny) {
+                        if (edge_x && dup_x >= 0) copy(dup_x);
+                        if (edge_y && dup_y >= 0) copy(dup_y);
+                        if (edge_x && edge_y && dup_xy >= 0) copy(dup_xy);
+                    } else {
+                        const int r = t.ty0 + (m_ep >> 4), x = t.tx0 + (m_ep & 15);
+                        if (r < g.H + g.he && x < g.W)
+                            for (int ky = g.wrap_y ? -2 * APRON : 0; ky <= (g.wrap_y ? 2 * APRON : 0); ++ky)
+                                for (int kx = -2 * APRON; kx <= 2 * APRON; ++kx) {
+                                    const int rr = r + ky * g.H, xx = x + kx * g.W;
+                                    if ((ky == 0 && kx == 0) || rr < -APRON || rr >= g.H + APRON || xx < -APRON || xx >= g.W + APRON) continue;
+                                    copy((rr + APRON) * g.ev_w + xx + APRON);
+                                }
+                    }
+                }
+            }
+        }
+        if (lane == 0) ptx::bulk_wait0();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) ptx::tmem_dealloc(tmem, k1f::TMEM_COLS);
+}
 
-    for (int h = 0; h < NH; ++h) {
-        const float* Eh = E + ((size_t)b * NH + h) * eplane;
-        const float* Vh = V + ((size_t)b * NH + h) * eplane;
-        __syncthreads();
-        for (int i = tid; i < 144 * 16; i += 256) {
-            const int cell = i >> 4, q = i & 15;
-            const int r = ty0 + cell / 12 - 2, x = g.wrap_x(tx0 + cell % 12 - 2);
-            reinterpret_cast<float4*>(es)[i] =
-                *reinterpret_cast<const float4*>(Eh + ((size_t)g.erow(r) * g.W + x) * HD + q * 4);
+// =============================================================================================================
+// k2: the marching scheme of the bf16 kernel (see there) on fp32 planes.  A head is taken as two half-heads of 32 dims, so
+// that a block of 4 rows has the byte shape of a bf16 block (128 bytes a cell) and a thread owns 4 dims.
+//   warps 0-7,19 A: R = V / box3(E) in place in the stage
+//   warps 8-15   B: V' = E * box3(R), split into the three parts of the A operand
+//   warp 16      TMA producer: per (macro tile, half-head) the parts of its Wo slice, per block E and V
+//   warp 17      UMMA issuer: the half-head's share of Y (N=64, K=32, six products) into one of two working accumulators
+//   warp 18      TMA producer of the epilogue's state tiles
+//   warps 20-23  P: adds every working accumulator to the tile's running sum in TMEM, rounded to nearest (16 half-heads:
+//                on the tensor core that sum would be truncated 192 times); after the last half-head X+ = scale X + dt Y,
+//                written back through shared memory, and the tile's channel sums in fp64
+namespace k2f {
+constexpr int SW = k2m::SW, BR = k2m::BR, NB = 6;       // strip width, rows per block, blocks per macro tile at most
+constexpr int NHH = 2 * NH;                             // half-heads
+constexpr int EW = k2m::EW, VW = k2m::VW;
+constexpr int E_BYTES = k2m::E_BYTES, STAGE_BYTES = k2m::STAGE_BYTES;
+constexpr int NSTAGE = 3;
+constexpr int STG = 0;
+constexpr int PART = 8192;                              // one part of the operand tile: [128 cells][32] bf16, 64-byte rows
+constexpr int A_VP = STG + NSTAGE * STAGE_BYTES;        // two operand tiles of 3 parts
+constexpr int WO_PART = 4096, WO = A_VP + 2 * 3 * PART; // two Wo slices of 3 parts [64][32]
+constexpr int XT = WO + 2 * 3 * WO_PART;                // state tile of the epilogue: two halves of 32 channels, 16 KB each
+constexpr int RED = XT + 2 * 16384;                     // [4 quads][64] fp64
+constexpr int BARS = RED + 4 * 64 * 8;
+constexpr int N_BARS = 2 * NSTAGE + 12;
+constexpr int TMEM_PTR = BARS + N_BARS * 8;
+constexpr int BYTES = TMEM_PTR + 16;
+constexpr int SMEM = BYTES + 1024;
+constexpr uint32_t TMEM_COLS = 512, WORK = NB * 64;     // running sums of up to six tiles, two working accumulators behind
+constexpr int A_THREADS = k2m::A_THREADS, B_THREADS = k2m::B_THREADS;
+constexpr int THREADS = 768;
+constexpr int HANDOFF = A_THREADS + B_THREADS;
+static_assert(A_VP % 1024 == 0 && WO % 1024 == 0 && XT % 1024 == 0, "swizzled tiles must be aligned");
+static_assert(SMEM <= 227 * 1024, "k2 (fp32) shared memory");
+}  // namespace k2f
+
+struct V4 { ptx::f2 a, b; };
+__device__ __forceinline__ V4 v4(const float4& f) { V4 r; r.a = ptx::make_f2(f.x, f.y); r.b = ptx::make_f2(f.z, f.w); return r; }
+__device__ __forceinline__ V4 v4_add(const V4& x, const V4& y) { V4 r; r.a = ptx::add2(x.a, y.a); r.b = ptx::add2(x.b, y.b); return r; }
+__device__ __forceinline__ V4 v4_mul(const V4& x, const V4& y) { V4 r; r.a = ptx::mul2(x.a, y.a); r.b = ptx::mul2(x.b, y.b); return r; }
+// x / z to the last bit or nearly: the quotient by the approximate reciprocal and one residual correction (Markstein).  The
+// compiler's own division costs four times the instructions, and its subnormal branch is not needed: z lies within
+// 9 exp(+-80).
+__device__ __forceinline__ ptx::f2 div2(ptx::f2 x, ptx::f2 z) {
+    float z0, z1;
+    ptx::split_f2(z, z0, z1);
+    const ptx::f2 r = ptx::make_f2(ptx::rcp(z0), ptx::rcp(z1)), q = ptx::mul2(x, r);
+    return ptx::fma2(ptx::fma2(ptx::mul2(z, ptx::make_f2(-1.f, -1.f)), q, x), r, q);
+}
+__device__ __forceinline__ V4 v4_div(const V4& x, const V4& z) { V4 r; r.a = div2(x.a, z.a); r.b = div2(x.b, z.b); return r; }
+__device__ __forceinline__ float4 v4_f4(const V4& x) { float4 f; ptx::split_f2(x.a, f.x, f.y); ptx::split_f2(x.b, f.z, f.w); return f; }
+
+__global__ void __launch_bounds__(k2f::THREADS, 1)
+k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUtensorMap map_e,
+       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ scale,
+       float* __restrict__ partial, size_t lo_offset, float* __restrict__ vprime, int* __restrict__ status, int n_mt,
+       int mt_per_grid, int strips, int tiles_per_grid, int nbmax, Geom g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = align1024(smem_raw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + k2f::BARS);
+    uint64_t* full = bars;                           // [3] block landed                              (waits: A)
+    uint64_t* empty = full + k2f::NSTAGE;            // [3] B is done with the stage (256 arrivals)   (waits: TMA producer)
+    uint64_t* vp_full = empty + k2f::NSTAGE;         // [2] operand tile written (256 arrivals)       (waits: UMMA issuer)
+    uint64_t* vp_empty = vp_full + 2;                // [2] the UMMAs reading it are done             (waits: B)
+    uint64_t* wo_full = vp_empty + 2;                // [2] Wo slice landed                           (waits: UMMA issuer)
+    uint64_t* wo_empty = wo_full + 2;                // [2] its half-head is issued and done          (waits: TMA producer)
+    uint64_t* wk_full = wo_empty + 2;                // [2] working accumulator complete              (waits: P)
+    uint64_t* wk_empty = wk_full + 2;                // [2] ... and added (128 arrivals)              (waits: UMMA issuer)
+    uint64_t* x_full = wk_empty + 2;                 // state tile landed                             (waits: P)
+    uint64_t* x_empty = x_full + 1;                  // ... and its X+ has left shared memory          (waits: state producer)
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k2f::TMEM_PTR);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < k2f::NSTAGE; ++i) { ptx::mbar_init(&full[i], 1); ptx::mbar_init(&empty[i], k2f::B_THREADS); }
+        for (int i = 0; i < 2; ++i) {
+            ptx::mbar_init(&vp_full[i], k2f::B_THREADS); ptx::mbar_init(&vp_empty[i], 1);
+            ptx::mbar_init(&wo_full[i], 1); ptx::mbar_init(&wo_empty[i], 1);
+            ptx::mbar_init(&wk_full[i], 1); ptx::mbar_init(&wk_empty[i], 128);
         }
-        for (int i = tid; i < 100 * 16; i += 256) {
-            const int cell = i >> 4, q = i & 15;
-            const int r = ty0 + cell / 10 - 1, x = g.wrap_x(tx0 + cell % 10 - 1);
-            reinterpret_cast<float4*>(vs)[i] =
-                *reinterpret_cast<const float4*>(Vh + ((size_t)g.erow(r) * g.W + x) * HD + q * 4);
-        }
-        const float* wsrc = Wo + ((size_t)set * NH + h) * HD * NC;
-        for (int i = tid; i < 64 * 64 / 4; i += 256)
-            reinterpret_cast<float4*>(wo)[i] = reinterpret_cast<const float4*>(wsrc)[i];
-        __syncthreads();
-        // R = V / box3(E) on the 10x10 ring-extended tile (each item owns its own 4 values: in place)
-        for (int i = tid; i < 100 * 16; i += 256) {
-            const int cell = i >> 4, q = i & 15;
-            const int vy = cell / 10, vx = cell % 10;
-            float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                const float4 e = *reinterpret_cast<const float4*>(es + ((vy + t / 3) * 12 + vx + t % 3) * 64 + q * 4);
-                z.x += e.x; z.y += e.y; z.z += e.z; z.w += e.w;
+        ptx::mbar_init(x_full, 1); ptx::mbar_init(x_empty, 1);
+        ptx::fence_barrier_init();
+        ptx::prefetch_tmap(&map_wo); ptx::prefetch_tmap(&map_e); ptx::prefetch_tmap(&map_v); ptx::prefetch_tmap(&map_x);
+    }
+    if (warp == 0) ptx::tmem_alloc(tmem_ptr, k2f::TMEM_COLS);
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_ptr;
+    const int my_mt = n_mt > (int)blockIdx.x ? (n_mt - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+
+    if (warp == 16) {
+        // ================= TMA producer ===================================================================
+        if (lane == 0) {
+            uint32_t it = 0, wit = 0;       // blocks and half-heads so far
+            for (int k = 0; k < my_mt; ++k) {
+                const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+                const int set = m.b / g.per_set;
+                for (int hh = 0; hh < k2f::NHH; ++hh, ++wit) {
+                    const int wb = wit & 1, plane = m.b * NH + (hh >> 1), d0 = (hh & 1) * 32;
+                    ptx::mbar_wait(&wo_empty[wb], ((wit >> 1) & 1) ^ 1, status, 510);
+                    ptx::mbar_expect_tx(&wo_full[wb], 3 * k2f::WO_PART);
+                    ptx::tma_load_2d(sm + k2f::WO + wb * 3 * k2f::WO_PART, &map_wo, 0, (set * k2f::NHH + hh) * 192, &wo_full[wb]);
+                    for (int b = -1; b < m.nb; ++b, ++it) {
+                        const int s = it % k2f::NSTAGE;
+                        uint8_t* st = sm + k2f::STG + s * k2f::STAGE_BYTES;
+                        ptx::mbar_wait(&empty[s], ((it / k2f::NSTAGE) & 1) ^ 1, status, 511);
+                        ptx::mbar_expect_tx(&full[s], k2f::STAGE_BYTES);
+                        ptx::tma_load_4d(st, &map_e, d0, m.mx0, m.my0 + 4 * b + 4, plane, &full[s]);
+                        ptx::tma_load_4d(st + k2f::E_BYTES, &map_v, d0, m.mx0 + 1, m.my0 + 4 * b + 3, plane, &full[s]);
+                    }
+                }
             }
-            float4 v = reinterpret_cast<float4*>(vs)[i];
-            v.x /= z.x; v.y /= z.y; v.z /= z.z; v.w /= z.w;
-            reinterpret_cast<float4*>(vs)[i] = v;
         }
-        __syncthreads();
-        // V' = E * box3(R) on the 8x8 tile
-        for (int i = tid; i < 64 * 16; i += 256) {
-            const int cell = i >> 4, q = i & 15;
-            const int cy = cell >> 3, cx = cell & 7;
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                const float4 r = *reinterpret_cast<const float4*>(vs + ((cy + t / 3) * 10 + cx + t % 3) * 64 + q * 4);
-                s.x += r.x; s.y += r.y; s.z += r.z; s.w += r.w;
+    } else if (warp == 18) {
+        // ================= TMA producer of the epilogue's state tiles ==========================================
+        if (lane == 0) {
+            uint32_t nx = 0;
+            for (int k = 0; k < my_mt; ++k) {
+                const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+                for (int b = 0; b < m.nb; ++b, ++nx) {
+                    ptx::mbar_wait(x_empty, (nx & 1) ^ 1, status, 512);
+                    ptx::mbar_expect_tx(x_full, 32768);
+                    ptx::tma_load_4d(sm + k2f::XT, &map_x, 0, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, x_full);
+                    ptx::tma_load_4d(sm + k2f::XT + 16384, &map_x, 32, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, x_full);
+                }
             }
-            const float4 e = *reinterpret_cast<const float4*>(es + ((cy + 2) * 12 + cx + 2) * 64 + q * 4);
-            s.x *= e.x; s.y *= e.y; s.z *= e.z; s.w *= e.w;
-            *reinterpret_cast<float4*>(vp + cell * XS32 + q * 4) = s;
-            if (vprime != nullptr && ty0 + cy < g.H && tx0 + cx < g.W)
-                *reinterpret_cast<float4*>(vprime + ((size_t)b * NH + h) * vplane +
-                                           ((size_t)(ty0 + cy) * g.W + tx0 + cx) * HD + q * 4) = s;
         }
-        __syncthreads();
-        for (int k4 = 0; k4 < 16; ++k4) {
-            float4 a4[4];
+    } else if (warp == 17) {
+        // ================= UMMA issuer (the whole warp, its leader executes) ==================================
+        const uint32_t leader = ptx::elect_one();
+        const uint32_t a0 = ptx::smem_u32(sm + k2f::A_VP) >> 4, w0 = ptx::smem_u32(sm + k2f::WO) >> 4;
+        uint32_t v = 0, wit = 0;     // operand tiles used, half-heads
+        for (int k = 0; k < my_mt; ++k) {
+            const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+            for (int hh = 0; hh < k2f::NHH; ++hh, ++wit) {
+                const int wb = wit & 1;
+                for (int b = 0; b < m.nb; ++b, ++v) {
+                    const int buf = v & 1;
+                    if (b == 0) ptx::mbar_wait(&wo_full[wb], (wit >> 1) & 1, status, 521);
+                    ptx::mbar_wait(&wk_empty[buf], ((v >> 1) & 1) ^ 1, status, 520);
+                    ptx::mbar_wait(&vp_full[buf], (v >> 1) & 1, status, 522);
+                    ptx::tc_fence_after();
+                    const uint32_t a = a0 + buf * (3 * k2f::PART >> 4), w = w0 + wb * (3 * k2f::WO_PART >> 4);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) a4[j] = *reinterpret_cast<const float4*>(vp + (cg * 4 + j) * XS32 + k4 * 4);
+                    for (int pw = 2; pw >= 0; --pw)
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                const float4 w = *reinterpret_cast<const float4*>(wo + (k4 * 4 + kk) * 64 + c0);
+                        for (int pa = 2 - pw; pa >= 0; --pa)
+                            ptx::umma2_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW64_HI>(leader, tmem + k2f::WORK + buf * 64, a + pa * (k2f::PART >> 4),
+                                                                                      w + pw * (k2f::WO_PART >> 4), pw < 2 || pa < 2 - pw);
+                    ptx::umma_commit_by(leader, &vp_empty[buf]);
+                    ptx::umma_commit_by(leader, &wk_full[buf]);
+                    if (b == m.nb - 1) ptx::umma_commit_by(leader, &wo_empty[wb]);
+                }
+            }
+        }
+    } else if (warp >= 20) {
+        // ================= P: running sums, then the epilogue ==================================================
+        const int quad = warp & 3, cell = quad * 32 + lane, pt = tid - 640;
+        const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16);
+        uint8_t* xt = sm + k2f::XT;
+        double* red = reinterpret_cast<double*>(sm + k2f::RED);
+        uint32_t v = 0, nx = 0;
+        for (int k = 0; k < my_mt; ++k) {
+            const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+            for (int hh = 0; hh < k2f::NHH; ++hh) {
+                for (int b = 0; b < m.nb; ++b, ++v) {
+                    const int buf = v & 1;
+                    const uint32_t run = t_lane + b * 64, work = t_lane + k2f::WORK + buf * 64;
+                    ptx::mbar_wait(&wk_full[buf], (v >> 1) & 1, status, 530);
+                    ptx::tc_fence_after();
+                    if (hh < k2f::NHH - 1) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float a = kk == 0 ? a4[j].x : kk == 1 ? a4[j].y : kk == 2 ? a4[j].z : a4[j].w;
-                    acc[j][0] = fmaf(a, w.x, acc[j][0]); acc[j][1] = fmaf(a, w.y, acc[j][1]);
-                    acc[j][2] = fmaf(a, w.z, acc[j][2]); acc[j][3] = fmaf(a, w.w, acc[j][3]);
+                        for (int c0 = 0; c0 < 64; c0 += 16) {
+                            uint32_t w[16];
+                            ptx::tmem_ld16(work + c0, w);
+                            if (hh > 0) {
+                                uint32_t y[16];
+                                ptx::tmem_ld16(run + c0, y);
+                                ptx::tmem_ld_wait();
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) w[j] = __float_as_uint(__uint_as_float(w[j]) + __uint_as_float(y[j]));
+                            } else {
+                                ptx::tmem_ld_wait();
+                            }
+                            ptx::tmem_st16(run + c0, w);
+                        }
+                        ptx::tmem_st_wait();
+                        ptx::tc_fence_before();
+                        ptx::mbar_arrive(&wk_empty[buf]);
+                    } else {
+                        // the tile's last half-head: X+ = scale X + dt Y, and the channel sums of what is stored, kept in
+                        // fp64 and handed on as a float pair (value, remainder): a state that has grown large and signed
+                        // makes the per-channel sum a small difference of large terms, and fp32 tile sums would then miss
+                        // the 1e-6 bound on the renormalised mass
+                        const int ty0 = m.my0 + b * k2f::BR;
+                        const bool valid = ty0 + (cell >> 5) < g.H && m.mx0 + (cell & 31) < g.W;
+                        const float* sc = scale + m.b * NC;
+                        ptx::mbar_wait(x_full, nx & 1, status, 531);
+#pragma unroll
+                        for (int c0 = 0; c0 < 64; c0 += 16) {
+                            uint32_t w[16], y[16];
+                            ptx::tmem_ld16(work + c0, w);
+                            ptx::tmem_ld16(run + c0, y);
+                            ptx::tmem_ld_wait();
+                            if (c0 == 48) { ptx::tc_fence_before(); ptx::mbar_arrive(&wk_empty[buf]); }
+                            double xo[16];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                float4* px = reinterpret_cast<float4*>(xt + (c0 >> 5) * 16384 + swz(cell, ((c0 & 31) >> 2) + q));
+                                float4 x = *px;
+                                const float4 s4 = __ldg(reinterpret_cast<const float4*>(sc + c0) + q);
+                                x.x = fmaf(g.dt, __uint_as_float(w[4 * q]) + __uint_as_float(y[4 * q]), x.x * s4.x);
+                                x.y = fmaf(g.dt, __uint_as_float(w[4 * q + 1]) + __uint_as_float(y[4 * q + 1]), x.y * s4.y);
+                                x.z = fmaf(g.dt, __uint_as_float(w[4 * q + 2]) + __uint_as_float(y[4 * q + 2]), x.z * s4.z);
+                                x.w = fmaf(g.dt, __uint_as_float(w[4 * q + 3]) + __uint_as_float(y[4 * q + 3]), x.w * s4.w);
+                                *px = x;
+                                xo[4 * q] = valid ? (double)x.x : 0.0; xo[4 * q + 1] = valid ? (double)x.y : 0.0;
+                                xo[4 * q + 2] = valid ? (double)x.z : 0.0; xo[4 * q + 3] = valid ? (double)x.w : 0.0;
+                            }
+                            // sum over the 32 cells of this warp, fixed tree: each step halves the channels a lane carries
+#pragma unroll
+                            for (int wd = 8; wd >= 1; wd >>= 1) {
+                                const bool up = (lane & (wd * 2)) != 0;
+#pragma unroll
+                                for (int j = 0; j < wd; ++j) {
+                                    const double send = up ? xo[j] : xo[j + wd];
+                                    const double keep = up ? xo[j + wd] : xo[j];
+                                    xo[j] = keep + __shfl_xor_sync(0xffffffffu, send, wd * 2);
+                                }
+                            }
+                            xo[0] += __shfl_xor_sync(0xffffffffu, xo[0], 1);
+                            if ((lane & 1) == 0) {
+                                const int ch = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+                                red[quad * 64 + c0 + ch] = xo[0];
+                            }
+                        }
+                        ptx::fence_proxy_async();      // X+ in shared memory, for the TMA stores issued behind the barrier
+                        ptx::bar_sync(7, 128);
+                        if (pt < NC) {
+                            const double t = (red[pt] + red[64 + pt]) + (red[128 + pt] + red[192 + pt]);
+                            const size_t o = (size_t)(m.b * tiles_per_grid + m.tile0 + b * strips) * NC + pt;
+                            const float hi = (float)t;
+                            partial[o] = hi;
+                            partial[o + lo_offset] = (float)(t - (double)hi);
+                        }
+                        if (pt == 0) {
+                            ptx::tma_store_4d(&map_x, xt, 0, m.mx0, g.hx + ty0, m.b);
+                            ptx::tma_store_4d(&map_x, xt + 16384, 32, m.mx0, g.hx + ty0, m.b);
+                            ptx::bulk_commit();
+                            ptx::bulk_wait_read0();
+                            ptx::mbar_arrive(x_empty);
+                        }
+                        ptx::bar_sync(7, 128);         // the reduction scratch is free again
+                        ++nx;
+                    }
+                }
+            }
+        }
+        if (pt == 0) ptx::bulk_wait0();
+    } else {
+        // ================= the two box-sum sets ==================================================================
+        const bool is_a = warp < 8 || warp == 19;
+        const int gt = warp == 19 ? 256 + lane : (is_a ? tid : tid - 256);     // thread within its set
+        const int q = gt & 7, col = gt >> 3;                    // 4-dim chunk; column (A: of the 34 R columns, B: of the 32)
+        uint32_t it = 0, v = 0;
+        const V4 zero = v4(make_float4(0.f, 0.f, 0.f, 0.f));
+        V4 h2 = zero, h1 = zero;             // running horizontal sums of the two rows above (of E in A, of R in B)
+        float4 ekeep0 = make_float4(0.f, 0.f, 0.f, 0.f), ekeep1 = ekeep0;      // B: centre E of the last two rows of the block before
+        const size_t vplane = (size_t)g.H * g.W * HD;
+        for (int k = 0; k < my_mt; ++k) {
+            const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+            for (int hh = 0; hh < k2f::NHH; ++hh) {
+                for (int b = -1; b < m.nb; ++b, ++it) {
+                    const int s = it % k2f::NSTAGE;
+                    uint8_t* es = sm + k2f::STG + s * k2f::STAGE_BYTES;     // [4][36] cells x 128 B
+                    uint8_t* vs = es + k2f::E_BYTES;                        // [4][34] cells: V, then R in place
+                    if (is_a) {
+                        ptx::mbar_wait(&full[s], (it / k2f::NSTAGE) & 1, status, 540);
+                        if (col < k2f::VW) {
+#pragma unroll
+                            for (int j = 0; j < k2f::BR; ++j) {
+                                const float4* row = reinterpret_cast<const float4*>(es + (j * k2f::EW + col) * 128 + q * 16);
+                                const V4 hs = v4_add(v4_add(v4(row[0]), v4(row[8])), v4(row[16]));
+                                if (b >= 0 || j >= 2) {      // block -1: only its last two rows have all three E rows
+                                    float4* pv = reinterpret_cast<float4*>(vs + (j * k2f::VW + col) * 128 + q * 16);
+                                    *pv = v4_f4(v4_div(v4(*pv), v4_add(v4_add(h2, h1), hs)));
+                                }
+                                h2 = h1; h1 = hs;
+                            }
+                        }
+                        ptx::bar_arrive(1 + s, k2f::HANDOFF);       // R of this block is in the stage
+                    } else {
+                        const int buf = v & 1;
+                        uint8_t* a_vp = sm + k2f::A_VP + buf * 3 * k2f::PART;
+                        ptx::bar_sync(1 + s, k2f::HANDOFF);
+                        if (b >= 0) ptx::mbar_wait(&vp_empty[buf], ((v >> 1) & 1) ^ 1, status, 541);   // its last UMMAs are done
+                        const uint8_t* ecol = es + (col + 2) * 128 + q * 16;      // this thread's column in the E rows
+#pragma unroll
+                        for (int j = 0; j < k2f::BR; ++j) {
+                            if (b >= 0 || j >= 2) {
+                                const float4* row = reinterpret_cast<const float4*>(vs + (j * k2f::VW + col) * 128 + q * 16);
+                                const V4 hs = v4_add(v4_add(v4(row[0]), v4(row[8])), v4(row[16]));
+                                if (b >= 0) {
+                                    // tile row j is macro-tile row 4b+j: its E came with the block before (j < 2, kept
+                                    // in registers) or is row j-2 of this block's E rows
+                                    const V4 e = v4(j == 0 ? ekeep0 : j == 1 ? ekeep1
+                                                    : *reinterpret_cast<const float4*>(ecol + (j - 2) * k2f::EW * 128));
+                                    const V4 out = v4_mul(e, v4_add(v4_add(h2, h1), hs));
+                                    uint32_t pa[3], pb[3];
+                                    split3(out.a, pa[0], pa[1], pa[2]);
+                                    split3(out.b, pb[0], pb[1], pb[2]);
+                                    uint8_t* dst = a_vp + swz64(j * k2f::SW + col, q >> 1) + (q & 1) * 8;
+#pragma unroll
+                                    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dst + p * k2f::PART) = make_uint2(pa[p], pb[p]);
+                                    const int orow = m.my0 + 4 * b + j, ocol = m.mx0 + col;
+                                    if (vprime != nullptr && orow < g.H && ocol < g.W)
+                                        *reinterpret_cast<float4*>(vprime + ((size_t)m.b * NH + (hh >> 1)) * vplane +
+                                                                   ((size_t)orow * g.W + ocol) * HD + (hh & 1) * 32 + q * 4) = v4_f4(out);
+                                }
+                                h2 = h1; h1 = hs;
+                            }
+                        }
+                        ekeep0 = *reinterpret_cast<const float4*>(ecol + 2 * k2f::EW * 128);
+                        ekeep1 = *reinterpret_cast<const float4*>(ecol + 3 * k2f::EW * 128);
+                        if (b >= 0) {
+                            ptx::fence_proxy_async();
+                            ptx::mbar_arrive(&vp_full[buf]);
+                            ++v;
+                        }
+                        ptx::mbar_arrive(&empty[s]);
+                    }
                 }
             }
         }
     }
-
-    // X+ = scale * X + dt * Y, in place, and the tile's per-channel sums of what was stored
-    const float4 s = *reinterpret_cast<const float4*>(scale + b * NC + c0);
-    // The tile's channel sums are kept in fp64 and handed on as a float pair (value, remainder): a state that has
-    // grown large and signed makes the per-channel sum a small difference of large terms, and fp32 tile sums would
-    // then miss the 1e-6 bound on the renormalised mass.
-    double psum[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int cell = cg * 4 + j;
-        const int r = ty0 + (cell >> 3), x = tx0 + (cell & 7);
-        if (r >= g.H || x >= g.W) continue;
-        float* px = X + (size_t)b * xplane + ((size_t)g.xrow(r) * g.W + x) * NC + c0;
-        float4 v = *reinterpret_cast<const float4*>(px);
-        v.x = fmaf(g.dt, acc[j][0], v.x * s.x); v.y = fmaf(g.dt, acc[j][1], v.y * s.y);
-        v.z = fmaf(g.dt, acc[j][2], v.z * s.z); v.w = fmaf(g.dt, acc[j][3], v.w * s.w);
-        *reinterpret_cast<float4*>(px) = v;
-        psum[0] += (double)v.x; psum[1] += (double)v.y; psum[2] += (double)v.z; psum[3] += (double)v.w;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) red[cg * 64 + c0 + k] = psum[k];
+    ptx::tc_fence_before();
     __syncthreads();
-    if (tid < 64) {
-        double t = 0.0;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) t += red[k * 64 + tid];
-        const size_t o = ((size_t)b * gridDim.x + blockIdx.x) * NC + tid;
-        const float hi = (float)t;
-        partial[o] = hi;
-        partial[o + lo_offset] = (float)(t - (double)hi);
+    if (warp == 0) ptx::tmem_dealloc(tmem, k2f::TMEM_COLS);
+}
+
+// =============================================================================================================
+// host side
+inline void f32_plan(F32Plan& p, const Geom& g) {
+    p.tiles_x = (g.W + TBW - 1) / TBW;
+    p.k1_tiles = p.tiles_x * ((g.H + 2 * g.he + TBH - 1) / TBH);
+    p.strips = (g.W + k2f::SW - 1) / k2f::SW;
+    p.k2_tiles = p.strips * ((g.H + k2f::BR - 1) / k2f::BR);
+}
+
+// Tensor map of `rank` dimensions over T = fp32 or bf16 values; byte strides of dimensions 1 .. rank-1.
+inline bool f32_map(EncodeTiledFn enc, CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims,
+                    const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(map, type, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// 0 on success, else the text is in bf16_error()
+inline int f32_setup(F32Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16* wo, int sets, const float* E, const float* V,
+                     const float* X, const Geom& g, int num_sms) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn ||
+        q != cudaDriverEntryPointSuccess) {
+        bf16_error_ref() = "cuTensorMapEncodeTiled is not available from the driver";
+        return -1;
     }
+    EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(fn);
+    const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, F32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+    const cuuint64_t d1[2] = {64, (cuuint64_t)sets * NH * 3 * 192}, s1[1] = {128};
+    const cuuint64_t d2[2] = {32, (cuuint64_t)sets * k2f::NHH * 192}, s2[1] = {64};
+    const cuuint32_t b1[2] = {64, 64}, b2[2] = {32, 192};
+    const cuuint64_t dp[4] = {64, (cuuint64_t)g.ev_w, (cuuint64_t)g.ev_h, (cuuint64_t)g.B * NH};
+    const cuuint64_t sp[3] = {256, (cuuint64_t)g.ev_w * 256, (cuuint64_t)g.ev_h * g.ev_w * 256};
+    const cuuint32_t be[4] = {32, k2f::EW, k2f::BR, 1}, bv[4] = {32, k2f::VW, k2f::BR, 1}, bs[4] = {16, TBW, 2, 1};
+    // the rows below the own rows (a stripe's bottom halo) are left out of the state's map, so that a store of a tile
+    // that hangs over the last own row is clipped there
+    const cuuint64_t dx[4] = {64, (cuuint64_t)g.W, (cuuint64_t)(g.hx + g.H), (cuuint64_t)g.B};
+    const cuuint64_t sx[3] = {256, (cuuint64_t)g.W * 256, (cuuint64_t)g.state_rows() * g.W * 256};
+    const cuuint32_t bx[4] = {32, k2f::SW, k2f::BR, 1};
+    if (!f32_map(enc, &p.map_w1, BF, 2, w1, d1, s1, b1, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !f32_map(enc, &p.map_wo, BF, 2, wo, d2, s2, b2, CU_TENSOR_MAP_SWIZZLE_64B) ||
+        !f32_map(enc, &p.map_e, F32, 4, E, dp, sp, be, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !f32_map(enc, &p.map_v, F32, 4, V, dp, sp, bv, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !f32_map(enc, &p.map_es, F32, 4, E, dp, sp, bs, CU_TENSOR_MAP_SWIZZLE_64B) ||
+        !f32_map(enc, &p.map_vs, F32, 4, V, dp, sp, bs, CU_TENSOR_MAP_SWIZZLE_64B) ||
+        !f32_map(enc, &p.map_x, F32, 4, X, dx, sx, bx, CU_TENSOR_MAP_SWIZZLE_128B)) {
+        bf16_error_ref() = "cuTensorMapEncodeTiled rejected a layout of the fp32 path";
+        return -1;
+    }
+    if (cudaFuncSetAttribute(k1_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, k1f::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k2_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, k2f::SMEM) != cudaSuccess) {
+        bf16_error_ref() = "could not opt in to the kernels' dynamic shared memory";
+        return -1;
+    }
+    const long long items = (long long)p.k1_tiles * g.B * NH;
+    p.k1_grid = (int)(items < num_sms ? items : num_sms);
+    const long long total_mt = k2_macro_tiles(g, p.strips, k2f::NB, num_sms, p.nbmax, p.mt_per_grid);
+    p.k2_grid = (int)(total_mt < num_sms ? total_mt : num_sms);
+    return 0;
 }
 
 }  // namespace slime

@@ -33,6 +33,18 @@ struct Geom {
     __host__ __device__ int state_rows() const { return H + 2 * hx; }
     __host__ __device__ int ev_rows() const { return ev_h; }
     __device__ int wrap_x(int x) const { x %= W; return x < 0 ? x + W : x; }
+    // the same for positions at most one tile outside the grid: no division (a handful of steps on grids smaller than that)
+    __device__ int wrap_x_near(int x) const {
+        if (x < 0) x += W;
+        while (x >= W) x -= W;
+        return x;
+    }
+    __device__ int xrow_near(int r) const {
+        if (!wrap_y) return xrow(r);
+        if (r < 0) r += H;
+        while (r >= H) r -= H;
+        return r;
+    }
     // physical row in the state buffer of own-coordinate row r
     __device__ int xrow(int r) const {
         if (wrap_y) { r %= H; return r < 0 ? r + H : r; }

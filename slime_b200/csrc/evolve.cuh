@@ -94,13 +94,23 @@ k_evolve_refill(float* __restrict__ master, const int* __restrict__ parent, Evol
 
 // grid (blocks, n_sets): master weights -> the layouts the step kernels read.  `only`, when given, restricts the
 // work to sets whose parent differs from themselves (the ones the refill just rewrote).
-//   fp32 path: wpiv [set][8][64 c][192] = Wp | Wi | Wv rows, wo [set][512][64] as stored, prm {taps, mu, -1/(2 sigma^2)}
 //   bf16 path: w1 [set][8][192 rows = output column][64 c] with Wp scaled by s = sqrt(log2(e) / (2 sigma^2)) and
 //              Wi by log2(e), wo [set][8][64 c][64 d], prm {taps, mu * s, s}
+//   fp32 path: the same constants, every value as the sum of three bf16 parts (hi, mid, lo: 24 bits and more): w1
+//              [set][8][3 parts][192 rows][64 c], wo [set][8][2 halves of d][3 parts][64 c][32 d], prm as for bf16
+// The tensor core truncates its fp32 sums, which shortens them by a constant share on average; that share goes back into
+// the weights' lo part (exact zeros stay zeros).  Measured on 128 x 128 grids, one step, by projection on the fp64
+// result: V' -6.0e-8 (four truncations at K = 64) and Y for given V' -4.0e-8 (two at K = 32).
+constexpr double TRUNC_K64 = 1.0 + 6.0e-8, TRUNC_K32 = 1.0 + 4.0e-8;
+__device__ __forceinline__ void store_parts(__nv_bfloat16* dst, size_t part_stride, double x) {
+    const __nv_bfloat16 hi = __double2bfloat16(x);
+    const double r = x - (double)__bfloat162float(hi);
+    const __nv_bfloat16 mid = __double2bfloat16(r);
+    dst[0] = hi; dst[part_stride] = mid; dst[2 * part_stride] = __double2bfloat16(r - (double)__bfloat162float(mid));
+}
 __global__ void __launch_bounds__(256)
 k_weights_layout(const float* __restrict__ master, const int* __restrict__ only, int first_set, int bf16,
-                 float* __restrict__ wpiv_f32, float* __restrict__ wo_f32, __nv_bfloat16* __restrict__ w1_bf16,
-                 __nv_bfloat16* __restrict__ wo_bf16, float* __restrict__ prm) {
+                 __nv_bfloat16* __restrict__ w1_all, __nv_bfloat16* __restrict__ wo_all, float* __restrict__ prm) {
     const int s = first_set + blockIdx.y;
     if (only != nullptr && only[s] == s) return;
     const float* m = master + (size_t)s * MW_STRIDE;
@@ -110,29 +120,31 @@ k_weights_layout(const float* __restrict__ master, const int* __restrict__ only,
         const float mu = m[MW_MU + hd], sg = m[MW_SIGMA + hd];
         float* q = prm + ((size_t)s * NH + hd) * PRM;
         for (int t = 0; t < 9; ++t) q[t] = m[MW_K + hd * 9 + t];
-        if (bf16) {
-            const float sc = sqrtf(1.4426950408889634f / (2.f * sg * sg));
-            q[9] = mu * sc; q[10] = sc;
-        } else {
-            q[9] = mu; q[10] = -1.f / (2.f * sg * sg);
-        }
+        const float sc = sqrtf(1.4426950408889634f / (2.f * sg * sg));
+        q[9] = bf16 ? mu * sc : (float)(mu * sqrt(1.4426950408889634 / (2.0 * sg * sg)));
+        q[10] = sc;
         q[11] = 0.f;
     }
+    const int parts = bf16 ? 1 : 3;
+    __nv_bfloat16* w1 = w1_all + (size_t)s * NH * parts * 192 * 64;
+    __nv_bfloat16* wo = wo_all + (size_t)s * NH * parts * 64 * 64;
     for (int i = t0; i < NH * NC * HD; i += nt) {
         const int hd = i >> 12, c = (i >> 6) & 63, d = i & 63;   // source index [hd][c][d]; for Wo: [hd][d'=c][c'=d]
         if (bf16) {
             const float sg = m[MW_SIGMA + hd];
             const float sc = sqrtf(1.4426950408889634f / (2.f * sg * sg));
-            __nv_bfloat16* w1 = w1_bf16 + (size_t)s * NH * 192 * 64;
             w1[((size_t)hd * 192 + d) * 64 + c] = __float2bfloat16_rn(m[MW_WP + i] * sc);
             w1[((size_t)hd * 192 + 64 + d) * 64 + c] = __float2bfloat16_rn(m[MW_WI + i] * 1.4426950408889634f);
             w1[((size_t)hd * 192 + 128 + d) * 64 + c] = __float2bfloat16_rn(m[MW_WV + i]);
             // Wo[(hd*64 + d')][c'] -> row c' (output channel), column d'
-            wo_bf16[(size_t)s * NH * 64 * 64 + ((size_t)hd * 64 + d) * 64 + c] = __float2bfloat16_rn(m[MW_WO + i]);
+            wo[((size_t)hd * 64 + d) * 64 + c] = __float2bfloat16_rn(m[MW_WO + i]);
         } else {
-            float* w = wpiv_f32 + (size_t)s * NH * NC * 192 + ((size_t)hd * NC + c) * 192 + d;
-            w[0] = m[MW_WP + i]; w[64] = m[MW_WI + i]; w[128] = m[MW_WV + i];
-            wo_f32[(size_t)s * NH * HD * NC + i] = m[MW_WO + i];
+            const double sg = m[MW_SIGMA + hd];
+            __nv_bfloat16* w = w1 + ((size_t)hd * 3 * 192 + d) * 64 + c;
+            store_parts(w, 192 * 64, m[MW_WP + i] * sqrt(1.4426950408889634 / (2.0 * sg * sg)) * TRUNC_K64);
+            store_parts(w + 64 * 64, 192 * 64, m[MW_WI + i] * 1.4426950408889634 * TRUNC_K64);
+            store_parts(w + 128 * 64, 192 * 64, m[MW_WV + i] * TRUNC_K64);
+            store_parts(wo + ((size_t)(hd * 2 + (c >> 5)) * 3 * 64 + d) * 32 + (c & 31), 64 * 32, m[MW_WO + i] * TRUNC_K32);
         }
     }
 }

@@ -95,6 +95,8 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void*
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all of this thread's bulk stores have finished reading shared memory
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// ... all but the last of them
+__device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // all of this thread's bulk stores have completed
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // named barrier among `count` threads of the CTA (ids 1..15; 0 is __syncthreads)
@@ -148,6 +150,50 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// The same two by a whole warp whose control flow is uniform, executed by its leader only: the operands then stay in
+// uniform registers.  Issued from inside an `if (lane == 0)` every product costs about 190 cycles of moves into uniform
+// registers, which is what bounds an issuer with many small products.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
+// The four K = 16 steps of a K = 64 (KS = 2: K = 32) product, issued in one go.  `a` and `b` are the low words of operand
+// descriptors (addresses in 16-byte units, a step is 32 B); HI is their common high word.
+constexpr uint32_t SW128_HI = (1024u >> 4) | (1u << 14) | (2u << 29);     // 8-row groups 1024 B apart, version, SWIZZLE_128B
+constexpr uint32_t SW64_HI = (512u >> 4) | (1u << 14) | (4u << 29);       // 8-row groups 512 B apart, SWIZZLE_64B
+#define SLIME_UMMA_SS(STEP, P) "add.u32 x, %1, " #STEP ";\n\tadd.u32 y, %2, " #STEP ";\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t" \
+                               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, " #P ";\n\t"
+#define SLIME_UMMA_TS(STEP, COL, P) "add.u32 x, %1, " #COL ";\n\tadd.u32 y, %2, " #STEP ";\n\tmov.b64 db, {y, %3};\n\t" \
+                                    "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [x], db, %4, " #P ";\n\t"
+#define SLIME_UMMA_HEAD "{\n\t.reg .pred p, q, one;\n\t.reg .b32 x, y;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\t" \
+                        "setp.ne.b32 q, %6, 0;\n\tsetp.eq.b32 one, 0, 0;\n\t"
+template <uint32_t IDESC, uint32_t HI>
+__device__ __forceinline__ void umma4_ss(uint32_t leader, uint32_t d, uint32_t a, uint32_t b, bool accumulate) {
+    asm volatile(SLIME_UMMA_HEAD SLIME_UMMA_SS(0, p) SLIME_UMMA_SS(2, one) SLIME_UMMA_SS(4, one) SLIME_UMMA_SS(6, one) "}"
+                 ::"r"(d), "r"(a | (1u << 16)), "r"(b | (1u << 16)), "r"(HI), "r"(IDESC), "r"((uint32_t)accumulate), "r"(leader) : "memory");
+}
+template <uint32_t IDESC, uint32_t HI>
+__device__ __forceinline__ void umma2_ss(uint32_t leader, uint32_t d, uint32_t a, uint32_t b, bool accumulate) {
+    asm volatile(SLIME_UMMA_HEAD SLIME_UMMA_SS(0, p) SLIME_UMMA_SS(2, one) "}"
+                 ::"r"(d), "r"(a | (1u << 16)), "r"(b | (1u << 16)), "r"(HI), "r"(IDESC), "r"((uint32_t)accumulate), "r"(leader) : "memory");
+}
+// ... with the A operand in TMEM: row m in lane m, two consecutive k per 32-bit column (a K = 16 step is 8 columns)
+template <uint32_t IDESC>
+__device__ __forceinline__ void umma4_ts(uint32_t leader, uint32_t d, uint32_t a, uint32_t b, bool accumulate) {
+    asm volatile(SLIME_UMMA_HEAD SLIME_UMMA_TS(0, 0, p) SLIME_UMMA_TS(2, 8, one) SLIME_UMMA_TS(4, 16, one) SLIME_UMMA_TS(6, 24, one) "}"
+                 ::"r"(d), "r"(a), "r"(b | (1u << 16)), "r"(SW128_HI), "r"(IDESC), "r"((uint32_t)accumulate), "r"(leader) : "memory");
+}
+#undef SLIME_UMMA_SS
+#undef SLIME_UMMA_TS
+#undef SLIME_UMMA_HEAD
+__device__ __forceinline__ void umma_commit_by(uint32_t leader, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader) : "memory");
+}
+
 // TMEM -> registers: this thread's lane (32 * (warp % 4) + lane), 16 consecutive fp32 columns from `taddr`.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -157,6 +203,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// registers -> TMEM, same addressing
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---- packed fp32 pairs (add/mul/fma.f32x2: one instruction for two lanes of fp32) ---------------------------
 struct f2 { unsigned long long v; };

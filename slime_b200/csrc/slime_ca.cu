@@ -44,11 +44,9 @@ struct slime_ca {
     int* tickets = nullptr;          // one per grid: blocks of the reduction that have finished (back at 0 after each launch)
     int k1_tiles = 0, k2_tiles = 0, tiles_x = 0;
     // weights
-    float* wpiv_f32 = nullptr;      // [sets][8][64][192]  rows c_in, columns Wp | Wi | Wv
-    float* wo_f32 = nullptr;        // [sets][8][64][64]   rows d, columns c_out
     float* prm = nullptr;           // [sets][8][PRM]
-    __nv_bfloat16* w1_bf16 = nullptr;  // [sets][8][192][64]  rows = output column (Wp|Wi|Wv), K = c_in contiguous
-    __nv_bfloat16* wo_bf16 = nullptr;  // [sets][8][64][64]   rows = c_out, K = d contiguous
+    __nv_bfloat16* w1 = nullptr;    // [sets][8][192][64]  rows = output column (Wp|Wi|Wv), K = c_in contiguous; the fp32 path
+    __nv_bfloat16* wo = nullptr;    // [sets][8][64][64]   rows = c_out, K = d contiguous; holds both in parts (k_weights_layout)
     float* master = nullptr;        // [sets][MW_STRIDE] fp32 master copy in the upload's own index order
     float* set_stats = nullptr;     // [sets][2] mean fitness, mean hunger of the last population step
     int* parent = nullptr;          // [sets] parent of each set after the last population step
@@ -76,6 +74,7 @@ struct slime_ca {
     long long launches = 0;
     std::string err = "";
     Bf16Plan bf{};
+    F32Plan f32{};
 };
 
 namespace {
@@ -154,12 +153,15 @@ int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nul
             return fail(h, SLIME_CA_ECUDA, std::string("bf16 k2 launch: ") + cudaGetErrorString(cudaGetLastError()));
         ++h->launches;
     } else {
-        k1_f32<<<dim3(h->k1_tiles, g.B), 256, K1F32_SMEM, st>>>((const float*)h->X, h->scale, h->wpiv_f32, h->prm,
-                                                                 (float*)h->E, (float*)h->V, g);
+        const F32Plan& p = h->f32;
+        k1_f32<<<p.k1_grid, k1f::THREADS, k1f::SMEM, st>>>(p.map_w1, p.map_es, p.map_vs, (const float*)h->X, h->scale, h->prm,
+                                                           (float*)h->E, (float*)h->V, h->dev_status, p.k1_tiles * g.B * NH,
+                                                           p.k1_tiles, g);
         LAUNCHED(h);
         if (ev) CK(h, cudaEventRecord(ev[1], st));
-        k2_f32<<<dim3(h->k2_tiles, g.B), 256, K2F32_SMEM, st>>>((float*)h->X, h->scale, h->wo_f32, (const float*)h->E,
-                                                                 (const float*)h->V, h->partial, h->partial_lo, (float*)emit, g);
+        k2_f32<<<p.k2_grid, k2f::THREADS, k2f::SMEM, st>>>(p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, h->partial, h->partial_lo,
+                                                           (float*)emit, h->dev_status, p.mt_per_grid * g.B, p.mt_per_grid,
+                                                           p.strips, p.k2_tiles, p.nbmax, g);
         LAUNCHED(h);
     }
     if (ev) CK(h, cudaEventRecord(ev[2], st));
@@ -302,8 +304,7 @@ int slime_ca_create(const slime_ca_config* cfg, slime_ca** out) {
     g.per_set = cfg->batch / cfg->n_weight_sets;
     g.dt = cfg->dt;
     h->esz = cfg->dtype == SLIME_CA_BF16 ? 2 : 4;
-    if (cfg->dtype == SLIME_CA_BF16) { g.ev_h = g.H + 2 * APRON; g.ev_w = g.W + 2 * APRON; }
-    else { g.ev_h = g.H + 2 * g.he; g.ev_w = g.W; }
+    g.ev_h = g.H + 2 * APRON; g.ev_w = g.W + 2 * APRON;
     h->weights_set.assign(cfg->n_weight_sets, 0);
 
     const size_t xn = (size_t)g.B * g.state_rows() * g.W * NC;
@@ -314,11 +315,9 @@ int slime_ca_create(const slime_ca_config* cfg, slime_ca** out) {
         g.tiles_x = h->bf.tiles_x;
         h->k1_tiles = h->bf.k1_tiles; h->k2_tiles = h->bf.k2_tiles;
     } else {
-        g.tiles_x = (g.W + T32 - 1) / T32;
-        h->k1_tiles = g.tiles_x * ((g.H + 2 * g.he + T32 - 1) / T32);
-        h->k2_tiles = g.tiles_x * ((g.H + T32 - 1) / T32);
-        CK(h, cudaFuncSetAttribute(k1_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, K1F32_SMEM));
-        CK(h, cudaFuncSetAttribute(k2_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, K2F32_SMEM));
+        f32_plan(h->f32, g);
+        g.tiles_x = h->f32.tiles_x;
+        h->k1_tiles = h->f32.k1_tiles; h->k2_tiles = h->f32.k2_tiles;
     }
     h->tiles_x = g.tiles_x;
     const int chunks = (int)(((size_t)g.H * g.W + 255) / 256);
@@ -367,17 +366,14 @@ int slime_ca_create(const slime_ca_config* cfg, slime_ca** out) {
     if ((rc = dev_alloc(h, &h->set_stats, sets * 2))) return rc;
     if ((rc = dev_alloc(h, &h->parent, sets))) return rc;
     if ((rc = dev_alloc(h, &h->evolve_info, 2))) return rc;
-    if (is_bf16(h)) {
-        if ((rc = dev_alloc(h, &h->w1_bf16, sets * NH * 192 * 64))) return rc;
-        if ((rc = dev_alloc(h, &h->wo_bf16, sets * NH * 64 * 64))) return rc;
-        if (bf16_setup(h->bf, h->w1_bf16, h->wo_bf16, (int)sets, (const __nv_bfloat16*)h->E, (const __nv_bfloat16*)h->V,
-                       (const __nv_bfloat16*)h->X, g,
-                       prop.multiProcessorCount) != 0)
-            return fail(h, SLIME_CA_ECUDA, "tensor-map / kernel attribute set-up failed: " + std::string(bf16_error()));
-    } else {
-        if ((rc = dev_alloc(h, &h->wpiv_f32, sets * NH * NC * 192))) return rc;
-        if ((rc = dev_alloc(h, &h->wo_f32, sets * NH * HD * NC))) return rc;
-    }
+    const size_t parts = is_bf16(h) ? 1 : 3;
+    if ((rc = dev_alloc(h, &h->w1, sets * NH * parts * 192 * 64))) return rc;
+    if ((rc = dev_alloc(h, &h->wo, sets * NH * parts * 64 * 64))) return rc;
+    const int bad = is_bf16(h) ? bf16_setup(h->bf, h->w1, h->wo, (int)sets, (const __nv_bfloat16*)h->E, (const __nv_bfloat16*)h->V,
+                                            (const __nv_bfloat16*)h->X, g, prop.multiProcessorCount)
+                               : f32_setup(h->f32, h->w1, h->wo, (int)sets, (const float*)h->E, (const float*)h->V,
+                                           (const float*)h->X, g, prop.multiProcessorCount);
+    if (bad) return fail(h, SLIME_CA_ECUDA, "tensor-map / kernel attribute set-up failed: " + std::string(bf16_error()));
     std::vector<float> ones((size_t)g.B * NC, 1.f);
     CK(h, cudaMemcpy(h->scale, ones.data(), ones.size() * sizeof(float), cudaMemcpyHostToDevice));
     return SLIME_CA_OK;
@@ -387,7 +383,7 @@ int slime_ca_destroy(slime_ca* h) {
     if (!h) return SLIME_CA_EINVAL;
     cudaSetDevice(h->cfg.device);
     void* ptrs[] = {h->X, h->E, h->V, h->vprime[0], h->vprime[1], h->scale, h->mass, h->sums, h->partial, h->seg_sums, h->tickets,
-                    h->wpiv_f32, h->wo_f32, h->prm, h->w1_bf16, h->wo_bf16, h->gram_part, h->head_rank,
+                    h->prm, h->w1, h->wo, h->gram_part, h->head_rank,
                     h->pearson_part, h->fit_dev, h->dev_status, h->master, h->set_stats, h->parent, h->evolve_info};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -422,8 +418,7 @@ int slime_ca_set_weights(slime_ca* h, int set_index, const float* Wp, const floa
     CK(h, cudaMemcpy(m + MW_K, K, NH * 9 * sizeof(float), cudaMemcpyHostToDevice));
     CK(h, cudaMemcpy(m + MW_MU, mu, NH * sizeof(float), cudaMemcpyHostToDevice));
     CK(h, cudaMemcpy(m + MW_SIGMA, sigma, NH * sizeof(float), cudaMemcpyHostToDevice));
-    k_weights_layout<<<dim3(32, 1), 256>>>(h->master, nullptr, set_index, is_bf16(h) ? 1 : 0, h->wpiv_f32, h->wo_f32,
-                                           h->w1_bf16, h->wo_bf16, h->prm);
+    k_weights_layout<<<dim3(32, 1), 256>>>(h->master, nullptr, set_index, is_bf16(h) ? 1 : 0, h->w1, h->wo, h->prm);
     LAUNCHED(h);
     CK(h, cudaStreamSynchronize(nullptr));
     h->weights_set[set_index] = 1;
@@ -683,8 +678,7 @@ int slime_ca_evolve(slime_ca* h, const slime_ca_evolve_params* p, int* parent, i
     LAUNCHED(h);
     k_evolve_refill<<<dim3(32, sets), 256, 0, st>>>(h->master, h->parent, ep);
     LAUNCHED(h);
-    k_weights_layout<<<dim3(32, sets), 256, 0, st>>>(h->master, h->parent, 0, is_bf16(h) ? 1 : 0, h->wpiv_f32, h->wo_f32,
-                                                     h->w1_bf16, h->wo_bf16, h->prm);
+    k_weights_layout<<<dim3(32, sets), 256, 0, st>>>(h->master, h->parent, 0, is_bf16(h) ? 1 : 0, h->w1, h->wo, h->prm);
     LAUNCHED(h);
     int info[2] = {-1, 0};
     CK(h, cudaMemcpyAsync(info, h->evolve_info, sizeof(info), cudaMemcpyDeviceToHost, st));
@@ -1134,9 +1128,9 @@ int slime_ca_occupancy(slime_ca* h, float* occupancy) {
         else CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_bf16<false>, t1, k1b::SMEM));
         CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k2_bf16, t2, k2m::SMEM));
     } else {
-        t1 = t2 = 256;
-        CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_f32, t1, K1F32_SMEM));
-        CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k2_f32, t2, K2F32_SMEM));
+        t1 = k1f::THREADS; t2 = k2f::THREADS;
+        CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_f32, t1, k1f::SMEM));
+        CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k2_f32, t2, k2f::SMEM));
     }
     const float o1 = (float)(b1 * t1) / (float)max_threads, o2 = (float)(b2 * t2) / (float)max_threads;
     *occupancy = o1 < o2 ? o1 : o2;
