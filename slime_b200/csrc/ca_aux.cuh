@@ -12,93 +12,189 @@ template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-// Per-channel sums of the own rows of the stored state, one partial per 256-cell chunk:
-// partial[b][chunk][c] (fp32 over 64 cells per thread, combined in a fixed order).
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_channel_partials(const T* __restrict__ X, float* __restrict__ partial, Geom g) {
-    __shared__ float red[4][64];
-    const int b = blockIdx.y, c = threadIdx.x & 63, sub = threadIdx.x >> 6;
-    const size_t cells = (size_t)g.H * g.W;
-    const size_t first = (size_t)blockIdx.x * 256 + sub * 64;
-    const T* base = X + ((size_t)b * g.state_rows() + g.hx) * g.W * NC;
-    float s = 0.f;
-    for (int i = 0; i < 64; ++i) {
-        const size_t cell = first + i;
-        if (cell < cells) s += to_f32<T>(base[cell * NC + c]);
+// Eight consecutive values, as two or one 16-byte loads where the address allows it (a caller's pointer may not).
+template <typename T> __device__ __forceinline__ void load8(const T* p, bool vec, float (&f)[8]) {
+    if (vec) {
+        if (sizeof(T) == 4) {
+            const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+        } else {
+            const uint4 v = *reinterpret_cast<const uint4*>(p);
+            f[0] = bf16_lo(v.x); f[1] = bf16_hi(v.x); f[2] = bf16_lo(v.y); f[3] = bf16_hi(v.y);
+            f[4] = bf16_lo(v.z); f[5] = bf16_hi(v.z); f[6] = bf16_lo(v.w); f[7] = bf16_hi(v.w);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = to_f32<T>(p[k]);
     }
-    red[sub][c] = s;
-    __syncthreads();
-    if (sub == 0) partial[((size_t)b * gridDim.x + blockIdx.x) * NC + c] = (red[0][c] + red[1][c]) + (red[2][c] + red[3][c]);
+}
+// ... and stored; f becomes what was stored (rounded to T)
+template <typename T> __device__ __forceinline__ void store8(T* p, bool vec, float (&f)[8]) {
+    if (sizeof(T) == 4) {
+        if (vec) {
+            reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
+            reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
+            return;
+        }
+    } else {
+        const uint4 v = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+        f[0] = bf16_lo(v.x); f[1] = bf16_hi(v.x); f[2] = bf16_lo(v.y); f[3] = bf16_hi(v.y);
+        f[4] = bf16_lo(v.z); f[5] = bf16_hi(v.z); f[6] = bf16_lo(v.w); f[7] = bf16_hi(v.w);
+        if (vec) { *reinterpret_cast<uint4*>(p) = v; return; }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p[k] = from_f32<T>(f[k]);
 }
 
-// Stage 1 of the cross-tile reduction: segment s of grid b sums its share of the partials in fp64.  lo_offset != 0:
+// What follows a grid's sums.  mode 0: sums only; 1: also mass = sums and scale = 1 (a freshly loaded state); 2: also
+// scale = mass / sums.
+struct SumsOut {
+    double* sums;
+    double* mass;
+    float* scale;
+    int mode;
+};
+__device__ __forceinline__ void sums_out(const SumsOut& o, int b, int c, double t) {
+    o.sums[b * NC + c] = t;
+    if (o.mode == 1) { o.mass[b * NC + c] = t; o.scale[b * NC + c] = 1.f; }
+    if (o.mode == 2) o.scale[b * NC + c] = (float)(o.mass[b * NC + c] / t);
+}
+
+// Fixed-order fp64 sum of one grid's n partials by NT threads of a block (bar: their barrier), red: [NT / 64][64] doubles
+// of shared memory.  Thread (c, sub) sums every (NT / 64)-th partial of channel c, eight loads in flight.  lo_offset != 0:
 // every partial is a float pair, the remainder lo_offset floats after the value (the fp32 step kernel's tile sums).
-__global__ void __launch_bounds__(256)
-k_reduce_partials(const float* __restrict__ partial, int n_partials, double* __restrict__ seg_sums, size_t lo_offset = 0) {
-    __shared__ double red[4][64];
-    const int b = blockIdx.y, c = threadIdx.x & 63, sub = threadIdx.x >> 6;
-    const int nseg = gridDim.x;
-    const int per_seg = (n_partials + nseg - 1) / nseg;
-    const int per_sub = (per_seg + 3) / 4;
-    const int lo = blockIdx.x * per_seg + sub * per_sub;
-    int hi = lo + per_sub;
-    const int seg_hi = min((blockIdx.x + 1) * per_seg, n_partials);
-    if (hi > seg_hi) hi = seg_hi;
+template <int NT, typename Bar>
+__device__ __forceinline__ void sum_partials(const float* part, int n, size_t lo_offset, double* red, int tid, Bar bar, const SumsOut& o, int b) {
+    constexpr int SUBS = NT / 64;
+    const int c = tid & 63, sub = tid >> 6;
     double s = 0.0;
-    for (int t = lo; t < hi; ++t) {
-        const size_t o = ((size_t)b * n_partials + t) * NC + c;
-        s += (double)partial[o];
-        if (lo_offset) s += (double)partial[o + lo_offset];
+    int t = sub;
+    for (; t + 7 * SUBS < n; t += 8 * SUBS) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = __ldcg(part + (size_t)(t + k * SUBS) * NC + c);
+        if (lo_offset) {
+            float w[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = __ldcg(part + (size_t)(t + k * SUBS) * NC + c + lo_offset);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s += (double)v[k] + (double)w[k];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s += (double)v[k];
+        }
     }
-    red[sub][c] = s;
-    __syncthreads();
-    if (sub == 0) seg_sums[((size_t)b * nseg + blockIdx.x) * NC + c] = (red[0][c] + red[1][c]) + (red[2][c] + red[3][c]);
-}
-
-// Both stages of the cross-tile reduction in one launch: segment s of grid b sums its share of the partials in fp64
-// (as k_reduce_partials), and the block that finishes last for its grid (a ticket per grid, handed back at zero) adds
-// the segments in their fixed order, so the result does not depend on which block that is.
-// mode 0: sums only; 1: also mass = sums and scale = 1 (a freshly loaded state); 2: also scale = mass / sums.
-__global__ void __launch_bounds__(256)
-k_reduce_finish(const float* __restrict__ partial, int n_partials, double* __restrict__ seg_sums, size_t lo_offset,
-                int* __restrict__ tickets, double* __restrict__ sums, double* __restrict__ mass,
-                float* __restrict__ scale, int mode) {
-    __shared__ double red[4][64];
-    __shared__ int is_last;
-    const int b = blockIdx.y, c = threadIdx.x & 63, sub = threadIdx.x >> 6;
-    const int nseg = gridDim.x;
-    const int per_seg = (n_partials + nseg - 1) / nseg;
-    const int per_sub = (per_seg + 3) / 4;
-    const int lo = blockIdx.x * per_seg + sub * per_sub;
-    int hi = lo + per_sub;
-    const int seg_hi = min((blockIdx.x + 1) * per_seg, n_partials);
-    if (hi > seg_hi) hi = seg_hi;
-    double s = 0.0;
-    for (int t = lo; t < hi; ++t) {
-        const size_t o = ((size_t)b * n_partials + t) * NC + c;
-        s += (double)partial[o];
-        if (lo_offset) s += (double)partial[o + lo_offset];
+    for (; t < n; t += SUBS) {
+        const size_t at = (size_t)t * NC + c;
+        s += (double)__ldcg(part + at) + (lo_offset ? (double)__ldcg(part + at + lo_offset) : 0.0);
     }
-    red[sub][c] = s;
-    __syncthreads();
+    red[sub * NC + c] = s;
+    bar();
     if (sub == 0) {
-        seg_sums[((size_t)b * nseg + blockIdx.x) * NC + c] = (red[0][c] + red[1][c]) + (red[2][c] + red[3][c]);
-        __threadfence();
+        double r = 0.0;
+#pragma unroll
+        for (int k = 0; k < SUBS; ++k) r += red[k * NC + c];
+        sums_out(o, b, c, r);
     }
+}
+// Grids with at most this many partials are finished by the block that writes the last of them (a ticket per grid):
+// that costs it 2 to 4 us at the end, a launch of its own 5 to 20 us.  Beyond, a separate launch spreads the sum.
+constexpr int FUSE_PARTIALS = 512;
+
+// Tail of a kernel whose 256-thread blocks each hold the sums of a 256-cell chunk of grid b: acc = the sums over this
+// thread's cells of channels 8 q .. 8 q + 7 (q = tid & 7) -> partial[b][chunk][64], and, with tickets, the grid's sums by
+// the block that comes last.  It also puts the step's own ticket of the grid back to zero (a fresh state starts afresh).
+struct ChunkSums {
+    float* partial;
+    int* tickets;            // null: partials only
+    int* step_tickets;
+    SumsOut out;
+};
+__device__ __forceinline__ void chunk_sums(const float (&acc)[8], const ChunkSums& o) {
+    __shared__ __align__(16) float red[32][64];
+    __shared__ double red64[4 * NC];
+    __shared__ int is_last;
+    const int tid = threadIdx.x, b = blockIdx.y, c = tid & 63, sub = tid >> 6;
+    float4* r4 = reinterpret_cast<float4*>(&red[tid >> 3][(tid & 7) * 8]);
+    r4[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    r4[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
     __syncthreads();
-    if (threadIdx.x == 0) is_last = atomicAdd(&tickets[b], 1) == nseg - 1;
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += red[sub * 8 + k][c];
+    __syncthreads();
+    red[sub][c] = s;
+    __syncthreads();
+    float* part = o.partial + (size_t)b * gridDim.x * NC;
+    if (sub == 0) {
+        part[(size_t)blockIdx.x * NC + c] = (red[0][c] + red[1][c]) + (red[2][c] + red[3][c]);
+        if (o.tickets) __threadfence();
+    }
+    if (!o.tickets) return;
+    __syncthreads();
+    if (tid == 0) is_last = atomicAdd(&o.tickets[b], 1) == (int)gridDim.x - 1;
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    if (sub == 0) {
-        double t = 0.0;
-        for (int i = 0; i < nseg; ++i) t += __ldcg(&seg_sums[((size_t)b * nseg + i) * NC + c]);
-        sums[b * NC + c] = t;
-        if (mode == 1) { mass[b * NC + c] = t; scale[b * NC + c] = 1.f; }
-        if (mode == 2) scale[b * NC + c] = (float)(mass[b * NC + c] / t);
+    sum_partials<256>(part, gridDim.x, 0, red64, tid, [] { __syncthreads(); }, o.out, b);
+    if (tid == 0) { o.tickets[b] = 0; if (o.step_tickets) o.step_tickets[b] = 0; }
+}
+
+// Per-channel sums of the own rows of the stored state.  Grid (256-cell chunks, grids).
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_channel_partials(const T* __restrict__ X, bool vec, ChunkSums out, Geom g) {
+    const size_t cells = (size_t)g.H * g.W;
+    const T* base = X + ((size_t)blockIdx.y * g.state_rows() + g.hx) * g.W * NC + (threadIdx.x & 7) * 8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const size_t cell = (size_t)blockIdx.x * 256 + i * 32 + (threadIdx.x >> 3);
+        if (cell < cells) {
+            float f[8];
+            load8<T>(base + cell * NC, vec, f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] += f[k];
+        }
     }
-    if (threadIdx.x == 0) tickets[b] = 0;
+    chunk_sums(acc, out);
+}
+
+// Stage 1 of the cross-tile reduction: segment s of grid b sums its share of the partials in fp64 (the channel sums that
+// allocate nothing).
+__global__ void __launch_bounds__(256)
+k_reduce_partials(const float* __restrict__ partial, int n_partials, double* __restrict__ sums) {
+    __shared__ double red[4 * NC];
+    const int b = blockIdx.y;
+    sum_partials<256>(partial + (size_t)b * n_partials * NC, n_partials, 0, red, threadIdx.x, [] { __syncthreads(); }, SumsOut{sums, nullptr, nullptr, 0}, b);
+}
+
+// The cross-tile reduction of grids with many partials, in one launch: segment s of grid b sums its share of the partials
+// in fp64, and the block that finishes last for its grid (a ticket per grid, handed back at zero) adds the segments in
+// their fixed order, so the result does not depend on which block that is.
+__global__ void __launch_bounds__(256)
+k_reduce_finish(const float* __restrict__ partial, int n_partials, double* __restrict__ seg_sums, size_t lo_offset,
+                int* __restrict__ tickets, SumsOut out) {
+    __shared__ double red[4 * NC];
+    __shared__ int is_last;
+    const int b = blockIdx.y, tid = threadIdx.x, c = tid & 63, sub = tid >> 6, nseg = gridDim.x;
+    const int per_seg = (n_partials + nseg - 1) / nseg;
+    const int lo = min((int)blockIdx.x * per_seg, n_partials), hi = min(lo + per_seg, n_partials);
+    sum_partials<256>(partial + ((size_t)b * n_partials + lo) * NC, hi - lo, lo_offset, red, tid, [] { __syncthreads(); },
+                      SumsOut{seg_sums, nullptr, nullptr, 0}, b * nseg + blockIdx.x);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) is_last = atomicAdd(&tickets[b], 1) == nseg - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    double s = 0.0;
+#pragma unroll 8
+    for (int i = sub; i < nseg; i += 4) s += __ldcg(&seg_sums[((size_t)b * nseg + i) * NC + c]);
+    red[sub * NC + c] = s;
+    __syncthreads();
+    if (sub == 0) sums_out(out, b, c, (red[c] + red[NC + c]) + (red[2 * NC + c] + red[3 * NC + c]));
+    if (tid == 0) tickets[b] = 0;
 }
 
 // scale = mass / sums from buffers the caller may have all-reduced.
@@ -108,45 +204,74 @@ __global__ void k_scale_from_sums(const double* __restrict__ sums, const double*
     if (i < n) scale[i] = (float)(mass[i] / sums[i]);
 }
 
-// dense [B][H][W][64] (TI) -> own rows of the state buffer (TO); halo rows untouched.
+// dense [B][H][W][64] (TI) -> own rows of the state buffer (TO), halo rows untouched, and the sums of what was stored.
+// Grid (256-cell chunks, grids).
 template <typename TI, typename TO>
-__global__ void k_state_in(const TI* __restrict__ src, TO* __restrict__ X, Geom g) {
-    const size_t per = (size_t)g.H * g.W * NC;
-    const size_t n = per * g.B;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t b = i / per, o = i % per;
-        X[(b * g.state_rows() + g.hx) * g.W * NC + o] = from_f32<TO>(to_f32<TI>(src[i]));
+__global__ void __launch_bounds__(256)
+k_state_in(const TI* __restrict__ src, bool vec, TO* __restrict__ X, ChunkSums out, Geom g) {
+    const size_t cells = (size_t)g.H * g.W, b = blockIdx.y;
+    const int q = (threadIdx.x & 7) * 8;
+    TO* dst = X + ((size_t)b * g.state_rows() + g.hx) * g.W * NC + q;
+    src += b * cells * NC + q;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const size_t cell = (size_t)blockIdx.x * 256 + i * 32 + (threadIdx.x >> 3);
+        if (cell < cells) {
+            float f[8];
+            load8<TI>(src + cell * NC, vec, f);
+            store8<TO>(dst + cell * NC, true, f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] += f[k];
+        }
+    }
+    chunk_sums(acc, out);
+}
+
+// own rows of the state buffer times the pending scale -> dense [B][H][W][64] (TO).  Grid (blocks, grids), eight values a thread.
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256)
+k_state_out(const TI* __restrict__ X, const float* __restrict__ scale, TO* __restrict__ dst, bool vec, Geom g) {
+    const size_t n = (size_t)g.H * g.W * 8, b = blockIdx.y;
+    const int q = (threadIdx.x & 7) * 8;                 // the same for all of a thread's chunks: the stride is a multiple of 8
+    const TI* src = X + ((size_t)b * g.state_rows() + g.hx) * g.W * NC;
+    dst += b * n * 8;
+    float s[8];
+    load8<float>(scale + b * NC + q, true, s);
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+        float f[8];
+        load8<TI>(src + i * 8, true, f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] *= s[k];
+        store8<TO>(dst + i * 8, vec, f);
     }
 }
 
-// own rows of the state buffer times the pending scale -> dense [B][H][W][64] (TO).
-template <typename TI, typename TO>
-__global__ void k_state_out(const TI* __restrict__ X, const float* __restrict__ scale, TO* __restrict__ dst, Geom g) {
-    const size_t per = (size_t)g.H * g.W * NC;
-    const size_t n = per * g.B;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t b = i / per, o = i % per;
-        const float v = to_f32<TI>(X[(b * g.state_rows() + g.hx) * g.W * NC + o]) * scale[b * NC + (o & 63)];
-        dst[i] = from_f32<TO>(v);
-    }
-}
-
-// X[b,y,x,c] = img[b,y-py,x-px] * L[c] inside the centred image, 0 in the padding.
+// X[b,y,x,c] = img[b,y-py,x-px] * L[c] inside the centred image, 0 in the padding, and the sums of what was stored.
 template <typename TO>
-__global__ void k_lift(const float* __restrict__ img, int ih, int iw, const float* __restrict__ L,
-                       TO* __restrict__ X, Geom g) {
+__global__ void __launch_bounds__(256)
+k_lift(const float* __restrict__ img, int ih, int iw, const float* __restrict__ L, TO* __restrict__ X, ChunkSums out, Geom g) {
     const int py = (g.H - ih) / 2, px = (g.W - iw) / 2;
-    const size_t per = (size_t)g.H * g.W * NC;
-    const size_t n = per * g.B;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t b = i / per, o = i % per;
-        const int c = (int)(o & 63);
-        const int x = (int)((o >> 6) % g.W), y = (int)((o >> 6) / g.W);
-        const int iy = y - py, ix = x - px;
-        float v = 0.f;
-        if (iy >= 0 && iy < ih && ix >= 0 && ix < iw) v = img[(b * ih + iy) * iw + ix] * L[c];
-        X[(b * g.state_rows() + g.hx) * g.W * NC + o] = from_f32<TO>(v);
+    const int cells = g.H * g.W, q = (threadIdx.x & 7) * 8;
+    const size_t b = blockIdx.y;
+    TO* dst = X + (b * g.state_rows() + g.hx) * g.W * NC + q;
+    float l[8], acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    load8<float>(L + q, true, l);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int cell = blockIdx.x * 256 + i * 32 + (threadIdx.x >> 3);
+        if (cell < cells) {
+            const int y = cell / g.W, iy = y - py, ix = cell - y * g.W - px;
+            const float v = iy >= 0 && iy < ih && ix >= 0 && ix < iw ? img[(b * ih + iy) * iw + ix] : 0.f;
+            float f[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) f[k] = v * l[k];
+            store8<TO>(dst + (size_t)cell * NC, true, f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] += f[k];
+        }
     }
+    chunk_sums(acc, out);
 }
 
 // field[b][cell] = mean over the 64 channels of the normalised state (stored value x pending scale).  Eight

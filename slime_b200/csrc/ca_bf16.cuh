@@ -20,6 +20,7 @@
 #pragma once
 #include <cuda.h>
 
+#include "ca_aux.cuh"
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -38,6 +39,30 @@ struct K1StoreMaps {
     CUtensorMap e_row, v_row;   // box 64 x 16 x 2 x 1
     CUtensorMap e_cor, v_cor;   // box 64 x 2 x 2 x 1
 };
+
+// Where k2 leaves the tiles' channel sums, and how they become the grids' sums: with tickets, whoever finishes a grid's
+// last macro tile adds them up.
+struct K2Sums {
+    float* partial;
+    size_t lo_offset;
+    int* tickets;
+    SumsOut out;
+};
+
+// A set of NT threads (bar: its barrier) has written its share of a macro tile's tile sums; `parts` shares make up grid
+// b's n tiles.  The set that comes last sums them.
+template <int NT, typename Bar>
+__device__ __forceinline__ void k2_finish(const K2Sums& k, int b, int n, int parts, double* red, int* flag, int tid, Bar bar) {
+    if (k.tickets == nullptr) return;
+    if (tid < NC) __threadfence();
+    bar();
+    if (tid == 0) *flag = atomicAdd(&k.tickets[b], 1) == parts - 1;
+    bar();
+    if (!*flag) return;
+    __threadfence();
+    sum_partials<NT>(k.partial + (size_t)b * n * NC, n, k.lo_offset, red, tid, bar, k.out, b);
+    if (tid == 0) k.tickets[b] = 0;
+}
 
 struct Bf16Plan {
     int tiles_x = 1, k1_tiles = 1, k2_tiles = 1, k1_grid = 1, k2_grid = 1;
@@ -641,8 +666,8 @@ constexpr int STG = 0;
 constexpr int A_VP = STG + NSTAGE * STAGE_BYTES;        // two 16 KB operand tiles
 constexpr int WO = A_VP + 2 * 16384;                    // two 8 KB Wo slices
 constexpr int XT = WO + 2 * 8192;                       // two 16 KB state tiles of the epilogue (one per box-sum set)
-constexpr int RED = XT + 2 * 16384;                     // [A, B][4 quads][64] fp32
-constexpr int BARS = RED + 2 * 4 * 64 * 4;
+constexpr int RED = XT + 2 * 16384;                     // [A, B]: [4 quads][64] fp32 of a drain, [4][64] fp64 and a flag of a grid's sums
+constexpr int BARS = RED + 2 * (4 * 64 * 8 + 8);
 constexpr int N_BARS = NSTAGE + NSTAGE + 2 + 2 + 2 + 2 + NB + NB + 2 + 2;
 constexpr int TMEM_PTR = BARS + N_BARS * 8;
 constexpr int BYTES = TMEM_PTR + 16;
@@ -675,7 +700,7 @@ __device__ __forceinline__ MacroTile macro_tile(int idx, int per_grid, int strip
 __global__ void __launch_bounds__(k2m::THREADS, 1)
 k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUtensorMap map_e,
               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ scale,
-              float* __restrict__ partial, __nv_bfloat16* __restrict__ vprime, int* __restrict__ status, int n_mt,
+              const K2Sums fin, __nv_bfloat16* __restrict__ vprime, int* __restrict__ status, int n_mt,
               int mt_per_grid, int strips, int tiles_per_grid, int nbmax, Geom g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
@@ -789,7 +814,7 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
         const bool is_a = warp < 8 || warp == 19;
         const int gt = warp == 19 ? 256 + lane : (is_a ? tid : tid - 256);     // thread within its set
         const int bar_ep = is_a ? 7 : 8;                        // named barrier of the set's drains (256 threads; 1-5 hand blocks over)
-        float* red = reinterpret_cast<float*>(sm + k2m::RED) + (is_a ? 0 : 256);
+        float* red = reinterpret_cast<float*>(sm + k2m::RED + (is_a ? 0 : 4 * 64 * 8 + 8));
         const int q = gt & 7, col = gt >> 3;                    // 8-dim chunk; column (A: of the 34 R columns, B: of the 32)
         uint32_t it = 0, v = 0, acc_par = 0, prev_par = 0;
         MacroTile prev;
@@ -806,7 +831,7 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
             ptx::mbar_wait(&acc_full[b], (par >> b) & 1, status, 232);
             ptx::mbar_wait(&x_full[is_a ? 0 : 1], nxs & 1, status, 233);
             ptx::tc_fence_after();
-            k2_epilogue(t, tmem + b * 64, xs, scale, partial, red, bar_ep, gt, warp, g);
+            k2_epilogue(t, tmem + b * 64, xs, scale, fin.partial, red, bar_ep, gt, warp, g);
             if (gt == 0) {
                 // X+ of the tile back to the state in one store (rows and columns past the grid are clipped); the
                 // buffer goes back to the producer once the store has read it
@@ -820,6 +845,12 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
             ++nxs;
         };
         const int mine = is_a ? 0 : 1;       // parity of the accumulators this set drains
+        // this set's tiles of macro tile `mt` are drained: its share (one of two per macro tile) of the grid's sums is there
+        auto finish = [&](const MacroTile& mt) {
+            if (mt.nb > 0)
+                k2_finish<256>(fin, mt.b, tiles_per_grid, 2 * mt_per_grid, reinterpret_cast<double*>(red), reinterpret_cast<int*>(red + 512), gt,
+                               [&] { ptx::bar_sync(bar_ep, 256); });
+        };
         V8 h2 = v8_zero(), h1 = v8_zero();   // running horizontal sums of the two rows above (of E in A, of R in B)
         uint4 ekeep0 = make_uint4(0, 0, 0, 0), ekeep1 = ekeep0;   // B: centre E of the last two rows of the block before
         const size_t vplane = (size_t)g.H * g.W * HD;
@@ -892,17 +923,21 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
                     }
                 }
                 // accumulators of the macro tile before that this one does not reach (it has fewer blocks)
-                if (h == 0 && gt < 256)
+                if (h == 0 && gt < 256) {
                     for (int b = m.nb; b < prev.nb; ++b)
                         if ((b & 1) == mine) drain(prev, b, prev_par);
+                    finish(prev);
+                }
             }
             prev = m;
             prev_par = acc_par;
             acc_par ^= (1u << m.nb) - 1u;
         }
-        if (gt < 256)
+        if (gt < 256) {
             for (int b = 0; b < prev.nb; ++b)
                 if ((b & 1) == mine) drain(prev, b, prev_par);
+            finish(prev);
+        }
         if (gt == 0) ptx::bulk_wait0();      // this set's stores of X+ are complete
     }
     ptx::tc_fence_before();
@@ -1036,8 +1071,8 @@ inline int bf16_k1(Bf16Plan& p, const __nv_bfloat16* X, const float* scale, cons
 }
 
 inline int bf16_k2(Bf16Plan& p, __nv_bfloat16* X, const float* scale, const __nv_bfloat16*, const __nv_bfloat16*,
-                   float* partial, __nv_bfloat16* vprime, int* status, const Geom& g, cudaStream_t st) {
-    k2_bf16<<<p.k2_grid, k2m::THREADS, k2m::SMEM, st>>>(p.map_wo, p.map_e, p.map_v, p.map_x, scale, partial, vprime, status,
+                   const K2Sums& fin, __nv_bfloat16* vprime, int* status, const Geom& g, cudaStream_t st) {
+    k2_bf16<<<p.k2_grid, k2m::THREADS, k2m::SMEM, st>>>(p.map_wo, p.map_e, p.map_v, p.map_x, scale, fin, vprime, status,
                                                         p.mt_per_grid * g.B, p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

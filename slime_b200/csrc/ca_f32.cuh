@@ -63,26 +63,27 @@ constexpr int WIV = A_CONV + 2 * A_BYTES, WIV_SLOT = 16384;          // two slot
 constexpr int WP = WIV + 2 * WIV_SLOT, WP_SLOT = 8192;               // two slots: one part of Wp
 constexpr int STG = WP + 2 * WP_SLOT;                    // 2 KB staging tiles [32 cells][16 dims]: one per E warp, two per V warp
 constexpr int XH = STG + 16 * 2048, XH_BYTES = 10 * 18 * 256;         // state halo tile, plain [10][18] cells x 64 fp32
-constexpr int PRM_ST = XH + XH_BYTES;                    // head parameters of the tile's weight set
-constexpr int BARS = PRM_ST + NH * PRM * 4, N_BARS = 18, TMEM_PTR = BARS + N_BARS * 8;
+constexpr int BARS = XH + XH_BYTES, N_BARS = 20, TMEM_PTR = BARS + N_BARS * 8;
 constexpr int BYTES = TMEM_PTR + 16;
 constexpr int SMEM = BYTES + 1024;                       // slack for manual 1024-byte alignment
 constexpr uint32_t TMEM_COLS = 512, AX = 384;            // two accumulator buffers of 192 columns, the X operand behind them
-constexpr int THREADS = 768;
+constexpr int THREADS = 800;
 static_assert(SMEM <= 227 * 1024, "k1 (fp32) shared memory");
 }  // namespace k1f
 
 // k1: one CTA per SM, warp-specialised.  The work is the list of (tile of 8 x 16 cells, head) items in order; a CTA
 // takes one contiguous stretch of it, so that the stretches differ by one item at most whatever the size of the grid.
-//   warps 0-7   stencil group: at a new tile loads the state halo (scale applied) and writes the parts of the X operand
-//               into TMEM; per item the 3x3 stencil, two columns x four channels x four rows per thread, written as the
-//               three parts of one of two operand tiles
+//   warps 0-7   stencil group: per item the 3x3 stencil of the state halo, two columns x four channels x four rows per
+//               thread, times the pending scale, written as the three parts of one of two operand tiles; once per tile,
+//               behind its first item, the parts of the X operand into TMEM
 //   warps 8-15  E group: TMEM -> growth bell, E = exp(G*I); warps 16-19 V group: TMEM -> V.  Each warp has its own staging
 //               tiles (its 32 cells x 16 dims) and its own TMA stores: no barrier among them
 //   warps 20,21 TMA producers of the weight chunks, parts lo, mid, hi of Wi | Wv and of Wp
 //   warps 22,23 UMMA issuers, one for I | V (N = 128, the X operand in TMEM: with both operands in shared memory the
 //               products, the stencil's loads and the stores of this kernel contend for its 128 bytes per cycle), one for U
 //               (N = 64).  One issuer for both was the longest chain of the kernel.
+//   warp 24     loads the tile's state halo, a bulk copy per row (two where the row wraps): with loads by the stencil group
+//               a change of tile cost 14 000 cycles, two to three items
 __global__ void __launch_bounds__(k1f::THREADS, 1)
 k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_es,
        const __grid_constant__ CUtensorMap map_vs, const float* __restrict__ X, const float* __restrict__ scale,
@@ -98,14 +99,21 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
     uint64_t* ac_empty = bars + 10;                // [2] ... and consumed                        (waits: stencil group)
     uint64_t* ax_full = bars + 12;                 // X operand of a tile written                 (waits: issuer of I|V)
     uint64_t* ax_empty = bars + 13;                // ... and consumed by the tile's last item    (waits: stencil group)
+    uint64_t* xh_full = bars + 18;                 // state halo of a tile landed                 (waits: stencil group)
+    uint64_t* xh_empty = bars + 19;                // ... and was used by its last item           (waits: halo loader)
     uint64_t* tm_full = bars + 14;                 // [2] accumulator buffer holds an item (both issuers arrive) (waits: E and V groups)
     uint64_t* tm_empty = bars + 16;                // [2] ... and was drained (384 arrivals)      (waits: both issuers)
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k1f::TMEM_PTR);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        for (int i = 0; i < 14; ++i) ptx::mbar_init(&bars[i], 1);
-        for (int i = 0; i < 2; ++i) { ptx::mbar_init(&tm_full[i], 2); ptx::mbar_init(&tm_empty[i], 384); }
+        for (int i = 0; i < 8; ++i) ptx::mbar_init(&bars[i], 1);
+        for (int i = 0; i < 2; ++i) {
+            ptx::mbar_init(&ac_full[i], 256); ptx::mbar_init(&ac_empty[i], 1);
+            ptx::mbar_init(&tm_full[i], 2); ptx::mbar_init(&tm_empty[i], 384);
+        }
+        ptx::mbar_init(ax_full, 256); ptx::mbar_init(ax_empty, 1);
+        ptx::mbar_init(xh_full, 1); ptx::mbar_init(xh_empty, 256);
         ptx::fence_barrier_init();
         ptx::prefetch_tmap(&map_w1); ptx::prefetch_tmap(&map_es); ptx::prefetch_tmap(&map_vs);
     }
@@ -190,72 +198,51 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
             ptx::umma_commit_by(leader, &ac_empty[tb]);
             ptx::umma_commit_by(leader, &tm_full[tb]);
         }
+    } else if (warp == 24) {
+        // ================= halo loader: lane r brings row r of the halo ==============================================
+        uint32_t tiles = 0;
+        for (int k = i0 >> 3; i0 < i1 && k <= (i1 - 1) >> 3; ++k, ++tiles) {
+            const CaTile t = ca_tile(k, tiles_per_grid, g.tiles_x, -g.he);
+            ptx::mbar_wait(xh_empty, (tiles & 1) ^ 1, status, 330);
+            if (lane == 0) ptx::mbar_expect_tx(xh_full, k1f::XH_BYTES);
+            __syncwarp();
+            if (lane < TBH + 2) {
+                const float* row = X + (size_t)t.b * xplane + (size_t)g.xrow_near(t.ty0 + lane - 1) * g.W * NC;
+                uint8_t* dst = sm + k1f::XH + lane * (TBW + 2) * 256;
+                int x = g.wrap_x_near(t.tx0 - 1);
+                for (int left = TBW + 2; left > 0; x = 0) {
+                    const int n = min(left, g.W - x);
+                    ptx::bulk_load(dst, row + (size_t)x * NC, n * 256, xh_full);
+                    dst += n * 256;
+                    left -= n;
+                }
+            }
+        }
     } else if (warp < 8) {
         // ================= stencil group ======================================================================
-        uint8_t* xh = sm + k1f::XH;
-        float* prm_s = reinterpret_cast<float*>(sm + k1f::PRM_ST);
+        const uint8_t* xh = sm + k1f::XH;
         const int c4 = tid & 15, p2 = (tid >> 4) & 7, y0 = (tid >> 7) * 4;
         uint32_t n = 0, tiles = 0;
+        CaTile t;
+        ptx::f2 sc[2];
         for (int i = i0; i < i1; ++i, ++n) {
             const int h = i & 7, tb = n & 1;
-            if (h == 0 || i == i0) {
-                const CaTile t = ca_tile(i >> 3, tiles_per_grid, g.tiles_x, -g.he);
-                const int set = t.b / g.per_set;
-                ptx::bar_sync(1, 256);                                    // everybody is done with the last halo
-                if (tid < NH * PRM) prm_s[tid] = __ldg(prm + (size_t)set * NH * PRM + tid);
-                // 180 cells x 16 chunks of 4 channels over 256 threads, every load issued before the first is used
-                const float* Xb = X + (size_t)t.b * xplane + c4 * 4;
+            const bool first = h == 0 || i == i0;
+            if (first) {
+                t = ca_tile(i >> 3, tiles_per_grid, g.tiles_x, -g.he);
                 const float4 s4 = __ldg(reinterpret_cast<const float4*>(scale + t.b * NC + c4 * 4));
-                float4 raw[12];
-#pragma unroll
-                for (int j = 0; j < 12; ++j) {
-                    const int cell = (tid >> 4) + j * 16, hy = cell / 18;
-                    if (cell < 180)
-                        raw[j] = *reinterpret_cast<const float4*>(Xb + ((size_t)g.xrow_near(t.ty0 + hy - 1) * g.W + g.wrap_x_near(t.tx0 + cell - hy * 18 - 1)) * NC);
-                }
-#pragma unroll
-                for (int j = 0; j < 12; ++j) {
-                    const int cell = (tid >> 4) + j * 16;
-                    if (cell < 180)
-                        *reinterpret_cast<float4*>(xh + cell * 256 + c4 * 16) =
-                            make_float4(raw[j].x * s4.x, raw[j].y * s4.y, raw[j].z * s4.z, raw[j].w * s4.w);
-                }
-                if ((i >> 3) + 1 <= (i1 - 1) >> 3) {                      // next tile's halo: two 128-byte lines a cell, into L2
-                    const CaTile tn = ca_tile((i >> 3) + 1, tiles_per_grid, g.tiles_x, -g.he);
-                    for (int j = tid; j < 360; j += 256) {
-                        const int cell = j >> 1, hy = cell / 18;
-                        ptx::prefetch_l2(X + (size_t)tn.b * xplane + (j & 1) * 32 +
-                                         ((size_t)g.xrow_near(tn.ty0 + hy - 1) * g.W + g.wrap_x_near(tn.tx0 + cell - hy * 18 - 1)) * NC);
-                    }
-                }
-                ptx::mbar_wait(ax_empty, (tiles & 1) ^ 1, status, 330);
-                ptx::bar_sync(1, 256);
-                // X operand: this thread's cell is TMEM lane m, half of its channels
-                {
-                    const int m = (warp & 3) * 32 + lane, half = warp >> 2;
-                    const uint8_t* src = xh + ((m >> 4) * 18 + 19 + (m & 15)) * 256 + half * 128;
-                    const uint32_t dst = tmem + ((uint32_t)((warp & 3) * 32) << 16) + k1f::AX + half * 16;
-                    uint32_t a[3][16];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const float4 v = *reinterpret_cast<const float4*>(src + q * 16);
-                        split3(ptx::make_f2(v.x, v.y), a[0][2 * q], a[1][2 * q], a[2][2 * q]);
-                        split3(ptx::make_f2(v.z, v.w), a[0][2 * q + 1], a[1][2 * q + 1], a[2][2 * q + 1]);
-                    }
-#pragma unroll
-                    for (int pa = 0; pa < 3; ++pa) ptx::tmem_st16(dst + pa * 32, a[pa]);
-                    ptx::tmem_st_wait();
-                    ptx::tc_fence_before();
-                }
-                ++tiles;
-                ptx::bar_sync(1, 256);
-                if (tid == 0) { ptx::tc_fence_after(); ptx::tc_fence_before(); ptx::mbar_arrive(ax_full); }
+                sc[0] = ptx::make_f2(s4.x, s4.y);
+                sc[1] = ptx::make_f2(s4.z, s4.w);
+                ptx::mbar_wait(xh_full, tiles & 1, status, 332);
             }
             // two adjacent columns x 4 channels x 4 rows per thread; input row j feeds output rows j (tap row 0), j-1 (tap
             // row 1) and j-2 (tap row 2)
             ptx::f2 kt[9], s1[2][2], s2[2][2];
 #pragma unroll
-            for (int tt = 0; tt < 9; ++tt) { const float kv = prm_s[h * PRM + tt]; kt[tt] = ptx::make_f2(kv, kv); }
+            for (int tt = 0; tt < 9; ++tt) {
+                const float kv = __ldg(prm + ((size_t)(t.b / g.per_set) * NH + h) * PRM + tt);
+                kt[tt] = ptx::make_f2(kv, kv);
+            }
             ptx::mbar_wait(&ac_empty[tb], ((n >> 1) & 1) ^ 1, status, 331);
             uint8_t* a_conv = sm + k1f::A_CONV + tb * k1f::A_BYTES + (c4 & 1) * 8;
 #pragma unroll
@@ -277,8 +264,8 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
 #pragma unroll
                         for (int e = 0; e < 2; ++e)
                             o[e] = ptx::fma2(kt[6], c[col][e], ptx::fma2(kt[7], c[col + 1][e], ptx::fma2(kt[8], c[col + 2][e], s2[col][e])));
-                        split3(o[0], a[0], a[1], a[2]);
-                        split3(o[1], b[0], b[1], b[2]);
+                        split3(ptx::mul2(o[0], sc[0]), a[0], a[1], a[2]);
+                        split3(ptx::mul2(o[1], sc[1]), b[0], b[1], b[2]);
                         uint8_t* dst = a_conv + swz((y0 + j - 2) * TBW + 2 * p2 + col, c4 >> 1);
 #pragma unroll
                         for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dst + p * k1f::PART) = make_uint2(a[p], b[p]);
@@ -292,8 +279,30 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                 }
             }
             ptx::fence_proxy_async();
-            ptx::bar_sync(2, 256);
-            if (tid == 0) ptx::mbar_arrive(&ac_full[tb]);
+            ptx::mbar_arrive(&ac_full[tb]);
+            if (first) {
+                // X operand: this thread's cell is TMEM lane m, half of its channels
+                const int m = (warp & 3) * 32 + lane, half = warp >> 2;
+                const uint8_t* src = xh + ((m >> 4) * 18 + 19 + (m & 15)) * 256 + half * 128;
+                const float4* ss = reinterpret_cast<const float4*>(scale + t.b * NC + half * 32);
+                const uint32_t dst = tmem + ((uint32_t)((warp & 3) * 32) << 16) + k1f::AX + half * 16;
+                ptx::mbar_wait(ax_empty, (tiles & 1) ^ 1, status, 333);
+                ptx::tc_fence_after();
+                uint32_t a[3][16];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float4 v = *reinterpret_cast<const float4*>(src + q * 16), s4 = __ldg(ss + q);
+                    split3(ptx::mul2(ptx::make_f2(v.x, v.y), ptx::make_f2(s4.x, s4.y)), a[0][2 * q], a[1][2 * q], a[2][2 * q]);
+                    split3(ptx::mul2(ptx::make_f2(v.z, v.w), ptx::make_f2(s4.z, s4.w)), a[0][2 * q + 1], a[1][2 * q + 1], a[2][2 * q + 1]);
+                }
+#pragma unroll
+                for (int pa = 0; pa < 3; ++pa) ptx::tmem_st16(dst + pa * 32, a[pa]);
+                ptx::tmem_st_wait();
+                ptx::tc_fence_before();
+                ptx::mbar_arrive(ax_full);
+                ++tiles;
+            }
+            if (h == NH - 1 || i == i1 - 1) ptx::mbar_arrive(xh_empty);
         }
     } else {
         // ================= E group (warps 8..15: a quarter of the cells, half of the dims) and V group (16..19: a quarter
@@ -426,7 +435,7 @@ constexpr int A_VP = STG + NSTAGE * STAGE_BYTES;        // two operand tiles of 
 constexpr int WO_PART = 4096, WO = A_VP + 2 * 3 * PART; // two Wo slices of 3 parts [64][32]
 constexpr int XT = WO + 2 * 3 * WO_PART;                // state tile of the epilogue: two halves of 32 channels, 16 KB each
 constexpr int RED = XT + 2 * 16384;                     // [4 quads][64] fp64
-constexpr int BARS = RED + 4 * 64 * 8;
+constexpr int FLAG = RED + 4 * 64 * 8, BARS = FLAG + 8;
 constexpr int N_BARS = 2 * NSTAGE + 12;
 constexpr int TMEM_PTR = BARS + N_BARS * 8;
 constexpr int BYTES = TMEM_PTR + 16;
@@ -458,7 +467,7 @@ __device__ __forceinline__ float4 v4_f4(const V4& x) { float4 f; ptx::split_f2(x
 __global__ void __launch_bounds__(k2f::THREADS, 1)
 k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUtensorMap map_e,
        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ scale,
-       float* __restrict__ partial, size_t lo_offset, float* __restrict__ vprime, int* __restrict__ status, int n_mt,
+       const K2Sums fin, float* __restrict__ vprime, int* __restrict__ status, int n_mt,
        int mt_per_grid, int strips, int tiles_per_grid, int nbmax, Geom g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
@@ -646,8 +655,8 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                             const double t = (red[pt] + red[64 + pt]) + (red[128 + pt] + red[192 + pt]);
                             const size_t o = (size_t)(m.b * tiles_per_grid + m.tile0 + b * strips) * NC + pt;
                             const float hi = (float)t;
-                            partial[o] = hi;
-                            partial[o + lo_offset] = (float)(t - (double)hi);
+                            fin.partial[o] = hi;
+                            fin.partial[o + fin.lo_offset] = (float)(t - (double)hi);
                         }
                         if (pt == 0) {
                             ptx::tma_store_4d(&map_x, xt, 0, m.mx0, g.hx + ty0, m.b);
@@ -658,6 +667,9 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                         }
                         ptx::bar_sync(7, 128);         // the reduction scratch is free again
                         ++nx;
+                        if (b == m.nb - 1)
+                            k2_finish<128>(fin, m.b, tiles_per_grid, mt_per_grid, red, reinterpret_cast<int*>(sm + k2f::FLAG), pt,
+                                           [] { ptx::bar_sync(7, 128); });
                     }
                 }
             }

@@ -41,7 +41,9 @@ struct slime_ca {
     int partial_cap = 0;
     size_t partial_lo = 0;          // fp32 path: offset (floats) of the remainders of the step's tile sums
     double* seg_sums = nullptr;
-    int* tickets = nullptr;          // one per grid: blocks of the reduction that have finished (back at 0 after each launch)
+    int* tickets = nullptr;          // one per grid: parts of the step's reduction that have finished (back at 0 after each)
+    int* load_tickets = nullptr;     // the same for the sums of a state being loaded
+    int n_sms = 1;
     int k1_tiles = 0, k2_tiles = 0, tiles_x = 0;
     // weights
     float* prm = nullptr;           // [sets][8][PRM]
@@ -78,6 +80,8 @@ struct slime_ca {
 };
 
 namespace {
+
+constexpr int MAX_SEGMENTS = 1024;      // of the reduction kernel, per grid
 
 int fail(slime_ca* h, int code, const std::string& msg) {
     if (h) h->err = msg;
@@ -119,21 +123,48 @@ int grid_for(size_t n) {
 
 bool is_bf16(const slime_ca* h) { return h->cfg.dtype == SLIME_CA_BF16; }
 
-// sums <- per-channel sums of the stored state's own rows; mode as in k_finish_sums
-int channel_sums(slime_ca* h, int mode, cudaStream_t st) {
-    const size_t cells = (size_t)h->g.H * h->g.W;
-    const int chunks = (int)((cells + 255) / 256);
-    dim3 grid(chunks, h->g.B);
-    // a fresh state also starts the reduction's tickets afresh (they are only non-zero if a launch before was cut short)
-    CK(h, cudaMemsetAsync(h->tickets, 0, (size_t)h->g.B * sizeof(int), st));
-    if (is_bf16(h)) k_channel_partials<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->partial, h->g);
-    else k_channel_partials<float><<<grid, 256, 0, st>>>((const float*)h->X, h->partial, h->g);
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Blocks per grid of the reduction kernel: enough to fill the GPU over all grids, eight partials or more each.
+int reduce_segments(const slime_ca* h, int n_partials) {
+    int n = (h->n_sms * 4 + h->g.B - 1) / h->g.B;
+    if (n > (n_partials + 7) / 8) n = (n_partials + 7) / 8;
+    return n < 1 ? 1 : n > MAX_SEGMENTS ? MAX_SEGMENTS : n;
+}
+
+// Runs launch(grid, ChunkSums), a kernel over 256-cell chunks of every grid that leaves chunk sums, and sees to the
+// grids' sums (mode as in SumsOut).
+template <typename Launch>
+int with_channel_sums(slime_ca* h, int mode, cudaStream_t st, Launch launch) {
+    const Geom& g = h->g;
+    const int chunks = (int)(((size_t)g.H * g.W + 255) / 256);
+    const bool fuse = chunks <= FUSE_PARTIALS;
+    const SumsOut out{h->sums, h->mass, h->scale, mode};
+    launch(dim3(chunks, g.B), ChunkSums{h->partial, fuse ? h->load_tickets : nullptr, mode == 1 ? h->tickets : nullptr, out});
     LAUNCHED(h);
-    const int nseg = chunks < 64 ? chunks : 64;
-    k_reduce_finish<<<dim3(nseg, h->g.B), 256, 0, st>>>(h->partial, chunks, h->seg_sums, 0, h->tickets, h->sums, h->mass,
-                                                        h->scale, mode);
-    LAUNCHED(h);
+    if (!fuse) {
+        // a fresh state also starts the reduction's tickets afresh (they are only non-zero if a launch before was cut short)
+        CK(h, cudaMemsetAsync(h->tickets, 0, (size_t)g.B * sizeof(int), st));
+        k_reduce_finish<<<dim3(reduce_segments(h, chunks), g.B), 256, 0, st>>>(h->partial, chunks, h->seg_sums, 0, h->tickets, out);
+        LAUNCHED(h);
+    }
     return SLIME_CA_OK;
+}
+
+// sums <- per-channel sums of the stored state's own rows
+int channel_sums(slime_ca* h, int mode, cudaStream_t st) {
+    return with_channel_sums(h, mode, st, [&](dim3 grid, const ChunkSums& cs) {
+        if (is_bf16(h)) k_channel_partials<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)h->X, true, cs, h->g);
+        else k_channel_partials<float><<<grid, 256, 0, st>>>((const float*)h->X, true, cs, h->g);
+    });
+}
+
+// X <- lifted images (device pointers), with the masses of the lifted state
+int lift(slime_ca* h, const float* img, int ih, int iw, const float* L, cudaStream_t st) {
+    return with_channel_sums(h, 1, st, [&](dim3 grid, const ChunkSums& cs) {
+        if (is_bf16(h)) k_lift<__nv_bfloat16><<<grid, 256, 0, st>>>(img, ih, iw, L, (__nv_bfloat16*)h->X, cs, h->g);
+        else k_lift<float><<<grid, 256, 0, st>>>(img, ih, iw, L, (float*)h->X, cs, h->g);
+    });
 }
 
 // the kernels of one step up to and including BUF_SUMS; `emit` = V' destination or null
@@ -141,6 +172,8 @@ int channel_sums(slime_ca* h, int mode, cudaStream_t st) {
 // scale from the local sums (a caller that all-reduces the sums first passes 0 and sets the scale afterwards)
 int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nullptr, int sums_mode = 0) {
     const Geom& g = h->g;
+    const SumsOut out{h->sums, h->mass, h->scale, sums_mode};
+    const K2Sums fin{h->partial, is_bf16(h) ? 0 : h->partial_lo, h->k2_tiles > FUSE_PARTIALS ? nullptr : h->tickets, out};
     if (ev) CK(h, cudaEventRecord(ev[0], st));
     if (is_bf16(h)) {
         if (bf16_k1(h->bf, (const __nv_bfloat16*)h->X, h->scale, h->prm, (__nv_bfloat16*)h->E, (__nv_bfloat16*)h->V,
@@ -149,7 +182,7 @@ int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nul
         ++h->launches;
         if (ev) CK(h, cudaEventRecord(ev[1], st));
         if (bf16_k2(h->bf, (__nv_bfloat16*)h->X, h->scale, (const __nv_bfloat16*)h->E, (const __nv_bfloat16*)h->V,
-                    h->partial, (__nv_bfloat16*)emit, h->dev_status, g, st) != 0)
+                    fin, (__nv_bfloat16*)emit, h->dev_status, g, st) != 0)
             return fail(h, SLIME_CA_ECUDA, std::string("bf16 k2 launch: ") + cudaGetErrorString(cudaGetLastError()));
         ++h->launches;
     } else {
@@ -159,16 +192,17 @@ int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nul
                                                            p.k1_tiles, g);
         LAUNCHED(h);
         if (ev) CK(h, cudaEventRecord(ev[1], st));
-        k2_f32<<<p.k2_grid, k2f::THREADS, k2f::SMEM, st>>>(p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, h->partial, h->partial_lo,
-                                                           (float*)emit, h->dev_status, p.mt_per_grid * g.B, p.mt_per_grid,
+        k2_f32<<<p.k2_grid, k2f::THREADS, k2f::SMEM, st>>>(p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, fin, (float*)emit,
+                                                           h->dev_status, p.mt_per_grid * g.B, p.mt_per_grid,
                                                            p.strips, p.k2_tiles, p.nbmax, g);
         LAUNCHED(h);
     }
     if (ev) CK(h, cudaEventRecord(ev[2], st));
-    const int nseg = h->k2_tiles < 64 ? h->k2_tiles : 64;
-    k_reduce_finish<<<dim3(nseg, g.B), 256, 0, st>>>(h->partial, h->k2_tiles, h->seg_sums, is_bf16(h) ? 0 : h->partial_lo,
-                                                     h->tickets, h->sums, h->mass, h->scale, sums_mode);
-    LAUNCHED(h);
+    if (h->k2_tiles > FUSE_PARTIALS) {        // else k2 has done it
+        k_reduce_finish<<<dim3(reduce_segments(h, h->k2_tiles), g.B), 256, 0, st>>>(h->partial, h->k2_tiles, h->seg_sums,
+                                                                                    is_bf16(h) ? 0 : h->partial_lo, h->tickets, out);
+        LAUNCHED(h);
+    }
     return SLIME_CA_OK;
 }
 
@@ -352,9 +386,11 @@ int slime_ca_create(const slime_ca_config* cfg, slime_ca** out) {
     if ((rc = dev_alloc(h, &h->sums, (size_t)g.B * NC))) return rc;
     h->partial_lo = is_bf16(h) ? 0 : (size_t)g.B * h->partial_cap * NC;
     if ((rc = dev_alloc(h, &h->partial, (size_t)g.B * h->partial_cap * NC + h->partial_lo))) return rc;
-    if ((rc = dev_alloc(h, &h->seg_sums, (size_t)g.B * 64 * NC))) return rc;
-    if ((rc = dev_alloc(h, &h->tickets, (size_t)g.B))) return rc;
-    CK(h, cudaMemset(h->tickets, 0, (size_t)g.B * sizeof(int)));
+    h->n_sms = prop.multiProcessorCount;
+    if ((rc = dev_alloc(h, &h->seg_sums, (size_t)g.B * reduce_segments(h, h->partial_cap) * NC))) return rc;
+    if ((rc = dev_alloc(h, &h->tickets, (size_t)g.B * 2))) return rc;
+    h->load_tickets = h->tickets + g.B;
+    CK(h, cudaMemset(h->tickets, 0, (size_t)g.B * 2 * sizeof(int)));
     if ((rc = dev_alloc(h, &h->dev_status, 1))) return rc;
     CK(h, cudaMemset(h->dev_status, 0, sizeof(int)));
     CK(h, cudaHostAlloc((void**)&h->host_status, sizeof(int), cudaHostAllocDefault));
@@ -434,18 +470,18 @@ int slime_ca_set_state_device(slime_ca* h, const void* dev_state, int dtype, voi
         const int bad = *reinterpret_cast<volatile int*>(h->host_status);   // a fresh state ends an earlier failure
         if (bad) { *reinterpret_cast<volatile int*>(h->host_status) = 0; cudaMemsetAsync(h->dev_status, 0, sizeof(int), st); }
     }
-    const Geom& g = h->g;
-    const size_t n = (size_t)g.B * g.H * g.W * NC;
-    const int blocks = grid_for(n);
-    if (is_bf16(h)) {
-        if (dtype == SLIME_CA_BF16) k_state_in<__nv_bfloat16, __nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)dev_state, (__nv_bfloat16*)h->X, g);
-        else k_state_in<float, __nv_bfloat16><<<blocks, 256, 0, st>>>((const float*)dev_state, (__nv_bfloat16*)h->X, g);
-    } else {
-        if (dtype == SLIME_CA_BF16) k_state_in<__nv_bfloat16, float><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)dev_state, (float*)h->X, g);
-        else k_state_in<float, float><<<blocks, 256, 0, st>>>((const float*)dev_state, (float*)h->X, g);
-    }
-    LAUNCHED(h);
-    int rc = channel_sums(h, 1, st);
+    const bool vec = aligned16(dev_state);
+    int rc = with_channel_sums(h, 1, st, [&](dim3 grid, const ChunkSums& cs) {
+        const __nv_bfloat16* s16 = (const __nv_bfloat16*)dev_state;
+        const float* s32 = (const float*)dev_state;
+        if (is_bf16(h)) {
+            if (dtype == SLIME_CA_BF16) k_state_in<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, st>>>(s16, vec, (__nv_bfloat16*)h->X, cs, h->g);
+            else k_state_in<float, __nv_bfloat16><<<grid, 256, 0, st>>>(s32, vec, (__nv_bfloat16*)h->X, cs, h->g);
+        } else {
+            if (dtype == SLIME_CA_BF16) k_state_in<__nv_bfloat16, float><<<grid, 256, 0, st>>>(s16, vec, (float*)h->X, cs, h->g);
+            else k_state_in<float, float><<<grid, 256, 0, st>>>(s32, vec, (float*)h->X, cs, h->g);
+        }
+    });
     if (rc) return rc;
     h->state_set = true;
     h->vp_steps = 0; h->fitness_valid = false;
@@ -461,13 +497,17 @@ int slime_ca_get_state_device(slime_ca* h, void* dev_state, int dtype, void* str
     int rcs = poll_status(h, st);
     if (rcs) return rcs;
     const Geom& g = h->g;
-    const int blocks = grid_for((size_t)g.B * g.H * g.W * NC);
+    const bool vec = aligned16(dev_state);
+    size_t per_grid = ((size_t)g.H * g.W * 8 + 255) / 256, most = (size_t)(h->n_sms * 16 + g.B - 1) / g.B;
+    const dim3 grid((unsigned)(per_grid < most ? per_grid : most), g.B);
+    __nv_bfloat16* d16 = (__nv_bfloat16*)dev_state;
+    float* d32 = (float*)dev_state;
     if (is_bf16(h)) {
-        if (dtype == SLIME_CA_BF16) k_state_out<__nv_bfloat16, __nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, (__nv_bfloat16*)dev_state, g);
-        else k_state_out<__nv_bfloat16, float><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, (float*)dev_state, g);
+        if (dtype == SLIME_CA_BF16) k_state_out<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, d16, vec, g);
+        else k_state_out<__nv_bfloat16, float><<<grid, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, d32, vec, g);
     } else {
-        if (dtype == SLIME_CA_BF16) k_state_out<float, __nv_bfloat16><<<blocks, 256, 0, st>>>((const float*)h->X, h->scale, (__nv_bfloat16*)dev_state, g);
-        else k_state_out<float, float><<<blocks, 256, 0, st>>>((const float*)h->X, h->scale, (float*)dev_state, g);
+        if (dtype == SLIME_CA_BF16) k_state_out<float, __nv_bfloat16><<<grid, 256, 0, st>>>((const float*)h->X, h->scale, d16, vec, g);
+        else k_state_out<float, float><<<grid, 256, 0, st>>>((const float*)h->X, h->scale, d32, vec, g);
     }
     LAUNCHED(h);
     return SLIME_CA_OK;
@@ -702,11 +742,7 @@ int slime_ca_lift_images(slime_ca* h, const float* host_img, int img_h, int img_
     float* d_L = (float*)h->V;
     CK(h, cudaMemcpyAsync(d_img, host_img, n_img * sizeof(float), cudaMemcpyHostToDevice, st));
     CK(h, cudaMemcpyAsync(d_L, host_L, NC * sizeof(float), cudaMemcpyHostToDevice, st));
-    const int blocks = grid_for((size_t)g.B * g.H * g.W * NC);
-    if (is_bf16(h)) k_lift<__nv_bfloat16><<<blocks, 256, 0, st>>>(d_img, img_h, img_w, d_L, (__nv_bfloat16*)h->X, g);
-    else k_lift<float><<<blocks, 256, 0, st>>>(d_img, img_h, img_w, d_L, (float*)h->X, g);
-    LAUNCHED(h);
-    int rc = channel_sums(h, 1, st);
+    int rc = lift(h, d_img, img_h, img_w, d_L, st);
     if (rc) return rc;
     CK(h, cudaStreamSynchronize(st));
     h->state_set = true;
@@ -750,14 +786,9 @@ int slime_ca_lift_field_device(slime_ca* h, const float* dev_field, const float*
     if (!dev_field || !host_L) return fail(h, SLIME_CA_EINVAL, "null field or lift vector");
     CK(h, cudaSetDevice(h->cfg.device));
     cudaStream_t st = (cudaStream_t)stream;
-    const Geom& g = h->g;
     float* d_L = (float*)h->V;
     CK(h, cudaMemcpyAsync(d_L, host_L, NC * sizeof(float), cudaMemcpyHostToDevice, st));
-    const int blocks = grid_for((size_t)g.B * g.H * g.W * NC);
-    if (is_bf16(h)) k_lift<__nv_bfloat16><<<blocks, 256, 0, st>>>(dev_field, g.H, g.W, d_L, (__nv_bfloat16*)h->X, g);
-    else k_lift<float><<<blocks, 256, 0, st>>>(dev_field, g.H, g.W, d_L, (float*)h->X, g);
-    LAUNCHED(h);
-    int rc = channel_sums(h, 1, st);
+    int rc = lift(h, dev_field, h->g.H, h->g.W, d_L, st);
     if (rc) return rc;
     CK(h, cudaStreamSynchronize(st));
     h->state_set = true;
@@ -1226,8 +1257,10 @@ int slime_ca_channel_sums_static(const void* dev_state, int dtype, int batch, in
     Geom g{};
     g.B = batch; g.H = cells_per_grid; g.W = 1; g.hx = 0; g.he = 0; g.wrap_y = 1; g.per_set = 1;
     const dim3 grid((unsigned)chunks, (unsigned)batch);
-    if (dtype == SLIME_CA_BF16) k_channel_partials<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dev_state, partial, g);
-    else k_channel_partials<float><<<grid, 256, 0, st>>>((const float*)dev_state, partial, g);
+    const bool vec = aligned16(dev_state);
+    const ChunkSums cs{partial, nullptr, nullptr, SumsOut{nullptr, nullptr, nullptr, 0}};
+    if (dtype == SLIME_CA_BF16) k_channel_partials<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dev_state, vec, cs, g);
+    else k_channel_partials<float><<<grid, 256, 0, st>>>((const float*)dev_state, vec, cs, g);
     e = cudaGetLastError();
     if (e != cudaSuccess) return static_fail(SLIME_CA_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     // one segment per grid: the fp64 second stage writes [batch][64] straight into the caller's buffer
