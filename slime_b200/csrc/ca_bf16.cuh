@@ -41,7 +41,7 @@ struct K1StoreMaps {
 };
 
 // Where k2 leaves the tiles' channel sums, and how they become the grids' sums: with tickets, whoever finishes a grid's
-// last macro tile adds them up.
+// last macro tile adds them up.  lo_offset != 0: every tile sum is a float pair, the remainder that many floats behind.
 struct K2Sums {
     float* partial;
     size_t lo_offset;
@@ -49,18 +49,61 @@ struct K2Sums {
     SumsOut out;
 };
 
-// A set of NT threads (bar: its barrier) has written its share of a macro tile's tile sums; `parts` shares make up grid
-// b's n tiles.  The set that comes last sums them.
-template <int NT, typename Bar>
-__device__ __forceinline__ void k2_finish(const K2Sums& k, int b, int n, int parts, double* red, int* flag, int tid, Bar bar) {
+// Channel sums of a grid's n tiles: sixteen interleaved partial sums, each in order, then those in order.  Whoever adds
+// them up, the result is the same.
+__device__ __forceinline__ double tile_sums(const float* part, size_t lo_offset, int n, int sub) {
+    double s = 0.0;
+    for (int t = sub; t < n; t += 128) {
+        float v[8], w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const bool in = t + 16 * i < n;
+            const float* p = part + (size_t)(t + 16 * i) * NC;
+            v[i] = in ? __ldcg(p) : 0.f;
+            w[i] = in && lo_offset ? __ldcg(p + lo_offset) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s += (double)v[i] + (double)w[i];
+    }
+    return s;
+}
+// A macro tile's tile sums have all been written (the caller has seen the writers' barrier); `parts` macro tiles make up
+// grid b's n tiles, and who comes last adds the tile sums.  By one warp, while the others go on with the next macro tile
+// (by the warps that drain the tiles the fence and the ticket cost 2 us per macro tile, 17 of 722 us a launch) ...
+__device__ __forceinline__ void k2_finish(const K2Sums& k, int b, int n, int parts) {
     if (k.tickets == nullptr) return;
-    if (tid < NC) __threadfence();
-    bar();
-    if (tid == 0) *flag = atomicAdd(&k.tickets[b], 1) == parts - 1;
-    bar();
+    const int lane = threadIdx.x & 31;
+    int last = 0;
+    __threadfence();
+    if (lane == 0) last = atomicAdd(&k.tickets[b], 1) == parts - 1;
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+#pragma unroll 1
+    for (int c = lane; c < NC; c += 32) {
+        double s = 0.0;
+#pragma unroll 1
+        for (int sub = 0; sub < 16; ++sub) s += tile_sums(k.partial + (size_t)b * n * NC + c, k.lo_offset, n, sub);
+        sums_out(k.out, b, c, s);
+    }
+    if (lane == 0) k.tickets[b] = 0;
+}
+// ... and by the whole CTA for its last macro tile, at whose end everybody waits (5 us less than by one warp at n = 128).
+// red: [16][64] doubles of shared memory, flag: an int of it.
+__device__ __forceinline__ void k2_finish_cta(const K2Sums& k, int b, int n, int parts, double* red, int* flag) {
+    if (k.tickets == nullptr) return;
+    const int tid = threadIdx.x, c = tid & 63;
+    if (tid == 0) { __threadfence(); *flag = atomicAdd(&k.tickets[b], 1) == parts - 1; }
+    __syncthreads();
     if (!*flag) return;
     __threadfence();
-    sum_partials<NT>(k.partial + (size_t)b * n * NC, n, k.lo_offset, red, tid, bar, k.out, b);
+    for (int sub = tid >> 6; sub < 16; sub += blockDim.x >> 6) red[sub * NC + c] = tile_sums(k.partial + (size_t)b * n * NC + c, k.lo_offset, n, sub);
+    __syncthreads();
+    if (tid < NC) {
+        double s = 0.0;
+#pragma unroll
+        for (int sub = 0; sub < 16; ++sub) s += red[sub * NC + c];
+        sums_out(k.out, b, c, s);
+    }
     if (tid == 0) k.tickets[b] = 0;
 }
 
@@ -111,6 +154,8 @@ __device__ __forceinline__ uint4 pack8p(const ptx::f2 (&f)[4]) {
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
     return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
+// the same for 64-byte rows and the 64-byte swizzle
+__device__ __forceinline__ uint32_t swz64(int m, int q) { return (uint32_t)(m * 64 + ((q ^ ((m >> 1) & 3)) << 4)); }
 __device__ __forceinline__ uint32_t swz(int m, int q) { return (uint32_t)(m * 128 + ((q ^ (m & 7)) << 4)); }
 
 // =============================================================================================================
@@ -128,7 +173,82 @@ __device__ __forceinline__ CaTile ca_tile(int t, int tiles_per_grid, int tiles_x
     return r;
 }
 
-// k1: persistent, warp-specialised, one CTA per SM (608 threads):
+// The (tile, head) items of one k1 CTA: as many whole tiles as every CTA gets, handed out in turn, so that the CTAs work
+// on neighbouring tiles at any time (a contiguous stretch each spreads the stores of E and V over 148 places: 12 % slower
+// on a 2048 x 2048 torus), and of the tiles that are left, which do not go round, a share of the items that differs by one
+// at most (as whole tiles they left a 32 x 32 grid on 8 of the SMs, and cost a 128 x 128 one 8 items where 7 do).
+struct K1Items {
+    int whole, base, r0, count;      // items of whole tiles; first of the tiles left over; first item of this CTA there
+    __device__ K1Items(int n_tiles) {
+        const int rounds = n_tiles / (int)gridDim.x, left = n_tiles - rounds * (int)gridDim.x;
+        whole = rounds * NH;
+        base = rounds * (int)gridDim.x;
+        r0 = (int)((long long)left * NH * blockIdx.x / gridDim.x);
+        count = whole + (int)((long long)left * NH * (blockIdx.x + 1) / gridDim.x) - r0;
+    }
+    __device__ int head(int n) const { return (n < whole ? n : r0 + n - whole) & 7; }
+    __device__ int tile(int n) const { return n < whole ? (int)blockIdx.x + (n >> 3) * (int)gridDim.x : base + ((r0 + n - whole) >> 3); }
+    __device__ bool first(int n) const { return n == whole || head(n) == 0; }                  // of its tile, for this CTA
+    __device__ bool last(int n) const { return n == count - 1 || head(n) == NH - 1; }
+    __device__ int end(int n) const { return min(n + NH - head(n), count); }                   // first item of the next tile, from a first item
+};
+
+// Apron copies of the cells of one epilogue warp of k1 (two rows of a tile, one cell per lane): the positions outside the
+// grid's own rows and columns that wrap onto them.  The TMA store of the warp's staging covers the cells and whatever
+// hangs over the far edge.  Copies at the high ends of the apron are the same staging stored once more at the shifted
+// position (all but the wanted part is clipped), and so is a pair of last rows at the low end; what is left - the last two
+// columns, which would have to start before the plane, and last rows that are not one warp's pair - the lanes store from
+// their registers.  Grids narrower or shorter than twice the apron can wrap more than once and take a general loop.
+struct ApronCopies {
+    bool tiny, wrap_x, lanes;         // general loop; staging again at x + W; any lane with a copy of its own
+    int dy;                           // staging again at y + dy (0: no)
+    int at_x, at_y, at_xy;            // this lane's own copies: cell offsets in the plane, -1 for none
+    __device__ void tile(const CaTile& t, int quad, int lane, const Geom& g) {
+        const int r0 = t.ty0 + quad * 2, r = r0 + (lane >> 4), x = t.tx0 + (lane & 15);
+        const bool valid = r < g.H + g.he && x < g.W, last_x = x >= g.W - APRON, last_y = g.wrap_y && r >= g.H - APRON;
+        tiny = g.W < 2 * APRON || (g.wrap_y && g.H < 2 * APRON);
+        wrap_x = t.tx0 == 0;
+        dy = !g.wrap_y ? 0 : r0 == 0 ? g.H : r0 == g.H - APRON ? -g.H : 0;
+        const int rd = dy ? dy : last_y ? -g.H : 0;           // where this lane's row goes, if anywhere
+        const bool own_y = rd != 0 && dy == 0;
+        const int here = (r + APRON) * g.ev_w + x + APRON, xd = last_x ? -g.W : x < APRON ? g.W : 0;
+        at_x = valid && last_x ? here - g.W : -1;
+        at_y = valid && own_y ? here + rd * g.ev_w : -1;
+        at_xy = valid && rd != 0 && xd != 0 && (last_x || own_y) ? here + rd * g.ev_w + xd : -1;
+        lanes = tiny || __any_sync(0xffffffffu, at_x >= 0 || at_y >= 0);
+    }
+    // copy(cell offset) for every copy of this lane's own
+    template <typename F> __device__ void own(const CaTile& t, int quad, int lane, const Geom& g, F copy) const {
+        if (!lanes) return;
+        if (!tiny) {
+            if (at_x >= 0) copy(at_x);
+            if (at_y >= 0) copy(at_y);
+            if (at_xy >= 0) copy(at_xy);
+            return;
+        }
+        const int r = t.ty0 + quad * 2 + (lane >> 4), x = t.tx0 + (lane & 15);
+        if (r >= g.H + g.he || x >= g.W) return;
+        for (int ky = g.wrap_y ? -2 * APRON : 0; ky <= (g.wrap_y ? 2 * APRON : 0); ++ky)
+            for (int kx = -2 * APRON; kx <= 2 * APRON; ++kx) {
+                const int rr = r + ky * g.H, xx = x + kx * g.W;
+                if ((ky == 0 && kx == 0) || rr < -APRON || rr >= g.H + APRON || xx < -APRON || xx >= g.W + APRON) continue;
+                copy((rr + APRON) * g.ev_w + xx + APRON);
+            }
+    }
+    // store(plane column, plane row) of the warp's staging: its place, and the copies
+    template <typename F> __device__ void staged(const CaTile& t, int quad, const Geom& g, F store) const {
+        const int px = t.tx0 + APRON, py = t.ty0 + quad * 2 + APRON;
+        store(px, py);
+        if (tiny) return;
+        if (wrap_x) store(px + g.W, py);
+        if (dy) {
+            store(px, py + dy);
+            if (wrap_x) store(px + g.W, py + dy);
+        }
+    }
+};
+
+// k1: persistent, warp-specialised, one CTA per SM (608 threads), over the items of K1Items:
 //   warps 0-7   stencil group: loads the tile's state halo (scale applied) and the X operand, then its two
 //               4-warp halves take alternate heads: 3x3 stencil marching down columns in packed fp32 -> A operand
 //   warps 8-15  epilogue group: TMEM -> growth bell, E = exp(G*I) -> swizzled staging tiles (+ register stores of
@@ -177,54 +297,41 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
-    const int my_tiles = n_tiles > (int)blockIdx.x ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    const K1Items items(n_tiles);
     const size_t xplane = (size_t)g.state_rows() * g.W * NC;
     const size_t eplane = (size_t)g.ev_h * g.ev_w * HD;
 
     if (warp == 16) {
-        // ================= TMA producer: weights of item i = (tile k, head h) into stage i % 3 ================
+        // ================= TMA producer: weights of the CTA's n-th item into stage n % 2 ==========================
         if (lane == 0) {
-            for (int k = 0; k < my_tiles; ++k) {
-                const CaTile t = ca_tile(blockIdx.x + k * gridDim.x, tiles_per_grid, g.tiles_x, -g.he);
-                const int set = t.b / g.per_set;
-                for (int h = 0; h < NH; ++h) {
-                    const int i = k * NH + h, ws = i & 1;
-                    ptx::mbar_wait(&w_empty[ws], ((i >> 1) & 1) ^ 1, status, 110);
-                    ptx::mbar_expect_tx(&w_full[ws], k1b::W_STAGE);
-                    ptx::tma_load_2d(sm + k1b::W0 + ws * k1b::W_STAGE, &map_w1, 0, (set * NH + h) * 192, &w_full[ws]);
-                }
+            for (int n = 0; n < items.count; ++n) {
+                const int ws = n & 1, set = items.tile(n) / tiles_per_grid / g.per_set;
+                ptx::mbar_wait(&w_empty[ws], ((n >> 1) & 1) ^ 1, status, 110);
+                ptx::mbar_expect_tx(&w_full[ws], k1b::W_STAGE);
+                ptx::tma_load_2d(sm + k1b::W0 + ws * k1b::W_STAGE, &map_w1, 0, (set * NH + items.head(n)) * 192, &w_full[ws]);
             }
         }
     } else if (warp == 17) {
-        // ================= UMMA issuer =======================================================================
-        if (lane == 0) {
-            const uint32_t idesc_u = ptx::umma_idesc_bf16(128, 64);
-            const uint32_t idesc_iv = ptx::umma_idesc_bf16(128, 128);
-            for (int k = 0; k < my_tiles; ++k) {
-                for (int h = 0; h < NH; ++h) {
-                    const int i = k * NH + h, ws = i & 1, half = h & 1, n = k * 4 + (h >> 1);
-                    const int slot = half * 2 + (n & 1), tb = i & 1;
-                    if (h == 0) ptx::mbar_wait(ax_full, k & 1, status, 120);
-                    ptx::mbar_wait(&w_full[ws], (i >> 1) & 1, status, 121);
-                    ptx::mbar_wait(&ac_full[slot], (n >> 1) & 1, status, 122);
-                    ptx::mbar_wait(&tm_empty[tb], ((i >> 1) & 1) ^ 1, status, 123);
-                    ptx::tc_fence_after();
-                    const uint32_t wb = ptx::smem_u32(sm + k1b::W0 + ws * k1b::W_STAGE);
-                    const uint64_t da = ptx::umma_desc_sw128(ptx::smem_u32(sm + k1b::A_CONV + slot * 16384));
-                    const uint64_t dx = ptx::umma_desc_sw128(ptx::smem_u32(sm + k1b::A_X));
-                    const uint64_t dwp = ptx::umma_desc_sw128(wb);
-                    const uint64_t dwiv = ptx::umma_desc_sw128(wb + 64 * 128);
-                    const uint32_t acc = tmem + tb * 192;
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) ptx::umma_bf16(acc, da + 2 * kk, dwp + 2 * kk, idesc_u, kk > 0);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) ptx::umma_bf16(acc + 64, dx + 2 * kk, dwiv + 2 * kk, idesc_iv, kk > 0);
-                    ptx::umma_commit(&w_empty[ws]);
-                    ptx::umma_commit(&ac_empty[slot]);
-                    ptx::umma_commit(&tm_full[tb]);
-                    if (h == NH - 1) ptx::umma_commit(ax_empty);
-                }
-            }
+        // ================= UMMA issuer (the whole warp, its leader executes) ======================================
+        const uint32_t leader = ptx::elect_one();
+        const uint32_t w0 = ptx::smem_u32(sm + k1b::W0) >> 4, a0 = ptx::smem_u32(sm + k1b::A_CONV) >> 4, x0 = ptx::smem_u32(sm + k1b::A_X) >> 4;
+        int k = -1;
+        for (int n = 0; n < items.count; ++n) {
+            const int tb = n & 1, slot = (n & 1) * 2 + ((n >> 1) & 1);
+            if (items.first(n)) { ++k; ptx::mbar_wait(ax_full, k & 1, status, 120); }
+            ptx::mbar_wait(&w_full[tb], (n >> 1) & 1, status, 121);
+            ptx::mbar_wait(&tm_empty[tb], ((n >> 1) & 1) ^ 1, status, 123);
+            ptx::mbar_wait(&ac_full[slot], (n >> 2) & 1, status, 122);
+            ptx::tc_fence_after();
+            const uint32_t w = w0 + tb * (k1b::W_STAGE >> 4), acc = tmem + tb * 192;
+            ptx::umma4_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW128_HI>(leader, acc, a0 + slot * (16384 >> 4), w, false);
+            ptx::umma4_ss<ptx::umma_idesc_bf16(128, 128), ptx::SW128_HI>(leader, acc + 64, x0, w + (64 * 128 >> 4), false);
+            ptx::umma_commit_by(leader, &w_empty[tb]);
+            ptx::umma_commit_by(leader, &ac_empty[slot]);
+            ptx::umma_commit_by(leader, &tm_full[tb]);
+            if (items.last(n)) ptx::umma_commit_by(leader, ax_empty);
         }
     } else if (warp == 18) {
         // ================= store warp: the TMA stores of every finished item ==================================
@@ -232,14 +339,17 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
         // tiles is written and go on to the next item; this thread issues the item's stores and hands the staging
         // back (stg_free) as soon as the stores have read it.
         if (lane == 0) {
-            for (int k = 0; k < my_tiles; ++k) {
-                const CaTile t = ca_tile(blockIdx.x + k * gridDim.x, tiles_per_grid, g.tiles_x, -g.he);
-                // whole-tile grids: which sides of the grid this tile touches
-                const bool left = t.tx0 == 0, right = t.tx0 + TBW == g.W;
-                const bool top = g.wrap_y && t.ty0 == 0, bottom = g.wrap_y && t.ty0 + TBH == g.H;
-                for (int h = 0; h < NH; ++h) {
-                    const int i = k * NH + h;
-                    ptx::mbar_wait(stg_full, i & 1, status, 150);
+            CaTile t;
+            bool left = false, right = false, top = false, bottom = false;
+            for (int n = 0; n < items.count; ++n) {
+                    const int h = items.head(n);
+                    if (items.first(n)) {
+                        t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
+                        // whole-tile grids: which sides of the grid this tile touches
+                        left = t.tx0 == 0; right = t.tx0 + TBW == g.W;
+                        top = g.wrap_y && t.ty0 == 0; bottom = g.wrap_y && t.ty0 + TBH == g.H;
+                    }
+                    ptx::mbar_wait(stg_full, n & 1, status, 150);
                     const int px = t.tx0 + APRON, py = t.ty0 + APRON, pl = t.b * NH + h;
                     ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, px, py, pl);
                     ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, px, py, pl);
@@ -275,7 +385,6 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
                     ptx::bulk_commit();
                     ptx::bulk_wait_read0();
                     ptx::mbar_arrive(stg_free);
-                }
             }
             ptx::bulk_wait0();
         }
@@ -284,17 +393,19 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
         const int half = warp >> 2, st = tid & 127;
         uint8_t* xh = sm + k1b::XH;
         float* prm_s = reinterpret_cast<float*>(sm + k1b::PRM_ST);
-        for (int k = 0; k < my_tiles; ++k) {
-            const CaTile t = ca_tile(blockIdx.x + k * gridDim.x, tiles_per_grid, g.tiles_x, -g.he);
+        for (int k = 0, first = 0, end; first < items.count; ++k, first = end) {
+            end = items.end(first);                                       // items first .. end - 1 are of this tile
+            const int h0 = items.head(first) - first;
+            const CaTile t = ca_tile(items.tile(first), tiles_per_grid, g.tiles_x, -g.he);
             const int set = t.b / g.per_set;
             uint8_t* a_x = sm + k1b::A_X;
             ptx::bar_sync(1, 256);                                        // both halves are done with the last halo
             const float* sc = scale + t.b * NC;
             if (tid < NH * PRM) prm_s[tid] = __ldg(prm + (size_t)set * NH * PRM + tid);
-            if (k + 1 < my_tiles && tid < 180) {       // next tile's halo cells: one 128-byte line each, into L2
-                const CaTile tn = ca_tile(blockIdx.x + (k + 1) * gridDim.x, tiles_per_grid, g.tiles_x, -g.he);
-                const int r = tn.ty0 + tid / 18 - 1, x = g.wrap_x(tn.tx0 + tid % 18 - 1);
-                ptx::prefetch_l2(X + (size_t)tn.b * xplane + ((size_t)g.xrow(r) * g.W + x) * NC);
+            if (end < items.count && tid < 180) {      // next tile's halo cells: one 128-byte line each, into L2
+                const CaTile tn = ca_tile(items.tile(end), tiles_per_grid, g.tiles_x, -g.he);
+                const int r = tn.ty0 + tid / 18 - 1, x = g.wrap_x_near(tn.tx0 + tid % 18 - 1);
+                ptx::prefetch_l2(X + (size_t)tn.b * xplane + ((size_t)g.xrow_near(r) * g.W + x) * NC);
             }
             {
                 // 180 cells x 8 chunks over 256 threads: issue every global load first, then scale, round to bf16
@@ -307,8 +418,8 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
                 for (int n = 0; n < 6; ++n) {
                     const int cell = (tid >> 3) + n * 32;
                     if (cell < 180) {
-                        const int r = t.ty0 + cell / 18 - 1, x = g.wrap_x(t.tx0 + cell % 18 - 1);
-                        raw[n] = *reinterpret_cast<const uint4*>(X + (size_t)t.b * xplane + ((size_t)g.xrow(r) * g.W + x) * NC + q * 8);
+                        const int r = t.ty0 + cell / 18 - 1, x = g.wrap_x_near(t.tx0 + cell % 18 - 1);
+                        raw[n] = *reinterpret_cast<const uint4*>(X + (size_t)t.b * xplane + ((size_t)g.xrow_near(r) * g.W + x) * NC + q * 8);
                     }
                 }
                 // the X operand is single-buffered: the last tile's products have long been issued by the time the
@@ -340,13 +451,13 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
             // a thread owns two adjacent columns x 4 channels: a row of the halo is four 16-byte loads (cells
             // 2p .. 2p+3), shared by the two outputs, and nothing is unpacked
             const int c4 = st & 15, p2 = st >> 4;
-            for (int h = half; h < NH; h += 2) {
-                const int n = k * 4 + (h >> 1), slot = half * 2 + (n & 1);
+            for (int n = first + ((first + half) & 1); n < end; n += 2) {
+                const int h = h0 + n, slot = half * 2 + ((n >> 1) & 1);
                 uint8_t* a_conv = sm + k1b::A_CONV + slot * 16384;
                 ptx::f2 kt[9];
 #pragma unroll
                 for (int tt = 0; tt < 9; ++tt) { const float kv = prm_s[h * PRM + tt]; kt[tt] = ptx::make_f2(kv, kv); }
-                ptx::mbar_wait(&ac_empty[slot], ((n >> 1) & 1) ^ 1, status, 131);
+                ptx::mbar_wait(&ac_empty[slot], ((n >> 2) & 1) ^ 1, status, 131);
                 // input row j feeds output rows j (tap row 0), j-1 (tap row 1) and j-2 (tap row 2)
                 ptx::f2 s1[2][2], s2[2][2];
 #pragma unroll
@@ -396,8 +507,10 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
         uint8_t* stg_e = sm + k1b::STG_E;
         uint8_t* stg_v = sm + k1b::STG_V;
         const bool tiny = g.W < 2 * APRON || (g.wrap_y && g.H < 2 * APRON);
-        for (int k = 0; k < my_tiles; ++k) {
-            const CaTile t = ca_tile(blockIdx.x + k * gridDim.x, tiles_per_grid, g.tiles_x, -g.he);
+        for (int first = 0, end; first < items.count; first = end) {
+            end = items.end(first);                        // items first .. end - 1 are of this tile
+            const int h0 = items.head(first) - first;
+            const CaTile t = ca_tile(items.tile(first), tiles_per_grid, g.tiles_x, -g.he);
             const int set = t.b / g.per_set;
             const int r_ep = t.ty0 + (m_ep >> 4), x_ep = t.tx0 + (m_ep & 15);
             const bool valid_ep = r_ep < g.H + g.he && x_ep < g.W;
@@ -422,8 +535,8 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
                 if (dup_x && dup_y) off_xy = ((size_t)(rd + APRON) * g.ev_w + xd + APRON) * HD;
             }
             const bool any_dup = !ALIGNED && valid_ep && (dup_x || dup_y || tiny);
-            for (int h = 0; h < NH; ++h) {
-                const int i = k * NH + h, tb = i & 1;
+            for (int i = first; i < end; ++i) {
+                const int h = h0 + i, tb = i & 1;
                 const float mus = __ldg(prm + ((size_t)set * NH + h) * PRM + 9);   // mu * s; Wp carries s and Wi carries log2(e)
                 const ptx::f2 neg_mus2 = ptx::make_f2(-mus, -mus), two2 = ptx::make_f2(2.f, 2.f), minus_one2 = ptx::make_f2(-1.f, -1.f);
                 // clamp(G*I) before the exponential = clamp of the rounded exponential (rounding to bf16 is monotone):
@@ -666,9 +779,9 @@ constexpr int STG = 0;
 constexpr int A_VP = STG + NSTAGE * STAGE_BYTES;        // two 16 KB operand tiles
 constexpr int WO = A_VP + 2 * 16384;                    // two 8 KB Wo slices
 constexpr int XT = WO + 2 * 8192;                       // two 16 KB state tiles of the epilogue (one per box-sum set)
-constexpr int RED = XT + 2 * 16384;                     // [A, B]: [4 quads][64] fp32 of a drain, [4][64] fp64 and a flag of a grid's sums
-constexpr int BARS = RED + 2 * (4 * 64 * 8 + 8);
-constexpr int N_BARS = NSTAGE + NSTAGE + 2 + 2 + 2 + 2 + NB + NB + 2 + 2;
+constexpr int RED = XT + 2 * 16384;                     // [A, B][4 quads][64] fp32
+constexpr int BARS = RED + 2 * 4 * 64 * 4;
+constexpr int N_BARS = NSTAGE + NSTAGE + 2 + 2 + 2 + 2 + NB + NB + 2 + 2 + 2;
 constexpr int TMEM_PTR = BARS + N_BARS * 8;
 constexpr int BYTES = TMEM_PTR + 16;
 constexpr int SMEM = BYTES + 1024;
@@ -714,7 +827,8 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
     uint64_t* acc_full = wo_empty + 2;               // [8] all 8 heads of the tile accumulated       (waits: who drains it)
     uint64_t* acc_empty = acc_full + k2m::NB;        // [8] drained (256 arrivals)                    (waits: UMMA issuer)
     uint64_t* x_full = acc_empty + k2m::NB;          // [2] a set's state tile landed                 (waits: that set)
-    uint64_t* x_empty = x_full + 2;                  // [2] ... and its X+ has left shared memory      (waits: TMA producer)
+    uint64_t* x_empty = x_full + 2;                  // [2] ... and its X+ has left shared memory      (waits: state producer)
+    uint64_t* summed = x_empty + 2;                  // [2] a set's tile sums are written (64 arrivals)  (waits: state producer)
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k2m::TMEM_PTR);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -726,7 +840,7 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
             ptx::mbar_init(&wo_full[i], 1); ptx::mbar_init(&wo_empty[i], 1);
         }
         for (int i = 0; i < k2m::NB; ++i) { ptx::mbar_init(&acc_full[i], 1); ptx::mbar_init(&acc_empty[i], 256); }
-        for (int i = 0; i < 2; ++i) { ptx::mbar_init(&x_full[i], 1); ptx::mbar_init(&x_empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { ptx::mbar_init(&x_full[i], 1); ptx::mbar_init(&x_empty[i], 1); ptx::mbar_init(&summed[i], NC); }
         ptx::fence_barrier_init();
         ptx::prefetch_tmap(&map_wo); ptx::prefetch_tmap(&map_e); ptx::prefetch_tmap(&map_v); ptx::prefetch_tmap(&map_x);
     }
@@ -735,6 +849,8 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const int my_mt = n_mt > (int)blockIdx.x ? (n_mt - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (warp == 16) {
@@ -764,57 +880,61 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
             }
         }
     } else if (warp == 18) {
-        // ================= TMA producer of the epilogues' state tiles ==========================================
+        // ================= TMA producer of the epilogues' state tiles, and the grids' sums ==========================
         // Tile b of a macro tile is drained by set A (even b) or B (odd b), in this order, while the next macro tile
         // runs its first head; its state goes into that set's buffer as soon as the buffer is free.  A producer of
         // its own, so that a wait for a buffer never holds back the E / V blocks.
-        if (lane == 0) {
-            uint32_t nx[2] = {0, 0};        // state tiles loaded for set A and set B
-            for (int k = 0; k < my_mt; ++k) {
-                const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
-                for (int b = 0; b < m.nb; ++b) {
-                    const int xb = b & 1;
-                    ptx::mbar_wait(&x_empty[xb], (nx[xb] & 1) ^ 1, status, 212);
+        uint32_t nx[2] = {0, 0}, seen[2] = {0, 0};        // state tiles loaded for set A and set B; their sums seen written
+        auto settle = [&](int xb) {
+            if (seen[xb] < nx[xb]) { ptx::mbar_wait(&summed[xb], seen[xb] & 1, status, 213); ++seen[xb]; }
+        };
+        int prev_b = -1;
+        for (int k = 0; k < my_mt; ++k) {
+            const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+            settle(0);
+            settle(1);
+            if (prev_b >= 0) k2_finish(fin, prev_b, tiles_per_grid, mt_per_grid);
+            prev_b = m.b;
+            for (int b = 0; b < m.nb; ++b) {
+                const int xb = b & 1;
+                ptx::mbar_wait(&x_empty[xb], (nx[xb] & 1) ^ 1, status, 212);
+                settle(xb);
+                if (lane == 0) {
                     ptx::mbar_expect_tx(&x_full[xb], 16384);
                     ptx::tma_load_4d(sm + k2m::XT + xb * 16384, &map_x, 0, m.mx0, g.hx + m.my0 + b * k2m::BR, m.b, &x_full[xb]);
-                    ++nx[xb];
                 }
+                ++nx[xb];
             }
         }
     } else if (warp == 17) {
-        // ================= UMMA issuer ====================================================================
-        if (lane == 0) {
-            const uint32_t idesc = ptx::umma_idesc_bf16(128, 64);
-            uint32_t v = 0, wit = 0, acc_par = 0;     // operand tiles used, heads, use parity of each accumulator
-            for (int k = 0; k < my_mt; ++k) {
-                const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
-                for (int h = 0; h < NH; ++h, ++wit) {
-                    const int wb = wit & 1;
-                    for (int b = 0; b < m.nb; ++b, ++v) {
-                        const int buf = v & 1;
-                        if (h == 0) ptx::mbar_wait(&acc_empty[b], ((acc_par >> b) & 1) ^ 1, status, 220);
-                        if (b == 0) ptx::mbar_wait(&wo_full[wb], (wit >> 1) & 1, status, 221);
-                        ptx::mbar_wait(&vp_full[buf], (v >> 1) & 1, status, 222);
-                        ptx::tc_fence_after();
-                        const uint64_t da = ptx::umma_desc_sw128(ptx::smem_u32(sm + k2m::A_VP + buf * 16384));
-                        const uint64_t dw = ptx::umma_desc_sw128(ptx::smem_u32(sm + k2m::WO + wb * 8192));
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            ptx::umma_bf16(tmem + b * 64, da + 2 * kk, dw + 2 * kk, idesc, h > 0 || kk > 0);
-                        ptx::umma_commit(&vp_empty[buf]);
-                        if (b == m.nb - 1) ptx::umma_commit(&wo_empty[wb]);
-                        if (h == NH - 1) ptx::umma_commit(&acc_full[b]);
-                    }
+        // ================= UMMA issuer (the whole warp, its leader executes) ==================================
+        const uint32_t leader = ptx::elect_one();
+        const uint32_t a0 = ptx::smem_u32(sm + k2m::A_VP) >> 4, w0 = ptx::smem_u32(sm + k2m::WO) >> 4;
+        uint32_t v = 0, wit = 0, acc_par = 0;     // operand tiles used, heads, use parity of each accumulator
+        for (int k = 0; k < my_mt; ++k) {
+            const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+            for (int h = 0; h < NH; ++h, ++wit) {
+                const int wb = wit & 1;
+                for (int b = 0; b < m.nb; ++b, ++v) {
+                    const int buf = v & 1;
+                    if (h == 0) ptx::mbar_wait(&acc_empty[b], ((acc_par >> b) & 1) ^ 1, status, 220);
+                    if (b == 0) ptx::mbar_wait(&wo_full[wb], (wit >> 1) & 1, status, 221);
+                    ptx::mbar_wait(&vp_full[buf], (v >> 1) & 1, status, 222);
+                    ptx::tc_fence_after();
+                    ptx::umma4_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW128_HI>(leader, tmem + b * 64, a0 + buf * (16384 >> 4), w0 + wb * (8192 >> 4), h > 0);
+                    ptx::umma_commit_by(leader, &vp_empty[buf]);
+                    if (b == m.nb - 1) ptx::umma_commit_by(leader, &wo_empty[wb]);
+                    if (h == NH - 1) ptx::umma_commit_by(leader, &acc_full[b]);
                 }
-                acc_par ^= (1u << m.nb) - 1u;
             }
+            acc_par ^= (1u << m.nb) - 1u;
         }
     } else {
         // ================= the two box-sum sets ==================================================================
         const bool is_a = warp < 8 || warp == 19;
         const int gt = warp == 19 ? 256 + lane : (is_a ? tid : tid - 256);     // thread within its set
         const int bar_ep = is_a ? 7 : 8;                        // named barrier of the set's drains (256 threads; 1-5 hand blocks over)
-        float* red = reinterpret_cast<float*>(sm + k2m::RED + (is_a ? 0 : 4 * 64 * 8 + 8));
+        float* red = reinterpret_cast<float*>(sm + k2m::RED) + (is_a ? 0 : 256);
         const int q = gt & 7, col = gt >> 3;                    // 8-dim chunk; column (A: of the 34 R columns, B: of the 32)
         uint32_t it = 0, v = 0, acc_par = 0, prev_par = 0;
         MacroTile prev;
@@ -832,6 +952,7 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
             ptx::mbar_wait(&x_full[is_a ? 0 : 1], nxs & 1, status, 233);
             ptx::tc_fence_after();
             k2_epilogue(t, tmem + b * 64, xs, scale, fin.partial, red, bar_ep, gt, warp, g);
+            if (gt < NC) ptx::mbar_arrive(&summed[is_a ? 0 : 1]);
             if (gt == 0) {
                 // X+ of the tile back to the state in one store (rows and columns past the grid are clipped); the
                 // buffer goes back to the producer once the store has read it
@@ -845,12 +966,6 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
             ++nxs;
         };
         const int mine = is_a ? 0 : 1;       // parity of the accumulators this set drains
-        // this set's tiles of macro tile `mt` are drained: its share (one of two per macro tile) of the grid's sums is there
-        auto finish = [&](const MacroTile& mt) {
-            if (mt.nb > 0)
-                k2_finish<256>(fin, mt.b, tiles_per_grid, 2 * mt_per_grid, reinterpret_cast<double*>(red), reinterpret_cast<int*>(red + 512), gt,
-                               [&] { ptx::bar_sync(bar_ep, 256); });
-        };
         V8 h2 = v8_zero(), h1 = v8_zero();   // running horizontal sums of the two rows above (of E in A, of R in B)
         uint4 ekeep0 = make_uint4(0, 0, 0, 0), ekeep1 = ekeep0;   // B: centre E of the last two rows of the block before
         const size_t vplane = (size_t)g.H * g.W * HD;
@@ -923,26 +1038,25 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
                     }
                 }
                 // accumulators of the macro tile before that this one does not reach (it has fewer blocks)
-                if (h == 0 && gt < 256) {
+                if (h == 0 && gt < 256)
                     for (int b = m.nb; b < prev.nb; ++b)
                         if ((b & 1) == mine) drain(prev, b, prev_par);
-                    finish(prev);
-                }
             }
             prev = m;
             prev_par = acc_par;
             acc_par ^= (1u << m.nb) - 1u;
         }
-        if (gt < 256) {
+        if (gt < 256)
             for (int b = 0; b < prev.nb; ++b)
                 if ((b & 1) == mine) drain(prev, b, prev_par);
-            finish(prev);
-        }
         if (gt == 0) ptx::bulk_wait0();      // this set's stores of X+ are complete
     }
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == 0) ptx::tmem_dealloc(tmem, k2m::TMEM_COLS);
+    if (my_mt > 0)       // the last macro tile's sums; the stages and the operand tiles are free by now
+        k2_finish_cta(fin, macro_tile(blockIdx.x + (my_mt - 1) * gridDim.x, mt_per_grid, strips, g.H, nbmax).b, tiles_per_grid, mt_per_grid,
+                      reinterpret_cast<double*>(sm + k2m::STG), reinterpret_cast<int*>(sm + k2m::A_VP));
 }
 
 // =============================================================================================================
@@ -1052,7 +1166,7 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
         bf16_error_ref() = "could not opt in to the kernels' dynamic shared memory";
         return -1;
     }
-    const long long total1 = (long long)p.k1_tiles * g.B;
+    const long long total1 = (long long)p.k1_tiles * g.B * NH;
     p.k1_grid = (int)(total1 < num_sms ? total1 : num_sms);
     const long long total_mt = k2_macro_tiles(g, p.strips, k2m::NB, num_sms, p.nbmax, p.mt_per_grid);
     p.k2_grid = (int)(total_mt < num_sms ? total_mt : num_sms);
@@ -1061,20 +1175,14 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
 
 inline int bf16_k1(Bf16Plan& p, const __nv_bfloat16* X, const float* scale, const float* prm, __nv_bfloat16* E,
                    __nv_bfloat16* V, int* status, const Geom& g, cudaStream_t st) {
-    if (p.k1_aligned)
-        k1_bf16<true><<<p.k1_grid, k1b::THREADS, k1b::SMEM, st>>>(p.map_w1, p.st, X, scale, prm, E, V, status,
-                                                                  p.k1_tiles * g.B, p.k1_tiles, g);
-    else
-        k1_bf16<false><<<p.k1_grid, k1b::THREADS, k1b::SMEM, st>>>(p.map_w1, p.st, X, scale, prm, E, V, status,
-                                                                   p.k1_tiles * g.B, p.k1_tiles, g);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_pdl(p.k1_aligned ? k1_bf16<true> : k1_bf16<false>, p.k1_grid, k1b::THREADS, k1b::SMEM, st, p.map_w1, p.st, X, scale, prm,
+                      E, V, status, p.k1_tiles * g.B, p.k1_tiles, g) == cudaSuccess ? 0 : -1;
 }
 
 inline int bf16_k2(Bf16Plan& p, __nv_bfloat16* X, const float* scale, const __nv_bfloat16*, const __nv_bfloat16*,
                    const K2Sums& fin, __nv_bfloat16* vprime, int* status, const Geom& g, cudaStream_t st) {
-    k2_bf16<<<p.k2_grid, k2m::THREADS, k2m::SMEM, st>>>(p.map_wo, p.map_e, p.map_v, p.map_x, scale, fin, vprime, status,
-                                                        p.mt_per_grid * g.B, p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_pdl(k2_bf16, p.k2_grid, k2m::THREADS, k2m::SMEM, st, p.map_wo, p.map_e, p.map_v, p.map_x, scale, fin, vprime, status,
+                      p.mt_per_grid * g.B, p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g) == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace slime

@@ -51,8 +51,6 @@ __device__ __forceinline__ void split3(ptx::f2 x, uint32_t& hi, uint32_t& mid, u
     lo = ptx::f2_to_bf16x2(ptx::fma2(ptx::bf16x2_to_f2(mid), m1, r));
 }
 
-__device__ __forceinline__ uint32_t swz64(int m, int q) { return (uint32_t)(m * 64 + ((q ^ ((m >> 1) & 3)) << 4)); }
-
 // The six products of a split contraction, smallest first, by part of the second operand: for part 2 (lo) of W only
 // hi of A, for part 1 mid and hi, for part 0 lo, mid and hi.  Part pw of W meets parts 2 - pw .. 0 of A.
 
@@ -67,27 +65,27 @@ constexpr int BARS = XH + XH_BYTES, N_BARS = 20, TMEM_PTR = BARS + N_BARS * 8;
 constexpr int BYTES = TMEM_PTR + 16;
 constexpr int SMEM = BYTES + 1024;                       // slack for manual 1024-byte alignment
 constexpr uint32_t TMEM_COLS = 512, AX = 384;            // two accumulator buffers of 192 columns, the X operand behind them
-constexpr int THREADS = 800;
+constexpr int THREADS = 768;
 static_assert(SMEM <= 227 * 1024, "k1 (fp32) shared memory");
 }  // namespace k1f
 
-// k1: one CTA per SM, warp-specialised.  The work is the list of (tile of 8 x 16 cells, head) items in order; a CTA
-// takes one contiguous stretch of it, so that the stretches differ by one item at most whatever the size of the grid.
+// k1: one CTA per SM, warp-specialised, over the (tile, head) items of K1Items (ca_bf16.cuh).
 //   warps 0-7   stencil group: per item the 3x3 stencil of the state halo, two columns x four channels x four rows per
 //               thread, times the pending scale, written as the three parts of one of two operand tiles; once per tile,
 //               behind its first item, the parts of the X operand into TMEM
 //   warps 8-15  E group: TMEM -> growth bell, E = exp(G*I); warps 16-19 V group: TMEM -> V.  Each warp has its own staging
 //               tiles (its 32 cells x 16 dims) and its own TMA stores: no barrier among them
-//   warps 20,21 TMA producers of the weight chunks, parts lo, mid, hi of Wi | Wv and of Wp
+//   warp 20     TMA producer of the weight chunks, per item the parts lo, mid, hi of Wi | Wv, then of Wp
 //   warps 22,23 UMMA issuers, one for I | V (N = 128, the X operand in TMEM: with both operands in shared memory the
 //               products, the stencil's loads and the stores of this kernel contend for its 128 bytes per cycle), one for U
 //               (N = 64).  One issuer for both was the longest chain of the kernel.
-//   warp 24     loads the tile's state halo, a bulk copy per row (two where the row wraps): with loads by the stencil group
+//   warp 21     loads the tile's state halo, a bulk copy per row (two where the row wraps): with loads by the stencil group
 //               a change of tile cost 14 000 cycles, two to three items
+// (24 warps: one more and a thread has 72 registers instead of 80.)
 __global__ void __launch_bounds__(k1f::THREADS, 1)
 k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_es,
        const __grid_constant__ CUtensorMap map_vs, const float* __restrict__ X, const float* __restrict__ scale,
-       const float* __restrict__ prm, float* __restrict__ E, float* __restrict__ V, int* __restrict__ status, int n_items,
+       const float* __restrict__ prm, float* __restrict__ E, float* __restrict__ V, int* __restrict__ status, int n_tiles,
        int tiles_per_grid, Geom g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
@@ -122,40 +120,44 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
-    const int i0 = (int)((long long)n_items * blockIdx.x / gridDim.x);
-    const int i1 = (int)((long long)n_items * (blockIdx.x + 1) / gridDim.x);
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    const K1Items items(n_tiles);
     const size_t xplane = (size_t)g.state_rows() * g.W * NC;
     const size_t eplane = (size_t)g.ev_h * g.ev_w * HD;
 
-    if (warp == 20 || warp == 21) {
-        // ================= TMA producers of the weight chunks =================================================
-        const int u = warp - 20;                               // 0: Wi | Wv, 1: Wp
+    if (warp == 20) {
+        // ================= TMA producer of the weight chunks ==================================================
         if (lane == 0) {
-            uint32_t c = 0;
-            for (int i = i0; i < i1; ++i) {
-                const int h = i & 7, b = (i >> 3) / tiles_per_grid, set = b / g.per_set;
-                for (int pw = 2; pw >= 0; --pw, ++c) {
-                    const int s = c & 1, row = ((set * NH + h) * 3 + pw) * 192;
-                    uint64_t* full = &w_full[2 * u + s];
-                    ptx::mbar_wait(&w_empty[2 * u + s], ((c >> 1) & 1) ^ 1, status, 310 + u);
-                    ptx::mbar_expect_tx(full, u ? k1f::WP_SLOT : k1f::WIV_SLOT);
-                    if (u) {
-                        ptx::tma_load_2d(sm + k1f::WP + s * k1f::WP_SLOT, &map_w1, 0, row, full);
-                    } else {
-                        ptx::tma_load_2d(sm + k1f::WIV + s * k1f::WIV_SLOT, &map_w1, 0, row + 64, full);
-                        ptx::tma_load_2d(sm + k1f::WIV + s * k1f::WIV_SLOT + 8192, &map_w1, 0, row + 128, full);
+            uint32_t c[2] = {0, 0};
+            for (int n = 0; n < items.count; ++n) {
+                const int set = items.tile(n) / tiles_per_grid / g.per_set;
+#pragma unroll
+                for (int u = 0; u < 2; ++u)                    // Wi | Wv, then Wp
+#pragma unroll 1
+                    for (int pw = 2; pw >= 0; --pw) {
+                        const int s = c[u] & 1, row = ((set * NH + items.head(n)) * 3 + pw) * 192;
+                        uint64_t* full = &w_full[2 * u + s];
+                        ptx::mbar_wait(&w_empty[2 * u + s], ((c[u] >> 1) & 1) ^ 1, status, 310 + u);
+                        ptx::mbar_expect_tx(full, u ? k1f::WP_SLOT : k1f::WIV_SLOT);
+                        if (u) {
+                            ptx::tma_load_2d(sm + k1f::WP + s * k1f::WP_SLOT, &map_w1, 0, row, full);
+                        } else {
+                            ptx::tma_load_2d(sm + k1f::WIV + s * k1f::WIV_SLOT, &map_w1, 0, row + 64, full);
+                            ptx::tma_load_2d(sm + k1f::WIV + s * k1f::WIV_SLOT + 8192, &map_w1, 0, row + 128, full);
+                        }
+                        ++c[u];
                     }
-                }
             }
         }
     } else if (warp == 22) {
         // ================= UMMA issuer of I | V (the whole warp, its leader executes) =================================
         const uint32_t leader = ptx::elect_one();
         const uint32_t wiv = ptx::smem_u32(sm + k1f::WIV) >> 4;
-        uint32_t c = 0, n = 0, tiles = 0;
-        for (int i = i0; i < i1; ++i, ++n) {
-            const int h = i & 7, tb = n & 1;
-            if (h == 0 || i == i0) { ptx::mbar_wait(ax_full, tiles & 1, status, 320); ++tiles; }
+        uint32_t c = 0, tiles = 0;
+        for (int n = 0; n < items.count; ++n) {
+            const int tb = n & 1;
+            if (items.first(n)) { ptx::mbar_wait(ax_full, tiles & 1, status, 320); ++tiles; }
             ptx::mbar_wait(&tm_empty[tb], ((n >> 1) & 1) ^ 1, status, 321);
             ptx::tc_fence_after();
             const uint32_t acc = tmem + tb * 192 + 64;
@@ -170,15 +172,15 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                     ptx::umma4_ts<ptx::umma_idesc_bf16(128, 128)>(leader, acc, tmem + k1f::AX + pa * 32, wiv + s * (k1f::WIV_SLOT >> 4), pw < 2 || pa < 2 - pw);
                 ptx::umma_commit_by(leader, &w_empty[s]);
             }
-            if (h == NH - 1 || i == i1 - 1) ptx::umma_commit_by(leader, ax_empty);
+            if (items.last(n)) ptx::umma_commit_by(leader, ax_empty);
             ptx::umma_commit_by(leader, &tm_full[tb]);
         }
     } else if (warp == 23) {
         // ================= UMMA issuer of U =======================================================================
         const uint32_t leader = ptx::elect_one();
         const uint32_t wp = ptx::smem_u32(sm + k1f::WP) >> 4, a0 = ptx::smem_u32(sm + k1f::A_CONV) >> 4;
-        uint32_t c = 0, n = 0;
-        for (int i = i0; i < i1; ++i, ++n) {
+        uint32_t c = 0;
+        for (int n = 0; n < items.count; ++n) {
             const int tb = n & 1;
             ptx::mbar_wait(&tm_empty[tb], ((n >> 1) & 1) ^ 1, status, 323);
             ptx::mbar_wait(&ac_full[tb], (n >> 1) & 1, status, 324);
@@ -198,11 +200,12 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
             ptx::umma_commit_by(leader, &ac_empty[tb]);
             ptx::umma_commit_by(leader, &tm_full[tb]);
         }
-    } else if (warp == 24) {
+    } else if (warp == 21) {
         // ================= halo loader: lane r brings row r of the halo ==============================================
         uint32_t tiles = 0;
-        for (int k = i0 >> 3; i0 < i1 && k <= (i1 - 1) >> 3; ++k, ++tiles) {
-            const CaTile t = ca_tile(k, tiles_per_grid, g.tiles_x, -g.he);
+        for (int n = 0; n < items.count; ++n) {
+            if (!items.first(n)) continue;
+            const CaTile t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
             ptx::mbar_wait(xh_empty, (tiles & 1) ^ 1, status, 330);
             if (lane == 0) ptx::mbar_expect_tx(xh_full, k1f::XH_BYTES);
             __syncwarp();
@@ -211,25 +214,26 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                 uint8_t* dst = sm + k1f::XH + lane * (TBW + 2) * 256;
                 int x = g.wrap_x_near(t.tx0 - 1);
                 for (int left = TBW + 2; left > 0; x = 0) {
-                    const int n = min(left, g.W - x);
-                    ptx::bulk_load(dst, row + (size_t)x * NC, n * 256, xh_full);
-                    dst += n * 256;
-                    left -= n;
+                    const int cells = min(left, g.W - x);
+                    ptx::bulk_load(dst, row + (size_t)x * NC, cells * 256, xh_full);
+                    dst += cells * 256;
+                    left -= cells;
                 }
             }
+            ++tiles;
         }
     } else if (warp < 8) {
         // ================= stencil group ======================================================================
         const uint8_t* xh = sm + k1f::XH;
         const int c4 = tid & 15, p2 = (tid >> 4) & 7, y0 = (tid >> 7) * 4;
-        uint32_t n = 0, tiles = 0;
+        uint32_t tiles = 0;
         CaTile t;
         ptx::f2 sc[2];
-        for (int i = i0; i < i1; ++i, ++n) {
-            const int h = i & 7, tb = n & 1;
-            const bool first = h == 0 || i == i0;
+        for (int n = 0; n < items.count; ++n) {
+            const int h = items.head(n), tb = n & 1;
+            const bool first = items.first(n);
             if (first) {
-                t = ca_tile(i >> 3, tiles_per_grid, g.tiles_x, -g.he);
+                t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
                 const float4 s4 = __ldg(reinterpret_cast<const float4*>(scale + t.b * NC + c4 * 4));
                 sc[0] = ptx::make_f2(s4.x, s4.y);
                 sc[1] = ptx::make_f2(s4.z, s4.w);
@@ -302,7 +306,7 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                 ptx::mbar_arrive(ax_full);
                 ++tiles;
             }
-            if (h == NH - 1 || i == i1 - 1) ptx::mbar_arrive(xh_empty);
+            if (items.last(n)) ptx::mbar_arrive(xh_empty);
         }
     } else {
         // ================= E group (warps 8..15: a quarter of the cells, half of the dims) and V group (16..19: a quarter
@@ -311,29 +315,14 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
         const int quad = warp & 3, m_ep = quad * 32 + lane;          // TMEM lane = cell of the tile this thread finishes
         const int d_first = is_e ? ((warp - 8) >> 2) * 32 : 0, d_last = is_e ? d_first + 16 : 48;
         uint8_t* stg = sm + k1f::STG + (is_e ? warp - 8 : 8 + quad * 2) * 2048;
-        const bool tiny = g.W < 2 * APRON || (g.wrap_y && g.H < 2 * APRON);
         const ptx::f2 two2 = ptx::make_f2(2.f, 2.f), minus_one2 = ptx::make_f2(-1.f, -1.f);
-        uint32_t n = 0;
         CaTile t;
-        // Apron positions that wrap onto this thread's cell (the TMA store covers the cell itself and whatever hangs over
-        // the far edge), as cell offsets in the plane, -1 for none.  Grids narrower or shorter than twice the apron can
-        // wrap more than once and take the general loop.
-        int dup_x = -1, dup_y = -1, dup_xy = -1;
-        bool edge_x = false, edge_y = false, edge = false;           // does any cell of the warp have one
-        for (int i = i0; i < i1; ++i, ++n) {
-            const int h = i & 7, tb = n & 1;
-            if (h == 0 || i == i0) {
-                t = ca_tile(i >> 3, tiles_per_grid, g.tiles_x, -g.he);
-                const int r = t.ty0 + (m_ep >> 4), x = t.tx0 + (m_ep & 15);
-                const bool valid = r < g.H + g.he && x < g.W;
-                const int xd = x < APRON ? x + g.W : x >= g.W - APRON ? x - g.W : -100;
-                const int rd = !g.wrap_y ? -100 : r < APRON ? r + g.H : r >= g.H - APRON ? r - g.H : -100;
-                dup_x = valid && xd != -100 ? (r + APRON) * g.ev_w + xd + APRON : -1;
-                dup_y = valid && rd != -100 ? (rd + APRON) * g.ev_w + x + APRON : -1;
-                dup_xy = dup_x >= 0 && dup_y >= 0 ? (rd + APRON) * g.ev_w + xd + APRON : -1;
-                edge_x = __any_sync(0xffffffffu, dup_x >= 0);
-                edge_y = __any_sync(0xffffffffu, dup_y >= 0);
-                edge = tiny || edge_x || edge_y;
+        ApronCopies apron;
+        for (int n = 0; n < items.count; ++n) {
+            const int h = items.head(n), tb = n & 1;
+            if (items.first(n)) {
+                t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
+                apron.tile(t, quad, lane, g);
             }
             const float mus = __ldg(prm + ((size_t)(t.b / g.per_set) * NH + h) * PRM + 9);   // mu * s; Wp carries s and Wi carries log2(e)
             const ptx::f2 neg_mus2 = ptx::make_f2(-mus, -mus);
@@ -377,32 +366,15 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                     *reinterpret_cast<float4*>(tile + swz64(lane, q)) = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
                 ptx::fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) {             // the warp's 32 cells are two rows of the tile
-                    ptx::tma_store_4d(is_e ? &map_es : &map_vs, tile, d0, t.tx0 + APRON, t.ty0 + quad * 2 + APRON, t.b * NH + h);
+                if (lane == 0) {
+                    apron.staged(t, quad, g, [&](int px, int py) { ptx::tma_store_4d(is_e ? &map_es : &map_vs, tile, d0, px, py, t.b * NH + h); });
                     ptx::bulk_commit();
                 }
-                if (edge) {
-                    float* plane = (is_e ? E : V) + ((size_t)t.b * NH + h) * eplane + d0;
-                    auto copy = [&](int cell) {
-                        float4* p = reinterpret_cast<float4*>(plane + (size_t)cell * HD);
+                apron.own(t, quad, lane, g, [&](int cell) {
+                    float4* p = reinterpret_cast<float4*>((is_e ? E : V) + ((size_t)t.b * NH + h) * eplane + (size_t)cell * HD + d0);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) p[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
-                    };
-                    if (!tiny) {
-                        if (edge_x && dup_x >= 0) copy(dup_x);
-                        if (edge_y && dup_y >= 0) copy(dup_y);
-                        if (edge_x && edge_y && dup_xy >= 0) copy(dup_xy);
-                    } else {
-                        const int r = t.ty0 + (m_ep >> 4), x = t.tx0 + (m_ep & 15);
-                        if (r < g.H + g.he && x < g.W)
-                            for (int ky = g.wrap_y ? -2 * APRON : 0; ky <= (g.wrap_y ? 2 * APRON : 0); ++ky)
-                                for (int kx = -2 * APRON; kx <= 2 * APRON; ++kx) {
-                                    const int rr = r + ky * g.H, xx = x + kx * g.W;
-                                    if ((ky == 0 && kx == 0) || rr < -APRON || rr >= g.H + APRON || xx < -APRON || xx >= g.W + APRON) continue;
-                                    copy((rr + APRON) * g.ev_w + xx + APRON);
-                                }
-                    }
-                }
+                    for (int q = 0; q < 4; ++q) p[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+                });
             }
         }
         if (lane == 0) ptx::bulk_wait0();
@@ -435,8 +407,8 @@ constexpr int A_VP = STG + NSTAGE * STAGE_BYTES;        // two operand tiles of 
 constexpr int WO_PART = 4096, WO = A_VP + 2 * 3 * PART; // two Wo slices of 3 parts [64][32]
 constexpr int XT = WO + 2 * 3 * WO_PART;                // state tile of the epilogue: two halves of 32 channels, 16 KB each
 constexpr int RED = XT + 2 * 16384;                     // [4 quads][64] fp64
-constexpr int FLAG = RED + 4 * 64 * 8, BARS = FLAG + 8;
-constexpr int N_BARS = 2 * NSTAGE + 12;
+constexpr int BARS = RED + 4 * 64 * 8;
+constexpr int N_BARS = 2 * NSTAGE + 13;
 constexpr int TMEM_PTR = BARS + N_BARS * 8;
 constexpr int BYTES = TMEM_PTR + 16;
 constexpr int SMEM = BYTES + 1024;
@@ -447,6 +419,11 @@ constexpr int HANDOFF = A_THREADS + B_THREADS;
 static_assert(A_VP % 1024 == 0 && WO % 1024 == 0 && XT % 1024 == 0, "swizzled tiles must be aligned");
 static_assert(SMEM <= 227 * 1024, "k2 (fp32) shared memory");
 }  // namespace k2f
+
+// The same two as calls: inlined, they cost this kernel 30 % (1.56 -> 2.03 ms at X[64,128,128,64]) by what they do to the
+// registers and the code of the others.
+__device__ __noinline__ void k2_finish_call(const K2Sums& k, int b, int n, int parts) { k2_finish(k, b, n, parts); }
+__device__ __noinline__ void k2_finish_cta_call(const K2Sums& k, int b, int n, int parts, double* red, int* flag) { k2_finish_cta(k, b, n, parts, red, flag); }
 
 struct V4 { ptx::f2 a, b; };
 __device__ __forceinline__ V4 v4(const float4& f) { V4 r; r.a = ptx::make_f2(f.x, f.y); r.b = ptx::make_f2(f.z, f.w); return r; }
@@ -482,6 +459,7 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
     uint64_t* wk_empty = wk_full + 2;                // [2] ... and added (128 arrivals)              (waits: UMMA issuer)
     uint64_t* x_full = wk_empty + 2;                 // state tile landed                             (waits: P)
     uint64_t* x_empty = x_full + 1;                  // ... and its X+ has left shared memory          (waits: state producer)
+    uint64_t* summed = x_full + 2;                   // the tile's sums are written (64 arrivals)       (waits: state producer)
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k2f::TMEM_PTR);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -492,7 +470,7 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
             ptx::mbar_init(&wo_full[i], 1); ptx::mbar_init(&wo_empty[i], 1);
             ptx::mbar_init(&wk_full[i], 1); ptx::mbar_init(&wk_empty[i], 128);
         }
-        ptx::mbar_init(x_full, 1); ptx::mbar_init(x_empty, 1);
+        ptx::mbar_init(x_full, 1); ptx::mbar_init(x_empty, 1); ptx::mbar_init(summed, NC);
         ptx::fence_barrier_init();
         ptx::prefetch_tmap(&map_wo); ptx::prefetch_tmap(&map_e); ptx::prefetch_tmap(&map_v); ptx::prefetch_tmap(&map_x);
     }
@@ -501,6 +479,8 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const int my_mt = n_mt > (int)blockIdx.x ? (n_mt - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (warp == 16) {
@@ -527,18 +507,21 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
             }
         }
     } else if (warp == 18) {
-        // ================= TMA producer of the epilogue's state tiles ==========================================
-        if (lane == 0) {
-            uint32_t nx = 0;
-            for (int k = 0; k < my_mt; ++k) {
-                const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
-                for (int b = 0; b < m.nb; ++b, ++nx) {
-                    ptx::mbar_wait(x_empty, (nx & 1) ^ 1, status, 512);
+        // ================= TMA producer of the epilogue's state tiles, and the grids' sums ==========================
+        uint32_t nx = 0;
+        for (int k = 0; k < my_mt; ++k) {
+            const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
+            for (int b = 0; b < m.nb; ++b, ++nx) {
+                ptx::mbar_wait(x_empty, (nx & 1) ^ 1, status, 512);
+                if (b > 0) ptx::mbar_wait(summed, (nx - 1) & 1, status, 513);
+                if (lane == 0) {
                     ptx::mbar_expect_tx(x_full, 32768);
                     ptx::tma_load_4d(sm + k2f::XT, &map_x, 0, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, x_full);
                     ptx::tma_load_4d(sm + k2f::XT + 16384, &map_x, 32, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, x_full);
                 }
             }
+            ptx::mbar_wait(summed, (nx - 1) & 1, status, 514);
+            if (k < my_mt - 1) k2_finish_call(fin, m.b, tiles_per_grid, mt_per_grid);
         }
     } else if (warp == 17) {
         // ================= UMMA issuer (the whole warp, its leader executes) ==================================
@@ -657,6 +640,7 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                             const float hi = (float)t;
                             fin.partial[o] = hi;
                             fin.partial[o + fin.lo_offset] = (float)(t - (double)hi);
+                            ptx::mbar_arrive(summed);
                         }
                         if (pt == 0) {
                             ptx::tma_store_4d(&map_x, xt, 0, m.mx0, g.hx + ty0, m.b);
@@ -667,9 +651,6 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                         }
                         ptx::bar_sync(7, 128);         // the reduction scratch is free again
                         ++nx;
-                        if (b == m.nb - 1)
-                            k2_finish<128>(fin, m.b, tiles_per_grid, mt_per_grid, red, reinterpret_cast<int*>(sm + k2f::FLAG), pt,
-                                           [] { ptx::bar_sync(7, 128); });
                     }
                 }
             }
@@ -754,6 +735,9 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == 0) ptx::tmem_dealloc(tmem, k2f::TMEM_COLS);
+    if (my_mt > 0)       // the last macro tile's sums; the stages and the operand tiles are free by now
+        k2_finish_cta_call(fin, macro_tile(blockIdx.x + (my_mt - 1) * gridDim.x, mt_per_grid, strips, g.H, nbmax).b, tiles_per_grid, mt_per_grid,
+                      reinterpret_cast<double*>(sm + k2f::STG), reinterpret_cast<int*>(sm + k2f::A_VP));
 }
 
 // =============================================================================================================

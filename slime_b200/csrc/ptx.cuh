@@ -116,6 +116,12 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
 
+// ---- programmatic dependent launch ---------------------------------------------------------------------------
+// The next kernel of the stream may take SMs as they fall free and set itself up ...
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// ... but touches nothing that the kernel before it writes until that has finished (and its writes are visible).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- TMEM ---------------------------------------------------------------------------------------------------
 // One full warp allocates `cols` (power of two >= 32) TMEM columns; the base address lands in *smem_out.
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_out, uint32_t cols) {

@@ -187,15 +187,13 @@ int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nul
         ++h->launches;
     } else {
         const F32Plan& p = h->f32;
-        k1_f32<<<p.k1_grid, k1f::THREADS, k1f::SMEM, st>>>(p.map_w1, p.map_es, p.map_vs, (const float*)h->X, h->scale, h->prm,
-                                                           (float*)h->E, (float*)h->V, h->dev_status, p.k1_tiles * g.B * NH,
-                                                           p.k1_tiles, g);
-        LAUNCHED(h);
+        CK(h, launch_pdl(k1_f32, p.k1_grid, k1f::THREADS, k1f::SMEM, st, p.map_w1, p.map_es, p.map_vs, (const float*)h->X, h->scale, h->prm,
+                         (float*)h->E, (float*)h->V, h->dev_status, p.k1_tiles * g.B, p.k1_tiles, g));
+        ++h->launches;
         if (ev) CK(h, cudaEventRecord(ev[1], st));
-        k2_f32<<<p.k2_grid, k2f::THREADS, k2f::SMEM, st>>>(p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, fin, (float*)emit,
-                                                           h->dev_status, p.mt_per_grid * g.B, p.mt_per_grid,
-                                                           p.strips, p.k2_tiles, p.nbmax, g);
-        LAUNCHED(h);
+        CK(h, launch_pdl(k2_f32, p.k2_grid, k2f::THREADS, k2f::SMEM, st, p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, fin, (float*)emit,
+                         h->dev_status, p.mt_per_grid * g.B, p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g));
+        ++h->launches;
     }
     if (ev) CK(h, cudaEventRecord(ev[2], st));
     if (h->k2_tiles > FUSE_PARTIALS) {        // else k2 has done it
