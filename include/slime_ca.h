@@ -102,9 +102,8 @@ int slime_ca_get_state(slime_ca* h, void* host_state, int host_dtype, void* stre
 
 /* Same with DEVICE pointers (no synchronisation).  A caller that never synchronises through this library
  * (set_state_device / step / get_state_device on its own stream) still learns of a kernel that gave up on a
- * bounded wait: every batch of steps copies the status word back to pinned host memory behind itself, and
- * slime_ca_step, slime_ca_step_partial, slime_ca_step_ring and slime_ca_get_state_device return
- * SLIME_CA_EDEVICE at their next call once that copy has run.  set_state_device clears the condition. */
+ * bounded wait: the kernel writes the status word to pinned host memory, and slime_ca_step, slime_ca_step_partial,
+ * slime_ca_step_ring and slime_ca_get_state_device return SLIME_CA_EDEVICE at their next call after that.  set_state_device clears the condition. */
 int slime_ca_set_state_device(slime_ca* h, const void* dev_state, int dtype, void* stream);
 int slime_ca_get_state_device(slime_ca* h, void* dev_state, int dtype, void* stream);
 
@@ -299,7 +298,7 @@ int slime_ca_occupancy(slime_ca* h, float* occupancy);
 /*
  * Self-test of the bounded device-side waits, with no counterpart in the reference: launches one thread that waits
  * `limit_ns` (at most 100 ms) on a barrier nobody arrives on, gives up, and records code 901 in the handle's status
- * word.  The next synchronising call on the handle (or the next step call, once the word has been copied back)
+ * word.  The next synchronising call on the handle (or the next step call after the kernel has run)
  * returns SLIME_CA_EDEVICE and clears the word; the context stays usable.
  */
 int slime_ca_selftest_bounded_wait(slime_ca* h, unsigned long long limit_ns, void* stream);

@@ -247,16 +247,18 @@ k_state_out(const TI* __restrict__ X, const float* __restrict__ scale, TO* __res
     }
 }
 
+struct LiftVector { float v[NC]; };      // a kernel argument: no copy to the device ahead of the launch
 // X[b,y,x,c] = img[b,y-py,x-px] * L[c] inside the centred image, 0 in the padding, and the sums of what was stored.
 template <typename TO>
 __global__ void __launch_bounds__(256)
-k_lift(const float* __restrict__ img, int ih, int iw, const float* __restrict__ L, TO* __restrict__ X, ChunkSums out, Geom g) {
+k_lift(const float* __restrict__ img, int ih, int iw, const LiftVector L, TO* __restrict__ X, ChunkSums out, Geom g) {
     const int py = (g.H - ih) / 2, px = (g.W - iw) / 2;
     const int cells = g.H * g.W, q = (threadIdx.x & 7) * 8;
     const size_t b = blockIdx.y;
     TO* dst = X + (b * g.state_rows() + g.hx) * g.W * NC + q;
     float l[8], acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    load8<float>(L + q, true, l);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) l[k] = L.v[q + k];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int cell = blockIdx.x * 256 + i * 32 + (threadIdx.x >> 3);
@@ -274,28 +276,29 @@ k_lift(const float* __restrict__ img, int ih, int iw, const float* __restrict__ 
     chunk_sums(acc, out);
 }
 
-// field[b][cell] = mean over the 64 channels of the normalised state (stored value x pending scale).  Eight
-// threads per cell, eight channels each, summed by a fixed shuffle tree.
+// field[b][cell] = mean over the 64 channels of the normalised state (stored value x pending scale).  Grid (blocks,
+// grids); eight threads per cell, eight channels each, summed by a fixed shuffle tree.
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_channel_mean(const T* __restrict__ X, const float* __restrict__ scale, float* __restrict__ field, Geom g) {
-    const size_t cells = (size_t)g.H * g.W, n = cells * g.B;
-    const int q = threadIdx.x & 7;
+    const size_t cells = (size_t)g.H * g.W, b = blockIdx.y;
+    const int q = (threadIdx.x & 7) * 8;
+    const T* src = X + (b * g.state_rows() + g.hx) * g.W * NC + q;
+    float sc[8];
+    load8<float>(scale + b * NC + q, true, sc);
     // a warp covers 4 consecutive cells; the loop condition is on the warp's first cell, so all 32 lanes shuffle
-    for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; (i & ~size_t(3)) < n;
-         i += ((size_t)gridDim.x * blockDim.x) >> 3) {
+    for (size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) >> 3; (i & ~size_t(3)) < cells; i += (size_t)gridDim.x * 32) {
         float s = 0.f;
-        const bool live = i < n;
-        const size_t b = live ? i / cells : 0, cell = live ? i % cells : 0;
-        if (live) {
-            const T* px = X + ((b * g.state_rows() + g.hx) * g.W) * NC + cell * NC + q * 8;
+        if (i < cells) {
+            float f[8];
+            load8<T>(src + i * NC, true, f);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) s = fmaf(to_f32<T>(px[k]), scale[b * NC + q * 8 + k], s);
+            for (int k = 0; k < 8; ++k) s = fmaf(f[k], sc[k], s);
         }
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
         s += __shfl_xor_sync(0xffffffffu, s, 4);
-        if (live && q == 0) field[i] = s * (1.f / NC);
+        if (i < cells && q == 0) field[b * cells + i] = s * (1.f / NC);
     }
 }
 

@@ -312,7 +312,7 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
         // ================= E group (warps 8..15: a quarter of the cells, half of the dims) and V group (16..19: a quarter
         // of the cells, all dims), sixteen dims at a time ===========================================================
         const bool is_e = warp < 16;
-        const int quad = warp & 3, m_ep = quad * 32 + lane;          // TMEM lane = cell of the tile this thread finishes
+        const int quad = warp & 3;
         const int d_first = is_e ? ((warp - 8) >> 2) * 32 : 0, d_last = is_e ? d_first + 16 : 48;
         uint8_t* stg = sm + k1f::STG + (is_e ? warp - 8 : 8 + quad * 2) * 2048;
         const ptx::f2 two2 = ptx::make_f2(2.f, 2.f), minus_one2 = ptx::make_f2(-1.f, -1.f);

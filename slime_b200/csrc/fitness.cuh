@@ -1,7 +1,6 @@
-// Fitness reduction: per (grid, head) 64x64 Gram of the redistributed value V', Jacobi eigenvalues,
-// exp-entropy rank, Pearson coherence between the last two steps, fitness = rank x coherence.
+// Fitness reduction: per (grid, head) 64x64 Gram of the redistributed value V', its eigenvalues, exp-entropy rank, Pearson coherence between the last two steps, fitness = rank x coherence.
 // Replaces gpu_svd_kernel / effective_rank_kernel / coherence_kernel / fitness_fused_kernel
-// (slime/kernels/warp_ca.cu:66-226).  Gram and Jacobi run in fp64: the small eigenvalues carry most of the
+// (slime/kernels/warp_ca.cu:66-226).  Gram and eigenvalues run in fp64: the small eigenvalues carry most of the
 // entropy's sensitivity, and an fp32 Gram loses them.
 #pragma once
 #include "ca_aux.cuh"
@@ -10,10 +9,9 @@
 
 namespace slime {
 
-constexpr int GRAM_CHUNK = 2048;   // cells per Gram partial
-constexpr int JSTRIDE = 65;        // padded row stride of the Jacobi matrix in shared memory (doubles)
+constexpr int GRAM_CHUNK = 2048;   // cells per Gram partial, at most; populations too small to fill the GPU take less
 
-// gram_part[((b*8+h)*splits + split)][64][64] (fp64) over cells [split*GRAM_CHUNK, ...) of plane (b,h).
+// gram_part[((b*8+h)*splits + split)][64][64] (fp64) over cells [split*chunk, ...) of plane (b,h).
 // The Gram matrix is symmetric: only the 136 4x4 blocks on or above the diagonal are accumulated (one thread
 // each, 160 threads per block) and each is written to both places.  A chunk of 64 cells is converted to fp64
 // once, on its way into shared memory (the conversion is the slow instruction here: converting at the point of
@@ -23,7 +21,7 @@ constexpr int JSTRIDE = 65;        // padded row stride of the Jacobi matrix in 
 constexpr int GRAM_THREADS = 160;
 template <typename T>
 __global__ void __launch_bounds__(GRAM_THREADS, 6)
-k_gram(const T* __restrict__ vp, int cells, double* __restrict__ gram_part) {
+k_gram(const T* __restrict__ vp, int cells, int chunk, double* __restrict__ gram_part) {
     __shared__ __align__(16) double2 flo[64][16];      // values 4 blk + 0, 4 blk + 1 of cell s
     __shared__ __align__(16) double2 fhi[64][16];      // values 4 blk + 2, 4 blk + 3
     const int split = blockIdx.x, h = blockIdx.y, b = blockIdx.z, splits = gridDim.x;
@@ -39,8 +37,8 @@ k_gram(const T* __restrict__ vp, int cells, double* __restrict__ gram_part) {
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    const int lo = split * GRAM_CHUNK;
-    const int hi = min(lo + GRAM_CHUNK, cells);
+    const int lo = split * chunk;
+    const int hi = min(lo + chunk, cells);
     for (int s0 = lo; s0 < hi; s0 += 64) {
         __syncthreads();
         for (int i = threadIdx.x; i < 64 * 32; i += GRAM_THREADS) {       // one pair of adjacent values per step
@@ -77,13 +75,13 @@ k_gram(const T* __restrict__ vp, int cells, double* __restrict__ gram_part) {
         }
 }
 
-// The same Gram partials for bf16 planes on the tensor cores.  One CTA per (grid, head) plane walks the plane in tiles
+// The same Gram partials for bf16 planes on the tensor cores.  One CTA per (grid, head) plane (several where there are few planes) walks its chunks in tiles
 // of 128 cells; a tile [128 cells][64 dims] lands in shared memory by TMA with the 128-byte swizzle, which is exactly
 // the MN-major operand layout of tcgen05 (one 128-byte row of the 64 dims per cell), so the one tile is both operands of
 // D[64 x 64] += F^T F: eight tcgen05.mma of M = 64, N = 64, K = 16 cells, fp32 accumulation in 64 TMEM columns (the
-// products of bf16 values are exact in fp32).  After every GRAM_CHUNK cells the accumulator is written out as one fp64
+// products of bf16 values are exact in fp32).  After every chunk of cells the accumulator is written out as one fp64
 // partial - the same [plane][split][64][64] layout the SIMT kernel fills - and cleared by the next chunk's first
-// instruction, so chunks are still summed in fp64 by k_jacobi_rank.  An M = 64 accumulator keeps row r in TMEM lane
+// instruction, so chunks are still summed in fp64 by k_gram_rank.  An M = 64 accumulator keeps row r in TMEM lane
 // 32 * (r / 16) + r % 16: warp w's first sixteen lanes hold rows 16 w .. 16 w + 15.
 namespace gtc {
 constexpr int TILE = 128, STAGES = 4, TILE_BYTES = TILE * 128;
@@ -91,7 +89,7 @@ constexpr int BARS = STAGES * TILE_BYTES, TMEM_PTR = BARS + (2 * STAGES + 2) * 8
 constexpr uint32_t IDESC = ptx::umma_idesc_bf16(64, 64) | (1u << 15) | (1u << 16);     // both operands MN-major
 }  // namespace gtc
 __global__ void __launch_bounds__(128)
-k_gram_tc(const __grid_constant__ CUtensorMap map_vp, int cells, int splits, double* __restrict__ gram_part,
+k_gram_tc(const __grid_constant__ CUtensorMap map_vp, int cells, int chunk, int splits, double* __restrict__ gram_part,
           int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
@@ -114,8 +112,9 @@ k_gram_tc(const __grid_constant__ CUtensorMap map_vp, int cells, int splits, dou
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
     uint32_t it = 0;       // tiles so far (the producer and the issuer count the same way)
-    for (int split = 0; split < splits; ++split) {
-        const int lo = split * GRAM_CHUNK, hi = min(lo + GRAM_CHUNK, cells);
+    const int split0 = (int)((long long)splits * blockIdx.y / gridDim.y), split1 = (int)((long long)splits * (blockIdx.y + 1) / gridDim.y);
+    for (int split = split0; split < split1; ++split) {
+        const int lo = split * chunk, hi = min(lo + chunk, cells), u = split - split0;
         const int n_tiles = (hi - lo + gtc::TILE - 1) / gtc::TILE;
         if (warp == 0 && lane == 0) {
             for (int t = 0; t < n_tiles; ++t) {
@@ -127,7 +126,7 @@ k_gram_tc(const __grid_constant__ CUtensorMap map_vp, int cells, int splits, dou
                 ptx::tma_load_3d(sm + s * gtc::TILE_BYTES, &map_vp, 0, lo + t * gtc::TILE, plane, &full[s]);
             }
         } else if (warp == 1 && lane == 0) {
-            ptx::mbar_wait(acc_empty, (split & 1) ^ 1, status, 411);
+            ptx::mbar_wait(acc_empty, (u & 1) ^ 1, status, 411);
             ptx::tc_fence_after();
             for (int t = 0; t < n_tiles; ++t) {
                 const uint32_t i = it + t, s = i % gtc::STAGES;
@@ -143,7 +142,7 @@ k_gram_tc(const __grid_constant__ CUtensorMap map_vp, int cells, int splits, dou
         }
         it += n_tiles;
         __syncwarp();
-        ptx::mbar_wait(acc_full, split & 1, status, 413);
+        ptx::mbar_wait(acc_full, u & 1, status, 413);
         ptx::tc_fence_after();
         double* out = gram_part + ((size_t)plane * splits + split) * (HD * HD) + (size_t)(warp * 16 + (lane & 15)) * HD;
 #pragma unroll
@@ -183,114 +182,155 @@ inline int gram_tc_map(CUtensorMap* map, const void* vp, int planes, int cells) 
     return cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, gtc::SMEM) == cudaSuccess ? 0 : -1;
 }
 
-// One 256-thread block per (grid, head): sum the Gram partials, diagonalise by two-sided Jacobi with a
-// round-robin (tournament) ordering - 32 disjoint rotations per round, applied as 1024 independent 2 x 2 blocks, 63
-// rounds per sweep - until the
-// off-diagonal Frobenius norm is <= 1e-6 x the matrix norm, plus one more sweep, at most 30 sweeps
-// (rotation formula of slime/kernels/warp_ca.cu:51-63, sweep limit :20), then the exp-entropy rank
+// One 256-thread block per (grid, head): the eigenvalues of the summed Gram matrix and the exp-entropy rank
 // p = l/(sum l + 1e-7), rank = exp(-sum p ln(p + 1e-7))  (slime/kernels/warp_ca.cu:107-144).
-constexpr int JACOBI_THREADS = 256;
-// pair `i` of round `r` of the 64-player round-robin tournament: 32 disjoint index pairs per round, 63 rounds
-__device__ __forceinline__ void jacobi_pair(int r, int i, int& p, int& q) {
-    if (i == 0) { p = 63; q = r; }
-    else { p = (r + i) % 63; q = (r + 63 - i) % 63; }
-}
-__device__ __forceinline__ double jacobi_block_sum(double v, double* red) {
+//
+// Householder reduction to tridiagonal form (Golub & Van Loan, Matrix Computations, 8.3.1), then every eigenvalue by
+// multisection on Sturm counts (Wilkinson, The Algebraic Eigenvalue Problem, 5.37-5.39), all in fp64: absolute errors of a
+// few 1e-15 of the trace from the first and 2e-14 from the second, where the entropy's sensitivity asks for 1e-9.
+// It replaces a cyclic Jacobi iteration of 7 sweeps x 63 rounds, whose 440 rounds of three barriers took 610 us however
+// few matrices there were, and 2.36 ms for 1024 of them; here 62 steps of two barriers and 18 of one.
+//   The matrix lives in registers, row r = lane + 32 (warp & 1) and 16 columns per thread, so a step's matrix-vector
+// product and rank-2 update touch shared memory only for the vectors, which every warp keeps a copy of.
+constexpr int RANK_THREADS = 256;
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    return ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+    return v;
 }
-__global__ void __launch_bounds__(JACOBI_THREADS)
-k_jacobi_rank(const double* __restrict__ gram_part, int splits, float* __restrict__ head_rank) {
-    __shared__ double A[64 * JSTRIDE];
-    __shared__ double red[8];
-    __shared__ double2 cs[32];          // (cos, sin) of the round's 32 rotations
-    const int m = blockIdx.x, tid = threadIdx.x;
-    const double* src = gram_part + (size_t)m * splits * (HD * HD);
-    double fro2 = 0.0;
-    for (int i = tid; i < HD * HD; i += JACOBI_THREADS) {
-        double s = 0.0;
-        for (int k = 0; k < splits; ++k) s += src[(size_t)k * (HD * HD) + i];
-        A[(i >> 6) * JSTRIDE + (i & 63)] = s;
-        fro2 += s * s;
-    }
-    fro2 = jacobi_block_sum(fro2, red);
-
-    int extra = 0;
-    for (int sweep = 0; sweep < 30; ++sweep) {
-        double off2 = 0.0;
-        for (int i = tid; i < HD * HD; i += JACOBI_THREADS) {
-            const int r = i >> 6, c = i & 63;
-            if (r != c) { const double v = A[r * JSTRIDE + c]; off2 += v * v; }
-        }
-        off2 = jacobi_block_sum(off2, red);          // the same value in every thread: the exit below is uniform
-        if (off2 <= 1e-12 * fro2) { if (extra) break; extra = 1; }
-        for (int round = 0; round < 63; ++round) {
-            // (p, q) of a pair is used as the tournament hands it out, not ordered: a warp's values of p, and of q, are
-            // then consecutive indices (mod 63), which land in distinct banks; the matrix keeps both triangles, so
-            // A[p][q] is there whichever of the two is larger, and the rotation zeroes it either way
-            if (tid < 32) {
-                int p, q;
-                jacobi_pair(round, tid, p, q);
-                const double apq = A[p * JSTRIDE + q];
-                double c = 1.0, sn = 0.0;
-                if (apq != 0.0) {
-                    // The tangent of the rotation angle only decides how much of A[p][q] the rotation removes (all of
-                    // it, to fp32 accuracy here: three fp64 divisions and square roots on one warp were the longest
-                    // serial stretch of a round); what has to be exact is that the rotation is orthogonal, and
-                    // c = 1 / sqrt(1 + t^2), s = t c in fp64 make it so for whatever t.
-                    const float tau = (float)(A[q * JSTRIDE + q] - A[p * JSTRIDE + p]) / (2.f * (float)apq);
-                    const float tf = (tau >= 0.f ? 1.f : -1.f) / (fabsf(tau) + sqrtf(1.f + tau * tau));
-                    const double t = isfinite(tf) ? (double)tf : 0.0;
-                    c = rsqrt(1.0 + t * t);
-                    sn = t * c;
-                }
-                cs[tid] = make_double2(c, sn);
-            }
-            __syncthreads();
-            // The round's 32 rotations touch disjoint index pairs, so A'' = J^T A J falls apart into 32 x 32 independent
-            // 2 x 2 blocks: rows (p, q) of one pair against columns (p', q') of another.  A thread takes 4 blocks:
-            // columns first, then rows, exactly the arithmetic of rotating all columns and then all rows, but every
-            // element is read and written once per round instead of twice, with one barrier fewer.
-            {
-                int p, q;
-                // a warp holds the 32 row pairs of one column pair: its 8-byte accesses go to (almost) consecutive rows
-                // of one column, i.e. distinct banks (the row stride is odd)
-                jacobi_pair(round, tid & 31, p, q);
-                const double2 rc = cs[tid & 31];
+__global__ void __launch_bounds__(RANK_THREADS)
+k_gram_rank(const double* __restrict__ gram_part, int splits, float* __restrict__ head_rank) {
+    __shared__ __align__(16) double xrow[2][HD];          // row of the matrix that the next step eliminates
+    __shared__ __align__(16) double vv[8][HD], ww[8][HD]; // per warp: the step's v and w
+    __shared__ double part[4][HD];
+    __shared__ __align__(16) double2 tri[HD];             // {d[i], e[i-1]^2} of the tridiagonal matrix over its trace
+    __shared__ double dd[HD], ee[HD];
+    __shared__ int cnt[RANK_THREADS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r = lane + 32 * (warp & 1), c0 = (warp >> 1) * 16;
+    double a[16];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int cp = (tid >> 5) * 4 + j;
-                    int p2, q2;
-                    jacobi_pair(round, cp, p2, q2);
-                    const double2 cc = cs[cp];
-                    const double a_pp = A[p * JSTRIDE + p2], a_pq = A[p * JSTRIDE + q2];
-                    const double a_qp = A[q * JSTRIDE + p2], a_qq = A[q * JSTRIDE + q2];
-                    const double b_pp = cc.x * a_pp - cc.y * a_pq, b_pq = cc.y * a_pp + cc.x * a_pq;      // columns p', q'
-                    const double b_qp = cc.x * a_qp - cc.y * a_qq, b_qq = cc.y * a_qp + cc.x * a_qq;
-                    A[p * JSTRIDE + p2] = rc.x * b_pp - rc.y * b_qp;                                        // rows p, q
-                    A[p * JSTRIDE + q2] = rc.x * b_pq - rc.y * b_qq;
-                    A[q * JSTRIDE + p2] = rc.y * b_pp + rc.x * b_qp;
-                    A[q * JSTRIDE + q2] = rc.y * b_pq + rc.x * b_qq;
-                }
-            }
-            __syncthreads();
-        }
+    for (int j = 0; j < 16; ++j) a[j] = 0.0;
+    {
+        // the matrix is symmetric: this thread's 16 values are read down a column, coalesced over the lanes
+        const double* src = gram_part + (size_t)blockIdx.x * splits * (HD * HD) + c0 * HD + r;
+        for (int k = 0; k < splits; ++k, src += HD * HD)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) a[j] += __ldcs(src + j * HD);
     }
+    if (r == 0) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) xrow[0][c0 + j] = a[j];
+    }
+    __syncthreads();
+    double* v = vv[warp];
+    double* w = ww[warp];
+    for (int k = 0; k < HD - 2; ++k) {
+        const double* x = xrow[k & 1];
+        double x0 = lane > k ? x[lane] : 0.0, x1 = lane + 32 > k ? x[lane + 32] : 0.0;
+        const double head = x[k + 1], diag = x[k];
+        const double tail = warp_sum((lane == k + 1 ? 0.0 : x0 * x0) + (lane + 32 == k + 1 ? 0.0 : x1 * x1));
+        double alpha = head, beta = 0.0;                   // tail = 0: nothing to eliminate
+        if (tail != 0.0) {
+            const double norm2 = fma(head, head, tail);
+            alpha = head > 0.0 ? -sqrt(norm2) : sqrt(norm2);
+            beta = 1.0 / fma(-head, alpha, norm2);
+        }
+        if (tid == 0) { dd[k] = diag; ee[k] = alpha; }
+        if (lane == k + 1) x0 -= alpha;
+        if (lane + 32 == k + 1) x1 -= alpha;
+        if (tail == 0.0) x0 = x1 = 0.0;
+        v[lane] = x0; v[lane + 32] = x1;
+        __syncwarp();
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+            const double2 vc = *reinterpret_cast<const double2*>(v + c0 + j);
+            s0 = fma(a[j], vc.x, s0);
+            s1 = fma(a[j + 1], vc.y, s1);
+        }
+        part[warp >> 1][r] = s0 + s1;
+        __syncthreads();
+        const double p0 = beta * ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]));
+        const double p1 = beta * ((part[0][lane + 32] + part[1][lane + 32]) + (part[2][lane + 32] + part[3][lane + 32]));
+        const double half = 0.5 * beta * warp_sum(fma(p0, x0, p1 * x1));
+        w[lane] = fma(-half, x0, p0); w[lane + 32] = fma(-half, x1, p1);
+        __syncwarp();
+        const double vr = v[r], wr = w[r];
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+            const double2 vc = *reinterpret_cast<const double2*>(v + c0 + j), wc = *reinterpret_cast<const double2*>(w + c0 + j);
+            a[j] = fma(-vr, wc.x, fma(-wr, vc.x, a[j]));
+            a[j + 1] = fma(-vr, wc.y, fma(-wr, vc.y, a[j + 1]));
+        }
+        if (r == k + 1) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) xrow[(k + 1) & 1][c0 + j] = a[j];
+        }
+        if (k == HD - 3 && r == HD - 1 && warp >> 1 == 3) dd[HD - 1] = a[15];
+        __syncthreads();
+    }
+    if (tid == 0) { dd[HD - 2] = xrow[0][HD - 2]; ee[HD - 2] = xrow[0][HD - 1]; }
+    __syncthreads();
+    // over the trace: the eigenvalues of the (positive semidefinite) matrix then lie in [0, 1]
+    const double trace = warp_sum(dd[lane] + dd[lane + 32]);
+    const double inv = 1.0 / trace;
+    if (tid < HD) {
+        const double e = tid > 0 ? ee[tid - 1] * inv : 0.0;
+        tri[tid] = make_double2(dd[tid] * inv, e * e);
+    }
+    __syncthreads();
+    if (!(trace > 0.0) || !isfinite(trace) || !isfinite(inv)) {      // no spread to measure: one direction
+        if (tid == 0) head_rank[blockIdx.x] = 1.f;
+        return;
+    }
+    // Eigenvalues below x: sign changes of the leading minors p(i) = (d(i) - x) p(i-1) - e(i-1)^2 p(i-2).  The two last are
+    // brought back to order 1 by a power of two every four steps; a minor that is exactly zero is taken as slightly of the
+    // other sign (a perturbation of d(i) by 2^-60).
+    auto below = [&](double x) {
+        double p2 = 0.0, p1 = 1.0;
+        int n = 0;
+#pragma unroll 1
+        for (int i = 0; i < HD; i += 4) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double2 t = tri[i + j];
+                double p = fma(t.x - x, p1, -(t.y * p2));
+                if (p == 0.0) p = p1 * -8.673617379884035e-19;
+                n += (__double2hiint(p) ^ __double2hiint(p1)) < 0;
+                p2 = p1; p1 = p;
+            }
+            const int e = max((__double2hiint(p1) >> 20) & 0x7ff, (__double2hiint(p2) >> 20) & 0x7ff);
+            const double sc = __hiloint2double(min(max(2046 - e, 1), 2046) << 20, 0);
+            p1 *= sc; p2 *= sc;
+        }
+        return n;
+    };
+    // all threads once, on a uniform grid: each eigenvalue within 1 / 256 ...
+    const double step0 = 1.0 / RANK_THREADS;
+    cnt[tid] = below((tid + 1) * step0);
+    __syncthreads();
+    // ... then four threads per eigenvalue, 16 rounds of five parts each (5^16 = 2^37)
+    const int ev = tid >> 2, q = tid & 3;
+    int lo_i = 0;                                          // first grid point with more than ev eigenvalues below it
+#pragma unroll
+    for (int b = RANK_THREADS / 2; b > 0; b >>= 1)
+        if (cnt[lo_i + b - 1] <= ev) lo_i += b;
+    double lo = lo_i * step0, width = step0;
+    for (int round = 0; round < 16; ++round) {
+        width *= 0.2;
+        const bool above = below(fma(q + 1.0, width, lo)) <= ev;
+        const unsigned m = (__ballot_sync(0xffffffffu, above) >> (lane & ~3)) & 15u;
+        lo = fma((double)__popc(m), width, lo);
+    }
+    if (q == 0) dd[ev] = lo * trace;
+    __syncthreads();
     if (tid >= 32) return;
-    const int lane = tid;
-    double l0 = fmax(A[lane * JSTRIDE + lane], 0.0), l1 = fmax(A[(lane + 32) * JSTRIDE + lane + 32], 0.0);
-    double sum = l0 + l1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const double p0 = l0 / (sum + 1e-7), p1 = l1 / (sum + 1e-7);
-    double ent = -(p0 * log(p0 + 1e-7) + p1 * log(p1 + 1e-7));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ent += __shfl_xor_sync(0xffffffffu, ent, o);
-    if (lane == 0) head_rank[m] = (float)exp(ent);
+    const double l0 = dd[lane], l1 = dd[lane + 32];
+    const double sum = warp_sum(l0 + l1);
+    const double e0 = l0 / (sum + 1e-7), e1 = l1 / (sum + 1e-7);
+    const double ent = warp_sum(-(e0 * log(e0 + 1e-7) + e1 * log(e1 + 1e-7)));
+    if (lane == 0) head_rank[blockIdx.x] = (float)exp(ent);
 }
 
 // Raw moments of (a, b) = (V' of step n-1, V' of step n) for one grid, fp64:
@@ -342,20 +382,21 @@ k_pearson(const T* __restrict__ va, const T* __restrict__ vb, size_t per_grid, d
 }
 
 // out[b] = {rank, coherence, fitness, hunger}: fitness = rank x coherence (slime/kernels/warp_ca.cu:219),
-// hunger = 1 - coherence (slime/kernels/warp_ca.cu:238).
-__global__ void k_fitness_final(const float* __restrict__ head_rank, const double* __restrict__ part, int splits,
-                                double n, float* __restrict__ out, int B) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
+// hunger = 1 - coherence (slime/kernels/warp_ca.cu:238).  A warp per grid.
+__global__ void __launch_bounds__(32)
+k_fitness_final(const float* __restrict__ head_rank, const double* __restrict__ part, int splits, double n, float* __restrict__ out) {
+    const int b = blockIdx.x, lane = threadIdx.x;
     double s[5] = {0, 0, 0, 0, 0};
-    for (int k = 0; k < splits; ++k)
+    for (int k = lane; k < splits; k += 32)
+#pragma unroll
         for (int j = 0; j < 5; ++j) s[j] += part[((size_t)b * splits + k) * 5 + j];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) s[j] = warp_sum(s[j]);
+    const double rk = warp_sum(lane < NH ? (double)head_rank[b * NH + lane] : 0.0) / NH;
+    if (lane != 0) return;
     const double cov = s[4] - s[0] * s[1] / n;
     const double va = s[2] - s[0] * s[0] / n, vb = s[3] - s[1] * s[1] / n;
     const double coh = cov / sqrt(va * vb);
-    double rk = 0.0;
-    for (int h = 0; h < NH; ++h) rk += (double)head_rank[b * NH + h];
-    rk /= NH;
     out[b * 4 + 0] = (float)rk;
     out[b * 4 + 1] = (float)coh;
     out[b * 4 + 2] = (float)(rk * coh);

@@ -55,7 +55,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
             else if (t - t0 > limit_ns) break;
         }
     }
-    atomicCAS(status, 0, code);
+    // the word, and (its address behind the word) the host's mirror of it: a caller learns of it without a copy per call
+    if (atomicCAS(status, 0, code) == 0) {
+        *reinterpret_cast<volatile int*>(*reinterpret_cast<int* const*>(status + 2)) = code;
+        __threadfence_system();
+    }
     return false;
 }
 

@@ -3,6 +3,7 @@
 // thread with dynamic parallelism is sequenced here from the host on one stream.
 #include "../../include/slime_ca.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -59,15 +60,16 @@ struct slime_ca {
     bool evolved = false;           // `parent` holds the result of a population step
     // fitness scratch
     double* gram_part = nullptr;
-    int gram_splits = 0;
+    int gram_splits = 0, gram_chunk = 0;
     CUtensorMap gram_map[2];        // bf16 path: tensor maps over the two V' buffers for the tensor-core Gram
     float* head_rank = nullptr;
     double* pearson_part = nullptr;
     int pearson_splits = 0;
     float* fit_dev = nullptr;
-    int* dev_status = nullptr;      // status word kernels with bounded waits report into
-    int* host_status = nullptr;     // pinned host mirror of it: copied back behind every batch of steps, read without
+    int* dev_status = nullptr;      // status word kernels with bounded waits report into, and the address of its host mirror
+    int* host_status = nullptr;     // pinned host mirror of it, written by the kernel that gives up, read without
                                     // synchronising at the start of the next call
+    float* host_fit = nullptr;      // pinned, behind it: [B][4] of the last fitness call
     // row-stripe ring (stripe mode): NCCL communicator over the ranks that hold the other stripes
     void* comm = nullptr;
     bool own_comm = false;
@@ -116,9 +118,10 @@ int dev_alloc(slime_ca* h, T** p, size_t n) {
     return SLIME_CA_OK;
 }
 
-int grid_for(size_t n) {
-    size_t b = (n + 255) / 256;
-    return (int)(b > 148 * 16 ? 148 * 16 : (b ? b : 1));
+// (blocks, grids) of 256 threads for kernels that go over all cells, eight threads each
+dim3 cell_blocks(const slime_ca* h) {
+    const size_t per_grid = ((size_t)h->g.H * h->g.W * 8 + 255) / 256, most = (size_t)(h->n_sms * 16 + h->g.B - 1) / h->g.B;
+    return dim3((unsigned)std::min(per_grid, most), h->g.B);
 }
 
 bool is_bf16(const slime_ca* h) { return h->cfg.dtype == SLIME_CA_BF16; }
@@ -160,7 +163,9 @@ int channel_sums(slime_ca* h, int mode, cudaStream_t st) {
 }
 
 // X <- lifted images (device pointers), with the masses of the lifted state
-int lift(slime_ca* h, const float* img, int ih, int iw, const float* L, cudaStream_t st) {
+int lift(slime_ca* h, const float* img, int ih, int iw, const float* host_L, cudaStream_t st) {
+    LiftVector L;
+    memcpy(L.v, host_L, sizeof L.v);
     return with_channel_sums(h, 1, st, [&](dim3 grid, const ChunkSums& cs) {
         if (is_bf16(h)) k_lift<__nv_bfloat16><<<grid, 256, 0, st>>>(img, ih, iw, L, (__nv_bfloat16*)h->X, cs, h->g);
         else k_lift<float><<<grid, 256, 0, st>>>(img, ih, iw, L, (float*)h->X, cs, h->g);
@@ -276,10 +281,9 @@ int ring_ready(slime_ca* h) {
 
 const char* const AFTER_EDEVICE = "); the state is no longer defined: load it again before further steps";
 
-// After a synchronisation: read the device status word itself.
+// After a synchronisation of the stream: whatever its kernels had to report is in the mirror.
 int check_status_word(slime_ca* h) {
-    int s = 0;
-    CK(h, cudaMemcpy(&s, h->dev_status, sizeof(int), cudaMemcpyDeviceToHost));
+    const int s = *reinterpret_cast<volatile int*>(h->host_status);
     if (s != 0) {
         cudaMemset(h->dev_status, 0, sizeof(int));
         *reinterpret_cast<volatile int*>(h->host_status) = 0;
@@ -288,20 +292,14 @@ int check_status_word(slime_ca* h) {
     return SLIME_CA_OK;
 }
 
-// Without synchronising: the mirror that the last batch of steps copied back, if that copy has run by now.  Lets a
-// caller that never leaves the device (set_state_device / step / get_state_device) learn of a failed wait at its
-// next call.
+// Without synchronising: what the kernels have reported by now.  Lets a caller that never leaves the device
+// (set_state_device / step / get_state_device) learn of a failed wait at its next call.
 int poll_status(slime_ca* h, cudaStream_t st) {
     const int s = *reinterpret_cast<volatile int*>(h->host_status);
     if (s == 0) return SLIME_CA_OK;
     *reinterpret_cast<volatile int*>(h->host_status) = 0;
     cudaMemsetAsync(h->dev_status, 0, sizeof(int), st);
     return fail(h, SLIME_CA_EDEVICE, "a kernel of an earlier call gave up on a bounded wait (status word " + std::to_string(s) + AFTER_EDEVICE);
-}
-
-int publish_status(slime_ca* h, cudaStream_t st) {
-    CK(h, cudaMemcpyAsync(h->host_status, h->dev_status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    return SLIME_CA_OK;
 }
 
 }  // namespace
@@ -364,18 +362,25 @@ int slime_ca_create(const slime_ca_config* cfg, slime_ca** out) {
         const size_t vn = (size_t)g.B * NH * g.H * g.W * HD;
         for (int i = 0; i < 2; ++i) { if ((rc = dev_alloc(h, &p, vn * h->esz))) return rc; h->vprime[i] = p; }
         const size_t cells = (size_t)g.H * g.W;
-        h->gram_splits = (int)((cells + GRAM_CHUNK - 1) / GRAM_CHUNK);
-        if (h->gram_splits > 64) h->gram_splits = 64;   // k_gram then covers GRAM_CHUNK * 64 cells at most
-        if ((size_t)h->gram_splits * GRAM_CHUNK < cells)
-            return fail(h, SLIME_CA_EINVAL, "keep_vprime supports grids of at most 131072 cells");
+        if (cells > (size_t)GRAM_CHUNK * 64) return fail(h, SLIME_CA_EINVAL, "keep_vprime supports grids of at most 131072 cells");
+        // Gram partials: chunks of GRAM_CHUNK cells, or shorter ones (down to 512) where the planes alone give the SMs less
+        // than three blocks each
+        int splits = (3 * prop.multiProcessorCount + g.B * NH - 1) / (g.B * NH);
+        splits = std::min(splits, (int)((cells + 511) / 512));
+        splits = std::max(splits, (int)((cells + GRAM_CHUNK - 1) / GRAM_CHUNK));
+        h->gram_chunk = (int)((cells + splits - 1) / splits + gtc::TILE - 1) / gtc::TILE * gtc::TILE;
+        h->gram_splits = (int)((cells + h->gram_chunk - 1) / h->gram_chunk);
         if ((rc = dev_alloc(h, &h->gram_part, (size_t)g.B * NH * h->gram_splits * HD * HD))) return rc;
         if (is_bf16(h))
             for (int i = 0; i < 2; ++i)
                 if (gram_tc_map(&h->gram_map[i], h->vprime[i], g.B * NH, (int)cells) != 0)
                     return fail(h, SLIME_CA_ECUDA, "tensor-map set-up of the Gram kernel failed");
         if ((rc = dev_alloc(h, &h->head_rank, (size_t)g.B * NH))) return rc;
-        h->pearson_splits = (int)((cells * HC + 262143) / 262144);
-        if (h->pearson_splits > 64) h->pearson_splits = 64;
+        // moments: 262144 values a block at most 64 times, or down to 16384 where that leaves the SMs less than four blocks each
+        const size_t values = cells * HC;
+        size_t parts = (4 * prop.multiProcessorCount + g.B - 1) / g.B;
+        parts = std::max(std::min(parts, (values + 16383) / 16384), std::min<size_t>((values + 262143) / 262144, 64));
+        h->pearson_splits = (int)parts;
         if ((rc = dev_alloc(h, &h->pearson_part, (size_t)g.B * h->pearson_splits * 5))) return rc;
         if ((rc = dev_alloc(h, &h->fit_dev, (size_t)g.B * 4))) return rc;
     }
@@ -389,10 +394,16 @@ int slime_ca_create(const slime_ca_config* cfg, slime_ca** out) {
     if ((rc = dev_alloc(h, &h->tickets, (size_t)g.B * 2))) return rc;
     h->load_tickets = h->tickets + g.B;
     CK(h, cudaMemset(h->tickets, 0, (size_t)g.B * 2 * sizeof(int)));
-    if ((rc = dev_alloc(h, &h->dev_status, 1))) return rc;
-    CK(h, cudaMemset(h->dev_status, 0, sizeof(int)));
-    CK(h, cudaHostAlloc((void**)&h->host_status, sizeof(int), cudaHostAllocDefault));
+    // one pinned block: the status mirror (which kernels write), then what fitness copies back
+    CK(h, cudaHostAlloc((void**)&h->host_status, 64 + (cfg->keep_vprime ? (size_t)g.B * 4 * sizeof(float) : 0), cudaHostAllocMapped));
     *h->host_status = 0;
+    h->host_fit = reinterpret_cast<float*>(h->host_status) + 16;
+    if ((rc = dev_alloc(h, &h->dev_status, 4))) return rc;
+    {
+        struct { int word, pad; void* mirror; } st{0, 0, nullptr};       // as ptx::mbar_wait takes it
+        CK(h, cudaHostGetDevicePointer(&st.mirror, h->host_status, 0));
+        CK(h, cudaMemcpy(h->dev_status, &st, sizeof st, cudaMemcpyHostToDevice));
+    }
     const size_t sets = cfg->n_weight_sets;
     if ((rc = dev_alloc(h, &h->prm, sets * NH * PRM))) return rc;
     if ((rc = dev_alloc(h, &h->master, sets * MW_STRIDE))) return rc;
@@ -496,8 +507,7 @@ int slime_ca_get_state_device(slime_ca* h, void* dev_state, int dtype, void* str
     if (rcs) return rcs;
     const Geom& g = h->g;
     const bool vec = aligned16(dev_state);
-    size_t per_grid = ((size_t)g.H * g.W * 8 + 255) / 256, most = (size_t)(h->n_sms * 16 + g.B - 1) / g.B;
-    const dim3 grid((unsigned)(per_grid < most ? per_grid : most), g.B);
+    const dim3 grid = cell_blocks(h);
     __nv_bfloat16* d16 = (__nv_bfloat16*)dev_state;
     float* d32 = (float*)dev_state;
     if (is_bf16(h)) {
@@ -563,7 +573,7 @@ int slime_ca_step_partial(slime_ca* h, void* stream) {
     rc = step_kernels(h, emit, (cudaStream_t)stream);
     if (rc) return rc;
     ++h->steps_done;
-    return publish_status(h, (cudaStream_t)stream);
+    return SLIME_CA_OK;
 }
 
 int slime_ca_step_finish(slime_ca* h, void* stream) {
@@ -590,7 +600,7 @@ int slime_ca_step(slime_ca* h, int n_steps, void* stream) {
         if (rc) return rc;
         ++h->steps_done;
     }
-    return n_steps > 0 ? publish_status(h, st) : SLIME_CA_OK;
+    return SLIME_CA_OK;
 }
 
 int slime_ca_step_timed(slime_ca* h, int n_steps, void* stream, float* ms) {
@@ -654,22 +664,25 @@ int slime_ca_fitness(slime_ca* h, float* rank, float* coherence, float* fitness,
     const void* vb = h->vprime[h->vp_last];
     const size_t per_grid = (size_t)cells * HC;
     if (is_bf16(h)) {
-        k_gram_tc<<<g.B * NH, 128, gtc::SMEM, st>>>(h->gram_map[h->vp_last], cells, h->gram_splits, h->gram_part, h->dev_status);
+        // a CTA per plane, two chunks and more each where there are too few planes to fill the GPU
+        const int per_plane = std::max(1, std::min(h->gram_splits / 2, 2 * h->n_sms / (g.B * NH)));
+        k_gram_tc<<<dim3(g.B * NH, per_plane), 128, gtc::SMEM, st>>>(h->gram_map[h->vp_last], cells, h->gram_chunk, h->gram_splits, h->gram_part,
+                                                                     h->dev_status);
         LAUNCHED(h);
         k_pearson<__nv_bfloat16><<<dim3(h->pearson_splits, g.B), 256, 0, st>>>((const __nv_bfloat16*)va, (const __nv_bfloat16*)vb, per_grid, h->pearson_part);
         LAUNCHED(h);
     } else {
-        k_gram<float><<<dim3(h->gram_splits, NH, g.B), GRAM_THREADS, 0, st>>>((const float*)vb, cells, h->gram_part);
+        k_gram<float><<<dim3(h->gram_splits, NH, g.B), GRAM_THREADS, 0, st>>>((const float*)vb, cells, h->gram_chunk, h->gram_part);
         LAUNCHED(h);
         k_pearson<float><<<dim3(h->pearson_splits, g.B), 256, 0, st>>>((const float*)va, (const float*)vb, per_grid, h->pearson_part);
         LAUNCHED(h);
     }
-    k_jacobi_rank<<<g.B * NH, JACOBI_THREADS, 0, st>>>(h->gram_part, h->gram_splits, h->head_rank);
+    k_gram_rank<<<g.B * NH, RANK_THREADS, 0, st>>>(h->gram_part, h->gram_splits, h->head_rank);
     LAUNCHED(h);
-    k_fitness_final<<<(g.B + 127) / 128, 128, 0, st>>>(h->head_rank, h->pearson_part, h->pearson_splits, (double)per_grid, h->fit_dev, g.B);
+    k_fitness_final<<<g.B, 32, 0, st>>>(h->head_rank, h->pearson_part, h->pearson_splits, (double)per_grid, h->fit_dev);
     LAUNCHED(h);
-    std::vector<float> out((size_t)g.B * 4);
-    CK(h, cudaMemcpyAsync(out.data(), h->fit_dev, out.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
+    const float* out = h->host_fit;
+    CK(h, cudaMemcpyAsync(h->host_fit, h->fit_dev, (size_t)g.B * 4 * sizeof(float), cudaMemcpyDeviceToHost, st));
     CK(h, cudaStreamSynchronize(st));
     for (int b = 0; b < g.B; ++b) {
         if (rank) rank[b] = out[b * 4 + 0];
@@ -737,10 +750,8 @@ int slime_ca_lift_images(slime_ca* h, const float* host_img, int img_h, int img_
     const Geom& g = h->g;
     const size_t n_img = (size_t)g.B * img_h * img_w;
     float* d_img = (float*)h->E;
-    float* d_L = (float*)h->V;
     CK(h, cudaMemcpyAsync(d_img, host_img, n_img * sizeof(float), cudaMemcpyHostToDevice, st));
-    CK(h, cudaMemcpyAsync(d_L, host_L, NC * sizeof(float), cudaMemcpyHostToDevice, st));
-    int rc = lift(h, d_img, img_h, img_w, d_L, st);
+    int rc = lift(h, d_img, img_h, img_w, host_L, st);
     if (rc) return rc;
     CK(h, cudaStreamSynchronize(st));
     h->state_set = true;
@@ -784,9 +795,7 @@ int slime_ca_lift_field_device(slime_ca* h, const float* dev_field, const float*
     if (!dev_field || !host_L) return fail(h, SLIME_CA_EINVAL, "null field or lift vector");
     CK(h, cudaSetDevice(h->cfg.device));
     cudaStream_t st = (cudaStream_t)stream;
-    float* d_L = (float*)h->V;
-    CK(h, cudaMemcpyAsync(d_L, host_L, NC * sizeof(float), cudaMemcpyHostToDevice, st));
-    int rc = lift(h, dev_field, h->g.H, h->g.W, d_L, st);
+    int rc = lift(h, dev_field, h->g.H, h->g.W, host_L, st);
     if (rc) return rc;
     CK(h, cudaStreamSynchronize(st));
     h->state_set = true;
@@ -801,7 +810,7 @@ int slime_ca_field_from_state_device(slime_ca* h, float* dev_field, void* stream
     CK(h, cudaSetDevice(h->cfg.device));
     cudaStream_t st = (cudaStream_t)stream;
     const Geom& g = h->g;
-    const int blocks = grid_for((size_t)g.B * g.H * g.W * 8);
+    const dim3 blocks = cell_blocks(h);
     if (is_bf16(h)) k_channel_mean<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, dev_field, g);
     else k_channel_mean<float><<<blocks, 256, 0, st>>>((const float*)h->X, h->scale, dev_field, g);
     LAUNCHED(h);
@@ -860,7 +869,7 @@ int slime_ca_evolution_record(slime_ca* h, int grid_index, int generation, doubl
     const float* field = dev_field;
     if (!field) {
         float* scratch = (float*)h->E;
-        const int blocks = grid_for((size_t)g.B * g.H * g.W * 8);
+        const dim3 blocks = cell_blocks(h);
         if (is_bf16(h)) k_channel_mean<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, scratch, g);
         else k_channel_mean<float><<<blocks, 256, 0, st>>>((const float*)h->X, h->scale, scratch, g);
         LAUNCHED(h);
@@ -1074,7 +1083,7 @@ int slime_ca_step_ring(slime_ca* h, int n_steps, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if ((rc = poll_status(h, st))) return rc;
     if ((rc = ring_steps(h, n_steps, st, nullptr))) return rc;
-    return n_steps > 0 ? publish_status(h, st) : SLIME_CA_OK;
+    return SLIME_CA_OK;
 }
 
 int slime_ca_step_ring_timed(slime_ca* h, int n_steps, void* stream, float* ms) {
@@ -1141,7 +1150,7 @@ int slime_ca_selftest_bounded_wait(slime_ca* h, unsigned long long limit_ns, voi
     cudaStream_t st = (cudaStream_t)stream;
     k_wait_selftest<<<1, 32, 0, st>>>(h->dev_status, limit_ns, 901);
     LAUNCHED(h);
-    return publish_status(h, st);
+    return SLIME_CA_OK;
 }
 
 int slime_ca_occupancy(slime_ca* h, float* occupancy) {

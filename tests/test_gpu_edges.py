@@ -1,0 +1,123 @@
+"""The sizes at which the kernels' divisions of the work change, against the CPU oracle: tiles that do not go round over
+the SMs, grids on either side of the limit of the fused channel sums, populations too small to fill the GPU with one
+Gram block per plane, and caller pointers that allow no wide loads."""
+import numpy as np
+import pytest
+
+from slime_b200 import inputs
+from tests.helpers import bf16_round, channel_mass, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    import torch
+    assert torch.cuda.is_available(), "these tests need a CUDA device"
+    from slime_b200 import capi, devmem
+    capi.lib()
+    return capi, devmem
+
+
+# (batch, height, width), weight sets: one item in all; tiles left over that share an item boundary; one whole round of tiles
+# and one tile more; 512 and 544 tile sums a grid (the limit of the fused sums); ragged in both directions
+SHAPES = [((1, 1, 5), 1), ((1, 8, 16), 1), ((3, 33, 47), 3), ((149, 8, 16), 1), ((1, 512, 128), 1), ((1, 544, 128), 1), ((2, 75, 53), 2)]
+
+
+@pytest.mark.parametrize("dtype_name", ["f32", "bf16"])
+@pytest.mark.parametrize("shape,n_sets", SHAPES)
+def test_work_divisions(gpu, shape, n_sets, dtype_name):
+    from oracle import ca_oracle
+    capi, devmem = gpu
+    B, H, W = shape
+    f32 = dtype_name == "f32"
+    X0 = inputs.make_state(B, H, W, seed=17, scale=0.45 * H * W)
+    w = inputs.make_weight_sets(n_sets, seed=17, bounded=True)
+    R1, _, rlast = ca_oracle.ca_steps(X0, w, 2, literal=False, want_vprime=True)
+    with capi.Handle(B, H, W, n_weight_sets=n_sets, dtype=capi.F32 if f32 else capi.BF16, keep_vprime=True) as h:
+        h.set_weights(w)
+        h.set_state(X0)
+        h.step(2)
+        X1, vlast = h.get_state(), devmem.vprime(h, capi.BUF_VPRIME_LAST)
+    # fp32: twice what the split products and fp32 sums leave on these shapes
+    assert rel_l2(X1, R1) < (1e-6 if f32 else 2e-2)
+    assert rel_l2(vlast, rlast) < (2e-6 if f32 else 2e-2)
+    m0 = channel_mass(X0 if f32 else bf16_round(X0))
+    assert np.max(np.abs(channel_mass(X1) - m0) / np.abs(m0)) < 1e-6
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 3), (1, 16, 16), (2, 40, 56), (60, 16, 24)])
+def test_fitness_of_small_populations(gpu, shape):
+    """Few planes: Gram chunks and moment blocks are shorter, and a plane may have several blocks."""
+    from oracle import ca_oracle
+    capi, devmem = gpu
+    B, H, W = shape
+    X0 = inputs.make_state(B, H, W, seed=23, scale=0.45 * H * W)
+    w = inputs.make_weight_sets(1, seed=23, bounded=True)
+    _, rprev, rlast = ca_oracle.ca_steps(X0, w, 2, literal=False, want_vprime=True)
+    ref = ca_oracle.fitness(rprev, rlast)
+    for dtype, tol in ((capi.F32, 1e-4), (capi.BF16, 5e-2)):
+        with capi.Handle(B, H, W, dtype=dtype, keep_vprime=True) as h:
+            h.set_weights(w)
+            h.set_state(X0)
+            h.step(2)
+            fit = h.fitness()
+        np.testing.assert_allclose(fit["rank"], ref["rank"], atol=tol if dtype == capi.F32 else 0, rtol=0 if dtype == capi.F32 else tol)
+
+
+def test_rank_of_known_spectra(gpu):
+    """V' with a Gram matrix of known rank: 1 (all heads' values equal over a uniform state), and a spectrum spread over
+    twelve decades, where the entropy hangs on the small eigenvalues."""
+    import torch
+    capi, devmem = gpu
+    H = W = 16
+    rng = np.random.default_rng(3)
+    with capi.Handle(1, H, W, dtype=capi.F32, keep_vprime=True) as h:
+        h.set_weights(inputs.make_weight_sets(1, seed=3))
+        h.set_state(inputs.make_state(1, H, W, seed=3))
+        h.step(2)
+        cells = H * W
+        basis = np.linalg.qr(rng.standard_normal((64, 64)))[0]
+        planes = np.empty((8, cells, 64), np.float32)
+        for i in range(8):
+            sv = np.zeros(64) if i == 0 else 10.0 ** (-6.0 * np.arange(64) / 63 * (i / 7))
+            sv[0] = 1.0
+            planes[i] = (np.linalg.qr(rng.standard_normal((cells, 64)))[0] * sv) @ basis.T
+        ptr, _ = h.buffer(capi.BUF_VPRIME_LAST)
+        devmem.view(ptr, (8, cells, 64), torch.float32).copy_(torch.from_numpy(planes))
+        torch.cuda.synchronize()
+        got = h.fitness()["rank"][0]
+    ranks = []
+    for p in planes.astype(np.float64):
+        lam = np.clip(np.linalg.eigvalsh(p.T @ p), 0, None)
+        q = lam / (lam.sum() + 1e-7)
+        ranks.append(np.exp(-np.sum(q * np.log(q + 1e-7))))
+    np.testing.assert_allclose(got, np.mean(ranks), rtol=1e-6)
+
+
+@pytest.mark.parametrize("dtype_name", ["f32", "bf16"])
+def test_unaligned_device_pointers(gpu, dtype_name):
+    """State pointers one element past a 16-byte boundary: the same bits as with aligned ones."""
+    import torch
+    capi, _ = gpu
+    f32 = dtype_name == "f32"
+    dt, code = (torch.float32, capi.F32) if f32 else (torch.bfloat16, capi.BF16)
+    B, H, W = 2, 9, 21
+    n = B * H * W * 64
+    X0 = torch.from_numpy(inputs.make_state(B, H, W, seed=5, scale=0.45 * H * W)).to(dt).cuda().flatten()
+    w = inputs.make_weight_sets(1, seed=5, bounded=True)
+    outs = []
+    for off in (0, 1):
+        src, dst = torch.zeros(n + 8, dtype=dt, device="cuda"), torch.zeros(n + 8, dtype=dt, device="cuda")
+        src[off:off + n] = X0
+        es = src.element_size()
+        torch.cuda.synchronize()
+        with capi.Handle(B, H, W, dtype=code) as h:
+            h.set_weights(w)
+            h.set_state_device(src.data_ptr() + off * es, code)
+            h.step(1)
+            h.get_state_device(dst.data_ptr() + off * es, code)
+            torch.cuda.synchronize()
+        outs.append(dst[off:off + n].clone())
+        assert int((dst[off + n:] != 0).sum()) == 0
+    assert torch.equal(outs[0], outs[1])
