@@ -1,5 +1,5 @@
-// fp32 path of the CA step: fp32 storage of state and intermediates, exact expf and division, fp32 sums.  This is the
-// path held to 1e-5 relative L2 against the CPU oracle.  The same two-kernel split as the bf16 path (ca_bf16.cuh), and
+// fp32 path of the CA step: fp32 storage of state and intermediates, fp32 sums and fp32-accurate products, division and
+// exponentials.  This is the path held to 1e-5 relative L2 against the CPU oracle.  The same two-kernel split as the bf16 path (ca_bf16.cuh), and
 // like there the projections run on the 5th-generation tensor cores:
 //
 //   every fp32 operand is the exact sum of three bf16 values, x = hi + mid + lo (8 + 8 + 8 bits of mantissa, split3
@@ -10,7 +10,9 @@
 //   inside one K = 16 step, then the sum is truncated to fp32), so the products are issued smallest first and a sum
 //   stays on the tensor core for K = 64 (k1) or K = 32 (k2) at most - only the last two to four instructions then
 //   truncate at the sum's own magnitude - and longer sums are continued in registers, rounded to nearest.
-//   Against the fp64 oracle this is as accurate as the fp32 fused multiply-add loops it replaced.
+//   Against the fp64 oracle this is more accurate than the fp32 fused multiply-add loops, expf and divisions it replaced:
+//   relative L2 error of V' after one step of 128 x 128 grids 7.3e-8 (9.1e-8) at unit mass, 1.4e-7 (2.2e-7) and 1.1e-6
+//   (1.9e-6) with the state 7000 and 40000 times that; of the state after 16 steps 2.2e-7 (3.5e-7), after 64 2.2e-7 (2.6e-7).
 //
 //   k1_f32  reads the state with a 1-cell halo, applies the pending per-channel scale, forms for every head the
 //           3x3-convolved input (the stencil commutes with the linear perception projection), projects to U | I | V
@@ -334,7 +336,8 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                 float f[16];
                 if (is_e) {
                     // G = 2 ex2(-(s (U - mu))^2) - 1, E = ex2(clamp(G I log2 e)): the constants sit in the weights, whose
-                    // three parts hold the products to 24 bits, so each exponential's argument is rounded once
+                    // three parts hold the products to 24 bits, so each exponential's argument is rounded once (as expf of
+                    // a product it was rounded twice, which weighs more than ex2's own 1.45e-7)
                     uint32_t ru[16], ri[16];
                     ptx::tmem_ld16(t_lane + d0, ru);
                     ptx::tmem_ld16(t_lane + 64 + d0, ri);
@@ -429,9 +432,9 @@ struct V4 { ptx::f2 a, b; };
 __device__ __forceinline__ V4 v4(const float4& f) { V4 r; r.a = ptx::make_f2(f.x, f.y); r.b = ptx::make_f2(f.z, f.w); return r; }
 __device__ __forceinline__ V4 v4_add(const V4& x, const V4& y) { V4 r; r.a = ptx::add2(x.a, y.a); r.b = ptx::add2(x.b, y.b); return r; }
 __device__ __forceinline__ V4 v4_mul(const V4& x, const V4& y) { V4 r; r.a = ptx::mul2(x.a, y.a); r.b = ptx::mul2(x.b, y.b); return r; }
-// x / z to the last bit or nearly: the quotient by the approximate reciprocal and one residual correction (Markstein).  The
-// compiler's own division costs four times the instructions, and its subnormal branch is not needed: z lies within
-// 9 exp(+-80).
+// x / z by the approximate reciprocal, the quotient and one residual correction in fused multiply-adds (Markstein, IA-64 and
+// Elementary Functions, chapter 8).  z lies within 9 exp(+-80), so that neither step leaves the normal range.  Equal to the
+// correctly rounded quotient on 67 million random pairs over that range; two quotients at a time in packed fp32.
 __device__ __forceinline__ ptx::f2 div2(ptx::f2 x, ptx::f2 z) {
     float z0, z1;
     ptx::split_f2(z, z0, z1);
