@@ -117,6 +117,7 @@ struct Bf16Plan {
     K1StoreMaps st;       // store maps of k1 (whole tile, last two columns, last two rows, their corner)
     bool k1_aligned = false;
     int strips = 1, mt_per_grid = 1, nbmax = 8;    // k2: 32-column strips, macro tiles per grid, blocks per macro tile
+    int split_grid = 0;   // CTAs of k2_split_bf16, 0: the launch is large enough for k2_bf16
 };
 
 // ---- shared-memory maps (byte offsets from a 1024-aligned base) -------------------------------------------
@@ -793,6 +794,50 @@ static_assert(STAGE_BYTES % 1024 == 0 && A_VP % 1024 == 0 && WO % 1024 == 0 && X
 static_assert(SMEM <= 227 * 1024, "k2 (marching) shared memory");
 }  // namespace k2m
 
+// Set A's part of a block: R = V / box3(E) for its four V rows, marching down, by the thread of column col and dims 8q..8q+7.
+// h2, h1: horizontal sums of the two E rows above.  Of a priming block only the last two rows have all three E rows.
+__device__ __forceinline__ void k2_box_e(const uint8_t* es, uint8_t* vs, int col, int q, bool prime, V8& h2, V8& h1) {
+#pragma unroll
+    for (int j = 0; j < k2m::BR; ++j) {
+        const uint8_t* row = es + (j * k2m::EW + col) * 128 + q * 16;
+        const uint4 e0 = *reinterpret_cast<const uint4*>(row);
+        const uint4 e1 = *reinterpret_cast<const uint4*>(row + 128);
+        const uint4 e2 = *reinterpret_cast<const uint4*>(row + 256);
+        const V8 hs = v8_sum3(e0, e1, e2);
+        if (!prime || j >= 2) {
+            uint4* pv = reinterpret_cast<uint4*>(vs + (j * k2m::VW + col) * 128 + q * 16);
+            *pv = v8_pack(v8_mul(v8_unpack(*pv), v8_rcp(v8_add(v8_add(h2, h1), hs))));
+        }
+        h2 = h1; h1 = hs;
+    }
+}
+// Set B's part: V' = E * box3(R) for tile rows 4b .. 4b+3 -> A operand, and emit(row, V').  Tile row j is macro-tile row 4b+j:
+// its E came with the block before (j < 2, kept in registers) or is row j-2 of this block's E rows.
+template <typename F>
+__device__ __forceinline__ void k2_box_r(const uint8_t* es, const uint8_t* vs, uint8_t* a_vp, int col, int q, bool prime, V8& h2, V8& h1,
+                                         uint4& ekeep0, uint4& ekeep1, F emit) {
+    const uint8_t* ecol = es + (col + 2) * 128 + q * 16;      // this thread's column in the E rows
+#pragma unroll
+    for (int j = 0; j < k2m::BR; ++j) {
+        if (!prime || j >= 2) {
+            const uint8_t* row = vs + (j * k2m::VW + col) * 128 + q * 16;
+            const uint4 a0 = *reinterpret_cast<const uint4*>(row);
+            const uint4 a1 = *reinterpret_cast<const uint4*>(row + 128);
+            const uint4 a2 = *reinterpret_cast<const uint4*>(row + 256);
+            const V8 hs = v8_sum3(a0, a1, a2);
+            if (!prime) {
+                const V8 e = v8_unpack(j == 0 ? ekeep0 : j == 1 ? ekeep1 : *reinterpret_cast<const uint4*>(ecol + (j - 2) * k2m::EW * 128));
+                const uint4 out = v8_pack(v8_mul(e, v8_add(v8_add(h2, h1), hs)));
+                *reinterpret_cast<uint4*>(a_vp + swz(j * k2m::SW + col, q)) = out;
+                emit(j, out);
+            }
+            h2 = h1; h1 = hs;
+        }
+    }
+    ekeep0 = *reinterpret_cast<const uint4*>(ecol + 2 * k2m::EW * 128);
+    ekeep1 = *reinterpret_cast<const uint4*>(ecol + 3 * k2m::EW * 128);
+}
+
 // Macro tile `idx` of the launch: grid, origin, number of 4-row blocks that hold own rows.
 struct MacroTile {
     int b, mx0, my0, nb, tile0;     // tile0: index of its first 4 x 32 tile among the grid's partial sums
@@ -981,21 +1026,7 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
                     if (is_a) {
                         // ---- A: R = V / box3(E) for the block's four V rows, marching down ----
                         ptx::mbar_wait(&full[s], (it / k2m::NSTAGE) & 1, status, 230);
-                        if (col < k2m::VW) {
-#pragma unroll
-                            for (int j = 0; j < k2m::BR; ++j) {
-                                const uint8_t* row = es + (j * k2m::EW + col) * 128 + q * 16;
-                                const uint4 e0 = *reinterpret_cast<const uint4*>(row);
-                                const uint4 e1 = *reinterpret_cast<const uint4*>(row + 128);
-                                const uint4 e2 = *reinterpret_cast<const uint4*>(row + 256);
-                                const V8 hs = v8_sum3(e0, e1, e2);
-                                if (b >= 0 || j >= 2) {      // block -1: only its last two rows have all three E rows
-                                    uint4* pv = reinterpret_cast<uint4*>(vs + (j * k2m::VW + col) * 128 + q * 16);
-                                    *pv = v8_pack(v8_mul(v8_unpack(*pv), v8_rcp(v8_add(v8_add(h2, h1), hs))));
-                                }
-                                h2 = h1; h1 = hs;
-                            }
-                        }
+                        if (col < k2m::VW) k2_box_e(es, vs, col, q, b < 0, h2, h1);
                         ptx::bar_arrive(1 + s, k2m::HANDOFF);       // R of this block is in the stage
                     } else {
                         // ---- B: V' = E * box3(R) for tile rows 4b .. 4b+3 -> A operand ----
@@ -1003,32 +1034,11 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
                         uint8_t* a_vp = sm + k2m::A_VP + buf * 16384;
                         ptx::bar_sync(1 + s, k2m::HANDOFF);
                         if (b >= 0) ptx::mbar_wait(&vp_empty[buf], ((v >> 1) & 1) ^ 1, status, 231);   // its last UMMAs are done
-                        const uint8_t* ecol = es + (col + 2) * 128 + q * 16;      // this thread's column in the E rows
-#pragma unroll
-                        for (int j = 0; j < k2m::BR; ++j) {
-                            if (b >= 0 || j >= 2) {
-                                const uint8_t* row = vs + (j * k2m::VW + col) * 128 + q * 16;
-                                const uint4 a0 = *reinterpret_cast<const uint4*>(row);
-                                const uint4 a1 = *reinterpret_cast<const uint4*>(row + 128);
-                                const uint4 a2 = *reinterpret_cast<const uint4*>(row + 256);
-                                const V8 hs = v8_sum3(a0, a1, a2);
-                                if (b >= 0) {
-                                    // tile row j is macro-tile row 4b+j: its E came with the block before (j < 2, kept
-                                    // in registers) or is row j-2 of this block's E rows
-                                    const V8 e = v8_unpack(j == 0 ? ekeep0 : j == 1 ? ekeep1
-                                                           : *reinterpret_cast<const uint4*>(ecol + (j - 2) * k2m::EW * 128));
-                                    const uint4 out = v8_pack(v8_mul(e, v8_add(v8_add(h2, h1), hs)));
-                                    *reinterpret_cast<uint4*>(a_vp + swz(j * k2m::SW + col, q)) = out;
-                                    const int orow = m.my0 + 4 * b + j, ocol = m.mx0 + col;
-                                    if (vprime != nullptr && orow < g.H && ocol < g.W)
-                                        *reinterpret_cast<uint4*>(vprime + ((size_t)m.b * NH + h) * vplane +
-                                                                  ((size_t)orow * g.W + ocol) * HD + q * 8) = out;
-                                }
-                                h2 = h1; h1 = hs;
-                            }
-                        }
-                        ekeep0 = *reinterpret_cast<const uint4*>(ecol + 2 * k2m::EW * 128);
-                        ekeep1 = *reinterpret_cast<const uint4*>(ecol + 3 * k2m::EW * 128);
+                        k2_box_r(es, vs, a_vp, col, q, b < 0, h2, h1, ekeep0, ekeep1, [&](int j, const uint4& out) {
+                            const int orow = m.my0 + 4 * b + j, ocol = m.mx0 + col;
+                            if (vprime != nullptr && orow < g.H && ocol < g.W)
+                                *reinterpret_cast<uint4*>(vprime + ((size_t)m.b * NH + h) * vplane + ((size_t)orow * g.W + ocol) * HD + q * 8) = out;
+                        });
                         if (b >= 0) {
                             ptx::fence_proxy_async();
                             ptx::mbar_arrive(&vp_full[buf]);
@@ -1057,6 +1067,194 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
     if (my_mt > 0)       // the last macro tile's sums; the stages and the operand tiles are free by now
         k2_finish_cta(fin, macro_tile(blockIdx.x + (my_mt - 1) * gridDim.x, mt_per_grid, strips, g.H, nbmax).b, tiles_per_grid, mt_per_grid,
                       reinterpret_cast<double*>(sm + k2m::STG), reinterpret_cast<int*>(sm + k2m::A_VP));
+}
+
+// =============================================================================================================
+// k2 for grids too small to fill the GPU: a cluster of four CTAs per macro tile of one, two or four blocks, CTA r doing the
+// box sums of heads r and r + 4.  One CTA alone marches 8 heads x (blocks + 1) however few macro tiles there are (16 blocks of
+// work at the least, 25 us for a 32 x 32 grid); here it is 2 x (blocks + 1).  A block's V' operand goes to the CTA that owns
+// the tile (tile b: CTA b), by a bulk copy through distributed shared memory, and the owner issues the products of the eight
+// heads in head order: the same products in the same order as k2_bf16, hence the same bits.
+//   warps 0-7,19 A, 8-15 B: as in k2_bf16; A's first eight warps drain the owner's tile
+//   warp 16      TMA producer of the E / V blocks, and behind them of the owner's state tile
+//   warp 17      owner: UMMA issuer;  warp 18  owner: TMA producer of the Wo slices;  warp 20  sends operand tiles to the owners
+namespace k2s {
+constexpr int C = 4, ROUNDS = NH / C;                    // CTAs per cluster; heads per CTA
+constexpr int NSTAGE = 3;
+constexpr int STG = 0;
+constexpr int A_VP = STG + NSTAGE * k2m::STAGE_BYTES;    // two 16 KB operand tiles of this CTA's heads
+constexpr int SLOT = A_VP + 2 * 16384;                   // the owned tile's operands, one from each CTA of the cluster
+constexpr int WO = SLOT + C * 16384;                     // two 8 KB Wo slices
+constexpr int RED = WO + 2 * 8192;                       // [4 quads][64] fp32
+constexpr int BARS = RED + 4 * 64 * 4;
+constexpr int N_BARS = 2 * NSTAGE + 8 + 2 * C + 1;
+constexpr int TMEM_PTR = BARS + N_BARS * 8;
+constexpr int SMEM = TMEM_PTR + 16 + 1024;
+constexpr int THREADS = 672;
+static_assert(A_VP % 1024 == 0 && SLOT % 1024 == 0 && WO % 1024 == 0, "swizzled tiles must be 1024-byte aligned");
+static_assert(SMEM <= 227 * 1024, "k2 (split) shared memory");
+}  // namespace k2s
+
+__global__ void __cluster_dims__(k2s::C, 1, 1) __launch_bounds__(k2s::THREADS, 1)
+k2_split_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUtensorMap map_e,
+              const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ scale,
+              const K2Sums fin, __nv_bfloat16* __restrict__ vprime, int* __restrict__ status,
+              int mt_per_grid, int strips, int tiles_per_grid, int nbmax, Geom g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = align1024(smem_raw);
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm + k2s::BARS);    // [3] block landed                               (waits: A)
+    uint64_t* empty = full + k2s::NSTAGE;            // [3] B is done with the stage (256 arrivals)   (waits: TMA producer)
+    uint64_t* vp_full = empty + k2s::NSTAGE;         // [2] operand tile written (256 arrivals)       (waits: sender)
+    uint64_t* vp_empty = vp_full + 2;                // [2] ... and landed at its owner (who arrives) (waits: B)
+    uint64_t* wo_full = vp_empty + 2;                // [2] Wo slice landed                           (waits: UMMA issuer)
+    uint64_t* wo_empty = wo_full + 2;                // [2] its head is issued and done               (waits: Wo producer)
+    uint64_t* slot_full = wo_empty + 2;              // [4] operand of CTA r landed                   (waits: UMMA issuer)
+    uint64_t* slot_ok = slot_full + k2s::C;          // [4] owner b's slot of this CTA is free again (the owner's commit)  (waits: sender)
+    uint64_t* acc_full = slot_ok + k2s::C;           // all 8 heads of the owned tile accumulated     (waits: A)
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k2s::TMEM_PTR);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x % k2s::C;
+    if (tid == 0) {
+        for (int i = 0; i < k2s::NSTAGE; ++i) { ptx::mbar_init(&full[i], 1); ptx::mbar_init(&empty[i], k2m::B_THREADS); }
+        for (int i = 0; i < 2; ++i) {
+            ptx::mbar_init(&vp_full[i], k2m::B_THREADS); ptx::mbar_init(&vp_empty[i], 1);
+            ptx::mbar_init(&wo_full[i], 1); ptx::mbar_init(&wo_empty[i], 1);
+        }
+        for (int i = 0; i < k2s::C; ++i) { ptx::mbar_init(&slot_full[i], 1); ptx::mbar_init(&slot_ok[i], 1); }
+        ptx::mbar_init(acc_full, 1);
+        ptx::fence_barrier_init();
+        for (int i = 0; i < k2s::C; ++i) ptx::mbar_expect_tx(&slot_full[i], 16384);      // round 0
+        ptx::prefetch_tmap(&map_wo); ptx::prefetch_tmap(&map_e); ptx::prefetch_tmap(&map_v); ptx::prefetch_tmap(&map_x);
+    }
+    if (warp == 0) ptx::tmem_alloc(tmem_ptr, 64);
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_ptr;
+    ptx::cluster_sync();                 // the others' barriers are there
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    const MacroTile m = macro_tile(blockIdx.x / k2s::C, mt_per_grid, strips, g.H, nbmax);
+    const bool owner = rank < m.nb;
+
+    if (warp == 16) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            for (int round = 0; round < k2s::ROUNDS; ++round)
+                for (int b = -1; b < m.nb; ++b, ++it) {
+                    const int s = it % k2s::NSTAGE, plane = m.b * NH + round * k2s::C + rank;
+                    uint8_t* st = sm + k2s::STG + s * k2m::STAGE_BYTES;
+                    ptx::mbar_wait(&empty[s], ((it / k2s::NSTAGE) & 1) ^ 1, status, 250);
+                    ptx::mbar_expect_tx(&full[s], k2m::STAGE_TX);
+                    ptx::tma_load_4d(st, &map_e, 0, m.mx0, m.my0 + 4 * b + 4, plane, &full[s]);
+                    ptx::tma_load_4d(st + k2m::E_BYTES, &map_v, 0, m.mx0 + 1, m.my0 + 4 * b + 3, plane, &full[s]);
+                }
+            if (owner) {                 // the owned tile's state, through the ring
+                const int s = it % k2s::NSTAGE;
+                ptx::mbar_wait(&empty[s], ((it / k2s::NSTAGE) & 1) ^ 1, status, 251);
+                ptx::mbar_expect_tx(&full[s], 16384);
+                ptx::tma_load_4d(sm + k2s::STG + s * k2m::STAGE_BYTES, &map_x, 0, m.mx0, g.hx + m.my0 + rank * k2m::BR, m.b, &full[s]);
+            }
+        }
+    } else if (warp == 18) {
+        if (lane == 0 && owner) {
+            const int set = m.b / g.per_set;
+            for (int h = 0; h < NH; ++h) {
+                const int wb = h & 1;
+                ptx::mbar_wait(&wo_empty[wb], ((h >> 1) & 1) ^ 1, status, 252);
+                ptx::mbar_expect_tx(&wo_full[wb], 8192);
+                ptx::tma_load_2d(sm + k2s::WO + wb * 8192, &map_wo, 0, (set * NH + h) * 64, &wo_full[wb]);
+            }
+        }
+    } else if (warp == 17) {
+        if (owner) {
+            const uint32_t leader = ptx::elect_one();
+            const uint32_t a0 = ptx::smem_u32(sm + k2s::SLOT) >> 4, w0 = ptx::smem_u32(sm + k2s::WO) >> 4;
+            for (int h = 0; h < NH; ++h) {
+                const int r = h % k2s::C, round = h / k2s::C, wb = h & 1;
+                ptx::mbar_wait(&wo_full[wb], (h >> 1) & 1, status, 253);
+                ptx::mbar_wait(&slot_full[r], round & 1, status, 254);
+                if (lane == 0) {
+                    // the sender may write its operand tile again (its use number round * nb + rank)
+                    ptx::mbar_arrive_remote(&vp_empty[(round * m.nb + rank) & 1], r);
+                    if (round + 1 < k2s::ROUNDS) ptx::mbar_expect_tx(&slot_full[r], 16384);
+                }
+                __syncwarp();
+                ptx::tc_fence_after();
+                ptx::umma4_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW128_HI>(leader, tmem, a0 + r * (16384 >> 4), w0 + wb * (8192 >> 4), h > 0);
+                ptx::umma_commit_by(leader, &wo_empty[wb]);
+                if (round + 1 < k2s::ROUNDS) ptx::umma_commit_remote_by(leader, &slot_ok[rank], 1u << r);
+                if (h == NH - 1) ptx::umma_commit_by(leader, acc_full);
+            }
+        }
+    } else if (warp == 20) {
+        if (lane == 0) {
+            uint32_t v = 0;
+            for (int round = 0; round < k2s::ROUNDS; ++round)
+                for (int b = 0; b < m.nb; ++b, ++v) {
+                    const int buf = v & 1;
+                    ptx::mbar_wait(&vp_full[buf], (v >> 1) & 1, status, 255);
+                    if (round > 0) ptx::mbar_wait(&slot_ok[b], (round - 1) & 1, status, 256);
+                    ptx::bulk_copy_to_cta(sm + k2s::SLOT + rank * 16384, sm + k2s::A_VP + buf * 16384, 16384, &slot_full[rank], b);
+                }
+        }
+    } else {
+        const bool is_a = warp < 8 || warp == 19;
+        const int gt = warp == 19 ? 256 + lane : (is_a ? tid : tid - 256);     // thread within its set
+        const int q = gt & 7, col = gt >> 3;
+        uint32_t it = 0, v = 0;
+        V8 h2 = v8_zero(), h1 = v8_zero();
+        uint4 ekeep0 = make_uint4(0, 0, 0, 0), ekeep1 = ekeep0;
+        const size_t vplane = (size_t)g.H * g.W * HD;
+        for (int round = 0; round < k2s::ROUNDS; ++round)
+            for (int b = -1; b < m.nb; ++b, ++it) {
+                const int s = it % k2s::NSTAGE, h = round * k2s::C + rank;
+                uint8_t* es = sm + k2s::STG + s * k2m::STAGE_BYTES;
+                uint8_t* vs = es + k2m::E_BYTES;
+                if (is_a) {
+                    ptx::mbar_wait(&full[s], (it / k2s::NSTAGE) & 1, status, 260);
+                    if (col < k2m::VW) k2_box_e(es, vs, col, q, b < 0, h2, h1);
+                    ptx::bar_arrive(1 + s, k2m::HANDOFF);
+                } else {
+                    const int buf = v & 1;
+                    ptx::bar_sync(1 + s, k2m::HANDOFF);
+                    if (b >= 0) ptx::mbar_wait(&vp_empty[buf], ((v >> 1) & 1) ^ 1, status, 261);
+                    k2_box_r(es, vs, sm + k2s::A_VP + buf * 16384, col, q, b < 0, h2, h1, ekeep0, ekeep1, [&](int j, const uint4& out) {
+                        const int orow = m.my0 + 4 * b + j, ocol = m.mx0 + col;
+                        if (vprime != nullptr && orow < g.H && ocol < g.W)
+                            *reinterpret_cast<uint4*>(vprime + ((size_t)m.b * NH + h) * vplane + ((size_t)orow * g.W + ocol) * HD + q * 8) = out;
+                    });
+                    if (b >= 0) {
+                        ptx::fence_proxy_async();
+                        ptx::mbar_arrive(&vp_full[buf]);
+                        ++v;
+                    }
+                    ptx::mbar_arrive(&empty[s]);
+                }
+            }
+        if (owner && is_a && gt < 256) {
+            CaTile t;
+            t.b = m.b; t.ty0 = m.my0 + rank * k2m::BR; t.tx0 = m.mx0;
+            t.index = m.b * tiles_per_grid + m.tile0 + rank * strips;
+            const int s = it % k2s::NSTAGE;
+            uint8_t* xs = sm + k2s::STG + s * k2m::STAGE_BYTES;
+            ptx::mbar_wait(&full[s], (it / k2s::NSTAGE) & 1, status, 262);
+            ptx::mbar_wait(acc_full, 0, status, 263);
+            ptx::tc_fence_after();
+            k2_epilogue(t, tmem, xs, scale, fin.partial, reinterpret_cast<float*>(sm + k2s::RED), 7, gt, warp, g);
+            if (gt == 0) {
+                ptx::tma_store_4d(&map_x, xs, 0, t.tx0, g.hx + t.ty0, t.b);
+                ptx::bulk_commit();
+                ptx::bulk_wait0();
+            }
+        }
+    }
+    ptx::tc_fence_before();
+    ptx::cluster_sync();                 // nobody's shared memory or barriers are written any more
+    if (warp == 0) ptx::tmem_dealloc(tmem, 64);
+    if (owner)                           // every tile is one CTA's
+        k2_finish_cta(fin, m.b, tiles_per_grid, tiles_per_grid, reinterpret_cast<double*>(sm + k2s::STG), reinterpret_cast<int*>(sm + k2s::A_VP));
 }
 
 // =============================================================================================================
@@ -1170,6 +1368,17 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
     p.k1_grid = (int)(total1 < num_sms ? total1 : num_sms);
     const long long total_mt = k2_macro_tiles(g, p.strips, k2m::NB, num_sms, p.nbmax, p.mt_per_grid);
     p.k2_grid = (int)(total_mt < num_sms ? total_mt : num_sms);
+    // a cluster per macro tile where all of them are resident at once: with the fewest blocks per macro tile that allows it
+    if (cudaFuncSetAttribute(k2_split_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, k2s::SMEM) != cudaSuccess) {
+        bf16_error_ref() = "could not opt in to the kernels' dynamic shared memory";
+        return -1;
+    }
+    const int most = max_clusters(k2_split_bf16, k2s::C, k2s::THREADS, k2s::SMEM), rows4 = (g.H + k2m::BR - 1) / k2m::BR;
+    p.split_grid = 0;
+    for (int nb = 1; nb <= k2s::C && p.split_grid == 0; nb *= 2) {
+        const int mt = p.strips * ((rows4 + nb - 1) / nb);
+        if ((long long)mt * g.B <= most) { p.split_grid = mt * g.B * k2s::C; p.nbmax = nb; p.mt_per_grid = mt; }
+    }
     return 0;
 }
 
@@ -1181,6 +1390,9 @@ inline int bf16_k1(Bf16Plan& p, const __nv_bfloat16* X, const float* scale, cons
 
 inline int bf16_k2(Bf16Plan& p, __nv_bfloat16* X, const float* scale, const __nv_bfloat16*, const __nv_bfloat16*,
                    const K2Sums& fin, __nv_bfloat16* vprime, int* status, const Geom& g, cudaStream_t st) {
+    if (p.split_grid)
+        return launch_pdl(k2_split_bf16, p.split_grid, k2s::THREADS, k2s::SMEM, st, p.map_wo, p.map_e, p.map_v, p.map_x, scale, fin, vprime, status,
+                          p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g) == cudaSuccess ? 0 : -1;
     return launch_pdl(k2_bf16, p.k2_grid, k2m::THREADS, k2m::SMEM, st, p.map_wo, p.map_e, p.map_v, p.map_x, scale, fin, vprime, status,
                       p.mt_per_grid * g.B, p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g) == cudaSuccess ? 0 : -1;
 }

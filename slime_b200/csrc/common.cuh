@@ -71,6 +71,19 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int 
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+// Clusters of c such blocks (of a kernel with __cluster_dims__) that the device holds at once; 0 if that can not be told.
+template <typename... P>
+inline int max_clusters(void (*kernel)(P...), int c, int threads, int smem) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = c; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(c); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return n;
+}
+
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {

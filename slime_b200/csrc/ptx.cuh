@@ -120,6 +120,26 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
 
+// ---- thread-block clusters ----------------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared::cluster address of this CTA's shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_to_cta(const void* p, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(bar, rank)) : "memory");
+}
+// bulk copy from this CTA's shared memory to the same layout's `dst` in CTA `rank`, completion on that CTA's `bar`
+__device__ __forceinline__ void bulk_copy_to_cta(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint32_t rank) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(map_to_cta(dst, rank)), "r"(smem_u32(src)), "r"(bytes), "r"(map_to_cta(bar, rank)) : "memory");
+}
+
 // ---- programmatic dependent launch ---------------------------------------------------------------------------
 // The next kernel of the stream may take SMs as they fall free and set itself up ...
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -207,6 +227,15 @@ __device__ __forceinline__ void umma_commit_by(uint32_t leader, uint64_t* bar) {
         "{\n\t.reg .pred q;\n\t"
         "setp.ne.b32 q, %1, 0;\n\t"
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader) : "memory");
+}
+
+// ... on the same barrier of the cluster's CTAs in `mask`
+__device__ __forceinline__ void umma_commit_remote_by(uint32_t leader, uint64_t* bar, uint32_t mask) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\tcvt.u16.u32 m, %2;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}"
+        ::"r"(smem_u32(bar)), "r"(leader), "r"(mask) : "memory");
 }
 
 // TMEM -> registers: this thread's lane (32 * (warp % 4) + lane), 16 consecutive fp32 columns from `taddr`.
