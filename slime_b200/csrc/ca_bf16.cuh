@@ -92,17 +92,22 @@ __device__ __forceinline__ void k2_finish(const K2Sums& k, int b, int n, int par
 __device__ __forceinline__ void k2_finish_cta(const K2Sums& k, int b, int n, int parts, double* red, int* flag) {
     if (k.tickets == nullptr) return;
     const int tid = threadIdx.x, c = tid & 63;
-    if (tid == 0) { __threadfence(); *flag = atomicAdd(&k.tickets[b], 1) == parts - 1; }
+    const double mass = tid < NC && k.out.mode == 2 ? k.out.mass[b * NC + c] : 0.0;
+    if (tid == 0) {          // its fences, with the barriers, order the whole CTA's accesses
+        __threadfence();
+        *flag = atomicAdd(&k.tickets[b], 1) == parts - 1;
+        __threadfence();
+    }
     __syncthreads();
     if (!*flag) return;
-    __threadfence();
     for (int sub = tid >> 6; sub < 16; sub += blockDim.x >> 6) red[sub * NC + c] = tile_sums(k.partial + (size_t)b * n * NC + c, k.lo_offset, n, sub);
     __syncthreads();
     if (tid < NC) {
         double s = 0.0;
 #pragma unroll
         for (int sub = 0; sub < 16; ++sub) s += red[sub * NC + c];
-        sums_out(k.out, b, c, s);
+        k.out.sums[b * NC + c] = s;
+        if (k.out.mode == 2) k.out.scale[b * NC + c] = (float)(mass / s);
     }
     if (tid == 0) k.tickets[b] = 0;
 }
@@ -1084,10 +1089,10 @@ constexpr int NSTAGE = 3;
 constexpr int STG = 0;
 constexpr int A_VP = STG + NSTAGE * k2m::STAGE_BYTES;    // two 16 KB operand tiles of this CTA's heads
 constexpr int SLOT = A_VP + 2 * 16384;                   // the owned tile's operands, one from each CTA of the cluster
-constexpr int WO = SLOT + C * 16384;                     // two 8 KB Wo slices
-constexpr int RED = WO + 2 * 8192;                       // [4 quads][64] fp32
-constexpr int BARS = RED + 4 * 64 * 4;
-constexpr int N_BARS = 2 * NSTAGE + 8 + 2 * C + 1;
+constexpr int NWO = 3, WO = SLOT + C * 16384;            // 8 KB Wo slices
+constexpr int RED = SLOT;                                // [4 quads][64] fp32, once the slots are done with
+constexpr int BARS = WO + NWO * 8192;
+constexpr int N_BARS = 2 * NSTAGE + 4 + 2 * NWO + 2 * C + 1;
 constexpr int TMEM_PTR = BARS + N_BARS * 8;
 constexpr int SMEM = TMEM_PTR + 16 + 1024;
 constexpr int THREADS = 672;
@@ -1106,9 +1111,9 @@ k2_split_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant_
     uint64_t* empty = full + k2s::NSTAGE;            // [3] B is done with the stage (256 arrivals)   (waits: TMA producer)
     uint64_t* vp_full = empty + k2s::NSTAGE;         // [2] operand tile written (256 arrivals)       (waits: sender)
     uint64_t* vp_empty = vp_full + 2;                // [2] ... and landed at its owner (who arrives) (waits: B)
-    uint64_t* wo_full = vp_empty + 2;                // [2] Wo slice landed                           (waits: UMMA issuer)
-    uint64_t* wo_empty = wo_full + 2;                // [2] its head is issued and done               (waits: Wo producer)
-    uint64_t* slot_full = wo_empty + 2;              // [4] operand of CTA r landed                   (waits: UMMA issuer)
+    uint64_t* wo_full = vp_empty + 2;                // [3] Wo slice landed                           (waits: UMMA issuer)
+    uint64_t* wo_empty = wo_full + k2s::NWO;         // [3] its head is issued and done               (waits: Wo producer)
+    uint64_t* slot_full = wo_empty + k2s::NWO;              // [4] operand of CTA r landed                   (waits: UMMA issuer)
     uint64_t* slot_ok = slot_full + k2s::C;          // [4] owner b's slot of this CTA is free again (the owner's commit)  (waits: sender)
     uint64_t* acc_full = slot_ok + k2s::C;           // all 8 heads of the owned tile accumulated     (waits: A)
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k2s::TMEM_PTR);
@@ -1117,10 +1122,8 @@ k2_split_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant_
     const int rank = blockIdx.x % k2s::C;
     if (tid == 0) {
         for (int i = 0; i < k2s::NSTAGE; ++i) { ptx::mbar_init(&full[i], 1); ptx::mbar_init(&empty[i], k2m::B_THREADS); }
-        for (int i = 0; i < 2; ++i) {
-            ptx::mbar_init(&vp_full[i], k2m::B_THREADS); ptx::mbar_init(&vp_empty[i], 1);
-            ptx::mbar_init(&wo_full[i], 1); ptx::mbar_init(&wo_empty[i], 1);
-        }
+        for (int i = 0; i < 2; ++i) { ptx::mbar_init(&vp_full[i], k2m::B_THREADS); ptx::mbar_init(&vp_empty[i], 1); }
+        for (int i = 0; i < 2 * k2s::NWO; ++i) ptx::mbar_init(&wo_full[i], 1);
         for (int i = 0; i < k2s::C; ++i) { ptx::mbar_init(&slot_full[i], 1); ptx::mbar_init(&slot_ok[i], 1); }
         ptx::mbar_init(acc_full, 1);
         ptx::fence_barrier_init();
@@ -1161,8 +1164,8 @@ k2_split_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant_
         if (lane == 0 && owner) {
             const int set = m.b / g.per_set;
             for (int h = 0; h < NH; ++h) {
-                const int wb = h & 1;
-                ptx::mbar_wait(&wo_empty[wb], ((h >> 1) & 1) ^ 1, status, 252);
+                const int wb = h % k2s::NWO;
+                ptx::mbar_wait(&wo_empty[wb], ((h / k2s::NWO) & 1) ^ 1, status, 252);
                 ptx::mbar_expect_tx(&wo_full[wb], 8192);
                 ptx::tma_load_2d(sm + k2s::WO + wb * 8192, &map_wo, 0, (set * NH + h) * 64, &wo_full[wb]);
             }
@@ -1172,8 +1175,7 @@ k2_split_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant_
             const uint32_t leader = ptx::elect_one();
             const uint32_t a0 = ptx::smem_u32(sm + k2s::SLOT) >> 4, w0 = ptx::smem_u32(sm + k2s::WO) >> 4;
             for (int h = 0; h < NH; ++h) {
-                const int r = h % k2s::C, round = h / k2s::C, wb = h & 1;
-                ptx::mbar_wait(&wo_full[wb], (h >> 1) & 1, status, 253);
+                const int r = h % k2s::C, round = h / k2s::C, wb = h % k2s::NWO;
                 ptx::mbar_wait(&slot_full[r], round & 1, status, 254);
                 if (lane == 0) {
                     // the sender may write its operand tile again (its use number round * nb + rank)
@@ -1181,6 +1183,7 @@ k2_split_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant_
                     if (round + 1 < k2s::ROUNDS) ptx::mbar_expect_tx(&slot_full[r], 16384);
                 }
                 __syncwarp();
+                ptx::mbar_wait(&wo_full[wb], (h / k2s::NWO) & 1, status, 253);
                 ptx::tc_fence_after();
                 ptx::umma4_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW128_HI>(leader, tmem, a0 + r * (16384 >> 4), w0 + wb * (8192 >> 4), h > 0);
                 ptx::umma_commit_by(leader, &wo_empty[wb]);
