@@ -1318,6 +1318,20 @@ inline long long k2_macro_tiles(const Geom& g, int strips, int most, int num_sms
     return total_mt;
 }
 
+// CTAs of the split k2, a cluster of c per macro tile, where all of them (at most `most` clusters) are resident at once: with
+// the fewest blocks per macro tile that allows it.  0 where there are too many macro tiles; nbmax and mt_per_grid then stay.
+inline int k2_split_grid(const Geom& g, int strips, int c, int most, int& nbmax, int& mt_per_grid) {
+    const int rows4 = (g.H + k2m::BR - 1) / k2m::BR;
+    for (int nb = 1; nb <= c; nb *= 2) {
+        const long long mt = (long long)strips * ((rows4 + nb - 1) / nb);
+        if (mt * g.B > most) continue;
+        nbmax = nb;
+        mt_per_grid = (int)mt;
+        return (int)(mt * g.B) * c;
+    }
+    return 0;
+}
+
 // Tensor maps over the weight arrays and the E/V planes, and the kernels' shared-memory opt-in.  0 on success.
 inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16* wo, int sets, const __nv_bfloat16* E,
                       const __nv_bfloat16* V, const __nv_bfloat16* X, const Geom& g, int num_sms) {
@@ -1371,17 +1385,11 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
     p.k1_grid = (int)(total1 < num_sms ? total1 : num_sms);
     const long long total_mt = k2_macro_tiles(g, p.strips, k2m::NB, num_sms, p.nbmax, p.mt_per_grid);
     p.k2_grid = (int)(total_mt < num_sms ? total_mt : num_sms);
-    // a cluster per macro tile where all of them are resident at once: with the fewest blocks per macro tile that allows it
     if (cudaFuncSetAttribute(k2_split_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, k2s::SMEM) != cudaSuccess) {
         bf16_error_ref() = "could not opt in to the kernels' dynamic shared memory";
         return -1;
     }
-    const int most = max_clusters(k2_split_bf16, k2s::C, k2s::THREADS, k2s::SMEM), rows4 = (g.H + k2m::BR - 1) / k2m::BR;
-    p.split_grid = 0;
-    for (int nb = 1; nb <= k2s::C && p.split_grid == 0; nb *= 2) {
-        const int mt = p.strips * ((rows4 + nb - 1) / nb);
-        if ((long long)mt * g.B <= most) { p.split_grid = mt * g.B * k2s::C; p.nbmax = nb; p.mt_per_grid = mt; }
-    }
+    p.split_grid = k2_split_grid(g, p.strips, k2s::C, max_clusters(k2_split_bf16, k2s::C, k2s::THREADS, k2s::SMEM), p.nbmax, p.mt_per_grid);
     return 0;
 }
 

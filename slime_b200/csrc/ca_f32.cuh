@@ -41,6 +41,7 @@ struct F32Plan {
     CUtensorMap map_x;        // the state, box 32 x 32 x 4 x 1, 128B swizzle
     CUtensorMap map_es, map_vs;   // stores of k1: box 16 x 16 x 2 x 1, 64B swizzle
     int strips = 1, mt_per_grid = 1, nbmax = 6;
+    int split_grid = 0;           // CTAs of k2_split_f32, 0: the launch is large enough for k2_f32
 };
 
 // x = hi + mid + lo, exactly: hi is x rounded to bf16, mid the rest rounded to bf16, lo what is left (at most 7 bits).
@@ -444,6 +445,131 @@ __device__ __forceinline__ ptx::f2 div2(ptx::f2 x, ptx::f2 z) {
 __device__ __forceinline__ V4 v4_div(const V4& x, const V4& z) { V4 r; r.a = div2(x.a, z.a); r.b = div2(x.b, z.b); return r; }
 __device__ __forceinline__ float4 v4_f4(const V4& x) { float4 f; ptx::split_f2(x.a, f.x, f.y); ptx::split_f2(x.b, f.z, f.w); return f; }
 
+// Set A's part of a block: R = V / box3(E) for its four V rows, marching down, by the thread of column col and dims 4q..4q+3.
+// h2, h1: horizontal sums of the two E rows above.  Of a priming block only the last two rows have all three E rows.
+__device__ __forceinline__ void k2f_box_e(const uint8_t* es, uint8_t* vs, int col, int q, bool prime, V4& h2, V4& h1) {
+#pragma unroll
+    for (int j = 0; j < k2f::BR; ++j) {
+        const float4* row = reinterpret_cast<const float4*>(es + (j * k2f::EW + col) * 128 + q * 16);
+        const V4 hs = v4_add(v4_add(v4(row[0]), v4(row[8])), v4(row[16]));
+        if (!prime || j >= 2) {
+            float4* pv = reinterpret_cast<float4*>(vs + (j * k2f::VW + col) * 128 + q * 16);
+            *pv = v4_f4(v4_div(v4(*pv), v4_add(v4_add(h2, h1), hs)));
+        }
+        h2 = h1; h1 = hs;
+    }
+}
+// Set B's part: V' = E * box3(R) for tile rows 4b .. 4b+3 -> the three parts of the A operand, and emit(row, V').  Tile row j is
+// macro-tile row 4b+j: its E came with the block before (j < 2, kept in registers) or is row j-2 of this block's E rows.
+template <typename F>
+__device__ __forceinline__ void k2f_box_r(const uint8_t* es, const uint8_t* vs, uint8_t* a_vp, int col, int q, bool prime, V4& h2, V4& h1,
+                                          float4& ekeep0, float4& ekeep1, F emit) {
+    const uint8_t* ecol = es + (col + 2) * 128 + q * 16;      // this thread's column in the E rows
+#pragma unroll
+    for (int j = 0; j < k2f::BR; ++j) {
+        if (!prime || j >= 2) {
+            const float4* row = reinterpret_cast<const float4*>(vs + (j * k2f::VW + col) * 128 + q * 16);
+            const V4 hs = v4_add(v4_add(v4(row[0]), v4(row[8])), v4(row[16]));
+            if (!prime) {
+                const V4 e = v4(j == 0 ? ekeep0 : j == 1 ? ekeep1 : *reinterpret_cast<const float4*>(ecol + (j - 2) * k2f::EW * 128));
+                const V4 out = v4_mul(e, v4_add(v4_add(h2, h1), hs));
+                uint32_t pa[3], pb[3];
+                split3(out.a, pa[0], pa[1], pa[2]);
+                split3(out.b, pb[0], pb[1], pb[2]);
+                uint8_t* dst = a_vp + swz64(j * k2f::SW + col, q >> 1) + (q & 1) * 8;
+#pragma unroll
+                for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dst + p * k2f::PART) = make_uint2(pa[p], pb[p]);
+                emit(j, out);
+            }
+            h2 = h1; h1 = hs;
+        }
+    }
+    ekeep0 = *reinterpret_cast<const float4*>(ecol + 2 * k2f::EW * 128);
+    ekeep1 = *reinterpret_cast<const float4*>(ecol + 3 * k2f::EW * 128);
+}
+// The six products of a half-head's operand parts (a) and Wo parts (w), smallest first, into accumulator d.
+__device__ __forceinline__ void k2f_products(uint32_t leader, uint32_t d, uint32_t a, uint32_t w) {
+#pragma unroll
+    for (int pw = 2; pw >= 0; --pw)
+#pragma unroll
+        for (int pa = 2 - pw; pa >= 0; --pa)
+            ptx::umma2_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW64_HI>(leader, d, a + pa * (k2f::PART >> 4), w + pw * (k2f::WO_PART >> 4),
+                                                                      pw < 2 || pa < 2 - pw);
+}
+// run (+)= work, this thread's TMEM lane, rounded to nearest
+__device__ __forceinline__ void k2f_add(uint32_t run, uint32_t work, bool accumulate) {
+#pragma unroll
+    for (int c0 = 0; c0 < 64; c0 += 16) {
+        uint32_t w[16];
+        ptx::tmem_ld16(work + c0, w);
+        if (accumulate) {
+            uint32_t y[16];
+            ptx::tmem_ld16(run + c0, y);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) w[j] = __float_as_uint(__uint_as_float(w[j]) + __uint_as_float(y[j]));
+        } else {
+            ptx::tmem_ld_wait();
+        }
+        ptx::tmem_st16(run + c0, w);
+    }
+    ptx::tmem_st_wait();
+}
+// A tile's last half-head: X+ = scale X + dt (run + work) in the state tile xt, and the channel sums of what is stored -> red,
+// kept in fp64 and handed on as a float pair (value, remainder): a state that has grown large and signed makes the
+// per-channel sum a small difference of large terms, and fp32 tile sums would then miss the 1e-6 bound on the renormalised
+// mass.  drained() once the accumulators are read.
+template <typename F>
+__device__ __forceinline__ void k2f_epilogue(uint32_t run, uint32_t work, uint8_t* xt, const float* sc, int cell, bool valid, double* red,
+                                             float dt, F drained) {
+    const int lane = cell & 31, quad = cell >> 5;
+#pragma unroll
+    for (int c0 = 0; c0 < 64; c0 += 16) {
+        uint32_t w[16], y[16];
+        ptx::tmem_ld16(work + c0, w);
+        ptx::tmem_ld16(run + c0, y);
+        ptx::tmem_ld_wait();
+        if (c0 == 48) drained();
+        double xo[16];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float4* px = reinterpret_cast<float4*>(xt + (c0 >> 5) * 16384 + swz(cell, ((c0 & 31) >> 2) + q));
+            float4 x = *px;
+            const float4 s4 = __ldg(reinterpret_cast<const float4*>(sc + c0) + q);
+            x.x = fmaf(dt, __uint_as_float(w[4 * q]) + __uint_as_float(y[4 * q]), x.x * s4.x);
+            x.y = fmaf(dt, __uint_as_float(w[4 * q + 1]) + __uint_as_float(y[4 * q + 1]), x.y * s4.y);
+            x.z = fmaf(dt, __uint_as_float(w[4 * q + 2]) + __uint_as_float(y[4 * q + 2]), x.z * s4.z);
+            x.w = fmaf(dt, __uint_as_float(w[4 * q + 3]) + __uint_as_float(y[4 * q + 3]), x.w * s4.w);
+            *px = x;
+            xo[4 * q] = valid ? (double)x.x : 0.0; xo[4 * q + 1] = valid ? (double)x.y : 0.0;
+            xo[4 * q + 2] = valid ? (double)x.z : 0.0; xo[4 * q + 3] = valid ? (double)x.w : 0.0;
+        }
+        // sum over the 32 cells of this warp, fixed tree: each step halves the channels a lane carries
+#pragma unroll
+        for (int wd = 8; wd >= 1; wd >>= 1) {
+            const bool up = (lane & (wd * 2)) != 0;
+#pragma unroll
+            for (int j = 0; j < wd; ++j) {
+                const double send = up ? xo[j] : xo[j + wd];
+                const double keep = up ? xo[j + wd] : xo[j];
+                xo[j] = keep + __shfl_xor_sync(0xffffffffu, send, wd * 2);
+            }
+        }
+        xo[0] += __shfl_xor_sync(0xffffffffu, xo[0], 1);
+        if ((lane & 1) == 0) {
+            const int ch = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+            red[quad * 64 + c0 + ch] = xo[0];
+        }
+    }
+    ptx::fence_proxy_async();      // X+ in shared memory, for the TMA stores issued behind the caller's barrier
+}
+__device__ __forceinline__ void k2f_store_sums(const K2Sums& fin, const double* red, size_t tile, int c) {
+    const double t = (red[c] + red[64 + c]) + (red[128 + c] + red[192 + c]);
+    const float hi = (float)t;
+    fin.partial[tile * NC + c] = hi;
+    fin.partial[tile * NC + c + fin.lo_offset] = (float)(t - (double)hi);
+}
+
 __global__ void __launch_bounds__(k2f::THREADS, 1)
 k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUtensorMap map_e,
        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ scale,
@@ -541,13 +667,7 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                     ptx::mbar_wait(&wk_empty[buf], ((v >> 1) & 1) ^ 1, status, 520);
                     ptx::mbar_wait(&vp_full[buf], (v >> 1) & 1, status, 522);
                     ptx::tc_fence_after();
-                    const uint32_t a = a0 + buf * (3 * k2f::PART >> 4), w = w0 + wb * (3 * k2f::WO_PART >> 4);
-#pragma unroll
-                    for (int pw = 2; pw >= 0; --pw)
-#pragma unroll
-                        for (int pa = 2 - pw; pa >= 0; --pa)
-                            ptx::umma2_ss<ptx::umma_idesc_bf16(128, 64), ptx::SW64_HI>(leader, tmem + k2f::WORK + buf * 64, a + pa * (k2f::PART >> 4),
-                                                                                      w + pw * (k2f::WO_PART >> 4), pw < 2 || pa < 2 - pw);
+                    k2f_products(leader, tmem + k2f::WORK + buf * 64, a0 + buf * (3 * k2f::PART >> 4), w0 + wb * (3 * k2f::WO_PART >> 4));
                     ptx::umma_commit_by(leader, &vp_empty[buf]);
                     ptx::umma_commit_by(leader, &wk_full[buf]);
                     if (b == m.nb - 1) ptx::umma_commit_by(leader, &wo_empty[wb]);
@@ -570,79 +690,17 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                     ptx::mbar_wait(&wk_full[buf], (v >> 1) & 1, status, 530);
                     ptx::tc_fence_after();
                     if (hh < k2f::NHH - 1) {
-#pragma unroll
-                        for (int c0 = 0; c0 < 64; c0 += 16) {
-                            uint32_t w[16];
-                            ptx::tmem_ld16(work + c0, w);
-                            if (hh > 0) {
-                                uint32_t y[16];
-                                ptx::tmem_ld16(run + c0, y);
-                                ptx::tmem_ld_wait();
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) w[j] = __float_as_uint(__uint_as_float(w[j]) + __uint_as_float(y[j]));
-                            } else {
-                                ptx::tmem_ld_wait();
-                            }
-                            ptx::tmem_st16(run + c0, w);
-                        }
-                        ptx::tmem_st_wait();
+                        k2f_add(run, work, hh > 0);
                         ptx::tc_fence_before();
                         ptx::mbar_arrive(&wk_empty[buf]);
                     } else {
-                        // the tile's last half-head: X+ = scale X + dt Y, and the channel sums of what is stored, kept in
-                        // fp64 and handed on as a float pair (value, remainder): a state that has grown large and signed
-                        // makes the per-channel sum a small difference of large terms, and fp32 tile sums would then miss
-                        // the 1e-6 bound on the renormalised mass
                         const int ty0 = m.my0 + b * k2f::BR;
                         const bool valid = ty0 + (cell >> 5) < g.H && m.mx0 + (cell & 31) < g.W;
-                        const float* sc = scale + m.b * NC;
                         ptx::mbar_wait(x_full, nx & 1, status, 531);
-#pragma unroll
-                        for (int c0 = 0; c0 < 64; c0 += 16) {
-                            uint32_t w[16], y[16];
-                            ptx::tmem_ld16(work + c0, w);
-                            ptx::tmem_ld16(run + c0, y);
-                            ptx::tmem_ld_wait();
-                            if (c0 == 48) { ptx::tc_fence_before(); ptx::mbar_arrive(&wk_empty[buf]); }
-                            double xo[16];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                float4* px = reinterpret_cast<float4*>(xt + (c0 >> 5) * 16384 + swz(cell, ((c0 & 31) >> 2) + q));
-                                float4 x = *px;
-                                const float4 s4 = __ldg(reinterpret_cast<const float4*>(sc + c0) + q);
-                                x.x = fmaf(g.dt, __uint_as_float(w[4 * q]) + __uint_as_float(y[4 * q]), x.x * s4.x);
-                                x.y = fmaf(g.dt, __uint_as_float(w[4 * q + 1]) + __uint_as_float(y[4 * q + 1]), x.y * s4.y);
-                                x.z = fmaf(g.dt, __uint_as_float(w[4 * q + 2]) + __uint_as_float(y[4 * q + 2]), x.z * s4.z);
-                                x.w = fmaf(g.dt, __uint_as_float(w[4 * q + 3]) + __uint_as_float(y[4 * q + 3]), x.w * s4.w);
-                                *px = x;
-                                xo[4 * q] = valid ? (double)x.x : 0.0; xo[4 * q + 1] = valid ? (double)x.y : 0.0;
-                                xo[4 * q + 2] = valid ? (double)x.z : 0.0; xo[4 * q + 3] = valid ? (double)x.w : 0.0;
-                            }
-                            // sum over the 32 cells of this warp, fixed tree: each step halves the channels a lane carries
-#pragma unroll
-                            for (int wd = 8; wd >= 1; wd >>= 1) {
-                                const bool up = (lane & (wd * 2)) != 0;
-#pragma unroll
-                                for (int j = 0; j < wd; ++j) {
-                                    const double send = up ? xo[j] : xo[j + wd];
-                                    const double keep = up ? xo[j + wd] : xo[j];
-                                    xo[j] = keep + __shfl_xor_sync(0xffffffffu, send, wd * 2);
-                                }
-                            }
-                            xo[0] += __shfl_xor_sync(0xffffffffu, xo[0], 1);
-                            if ((lane & 1) == 0) {
-                                const int ch = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
-                                red[quad * 64 + c0 + ch] = xo[0];
-                            }
-                        }
-                        ptx::fence_proxy_async();      // X+ in shared memory, for the TMA stores issued behind the barrier
+                        k2f_epilogue(run, work, xt, scale + m.b * NC, cell, valid, red, g.dt, [&] { ptx::tc_fence_before(); ptx::mbar_arrive(&wk_empty[buf]); });
                         ptx::bar_sync(7, 128);
                         if (pt < NC) {
-                            const double t = (red[pt] + red[64 + pt]) + (red[128 + pt] + red[192 + pt]);
-                            const size_t o = (size_t)(m.b * tiles_per_grid + m.tile0 + b * strips) * NC + pt;
-                            const float hi = (float)t;
-                            fin.partial[o] = hi;
-                            fin.partial[o + fin.lo_offset] = (float)(t - (double)hi);
+                            k2f_store_sums(fin, red, (size_t)(m.b * tiles_per_grid + m.tile0 + b * strips), pt);
                             ptx::mbar_arrive(summed);
                         }
                         if (pt == 0) {
@@ -678,52 +736,19 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                     uint8_t* vs = es + k2f::E_BYTES;                        // [4][34] cells: V, then R in place
                     if (is_a) {
                         ptx::mbar_wait(&full[s], (it / k2f::NSTAGE) & 1, status, 540);
-                        if (col < k2f::VW) {
-#pragma unroll
-                            for (int j = 0; j < k2f::BR; ++j) {
-                                const float4* row = reinterpret_cast<const float4*>(es + (j * k2f::EW + col) * 128 + q * 16);
-                                const V4 hs = v4_add(v4_add(v4(row[0]), v4(row[8])), v4(row[16]));
-                                if (b >= 0 || j >= 2) {      // block -1: only its last two rows have all three E rows
-                                    float4* pv = reinterpret_cast<float4*>(vs + (j * k2f::VW + col) * 128 + q * 16);
-                                    *pv = v4_f4(v4_div(v4(*pv), v4_add(v4_add(h2, h1), hs)));
-                                }
-                                h2 = h1; h1 = hs;
-                            }
-                        }
+                        if (col < k2f::VW) k2f_box_e(es, vs, col, q, b < 0, h2, h1);
                         ptx::bar_arrive(1 + s, k2f::HANDOFF);       // R of this block is in the stage
                     } else {
                         const int buf = v & 1;
                         uint8_t* a_vp = sm + k2f::A_VP + buf * 3 * k2f::PART;
                         ptx::bar_sync(1 + s, k2f::HANDOFF);
                         if (b >= 0) ptx::mbar_wait(&vp_empty[buf], ((v >> 1) & 1) ^ 1, status, 541);   // its last UMMAs are done
-                        const uint8_t* ecol = es + (col + 2) * 128 + q * 16;      // this thread's column in the E rows
-#pragma unroll
-                        for (int j = 0; j < k2f::BR; ++j) {
-                            if (b >= 0 || j >= 2) {
-                                const float4* row = reinterpret_cast<const float4*>(vs + (j * k2f::VW + col) * 128 + q * 16);
-                                const V4 hs = v4_add(v4_add(v4(row[0]), v4(row[8])), v4(row[16]));
-                                if (b >= 0) {
-                                    // tile row j is macro-tile row 4b+j: its E came with the block before (j < 2, kept
-                                    // in registers) or is row j-2 of this block's E rows
-                                    const V4 e = v4(j == 0 ? ekeep0 : j == 1 ? ekeep1
-                                                    : *reinterpret_cast<const float4*>(ecol + (j - 2) * k2f::EW * 128));
-                                    const V4 out = v4_mul(e, v4_add(v4_add(h2, h1), hs));
-                                    uint32_t pa[3], pb[3];
-                                    split3(out.a, pa[0], pa[1], pa[2]);
-                                    split3(out.b, pb[0], pb[1], pb[2]);
-                                    uint8_t* dst = a_vp + swz64(j * k2f::SW + col, q >> 1) + (q & 1) * 8;
-#pragma unroll
-                                    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dst + p * k2f::PART) = make_uint2(pa[p], pb[p]);
-                                    const int orow = m.my0 + 4 * b + j, ocol = m.mx0 + col;
-                                    if (vprime != nullptr && orow < g.H && ocol < g.W)
-                                        *reinterpret_cast<float4*>(vprime + ((size_t)m.b * NH + (hh >> 1)) * vplane +
-                                                                   ((size_t)orow * g.W + ocol) * HD + (hh & 1) * 32 + q * 4) = v4_f4(out);
-                                }
-                                h2 = h1; h1 = hs;
-                            }
-                        }
-                        ekeep0 = *reinterpret_cast<const float4*>(ecol + 2 * k2f::EW * 128);
-                        ekeep1 = *reinterpret_cast<const float4*>(ecol + 3 * k2f::EW * 128);
+                        k2f_box_r(es, vs, a_vp, col, q, b < 0, h2, h1, ekeep0, ekeep1, [&](int j, const V4& out) {
+                            const int orow = m.my0 + 4 * b + j, ocol = m.mx0 + col;
+                            if (vprime != nullptr && orow < g.H && ocol < g.W)
+                                *reinterpret_cast<float4*>(vprime + ((size_t)m.b * NH + (hh >> 1)) * vplane +
+                                                           ((size_t)orow * g.W + ocol) * HD + (hh & 1) * 32 + q * 4) = v4_f4(out);
+                        });
                         if (b >= 0) {
                             ptx::fence_proxy_async();
                             ptx::mbar_arrive(&vp_full[buf]);
@@ -741,6 +766,219 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
     if (my_mt > 0)       // the last macro tile's sums; the stages and the operand tiles are free by now
         k2_finish_cta_call(fin, macro_tile(blockIdx.x + (my_mt - 1) * gridDim.x, mt_per_grid, strips, g.H, nbmax).b, tiles_per_grid, mt_per_grid,
                       reinterpret_cast<double*>(sm + k2f::STG), reinterpret_cast<int*>(sm + k2f::A_VP));
+}
+
+// =============================================================================================================
+// k2 for grids too small to fill the GPU: as k2_split_bf16, a cluster of four CTAs per macro tile, CTA r doing half-heads r,
+// r + 4, r + 8 and r + 12.  The 24 KB operands go to the tile's owner by bulk copies through distributed shared memory, into one
+// of two slots (use hh of slot hh % 2 waits for the owner's products of hh - 2), the owner issues the products and adds the
+// half-heads in their order: the same bits as k2_f32.  Measured, k2_f32 -> this: one grid of 32 x 32 47.4 -> 31.4 us, of 64 x 64
+// 49.2 -> 33.2 us, of 128 x 128 52.4 -> 46.8 us.  What bounds it is the chain of the two slots, copy, products, credit, eight
+// times over; more slots do not fit beside three stages of fp32 blocks.
+//   warps 0-7,19 A, 8-15 B;  warp 16 TMA producer of the E / V blocks, and behind them of the owner's state tile
+//   warp 18      sends operand tiles to the owners
+//   warp 17      owner: Wo slices and UMMA issuer;  warps 20-23 owner: P
+namespace k2fs {
+constexpr int C = 4, ROUNDS = k2f::NHH / C, NSTAGE = 3;
+constexpr int OPERAND = 3 * k2f::PART, WO_SLICE = 3 * k2f::WO_PART;
+constexpr int STG = 0;
+constexpr int A_VP = STG + NSTAGE * k2f::STAGE_BYTES;    // two operand tiles of this CTA's half-heads
+constexpr int SLOT = A_VP + 2 * OPERAND;                 // two of the owned tile's
+constexpr int WO = SLOT + 2 * OPERAND;                   // two Wo slices
+constexpr int RED = SLOT;                                // [4 quads][64] fp64, once the slots are done with
+constexpr int BARS = WO + 2 * WO_SLICE;
+constexpr int N_BARS = 2 * NSTAGE + 14 + C;
+constexpr int TMEM_PTR = BARS + N_BARS * 8;
+constexpr int SMEM = TMEM_PTR + 16 + 1024;
+constexpr uint32_t TMEM_COLS = 256, WORK = 64;           // the running sum, two working accumulators behind
+static_assert(A_VP % 1024 == 0 && SLOT % 1024 == 0 && WO % 1024 == 0, "swizzled tiles must be aligned");
+static_assert(SMEM <= 227 * 1024, "k2 (split, fp32) shared memory");
+}  // namespace k2fs
+
+__global__ void __cluster_dims__(k2fs::C, 1, 1) __launch_bounds__(k2f::THREADS, 1)
+k2_split_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUtensorMap map_e,
+             const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ scale,
+             const K2Sums fin, float* __restrict__ vprime, int* __restrict__ status,
+             int mt_per_grid, int strips, int tiles_per_grid, int nbmax, Geom g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = align1024(smem_raw);
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm + k2fs::BARS);   // [3] block landed                               (waits: A)
+    uint64_t* empty = full + k2fs::NSTAGE;           // [3] B is done with the stage (256 arrivals)   (waits: TMA producer)
+    uint64_t* vp_full = empty + k2fs::NSTAGE;        // [2] operand tile written (256 arrivals)       (waits: sender)
+    uint64_t* vp_empty = vp_full + 2;                // [2] ... and landed at its owner (who arrives) (waits: B)
+    uint64_t* wo_full = vp_empty + 2;                // [2] Wo slice landed                           (waits: UMMA issuer)
+    uint64_t* wo_empty = wo_full + 2;                // [2] its half-head is issued and done          (waits: UMMA issuer)
+    uint64_t* wk_full = wo_empty + 2;                // [2] working accumulator complete              (waits: P)
+    uint64_t* wk_empty = wk_full + 2;                // [2] ... and added (128 arrivals)              (waits: UMMA issuer)
+    uint64_t* slot_full = wk_empty + 2;              // [2] operand landed                            (waits: UMMA issuer)
+    uint64_t* slot_ok = slot_full + 2;               // [4] this CTA's next slot at owner b is free (the owner's commit)  (waits: sender)
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k2fs::TMEM_PTR);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x % k2fs::C;
+    if (tid == 0) {
+        for (int i = 0; i < k2fs::NSTAGE; ++i) { ptx::mbar_init(&full[i], 1); ptx::mbar_init(&empty[i], k2f::B_THREADS); }
+        for (int i = 0; i < 2; ++i) {
+            ptx::mbar_init(&vp_full[i], k2f::B_THREADS); ptx::mbar_init(&vp_empty[i], 1);
+            ptx::mbar_init(&wo_full[i], 1); ptx::mbar_init(&wo_empty[i], 1);
+            ptx::mbar_init(&wk_full[i], 1); ptx::mbar_init(&wk_empty[i], 128);
+            ptx::mbar_init(&slot_full[i], 1);
+        }
+        for (int i = 0; i < k2fs::C; ++i) ptx::mbar_init(&slot_ok[i], 1);
+        ptx::fence_barrier_init();
+        for (int i = 0; i < 2; ++i) ptx::mbar_expect_tx(&slot_full[i], k2fs::OPERAND);       // half-heads 0 and 1
+        ptx::prefetch_tmap(&map_wo); ptx::prefetch_tmap(&map_e); ptx::prefetch_tmap(&map_v); ptx::prefetch_tmap(&map_x);
+    }
+    if (warp == 0) ptx::tmem_alloc(tmem_ptr, k2fs::TMEM_COLS);
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = *tmem_ptr;
+    ptx::cluster_sync();                 // the others' barriers are there
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    const MacroTile m = macro_tile(blockIdx.x / k2fs::C, mt_per_grid, strips, g.H, nbmax);
+    const bool owner = rank < m.nb;
+    const int blocks = k2fs::ROUNDS * (m.nb + 1), x_stage = blocks % k2fs::NSTAGE;     // the state tile comes behind the blocks
+    uint8_t* xt = sm + k2fs::STG + x_stage * k2f::STAGE_BYTES;
+
+    if (warp == 16) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            for (int round = 0; round < k2fs::ROUNDS; ++round)
+                for (int b = -1; b < m.nb; ++b, ++it) {
+                    const int s = it % k2fs::NSTAGE, hh = round * k2fs::C + rank, plane = m.b * NH + (hh >> 1), d0 = (hh & 1) * 32;
+                    uint8_t* st = sm + k2fs::STG + s * k2f::STAGE_BYTES;
+                    ptx::mbar_wait(&empty[s], ((it / k2fs::NSTAGE) & 1) ^ 1, status, 550);
+                    ptx::mbar_expect_tx(&full[s], k2f::STAGE_BYTES);
+                    ptx::tma_load_4d(st, &map_e, d0, m.mx0, m.my0 + 4 * b + 4, plane, &full[s]);
+                    ptx::tma_load_4d(st + k2f::E_BYTES, &map_v, d0, m.mx0 + 1, m.my0 + 4 * b + 3, plane, &full[s]);
+                }
+            if (owner) {
+                ptx::mbar_wait(&empty[x_stage], ((it / k2fs::NSTAGE) & 1) ^ 1, status, 551);
+                ptx::mbar_expect_tx(&full[x_stage], 32768);
+                ptx::tma_load_4d(xt, &map_x, 0, m.mx0, g.hx + m.my0 + rank * k2f::BR, m.b, &full[x_stage]);
+                ptx::tma_load_4d(xt + 16384, &map_x, 32, m.mx0, g.hx + m.my0 + rank * k2f::BR, m.b, &full[x_stage]);
+            }
+        }
+    } else if (warp == 18) {
+        if (lane == 0) {
+            uint32_t v = 0;
+            for (int round = 0; round < k2fs::ROUNDS; ++round)
+                for (int b = 0; b < m.nb; ++b, ++v) {
+                    const int buf = v & 1, hh = round * k2fs::C + rank, slot = hh & 1;
+                    ptx::mbar_wait(&vp_full[buf], (v >> 1) & 1, status, 552);
+                    if (hh >= 2) ptx::mbar_wait(&slot_ok[b], ((hh - 2) >> 2) & 1, status, 553);
+                    ptx::bulk_copy_to_cta(sm + k2fs::SLOT + slot * k2fs::OPERAND, sm + k2fs::A_VP + buf * k2fs::OPERAND, k2fs::OPERAND,
+                                          &slot_full[slot], b);
+                }
+        }
+    } else if (warp == 17) {
+        if (owner) {
+            const uint32_t leader = ptx::elect_one();
+            const uint32_t a0 = ptx::smem_u32(sm + k2fs::SLOT) >> 4, w0 = ptx::smem_u32(sm + k2fs::WO) >> 4;
+            const int set = m.b / g.per_set;
+            auto load_wo = [&](int hh) {
+                const int i = hh & 1;
+                ptx::mbar_wait(&wo_empty[i], ((hh >> 1) & 1) ^ 1, status, 554);
+                if (lane == 0) {
+                    ptx::mbar_expect_tx(&wo_full[i], k2fs::WO_SLICE);
+                    ptx::tma_load_2d(sm + k2fs::WO + i * k2fs::WO_SLICE, &map_wo, 0, (set * k2f::NHH + hh) * 192, &wo_full[i]);
+                }
+                __syncwarp();
+            };
+            load_wo(0);
+            for (int hh = 0; hh < k2f::NHH; ++hh) {
+                const int i = hh & 1, r = hh % k2fs::C, round = hh / k2fs::C;
+                if (hh + 1 < k2f::NHH) load_wo(hh + 1);
+                ptx::mbar_wait(&slot_full[i], (hh >> 1) & 1, status, 555);
+                if (lane == 0) {
+                    // the sender may write its operand tile again (its use number round * nb + rank)
+                    ptx::mbar_arrive_remote(&vp_empty[(round * m.nb + rank) & 1], r);
+                    if (hh + 2 < k2f::NHH) ptx::mbar_expect_tx(&slot_full[i], k2fs::OPERAND);
+                }
+                __syncwarp();
+                ptx::mbar_wait(&wo_full[i], (hh >> 1) & 1, status, 556);
+                ptx::mbar_wait(&wk_empty[i], ((hh >> 1) & 1) ^ 1, status, 557);
+                ptx::tc_fence_after();
+                k2f_products(leader, tmem + k2fs::WORK + i * 64, a0 + i * (k2fs::OPERAND >> 4), w0 + i * (k2fs::WO_SLICE >> 4));
+                ptx::umma_commit_by(leader, &wo_empty[i]);
+                if (hh + 2 < k2f::NHH) ptx::umma_commit_remote_by(leader, &slot_ok[rank], 1u << ((hh + 2) % k2fs::C));
+                ptx::umma_commit_by(leader, &wk_full[i]);
+            }
+        }
+    } else if (warp >= 20) {
+        if (owner) {
+            const int quad = warp & 3, cell = quad * 32 + lane, pt = tid - 640;
+            const uint32_t run = tmem + ((uint32_t)(quad * 32) << 16);
+            double* red = reinterpret_cast<double*>(sm + k2fs::RED);
+            for (int hh = 0; hh < k2f::NHH; ++hh) {
+                const int i = hh & 1;
+                const uint32_t work = run + k2fs::WORK + i * 64;
+                ptx::mbar_wait(&wk_full[i], (hh >> 1) & 1, status, 560);
+                ptx::tc_fence_after();
+                if (hh < k2f::NHH - 1) {
+                    k2f_add(run, work, hh > 0);
+                    ptx::tc_fence_before();
+                    ptx::mbar_arrive(&wk_empty[i]);
+                } else {
+                    const int ty0 = m.my0 + rank * k2f::BR;
+                    const bool valid = ty0 + (cell >> 5) < g.H && m.mx0 + (cell & 31) < g.W;
+                    ptx::mbar_wait(&full[x_stage], (blocks / k2fs::NSTAGE) & 1, status, 561);
+                    k2f_epilogue(run, work, xt, scale + m.b * NC, cell, valid, red, g.dt, [] {});
+                    ptx::bar_sync(7, 128);
+                    if (pt < NC) k2f_store_sums(fin, red, (size_t)(m.b * tiles_per_grid + m.tile0 + rank * strips), pt);
+                    if (pt == 0) {
+                        ptx::tma_store_4d(&map_x, xt, 0, m.mx0, g.hx + ty0, m.b);
+                        ptx::tma_store_4d(&map_x, xt + 16384, 32, m.mx0, g.hx + ty0, m.b);
+                        ptx::bulk_commit();
+                        ptx::bulk_wait0();
+                    }
+                }
+            }
+        }
+    } else {
+        const bool is_a = warp < 8 || warp == 19;
+        const int gt = warp == 19 ? 256 + lane : (is_a ? tid : tid - 256);     // thread within its set
+        const int q = gt & 7, col = gt >> 3;
+        uint32_t it = 0, v = 0;
+        const V4 zero = v4(make_float4(0.f, 0.f, 0.f, 0.f));
+        V4 h2 = zero, h1 = zero;
+        float4 ekeep0 = make_float4(0.f, 0.f, 0.f, 0.f), ekeep1 = ekeep0;
+        const size_t vplane = (size_t)g.H * g.W * HD;
+        for (int round = 0; round < k2fs::ROUNDS; ++round)
+            for (int b = -1; b < m.nb; ++b, ++it) {
+                const int s = it % k2fs::NSTAGE, hh = round * k2fs::C + rank;
+                uint8_t* es = sm + k2fs::STG + s * k2f::STAGE_BYTES;
+                uint8_t* vs = es + k2f::E_BYTES;
+                if (is_a) {
+                    ptx::mbar_wait(&full[s], (it / k2fs::NSTAGE) & 1, status, 570);
+                    if (col < k2f::VW) k2f_box_e(es, vs, col, q, b < 0, h2, h1);
+                    ptx::bar_arrive(1 + s, k2f::HANDOFF);
+                } else {
+                    const int buf = v & 1;
+                    ptx::bar_sync(1 + s, k2f::HANDOFF);
+                    if (b >= 0) ptx::mbar_wait(&vp_empty[buf], ((v >> 1) & 1) ^ 1, status, 571);
+                    k2f_box_r(es, vs, sm + k2fs::A_VP + buf * k2fs::OPERAND, col, q, b < 0, h2, h1, ekeep0, ekeep1, [&](int j, const V4& out) {
+                        const int orow = m.my0 + 4 * b + j, ocol = m.mx0 + col;
+                        if (vprime != nullptr && orow < g.H && ocol < g.W)
+                            *reinterpret_cast<float4*>(vprime + ((size_t)m.b * NH + (hh >> 1)) * vplane + ((size_t)orow * g.W + ocol) * HD +
+                                                       (hh & 1) * 32 + q * 4) = v4_f4(out);
+                    });
+                    if (b >= 0) {
+                        ptx::fence_proxy_async();
+                        ptx::mbar_arrive(&vp_full[buf]);
+                        ++v;
+                    }
+                    ptx::mbar_arrive(&empty[s]);
+                }
+            }
+    }
+    ptx::tc_fence_before();
+    ptx::cluster_sync();                 // nobody's shared memory or barriers are written any more
+    if (warp == 0) ptx::tmem_dealloc(tmem, k2fs::TMEM_COLS);
+    if (owner)                           // every tile is one CTA's
+        k2_finish_cta(fin, m.b, tiles_per_grid, tiles_per_grid, reinterpret_cast<double*>(sm + k2fs::STG), reinterpret_cast<int*>(sm + k2fs::A_VP));
 }
 
 // =============================================================================================================
@@ -794,7 +1032,8 @@ inline int f32_setup(F32Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16* w
         return -1;
     }
     if (cudaFuncSetAttribute(k1_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, k1f::SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(k2_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, k2f::SMEM) != cudaSuccess) {
+        cudaFuncSetAttribute(k2_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, k2f::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k2_split_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, k2fs::SMEM) != cudaSuccess) {
         bf16_error_ref() = "could not opt in to the kernels' dynamic shared memory";
         return -1;
     }
@@ -802,6 +1041,7 @@ inline int f32_setup(F32Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16* w
     p.k1_grid = (int)(items < num_sms ? items : num_sms);
     const long long total_mt = k2_macro_tiles(g, p.strips, k2f::NB, num_sms, p.nbmax, p.mt_per_grid);
     p.k2_grid = (int)(total_mt < num_sms ? total_mt : num_sms);
+    p.split_grid = k2_split_grid(g, p.strips, k2fs::C, max_clusters(k2_split_f32, k2fs::C, k2f::THREADS, k2fs::SMEM), p.nbmax, p.mt_per_grid);
     return 0;
 }
 

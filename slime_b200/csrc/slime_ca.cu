@@ -196,7 +196,11 @@ int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nul
                          (float*)h->E, (float*)h->V, h->dev_status, p.k1_tiles * g.B, p.k1_tiles, g));
         ++h->launches;
         if (ev) CK(h, cudaEventRecord(ev[1], st));
-        CK(h, launch_pdl(k2_f32, p.k2_grid, k2f::THREADS, k2f::SMEM, st, p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, fin, (float*)emit,
+        if (p.split_grid)
+            CK(h, launch_pdl(k2_split_f32, p.split_grid, k2f::THREADS, k2fs::SMEM, st, p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, fin,
+                             (float*)emit, h->dev_status, p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g));
+        else
+            CK(h, launch_pdl(k2_f32, p.k2_grid, k2f::THREADS, k2f::SMEM, st, p.map_wo, p.map_e, p.map_v, p.map_x, h->scale, fin, (float*)emit,
                          h->dev_status, p.mt_per_grid * g.B, p.mt_per_grid, p.strips, p.k2_tiles, p.nbmax, g));
         ++h->launches;
     }

@@ -124,17 +124,19 @@ def test_unaligned_device_pointers(gpu, dtype_name):
 
 
 @pytest.mark.parametrize("shape,copies", [((1, 5, 9), 150), ((1, 16, 33), 64), ((2, 30, 70), 40), ((1, 128, 128), 6)])
-def test_bf16_grids_do_not_depend_on_the_batch(gpu, shape, copies):
+@pytest.mark.parametrize("dtype_name", ["f32", "bf16"])
+def test_grids_do_not_depend_on_the_batch(gpu, shape, copies, dtype_name):
     """A few grids alone (a cluster of CTAs per macro tile of one, two or four blocks) and many times over in one batch
     (one CTA per macro tile): the same bits, V' included."""
     import torch
     capi, devmem = gpu
     B, H, W = shape
+    dtype = capi.F32 if dtype_name == "f32" else capi.BF16
     X0 = bf16_round(inputs.make_state(B, H, W, seed=29, scale=0.45 * H * W))
     w = inputs.make_weight_sets(1, seed=29, bounded=True)
     outs = []
     for n in (1, copies):
-        with capi.Handle(B * n, H, W, dtype=capi.BF16, keep_vprime=True) as h:
+        with capi.Handle(B * n, H, W, dtype=dtype, keep_vprime=True) as h:
             h.set_weights(w)
             h.set_state(np.tile(X0, (n, 1, 1, 1)))
             h.step(3)
