@@ -393,9 +393,11 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
 // that a block of 4 rows has the byte shape of a bf16 block (128 bytes a cell) and a thread owns 4 dims.
 //   warps 0-7,19 A: R = V / box3(E) in place in the stage
 //   warps 8-15   B: V' = E * box3(R), split into the three parts of the A operand
-//   warp 16      TMA producer: per (macro tile, half-head) the parts of its Wo slice, per block E and V
+//   warp 16      TMA producer: per (macro tile, half-head) the parts of its Wo slice, per block E and V; behind the blocks of
+//                the last half-head the tiles' state, through the same ring (three stages and a state buffer of its own: 1 to
+//                3 % slower)
 //   warp 17      UMMA issuer: the half-head's share of Y (N=64, K=32, six products) into one of two working accumulators
-//   warp 18      TMA producer of the epilogue's state tiles
+//   warp 18      the grids' sums
 //   warps 20-23  P: adds every working accumulator to the tile's running sum in TMEM, rounded to nearest (16 half-heads:
 //                on the tensor core that sum would be truncated 192 times); after the last half-head X+ = scale X + dt Y,
 //                written back through shared memory, and the tile's channel sums in fp64
@@ -404,15 +406,14 @@ constexpr int SW = k2m::SW, BR = k2m::BR, NB = 6;       // strip width, rows per
 constexpr int NHH = 2 * NH;                             // half-heads
 constexpr int EW = k2m::EW, VW = k2m::VW;
 constexpr int E_BYTES = k2m::E_BYTES, STAGE_BYTES = k2m::STAGE_BYTES;
-constexpr int NSTAGE = 3;
+constexpr int NSTAGE = 4;
 constexpr int STG = 0;
 constexpr int PART = 8192;                              // one part of the operand tile: [128 cells][32] bf16, 64-byte rows
 constexpr int A_VP = STG + NSTAGE * STAGE_BYTES;        // two operand tiles of 3 parts
 constexpr int WO_PART = 4096, WO = A_VP + 2 * 3 * PART; // two Wo slices of 3 parts [64][32]
-constexpr int XT = WO + 2 * 3 * WO_PART;                // state tile of the epilogue: two halves of 32 channels, 16 KB each
-constexpr int RED = XT + 2 * 16384;                     // [4 quads][64] fp64
+constexpr int RED = WO + 2 * 3 * WO_PART;               // [4 quads][64] fp64
 constexpr int BARS = RED + 4 * 64 * 8;
-constexpr int N_BARS = 2 * NSTAGE + 13;
+constexpr int N_BARS = 2 * NSTAGE + 16;
 constexpr int TMEM_PTR = BARS + N_BARS * 8;
 constexpr int BYTES = TMEM_PTR + 16;
 constexpr int SMEM = BYTES + 1024;
@@ -420,7 +421,7 @@ constexpr uint32_t TMEM_COLS = 512, WORK = NB * 64;     // running sums of up to
 constexpr int A_THREADS = k2m::A_THREADS, B_THREADS = k2m::B_THREADS;
 constexpr int THREADS = 768;
 constexpr int HANDOFF = A_THREADS + B_THREADS;
-static_assert(A_VP % 1024 == 0 && WO % 1024 == 0 && XT % 1024 == 0, "swizzled tiles must be aligned");
+static_assert(A_VP % 1024 == 0 && WO % 1024 == 0 && STAGE_BYTES % 1024 == 0, "swizzled tiles must be aligned");
 static_assert(SMEM <= 227 * 1024, "k2 (fp32) shared memory");
 }  // namespace k2f
 
@@ -578,17 +579,17 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + k2f::BARS);
-    uint64_t* full = bars;                           // [3] block landed                              (waits: A)
-    uint64_t* empty = full + k2f::NSTAGE;            // [3] B is done with the stage (256 arrivals)   (waits: TMA producer)
+    uint64_t* full = bars;                           // [4] block landed                              (waits: A)
+    uint64_t* empty = full + k2f::NSTAGE;            // [4] B is done with the block, P with the state tile (256 arrivals)  (waits: TMA producer)
     uint64_t* vp_full = empty + k2f::NSTAGE;         // [2] operand tile written (256 arrivals)       (waits: UMMA issuer)
     uint64_t* vp_empty = vp_full + 2;                // [2] the UMMAs reading it are done             (waits: B)
     uint64_t* wo_full = vp_empty + 2;                // [2] Wo slice landed                           (waits: UMMA issuer)
     uint64_t* wo_empty = wo_full + 2;                // [2] its half-head is issued and done          (waits: TMA producer)
     uint64_t* wk_full = wo_empty + 2;                // [2] working accumulator complete              (waits: P)
     uint64_t* wk_empty = wk_full + 2;                // [2] ... and added (128 arrivals)              (waits: UMMA issuer)
-    uint64_t* x_full = wk_empty + 2;                 // state tile landed                             (waits: P)
-    uint64_t* x_empty = x_full + 1;                  // ... and its X+ has left shared memory          (waits: state producer)
-    uint64_t* summed = x_full + 2;                   // the tile's sums are written (64 arrivals)       (waits: state producer)
+    uint64_t* x_full = wk_empty + 2;                 // [2] state tile landed (no more than two are under way)  (waits: P)
+    uint64_t* summed = x_full + 2;                   // the macro tile's sums are written (64 arrivals) (waits: warp 18)
+    uint64_t* added = summed + 1;                    // ... and warp 18 is done with them               (waits: P)
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(sm + k2f::TMEM_PTR);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -598,8 +599,9 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
             ptx::mbar_init(&vp_full[i], k2f::B_THREADS); ptx::mbar_init(&vp_empty[i], 1);
             ptx::mbar_init(&wo_full[i], 1); ptx::mbar_init(&wo_empty[i], 1);
             ptx::mbar_init(&wk_full[i], 1); ptx::mbar_init(&wk_empty[i], 128);
+            ptx::mbar_init(&x_full[i], 1);
         }
-        ptx::mbar_init(x_full, 1); ptx::mbar_init(x_empty, 1); ptx::mbar_init(summed, NC);
+        ptx::mbar_init(summed, NC); ptx::mbar_init(added, 1);
         ptx::fence_barrier_init();
         ptx::prefetch_tmap(&map_wo); ptx::prefetch_tmap(&map_e); ptx::prefetch_tmap(&map_v); ptx::prefetch_tmap(&map_x);
     }
@@ -615,7 +617,7 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
     if (warp == 16) {
         // ================= TMA producer ===================================================================
         if (lane == 0) {
-            uint32_t it = 0, wit = 0;       // blocks and half-heads so far
+            uint32_t it = 0, wit = 0, nx = 0;       // stage uses, half-heads and state tiles so far
             for (int k = 0; k < my_mt; ++k) {
                 const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
                 const int set = m.b / g.per_set;
@@ -631,26 +633,26 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                         ptx::mbar_expect_tx(&full[s], k2f::STAGE_BYTES);
                         ptx::tma_load_4d(st, &map_e, d0, m.mx0, m.my0 + 4 * b + 4, plane, &full[s]);
                         ptx::tma_load_4d(st + k2f::E_BYTES, &map_v, d0, m.mx0 + 1, m.my0 + 4 * b + 3, plane, &full[s]);
+                        if (b >= 0 && hh == k2f::NHH - 1) {      // behind a tile's last block its state, for the epilogue
+                            const int sx = ++it % k2f::NSTAGE;
+                            uint8_t* xt = sm + k2f::STG + sx * k2f::STAGE_BYTES;
+                            ptx::mbar_wait(&empty[sx], ((it / k2f::NSTAGE) & 1) ^ 1, status, 512);
+                            uint64_t* bar = &x_full[nx++ & 1];
+                            ptx::mbar_expect_tx(bar, 32768);
+                            ptx::tma_load_4d(xt, &map_x, 0, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, bar);
+                            ptx::tma_load_4d(xt + 16384, &map_x, 32, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, bar);
+                        }
                     }
                 }
             }
         }
     } else if (warp == 18) {
-        // ================= TMA producer of the epilogue's state tiles, and the grids' sums ==========================
-        uint32_t nx = 0;
+        // ================= the grids' sums, but for the last macro tile's ==============================================
         for (int k = 0; k < my_mt; ++k) {
-            const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
-            for (int b = 0; b < m.nb; ++b, ++nx) {
-                ptx::mbar_wait(x_empty, (nx & 1) ^ 1, status, 512);
-                if (b > 0) ptx::mbar_wait(summed, (nx - 1) & 1, status, 513);
-                if (lane == 0) {
-                    ptx::mbar_expect_tx(x_full, 32768);
-                    ptx::tma_load_4d(sm + k2f::XT, &map_x, 0, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, x_full);
-                    ptx::tma_load_4d(sm + k2f::XT + 16384, &map_x, 32, m.mx0, g.hx + m.my0 + b * k2f::BR, m.b, x_full);
-                }
-            }
-            ptx::mbar_wait(summed, (nx - 1) & 1, status, 514);
-            if (k < my_mt - 1) k2_finish_call(fin, m.b, tiles_per_grid, mt_per_grid);
+            ptx::mbar_wait(summed, k & 1, status, 514);
+            if (k < my_mt - 1) k2_finish_call(fin, macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax).b, tiles_per_grid, mt_per_grid);
+            if (lane == 0) ptx::mbar_arrive(added);
+            __syncwarp();
         }
     } else if (warp == 17) {
         // ================= UMMA issuer (the whole warp, its leader executes) ==================================
@@ -678,9 +680,8 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
         // ================= P: running sums, then the epilogue ==================================================
         const int quad = warp & 3, cell = quad * 32 + lane, pt = tid - 640;
         const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16);
-        uint8_t* xt = sm + k2f::XT;
         double* red = reinterpret_cast<double*>(sm + k2f::RED);
-        uint32_t v = 0, nx = 0;
+        uint32_t v = 0, it = 0, nx = 0;      // operand tiles added; stage uses before this macro tile; state tiles
         for (int k = 0; k < my_mt; ++k) {
             const MacroTile m = macro_tile(blockIdx.x + k * gridDim.x, mt_per_grid, strips, g.H, nbmax);
             for (int hh = 0; hh < k2f::NHH; ++hh) {
@@ -696,25 +697,28 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                     } else {
                         const int ty0 = m.my0 + b * k2f::BR;
                         const bool valid = ty0 + (cell >> 5) < g.H && m.mx0 + (cell & 31) < g.W;
-                        ptx::mbar_wait(x_full, nx & 1, status, 531);
+                        const int sx = (it + (k2f::NHH - 1) * (m.nb + 1) + 2 + 2 * b) % k2f::NSTAGE;     // the state tile's stage
+                        uint8_t* xt = sm + k2f::STG + sx * k2f::STAGE_BYTES;
+                        ptx::mbar_wait(&x_full[nx & 1], (nx >> 1) & 1, status, 531);
+                        ++nx;
                         k2f_epilogue(run, work, xt, scale + m.b * NC, cell, valid, red, g.dt, [&] { ptx::tc_fence_before(); ptx::mbar_arrive(&wk_empty[buf]); });
                         ptx::bar_sync(7, 128);
                         if (pt < NC) {
                             k2f_store_sums(fin, red, (size_t)(m.b * tiles_per_grid + m.tile0 + b * strips), pt);
-                            ptx::mbar_arrive(summed);
+                            if (b == m.nb - 1) { ptx::mbar_wait(added, (k & 1) ^ 1, status, 532); ptx::mbar_arrive(summed); }
                         }
                         if (pt == 0) {
                             ptx::tma_store_4d(&map_x, xt, 0, m.mx0, g.hx + ty0, m.b);
                             ptx::tma_store_4d(&map_x, xt + 16384, 32, m.mx0, g.hx + ty0, m.b);
                             ptx::bulk_commit();
                             ptx::bulk_wait_read0();
-                            ptx::mbar_arrive(x_empty);
+                            ptx::mbar_arrive_n(&empty[sx], k2f::B_THREADS);
                         }
                         ptx::bar_sync(7, 128);         // the reduction scratch is free again
-                        ++nx;
                     }
                 }
             }
+            it += k2f::NHH * (m.nb + 1) + m.nb;
         }
         if (pt == 0) ptx::bulk_wait0();
     } else {
@@ -722,7 +726,7 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
         const bool is_a = warp < 8 || warp == 19;
         const int gt = warp == 19 ? 256 + lane : (is_a ? tid : tid - 256);     // thread within its set
         const int q = gt & 7, col = gt >> 3;                    // 4-dim chunk; column (A: of the 34 R columns, B: of the 32)
-        uint32_t it = 0, v = 0;
+        uint32_t it = 0, v = 0, phase = 0;      // stage uses, operand tiles; A: parity of each stage's next block
         const V4 zero = v4(make_float4(0.f, 0.f, 0.f, 0.f));
         V4 h2 = zero, h1 = zero;             // running horizontal sums of the two rows above (of E in A, of R in B)
         float4 ekeep0 = make_float4(0.f, 0.f, 0.f, 0.f), ekeep1 = ekeep0;      // B: centre E of the last two rows of the block before
@@ -735,7 +739,8 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                     uint8_t* es = sm + k2f::STG + s * k2f::STAGE_BYTES;     // [4][36] cells x 128 B
                     uint8_t* vs = es + k2f::E_BYTES;                        // [4][34] cells: V, then R in place
                     if (is_a) {
-                        ptx::mbar_wait(&full[s], (it / k2f::NSTAGE) & 1, status, 540);
+                        ptx::mbar_wait(&full[s], (phase >> s) & 1, status, 540);
+                        phase ^= 1u << s;
                         if (col < k2f::VW) k2f_box_e(es, vs, col, q, b < 0, h2, h1);
                         ptx::bar_arrive(1 + s, k2f::HANDOFF);       // R of this block is in the stage
                     } else {
@@ -756,6 +761,7 @@ k2_f32(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUten
                         }
                         ptx::mbar_arrive(&empty[s]);
                     }
+                    if (b >= 0 && hh == k2f::NHH - 1) ++it;      // the next stage use is a state tile
                 }
             }
         }
