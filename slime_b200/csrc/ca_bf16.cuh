@@ -847,7 +847,7 @@ __device__ __forceinline__ void k2_box_r(const uint8_t* es, const uint8_t* vs, u
 struct MacroTile {
     int b, mx0, my0, nb, tile0;     // tile0: index of its first 4 x 32 tile among the grid's partial sums
 };
-// nbmax: blocks per full macro tile of this launch (8, 4, 2 or 1)
+// nbmax: blocks per full macro tile of this launch
 __device__ __forceinline__ MacroTile macro_tile(int idx, int per_grid, int strips, int H, int nbmax) {
     MacroTile m;
     m.b = idx / per_grid;
@@ -1075,7 +1075,7 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
 }
 
 // =============================================================================================================
-// k2 for grids too small to fill the GPU: a cluster of four CTAs per macro tile of one, two or four blocks, CTA r doing the
+// k2 for grids too small to fill the GPU: a cluster of four CTAs per macro tile of one to four blocks, CTA r doing the
 // box sums of heads r and r + 4.  One CTA alone marches 8 heads x (blocks + 1) however few macro tiles there are (16 blocks of
 // work at the least, 25 us for a 32 x 32 grid); here it is 2 x (blocks + 1).  A block's V' operand goes to the CTA that owns
 // the tile (tile b: CTA b), by a bulk copy through distributed shared memory, and the owner issues the products of the eight
@@ -1301,19 +1301,26 @@ inline int make_plane_map(EncodeTiledFn enc, CUtensorMap* map, const void* base,
 }
 
 // Blocks per macro tile of k2 (at most `most`).  A taller macro tile re-primes its march less often (nb + 1 blocks of work
-// for nb tiles) but gives fewer, coarser units to spread over the SMs: take the height with the best product of the two.
-// -> macro tiles of the launch.
+// for nb tiles) but gives fewer, coarser units to spread over the SMs: take the height whose busiest CTA has the fewest
+// blocks, counted out, the taller at a tie.  (Macro tiles x waves as the measure, as it was, took 5 + 5 + 5 + 1 blocks a
+// strip where 4 + 4 + 4 + 4 has five sixths of the march, and 8 + 2 for 5 + 5.)  -> macro tiles of the launch.
 inline long long k2_macro_tiles(const Geom& g, int strips, int most, int num_sms, int& nbmax, int& mt_per_grid) {
-    long long total_mt = 0;
-    double best = -1.0;
+    long long total_mt = 0, best = -1;
     const int rows4 = (g.H + k2m::BR - 1) / k2m::BR;
-    for (int nb = most; nb >= 1; --nb) {
+    for (int nb = most < rows4 ? most : rows4; nb >= 1; --nb) {
         const int mt_rows = (rows4 + nb - 1) / nb;
-        const long long total = (long long)strips * mt_rows * g.B;
-        const double per_mt = (double)rows4 / mt_rows;                         // tiles per macro tile on average
-        const long long waves = (total + num_sms - 1) / num_sms;
-        const double eff = per_mt / (per_mt + 1.0) * (double)total / (double)(waves * num_sms);
-        if (eff > best) { best = eff; nbmax = nb; mt_per_grid = strips * mt_rows; total_mt = total; }
+        const long long total = (long long)strips * mt_rows * g.B, blocks = (long long)strips * g.B * (rows4 + mt_rows);
+        if (best >= 0 && blocks >= best * num_sms) continue;                   // not even if spread evenly
+        long long busiest = 0;
+        for (int cta = 0; cta < num_sms && cta < total; ++cta) {
+            long long mine = 0;
+            for (long long t = cta; t < total; t += num_sms) {
+                const int left = rows4 - (int)(t / strips % mt_rows) * nb;
+                mine += (left < nb ? left : nb) + 1;
+            }
+            if (mine > busiest) busiest = mine;
+        }
+        if (best < 0 || busiest < best) { best = busiest; nbmax = nb; mt_per_grid = strips * mt_rows; total_mt = total; }
     }
     return total_mt;
 }
@@ -1322,7 +1329,7 @@ inline long long k2_macro_tiles(const Geom& g, int strips, int most, int num_sms
 // the fewest blocks per macro tile that allows it.  0 where there are too many macro tiles; nbmax and mt_per_grid then stay.
 inline int k2_split_grid(const Geom& g, int strips, int c, int most, int& nbmax, int& mt_per_grid) {
     const int rows4 = (g.H + k2m::BR - 1) / k2m::BR;
-    for (int nb = 1; nb <= c; nb *= 2) {
+    for (int nb = 1; nb <= c; ++nb) {
         const long long mt = (long long)strips * ((rows4 + nb - 1) / nb);
         if (mt * g.B > most) continue;
         nbmax = nb;

@@ -123,10 +123,10 @@ def test_unaligned_device_pointers(gpu, dtype_name):
     assert torch.equal(outs[0], outs[1])
 
 
-@pytest.mark.parametrize("shape,copies", [((1, 5, 9), 150), ((1, 16, 33), 64), ((2, 30, 70), 40), ((1, 128, 128), 6)])
+@pytest.mark.parametrize("shape,copies", [((1, 5, 9), 150), ((1, 16, 33), 64), ((2, 30, 70), 40), ((1, 90, 110), 17), ((1, 128, 128), 6)])
 @pytest.mark.parametrize("dtype_name", ["f32", "bf16"])
 def test_grids_do_not_depend_on_the_batch(gpu, shape, copies, dtype_name):
-    """A few grids alone (a cluster of CTAs per macro tile of one, two or four blocks) and many times over in one batch
+    """A few grids alone (a cluster of CTAs per macro tile of one to four blocks) and many times over in one batch
     (one CTA per macro tile): the same bits, V' included."""
     import torch
     capi, devmem = gpu
