@@ -120,7 +120,7 @@ struct Bf16Plan {
     CUtensorMap map_v;    // V planes, box 64 x 34 x 4 x 1
     CUtensorMap map_x;    // the state's own rows (and the halo rows above them) [B][hx + H][W][64], box 64 x 32 x 4 x 1, 128B swizzle
     K1StoreMaps st;       // store maps of k1 (whole tile, last two columns, last two rows, their corner)
-    bool k1_aligned = false;
+    bool k1_pieces = false;
     int strips = 1, mt_per_grid = 1, nbmax = 8;    // k2: 32-column strips, macro tiles per grid, blocks per macro tile
     int split_grid = 0;   // CTAs of k2_split_bf16, 0: the launch is large enough for k2_bf16
 };
@@ -258,15 +258,16 @@ struct ApronCopies {
 //   warps 0-7   stencil group: loads the tile's state halo (scale applied) and the X operand, then its two
 //               4-warp halves take alternate heads: 3x3 stencil marching down columns in packed fp32 -> A operand
 //   warps 8-15  epilogue group: TMEM -> growth bell, E = exp(G*I) -> swizzled staging tiles (+ register stores of
-//               the apron duplicates of edge cells on ragged grids)
+//               the apron duplicates of edge cells without PIECES)
 //   warp 16     TMA producer of the per-head weight tiles (2-stage ring)
 //   warp 17     UMMA issuer: U (N=64) and I|V (N=128) into a double-buffered 192-column TMEM accumulator
 //   warp 18     store warp: issues the TMA stores of every finished item, so that the epilogue group never meets at
 //               a barrier (its threads arrive on an mbarrier when their staging is written and move on)
-// ALIGNED: the grid is made of whole tiles (W a multiple of 16, and H a multiple of 8 on a torus), so the wrapped
-// copies of edge cells are whole pieces of a tile and go out as extra TMA stores; otherwise the threads that own
-// edge cells store the copies from registers.
-template <bool ALIGNED>
+// PIECES: the last two columns, and on a torus the last two rows, each lie within one tile, so the wrapped copies of edge
+// cells are pieces of a tile and go out as extra TMA stores.  (What hangs over the grid's far edges is computed from the
+// wrapped state and lands in the apron by the tile's own store: the same bits as a copy.)  Otherwise, and on tiny grids, the
+// threads that own edge cells store the copies from registers, with which k1 took 66 us at X[32,40,40,64] and 359 us at X[100,50,70,64] for the 56 and 305 it takes so.
+template <bool PIECES>
 __global__ void __launch_bounds__(k1b::THREADS, 1)
 k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1StoreMaps sm_maps,
         const __nv_bfloat16* __restrict__ X,
@@ -347,19 +348,21 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
         if (lane == 0) {
             CaTile t;
             bool left = false, right = false, top = false, bottom = false;
+            const bool far_x = (g.W & (TBW - 1)) == 0 || (g.W & (TBW - 1)) == TBW - 1, far_y = (g.H & (TBH - 1)) == 0 || (g.H & (TBH - 1)) == TBH - 1;
             for (int n = 0; n < items.count; ++n) {
                     const int h = items.head(n);
                     if (items.first(n)) {
                         t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
-                        // whole-tile grids: which sides of the grid this tile touches
-                        left = t.tx0 == 0; right = t.tx0 + TBW == g.W;
-                        top = g.wrap_y && t.ty0 == 0; bottom = g.wrap_y && t.ty0 + TBH == g.H;
+                        // the sides of the grid whose copies are this tile's to store; on the left and at the top none where
+                        // the last tile hangs over by the two columns or rows
+                        left = far_x && t.tx0 == 0; right = t.tx0 + TBW >= g.W;
+                        top = far_y && g.wrap_y && t.ty0 == 0; bottom = g.wrap_y && t.ty0 + TBH >= g.H;
                     }
                     ptx::mbar_wait(stg_full, n & 1, status, 150);
                     const int px = t.tx0 + APRON, py = t.ty0 + APRON, pl = t.b * NH + h;
                     ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, px, py, pl);
                     ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, px, py, pl);
-                    if (ALIGNED) {
+                    if (PIECES) {
                         // wrapped copies: pieces that land at the high end of an apron are the whole tile stored at the
                         // shifted position (all but the first two columns / rows are clipped); pieces that land at
                         // the low end come from the small staging tiles
@@ -523,15 +526,16 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
             // Apron positions that wrap onto this thread's cell (the store warp's TMA store covers the cell itself
             // and whatever hangs over the far edge).
             const int cy = m_ep >> 4, cx = m_ep & 15;
-            // whole-tile grids: does this tile touch the right / bottom side of the grid (uniform over the tile)
-            const bool right = t.tx0 + TBW == g.W, bottom = g.wrap_y && t.ty0 + TBH == g.H;
-            const bool in_col = right && cx >= TBW - APRON, in_row = bottom && cy >= TBH - APRON;
-            // ragged or tiny grids: per-thread targets (named registers, not an indexed array: an array would live
+            // the last two columns and rows of the grid, where this tile has them (PIECES: both or neither)
+            const int c2 = x_ep - (g.W - APRON), r2 = r_ep - (g.H - APRON);
+            const int mc = c2 >= 0 && c2 < APRON ? cy * APRON + c2 : -1;                      // cell of the small staging tiles,
+            const int mr = g.wrap_y && r2 >= 0 && r2 < APRON ? r2 * TBW + cx : -1;            // -1 for none
+            // without PIECES: per-thread targets (named registers, not an indexed array: an array would live
             // in local memory and put a load in front of every duplicate store).  Grids narrower or shorter than
             // twice the apron can wrap more than once and take the general loop.
             size_t off_x = 0, off_y = 0, off_xy = 0;
             bool dup_x = false, dup_y = false;
-            if (!ALIGNED && valid_ep && !tiny) {
+            if (!PIECES && valid_ep && !tiny) {
                 const int xd = x_ep < APRON ? x_ep + g.W : (x_ep >= g.W - APRON ? x_ep - g.W : -100);
                 const int rd = !g.wrap_y ? -100 : (r_ep < APRON ? r_ep + g.H : (r_ep >= g.H - APRON ? r_ep - g.H : -100));
                 dup_x = xd != -100;
@@ -540,7 +544,7 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
                 if (dup_y) off_y = ((size_t)(rd + APRON) * g.ev_w + x_ep + APRON) * HD;
                 if (dup_x && dup_y) off_xy = ((size_t)(rd + APRON) * g.ev_w + xd + APRON) * HD;
             }
-            const bool any_dup = !ALIGNED && valid_ep && (dup_x || dup_y || tiny);
+            const bool any_dup = !PIECES && valid_ep && (dup_x || dup_y || tiny);
             for (int i = first; i < end; ++i) {
                 const int h = h0 + i, tb = i & 1;
                 const float mus = __ldg(prm + ((size_t)set * NH + h) * PRM + 9);   // mu * s; Wp carries s and Wi carries log2(e)
@@ -588,23 +592,21 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
                     *reinterpret_cast<uint4*>(stg_e + swz(m_ep, qa + 1)) = e_hi;
                     *reinterpret_cast<uint4*>(stg_v + swz(m_ep, qa)) = v_lo;
                     *reinterpret_cast<uint4*>(stg_v + swz(m_ep, qa + 1)) = v_hi;
-                    if (ALIGNED) {
-                        if (in_col) {
-                            const int mc = cy * APRON + cx - (TBW - APRON);
+                    if (PIECES) {
+                        if (mc >= 0) {
                             *reinterpret_cast<uint4*>(sm + k1b::STG_COL_E + swz(mc, qa)) = e_lo;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_COL_E + swz(mc, qa + 1)) = e_hi;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_COL_V + swz(mc, qa)) = v_lo;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_COL_V + swz(mc, qa + 1)) = v_hi;
                         }
-                        if (in_row) {
-                            const int mr = (cy - (TBH - APRON)) * TBW + cx;
+                        if (mr >= 0) {
                             *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_E + swz(mr, qa)) = e_lo;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_E + swz(mr, qa + 1)) = e_hi;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_V + swz(mr, qa)) = v_lo;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_V + swz(mr, qa + 1)) = v_hi;
                         }
-                        if (in_col && in_row) {
-                            const int mq = (cy - (TBH - APRON)) * APRON + cx - (TBW - APRON);
+                        if (mc >= 0 && mr >= 0) {
+                            const int mq = mr / TBW * APRON + mc % APRON;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_COR_E + swz(mq, qa)) = e_lo;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_COR_E + swz(mq, qa + 1)) = e_hi;
                             *reinterpret_cast<uint4*>(sm + k1b::STG_COR_V + swz(mq, qa)) = v_lo;
@@ -1381,7 +1383,7 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
             return -1;
         }
     }
-    p.k1_aligned = g.W % TBW == 0 && (!g.wrap_y || g.H % TBH == 0);
+    p.k1_pieces = g.W >= 2 * APRON && g.W % TBW != 1 && (!g.wrap_y || (g.H >= 2 * APRON && g.H % TBH != 1));
     if (cudaFuncSetAttribute(k1_bf16<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, k1b::SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(k1_bf16<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, k1b::SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(k2_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, k2m::SMEM) != cudaSuccess) {
@@ -1402,7 +1404,7 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
 
 inline int bf16_k1(Bf16Plan& p, const __nv_bfloat16* X, const float* scale, const float* prm, __nv_bfloat16* E,
                    __nv_bfloat16* V, int* status, const Geom& g, cudaStream_t st) {
-    return launch_pdl(p.k1_aligned ? k1_bf16<true> : k1_bf16<false>, p.k1_grid, k1b::THREADS, k1b::SMEM, st, p.map_w1, p.st, X, scale, prm,
+    return launch_pdl(p.k1_pieces ? k1_bf16<true> : k1_bf16<false>, p.k1_grid, k1b::THREADS, k1b::SMEM, st, p.map_w1, p.st, X, scale, prm,
                       E, V, status, p.k1_tiles * g.B, p.k1_tiles, g) == cudaSuccess ? 0 : -1;
 }
 

@@ -1166,7 +1166,7 @@ int slime_ca_occupancy(slime_ca* h, float* occupancy) {
     int b1 = 0, b2 = 0, t1, t2;
     if (is_bf16(h)) {
         t1 = k1b::THREADS; t2 = k2m::THREADS;
-        if (h->bf.k1_aligned) CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_bf16<true>, t1, k1b::SMEM));
+        if (h->bf.k1_pieces) CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_bf16<true>, t1, k1b::SMEM));
         else CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_bf16<false>, t1, k1b::SMEM));
         CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k2_bf16, t2, k2m::SMEM));
     } else {

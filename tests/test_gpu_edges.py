@@ -20,8 +20,9 @@ def gpu():
 
 
 # (batch, height, width), weight sets: one item in all; tiles left over that share an item boundary; one whole round of tiles
-# and one tile more; 512 and 544 tile sums a grid (the limit of the fused sums); ragged in both directions
-SHAPES = [((1, 1, 5), 1), ((1, 8, 16), 1), ((3, 33, 47), 3), ((149, 8, 16), 1), ((1, 512, 128), 1), ((1, 544, 128), 1), ((2, 75, 53), 2)]
+# and one tile more; 512 and 544 tile sums a grid (the limit of the fused sums); ragged in both directions: the far edge one cell, two and more inside the last tile
+SHAPES = [((1, 1, 5), 1), ((1, 8, 16), 1), ((3, 33, 47), 3), ((149, 8, 16), 1), ((1, 512, 128), 1), ((1, 544, 128), 1), ((2, 75, 53), 2),
+          ((1, 39, 63), 1), ((1, 34, 50), 1), ((1, 4, 4), 1)]
 
 
 @pytest.mark.parametrize("dtype_name", ["f32", "bf16"])
