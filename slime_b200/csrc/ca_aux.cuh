@@ -1,7 +1,10 @@
 // Small kernels around the step: deterministic per-channel sums, the lazy renormalisation scale,
 // dtype conversion on the way in and out, the 1-channel lift and the pooled readout.
+// Those that run next to a step start while the kernel before them drains (launch_pdl), as the step's own kernels do: state
+// in, one step of a 32 x 32 bf16 grid and state out took 33.1 us without and take 29.2 us with it.
 #pragma once
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace slime {
 
@@ -144,6 +147,8 @@ __device__ __forceinline__ void chunk_sums(const float (&acc)[8], const ChunkSum
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_channel_partials(const T* __restrict__ X, bool vec, ChunkSums out, Geom g) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const size_t cells = (size_t)g.H * g.W;
     const T* base = X + ((size_t)blockIdx.y * g.state_rows() + g.hx) * g.W * NC + (threadIdx.x & 7) * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -175,6 +180,8 @@ k_reduce_partials(const float* __restrict__ partial, int n_partials, double* __r
 __global__ void __launch_bounds__(256)
 k_reduce_finish(const float* __restrict__ partial, int n_partials, double* __restrict__ seg_sums, size_t lo_offset,
                 int* __restrict__ tickets, SumsOut out) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     __shared__ double red[4 * NC];
     __shared__ int is_last;
     const int b = blockIdx.y, tid = threadIdx.x, c = tid & 63, sub = tid >> 6, nseg = gridDim.x;
@@ -209,6 +216,8 @@ __global__ void k_scale_from_sums(const double* __restrict__ sums, const double*
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
 k_state_in(const TI* __restrict__ src, bool vec, TO* __restrict__ X, ChunkSums out, Geom g) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const size_t cells = (size_t)g.H * g.W, b = blockIdx.y;
     const int q = (threadIdx.x & 7) * 8;
     TO* dst = X + ((size_t)b * g.state_rows() + g.hx) * g.W * NC + q;
@@ -232,6 +241,8 @@ k_state_in(const TI* __restrict__ src, bool vec, TO* __restrict__ X, ChunkSums o
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
 k_state_out(const TI* __restrict__ X, const float* __restrict__ scale, TO* __restrict__ dst, bool vec, Geom g) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const size_t n = (size_t)g.H * g.W * 8, b = blockIdx.y;
     const int q = (threadIdx.x & 7) * 8;                 // the same for all of a thread's chunks: the stride is a multiple of 8
     const TI* src = X + ((size_t)b * g.state_rows() + g.hx) * g.W * NC;
@@ -252,6 +263,8 @@ struct LiftVector { float v[NC]; };      // a kernel argument: no copy to the de
 template <typename TO>
 __global__ void __launch_bounds__(256)
 k_lift(const float* __restrict__ img, int ih, int iw, const LiftVector L, TO* __restrict__ X, ChunkSums out, Geom g) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const int py = (g.H - ih) / 2, px = (g.W - iw) / 2;
     const int cells = g.H * g.W, q = (threadIdx.x & 7) * 8;
     const size_t b = blockIdx.y;
@@ -281,6 +294,8 @@ k_lift(const float* __restrict__ img, int ih, int iw, const LiftVector L, TO* __
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_channel_mean(const T* __restrict__ X, const float* __restrict__ scale, float* __restrict__ field, Geom g) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const size_t cells = (size_t)g.H * g.W, b = blockIdx.y;
     const int q = (threadIdx.x & 7) * 8;
     const T* src = X + (b * g.state_rows() + g.hx) * g.W * NC + q;

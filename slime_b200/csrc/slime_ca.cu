@@ -148,7 +148,7 @@ int with_channel_sums(slime_ca* h, int mode, cudaStream_t st, Launch launch) {
     if (!fuse) {
         // a fresh state also starts the reduction's tickets afresh (they are only non-zero if a launch before was cut short)
         CK(h, cudaMemsetAsync(h->tickets, 0, (size_t)g.B * sizeof(int), st));
-        k_reduce_finish<<<dim3(reduce_segments(h, chunks), g.B), 256, 0, st>>>(h->partial, chunks, h->seg_sums, 0, h->tickets, out);
+        launch_pdl(k_reduce_finish, dim3(reduce_segments(h, chunks), g.B), 256, 0, st, h->partial, chunks, h->seg_sums, 0, h->tickets, out);
         LAUNCHED(h);
     }
     return SLIME_CA_OK;
@@ -157,8 +157,8 @@ int with_channel_sums(slime_ca* h, int mode, cudaStream_t st, Launch launch) {
 // sums <- per-channel sums of the stored state's own rows
 int channel_sums(slime_ca* h, int mode, cudaStream_t st) {
     return with_channel_sums(h, mode, st, [&](dim3 grid, const ChunkSums& cs) {
-        if (is_bf16(h)) k_channel_partials<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)h->X, true, cs, h->g);
-        else k_channel_partials<float><<<grid, 256, 0, st>>>((const float*)h->X, true, cs, h->g);
+        if (is_bf16(h)) launch_pdl(k_channel_partials<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)h->X, true, cs, h->g);
+        else launch_pdl(k_channel_partials<float>, grid, 256, 0, st, (const float*)h->X, true, cs, h->g);
     });
 }
 
@@ -167,8 +167,8 @@ int lift(slime_ca* h, const float* img, int ih, int iw, const float* host_L, cud
     LiftVector L;
     memcpy(L.v, host_L, sizeof L.v);
     return with_channel_sums(h, 1, st, [&](dim3 grid, const ChunkSums& cs) {
-        if (is_bf16(h)) k_lift<__nv_bfloat16><<<grid, 256, 0, st>>>(img, ih, iw, L, (__nv_bfloat16*)h->X, cs, h->g);
-        else k_lift<float><<<grid, 256, 0, st>>>(img, ih, iw, L, (float*)h->X, cs, h->g);
+        if (is_bf16(h)) launch_pdl(k_lift<__nv_bfloat16>, grid, 256, 0, st, img, ih, iw, L, (__nv_bfloat16*)h->X, cs, h->g);
+        else launch_pdl(k_lift<float>, grid, 256, 0, st, img, ih, iw, L, (float*)h->X, cs, h->g);
     });
 }
 
@@ -206,7 +206,7 @@ int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nul
     }
     if (ev) CK(h, cudaEventRecord(ev[2], st));
     if (h->k2_tiles > FUSE_PARTIALS) {        // else k2 has done it
-        k_reduce_finish<<<dim3(reduce_segments(h, h->k2_tiles), g.B), 256, 0, st>>>(h->partial, h->k2_tiles, h->seg_sums,
+        launch_pdl(k_reduce_finish, dim3(reduce_segments(h, h->k2_tiles), g.B), 256, 0, st, h->partial, h->k2_tiles, h->seg_sums,
                                                                                     is_bf16(h) ? 0 : h->partial_lo, h->tickets, out);
         LAUNCHED(h);
     }
@@ -488,11 +488,11 @@ int slime_ca_set_state_device(slime_ca* h, const void* dev_state, int dtype, voi
         const __nv_bfloat16* s16 = (const __nv_bfloat16*)dev_state;
         const float* s32 = (const float*)dev_state;
         if (is_bf16(h)) {
-            if (dtype == SLIME_CA_BF16) k_state_in<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, st>>>(s16, vec, (__nv_bfloat16*)h->X, cs, h->g);
-            else k_state_in<float, __nv_bfloat16><<<grid, 256, 0, st>>>(s32, vec, (__nv_bfloat16*)h->X, cs, h->g);
+            if (dtype == SLIME_CA_BF16) launch_pdl(k_state_in<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, st, s16, vec, (__nv_bfloat16*)h->X, cs, h->g);
+            else launch_pdl(k_state_in<float, __nv_bfloat16>, grid, 256, 0, st, s32, vec, (__nv_bfloat16*)h->X, cs, h->g);
         } else {
-            if (dtype == SLIME_CA_BF16) k_state_in<__nv_bfloat16, float><<<grid, 256, 0, st>>>(s16, vec, (float*)h->X, cs, h->g);
-            else k_state_in<float, float><<<grid, 256, 0, st>>>(s32, vec, (float*)h->X, cs, h->g);
+            if (dtype == SLIME_CA_BF16) launch_pdl(k_state_in<__nv_bfloat16, float>, grid, 256, 0, st, s16, vec, (float*)h->X, cs, h->g);
+            else launch_pdl(k_state_in<float, float>, grid, 256, 0, st, s32, vec, (float*)h->X, cs, h->g);
         }
     });
     if (rc) return rc;
@@ -515,11 +515,11 @@ int slime_ca_get_state_device(slime_ca* h, void* dev_state, int dtype, void* str
     __nv_bfloat16* d16 = (__nv_bfloat16*)dev_state;
     float* d32 = (float*)dev_state;
     if (is_bf16(h)) {
-        if (dtype == SLIME_CA_BF16) k_state_out<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, d16, vec, g);
-        else k_state_out<__nv_bfloat16, float><<<grid, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, d32, vec, g);
+        if (dtype == SLIME_CA_BF16) launch_pdl(k_state_out<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)h->X, h->scale, d16, vec, g);
+        else launch_pdl(k_state_out<__nv_bfloat16, float>, grid, 256, 0, st, (const __nv_bfloat16*)h->X, h->scale, d32, vec, g);
     } else {
-        if (dtype == SLIME_CA_BF16) k_state_out<float, __nv_bfloat16><<<grid, 256, 0, st>>>((const float*)h->X, h->scale, d16, vec, g);
-        else k_state_out<float, float><<<grid, 256, 0, st>>>((const float*)h->X, h->scale, d32, vec, g);
+        if (dtype == SLIME_CA_BF16) launch_pdl(k_state_out<float, __nv_bfloat16>, grid, 256, 0, st, (const float*)h->X, h->scale, d16, vec, g);
+        else launch_pdl(k_state_out<float, float>, grid, 256, 0, st, (const float*)h->X, h->scale, d32, vec, g);
     }
     LAUNCHED(h);
     return SLIME_CA_OK;
@@ -815,8 +815,8 @@ int slime_ca_field_from_state_device(slime_ca* h, float* dev_field, void* stream
     cudaStream_t st = (cudaStream_t)stream;
     const Geom& g = h->g;
     const dim3 blocks = cell_blocks(h);
-    if (is_bf16(h)) k_channel_mean<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, dev_field, g);
-    else k_channel_mean<float><<<blocks, 256, 0, st>>>((const float*)h->X, h->scale, dev_field, g);
+    if (is_bf16(h)) launch_pdl(k_channel_mean<__nv_bfloat16>, blocks, 256, 0, st, (const __nv_bfloat16*)h->X, h->scale, dev_field, g);
+    else launch_pdl(k_channel_mean<float>, blocks, 256, 0, st, (const float*)h->X, h->scale, dev_field, g);
     LAUNCHED(h);
     return SLIME_CA_OK;
 }
@@ -874,8 +874,8 @@ int slime_ca_evolution_record(slime_ca* h, int grid_index, int generation, doubl
     if (!field) {
         float* scratch = (float*)h->E;
         const dim3 blocks = cell_blocks(h);
-        if (is_bf16(h)) k_channel_mean<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)h->X, h->scale, scratch, g);
-        else k_channel_mean<float><<<blocks, 256, 0, st>>>((const float*)h->X, h->scale, scratch, g);
+        if (is_bf16(h)) launch_pdl(k_channel_mean<__nv_bfloat16>, blocks, 256, 0, st, (const __nv_bfloat16*)h->X, h->scale, scratch, g);
+        else launch_pdl(k_channel_mean<float>, blocks, 256, 0, st, (const float*)h->X, h->scale, scratch, g);
         LAUNCHED(h);
         field = scratch + (size_t)grid_index * g.H * g.W;
     }
@@ -1270,8 +1270,8 @@ int slime_ca_channel_sums_static(const void* dev_state, int dtype, int batch, in
     const dim3 grid((unsigned)chunks, (unsigned)batch);
     const bool vec = aligned16(dev_state);
     const ChunkSums cs{partial, nullptr, nullptr, SumsOut{nullptr, nullptr, nullptr, 0}};
-    if (dtype == SLIME_CA_BF16) k_channel_partials<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dev_state, vec, cs, g);
-    else k_channel_partials<float><<<grid, 256, 0, st>>>((const float*)dev_state, vec, cs, g);
+    if (dtype == SLIME_CA_BF16) launch_pdl(k_channel_partials<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)dev_state, vec, cs, g);
+    else launch_pdl(k_channel_partials<float>, grid, 256, 0, st, (const float*)dev_state, vec, cs, g);
     e = cudaGetLastError();
     if (e != cudaSuccess) return static_fail(SLIME_CA_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     // one segment per grid: the fp64 second stage writes [batch][64] straight into the caller's buffer
