@@ -120,7 +120,6 @@ struct Bf16Plan {
     CUtensorMap map_v;    // V planes, box 64 x 34 x 4 x 1
     CUtensorMap map_x;    // the state's own rows (and the halo rows above them) [B][hx + H][W][64], box 64 x 32 x 4 x 1, 128B swizzle
     K1StoreMaps st;       // store maps of k1 (whole tile, last two columns, last two rows, their corner)
-    bool k1_pieces = false;
     int strips = 1, mt_per_grid = 1, nbmax = 8;    // k2: 32-column strips, macro tiles per grid, blocks per macro tile
     int split_grid = 0;   // CTAs of k2_split_bf16, 0: the launch is large enough for k2_bf16
 };
@@ -169,13 +168,13 @@ __device__ __forceinline__ uint32_t swz(int m, int q) { return (uint32_t)(m * 12
 struct CaTile {
     int b, ty0, tx0, index;
 };
-__device__ __forceinline__ CaTile ca_tile(int t, int tiles_per_grid, int tiles_x, int row0) {
+__device__ __forceinline__ CaTile ca_tile(int t, int tiles_per_grid, const Geom& g) {
     CaTile r;
     r.index = t;
     r.b = t / tiles_per_grid;
     const int tt = t - r.b * tiles_per_grid;
-    r.ty0 = (tt / tiles_x) * TBH + row0;
-    r.tx0 = (tt % tiles_x) * TBW;
+    r.ty0 = (tt / g.tiles_x) * TBH + g.row0;
+    r.tx0 = (tt % g.tiles_x) * TBW + g.col0;
     return r;
 }
 
@@ -199,53 +198,41 @@ struct K1Items {
     __device__ int end(int n) const { return min(n + NH - head(n), count); }                   // first item of the next tile, from a first item
 };
 
-// Apron copies of the cells of one epilogue warp of k1 (two rows of a tile, one cell per lane): the positions outside the
-// grid's own rows and columns that wrap onto them.  The TMA store of the warp's staging covers the cells and whatever
-// hangs over the far edge.  Copies at the high ends of the apron are the same staging stored once more at the shifted
-// position (all but the wanted part is clipped), and so is a pair of last rows at the low end; what is left - the last two
-// columns, which would have to start before the plane, and last rows that are not one warp's pair - the lanes store from
-// their registers.  Grids narrower or shorter than twice the apron can wrap more than once and take a general loop.
+// Apron copies of the cells of one epilogue warp of k1 (two rows of a tile, one cell per lane), where the tiles start at the
+// grid: the positions outside the grid's own rows and columns that wrap onto them.  The TMA store of the warp's staging covers
+// the cells and whatever hangs over the far edge.  Copies at the high ends of the apron are the same staging stored once more
+// at the shifted position (all but the wanted part is clipped), and so is a pair of last rows at the low end; what is left -
+// the last two columns, which would have to start before the plane, and last rows that are not one warp's pair - the lanes
+// store from their registers.
 struct ApronCopies {
-    bool tiny, wrap_x, lanes;         // general loop; staging again at x + W; any lane with a copy of its own
+    bool wrap_x, lanes;               // staging again at x + W; any lane with a copy of its own
     int dy;                           // staging again at y + dy (0: no)
     int at_x, at_y, at_xy;            // this lane's own copies: cell offsets in the plane, -1 for none
     __device__ void tile(const CaTile& t, int quad, int lane, const Geom& g) {
         const int r0 = t.ty0 + quad * 2, r = r0 + (lane >> 4), x = t.tx0 + (lane & 15);
-        const bool valid = r < g.H + g.he && x < g.W, last_x = x >= g.W - APRON, last_y = g.wrap_y && r >= g.H - APRON;
-        tiny = g.W < 2 * APRON || (g.wrap_y && g.H < 2 * APRON);
-        wrap_x = t.tx0 == 0;
-        dy = !g.wrap_y ? 0 : r0 == 0 ? g.H : r0 == g.H - APRON ? -g.H : 0;
+        const bool valid = r < g.H + (g.copy_y ? 0 : APRON) && x < g.W + (g.copy_x ? 0 : APRON);
+        const bool last_x = g.copy_x && x >= g.W - APRON, last_y = g.copy_y && r >= g.H - APRON;
+        wrap_x = g.copy_x && t.tx0 == 0;
+        dy = !g.copy_y ? 0 : r0 == 0 ? g.H : r0 == g.H - APRON ? -g.H : 0;
         const int rd = dy ? dy : last_y ? -g.H : 0;           // where this lane's row goes, if anywhere
         const bool own_y = rd != 0 && dy == 0;
-        const int here = (r + APRON) * g.ev_w + x + APRON, xd = last_x ? -g.W : x < APRON ? g.W : 0;
+        const int here = (r + APRON) * g.ev_w + x + APRON, xd = last_x ? -g.W : g.copy_x && x < APRON ? g.W : 0;
         at_x = valid && last_x ? here - g.W : -1;
         at_y = valid && own_y ? here + rd * g.ev_w : -1;
         at_xy = valid && rd != 0 && xd != 0 && (last_x || own_y) ? here + rd * g.ev_w + xd : -1;
-        lanes = tiny || __any_sync(0xffffffffu, at_x >= 0 || at_y >= 0);
+        lanes = __any_sync(0xffffffffu, at_x >= 0 || at_y >= 0);
     }
     // copy(cell offset) for every copy of this lane's own
-    template <typename F> __device__ void own(const CaTile& t, int quad, int lane, const Geom& g, F copy) const {
+    template <typename F> __device__ void own(F copy) const {
         if (!lanes) return;
-        if (!tiny) {
-            if (at_x >= 0) copy(at_x);
-            if (at_y >= 0) copy(at_y);
-            if (at_xy >= 0) copy(at_xy);
-            return;
-        }
-        const int r = t.ty0 + quad * 2 + (lane >> 4), x = t.tx0 + (lane & 15);
-        if (r >= g.H + g.he || x >= g.W) return;
-        for (int ky = g.wrap_y ? -2 * APRON : 0; ky <= (g.wrap_y ? 2 * APRON : 0); ++ky)
-            for (int kx = -2 * APRON; kx <= 2 * APRON; ++kx) {
-                const int rr = r + ky * g.H, xx = x + kx * g.W;
-                if ((ky == 0 && kx == 0) || rr < -APRON || rr >= g.H + APRON || xx < -APRON || xx >= g.W + APRON) continue;
-                copy((rr + APRON) * g.ev_w + xx + APRON);
-            }
+        if (at_x >= 0) copy(at_x);
+        if (at_y >= 0) copy(at_y);
+        if (at_xy >= 0) copy(at_xy);
     }
     // store(plane column, plane row) of the warp's staging: its place, and the copies
     template <typename F> __device__ void staged(const CaTile& t, int quad, const Geom& g, F store) const {
         const int px = t.tx0 + APRON, py = t.ty0 + quad * 2 + APRON;
         store(px, py);
-        if (tiny) return;
         if (wrap_x) store(px + g.W, py);
         if (dy) {
             store(px, py + dy);
@@ -257,22 +244,19 @@ struct ApronCopies {
 // k1: persistent, warp-specialised, one CTA per SM (608 threads), over the items of K1Items:
 //   warps 0-7   stencil group: loads the tile's state halo (scale applied) and the X operand, then its two
 //               4-warp halves take alternate heads: 3x3 stencil marching down columns in packed fp32 -> A operand
-//   warps 8-15  epilogue group: TMEM -> growth bell, E = exp(G*I) -> swizzled staging tiles (+ register stores of
-//               the apron duplicates of edge cells without PIECES)
+//   warps 8-15  epilogue group: TMEM -> growth bell, E = exp(G*I) -> swizzled staging tiles
 //   warp 16     TMA producer of the per-head weight tiles (2-stage ring)
 //   warp 17     UMMA issuer: U (N=64) and I|V (N=128) into a double-buffered 192-column TMEM accumulator
 //   warp 18     store warp: issues the TMA stores of every finished item, so that the epilogue group never meets at
 //               a barrier (its threads arrive on an mbarrier when their staging is written and move on)
-// PIECES: the last two columns, and on a torus the last two rows, each lie within one tile, so the wrapped copies of edge
-// cells are pieces of a tile and go out as extra TMA stores.  (What hangs over the grid's far edges is computed from the
-// wrapped state and lands in the apron by the tile's own store: the same bits as a copy.)  Otherwise, and on tiny grids, the
-// threads that own edge cells store the copies from registers, with which k1 took 66 us at X[32,40,40,64] and 359 us at X[100,50,70,64] for the 56 and 305 it takes so.
-template <bool PIECES>
+// The apron of E and V: k1_origin.  Copies of edge cells are pieces of a tile and go out as extra TMA stores.  (As register
+// stores by the threads that own the edge cells, on all grids not made of whole tiles, k1 took 66 us at X[32,40,40,64] and
+// 359 us at X[100,50,70,64]; all as TMA pieces 56 and 305; with the apron computed where that costs no tile 54 and 298.)
 __global__ void __launch_bounds__(k1b::THREADS, 1)
 k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1StoreMaps sm_maps,
         const __nv_bfloat16* __restrict__ X,
-        const float* __restrict__ scale, const float* __restrict__ prm, __nv_bfloat16* __restrict__ E,
-        __nv_bfloat16* __restrict__ V, int* __restrict__ status, int n_tiles, int tiles_per_grid, Geom g) {
+        const float* __restrict__ scale, const float* __restrict__ prm, int* __restrict__ status, int n_tiles, int tiles_per_grid,
+        Geom g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + k1b::BARS);
@@ -308,7 +292,6 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
     ptx::pdl_wait();
     const K1Items items(n_tiles);
     const size_t xplane = (size_t)g.state_rows() * g.W * NC;
-    const size_t eplane = (size_t)g.ev_h * g.ev_w * HD;
 
     if (warp == 16) {
         // ================= TMA producer: weights of the CTA's n-th item into stage n % 2 ==========================
@@ -352,43 +335,41 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
             for (int n = 0; n < items.count; ++n) {
                     const int h = items.head(n);
                     if (items.first(n)) {
-                        t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
+                        t = ca_tile(items.tile(n), tiles_per_grid, g);
                         // the sides of the grid whose copies are this tile's to store; on the left and at the top none where
                         // the last tile hangs over by the two columns or rows
-                        left = far_x && t.tx0 == 0; right = t.tx0 + TBW >= g.W;
-                        top = far_y && g.wrap_y && t.ty0 == 0; bottom = g.wrap_y && t.ty0 + TBH >= g.H;
+                        left = g.copy_x && far_x && t.tx0 == 0; right = g.copy_x && t.tx0 + TBW >= g.W;
+                        top = g.copy_y && far_y && t.ty0 == 0; bottom = g.copy_y && t.ty0 + TBH >= g.H;
                     }
                     ptx::mbar_wait(stg_full, n & 1, status, 150);
                     const int px = t.tx0 + APRON, py = t.ty0 + APRON, pl = t.b * NH + h;
                     ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, px, py, pl);
                     ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, px, py, pl);
-                    if (PIECES) {
-                        // wrapped copies: pieces that land at the high end of an apron are the whole tile stored at the
-                        // shifted position (all but the first two columns / rows are clipped); pieces that land at
-                        // the low end come from the small staging tiles
-                        const int hx = g.W + APRON, hy = g.H + APRON;
-                        if (left) { ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, hx, py, pl); ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, hx, py, pl); }
-                        if (top) { ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, px, hy, pl); ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, px, hy, pl); }
-                        if (left && top) { ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, hx, hy, pl); ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, hx, hy, pl); }
-                        if (right) {
-                            ptx::tma_store_4d(&sm_maps.e_col, sm + k1b::STG_COL_E, 0, 0, py, pl);
-                            ptx::tma_store_4d(&sm_maps.v_col, sm + k1b::STG_COL_V, 0, 0, py, pl);
-                            if (top) {
-                                ptx::tma_store_4d(&sm_maps.e_col, sm + k1b::STG_COL_E, 0, 0, hy, pl);
-                                ptx::tma_store_4d(&sm_maps.v_col, sm + k1b::STG_COL_V, 0, 0, hy, pl);
-                            }
+                    // wrapped copies: pieces that land at the high end of an apron are the whole tile stored at the
+                    // shifted position (all but the first two columns / rows are clipped); pieces that land at
+                    // the low end come from the small staging tiles
+                    const int hx = g.W + APRON, hy = g.H + APRON;
+                    if (left) { ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, hx, py, pl); ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, hx, py, pl); }
+                    if (top) { ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, px, hy, pl); ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, px, hy, pl); }
+                    if (left && top) { ptx::tma_store_4d(&sm_maps.e, sm + k1b::STG_E, 0, hx, hy, pl); ptx::tma_store_4d(&sm_maps.v, sm + k1b::STG_V, 0, hx, hy, pl); }
+                    if (right) {
+                        ptx::tma_store_4d(&sm_maps.e_col, sm + k1b::STG_COL_E, 0, 0, py, pl);
+                        ptx::tma_store_4d(&sm_maps.v_col, sm + k1b::STG_COL_V, 0, 0, py, pl);
+                        if (top) {
+                            ptx::tma_store_4d(&sm_maps.e_col, sm + k1b::STG_COL_E, 0, 0, hy, pl);
+                            ptx::tma_store_4d(&sm_maps.v_col, sm + k1b::STG_COL_V, 0, 0, hy, pl);
                         }
-                        if (bottom) {
-                            ptx::tma_store_4d(&sm_maps.e_row, sm + k1b::STG_ROW_E, 0, px, 0, pl);
-                            ptx::tma_store_4d(&sm_maps.v_row, sm + k1b::STG_ROW_V, 0, px, 0, pl);
-                            if (left) {
-                                ptx::tma_store_4d(&sm_maps.e_row, sm + k1b::STG_ROW_E, 0, hx, 0, pl);
-                                ptx::tma_store_4d(&sm_maps.v_row, sm + k1b::STG_ROW_V, 0, hx, 0, pl);
-                            }
-                            if (right) {
-                                ptx::tma_store_4d(&sm_maps.e_cor, sm + k1b::STG_COR_E, 0, 0, 0, pl);
-                                ptx::tma_store_4d(&sm_maps.v_cor, sm + k1b::STG_COR_V, 0, 0, 0, pl);
-                            }
+                    }
+                    if (bottom) {
+                        ptx::tma_store_4d(&sm_maps.e_row, sm + k1b::STG_ROW_E, 0, px, 0, pl);
+                        ptx::tma_store_4d(&sm_maps.v_row, sm + k1b::STG_ROW_V, 0, px, 0, pl);
+                        if (left) {
+                            ptx::tma_store_4d(&sm_maps.e_row, sm + k1b::STG_ROW_E, 0, hx, 0, pl);
+                            ptx::tma_store_4d(&sm_maps.v_row, sm + k1b::STG_ROW_V, 0, hx, 0, pl);
+                        }
+                        if (right) {
+                            ptx::tma_store_4d(&sm_maps.e_cor, sm + k1b::STG_COR_E, 0, 0, 0, pl);
+                            ptx::tma_store_4d(&sm_maps.v_cor, sm + k1b::STG_COR_V, 0, 0, 0, pl);
                         }
                     }
                     ptx::bulk_commit();
@@ -405,14 +386,14 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
         for (int k = 0, first = 0, end; first < items.count; ++k, first = end) {
             end = items.end(first);                                       // items first .. end - 1 are of this tile
             const int h0 = items.head(first) - first;
-            const CaTile t = ca_tile(items.tile(first), tiles_per_grid, g.tiles_x, -g.he);
+            const CaTile t = ca_tile(items.tile(first), tiles_per_grid, g);
             const int set = t.b / g.per_set;
             uint8_t* a_x = sm + k1b::A_X;
             ptx::bar_sync(1, 256);                                        // both halves are done with the last halo
             const float* sc = scale + t.b * NC;
             if (tid < NH * PRM) prm_s[tid] = __ldg(prm + (size_t)set * NH * PRM + tid);
             if (end < items.count && tid < 180) {      // next tile's halo cells: one 128-byte line each, into L2
-                const CaTile tn = ca_tile(items.tile(end), tiles_per_grid, g.tiles_x, -g.he);
+                const CaTile tn = ca_tile(items.tile(end), tiles_per_grid, g);
                 const int r = tn.ty0 + tid / 18 - 1, x = g.wrap_x_near(tn.tx0 + tid % 18 - 1);
                 ptx::prefetch_l2(X + (size_t)tn.b * xplane + ((size_t)g.xrow_near(r) * g.W + x) * NC);
             }
@@ -515,36 +496,16 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
         const int m_ep = quad * 32 + lane;                 // TMEM lane = cell of the tile this thread finishes
         uint8_t* stg_e = sm + k1b::STG_E;
         uint8_t* stg_v = sm + k1b::STG_V;
-        const bool tiny = g.W < 2 * APRON || (g.wrap_y && g.H < 2 * APRON);
         for (int first = 0, end; first < items.count; first = end) {
             end = items.end(first);                        // items first .. end - 1 are of this tile
             const int h0 = items.head(first) - first;
-            const CaTile t = ca_tile(items.tile(first), tiles_per_grid, g.tiles_x, -g.he);
+            const CaTile t = ca_tile(items.tile(first), tiles_per_grid, g);
             const int set = t.b / g.per_set;
-            const int r_ep = t.ty0 + (m_ep >> 4), x_ep = t.tx0 + (m_ep & 15);
-            const bool valid_ep = r_ep < g.H + g.he && x_ep < g.W;
-            // Apron positions that wrap onto this thread's cell (the store warp's TMA store covers the cell itself
-            // and whatever hangs over the far edge).
             const int cy = m_ep >> 4, cx = m_ep & 15;
-            // the last two columns and rows of the grid, where this tile has them (PIECES: both or neither)
-            const int c2 = x_ep - (g.W - APRON), r2 = r_ep - (g.H - APRON);
-            const int mc = c2 >= 0 && c2 < APRON ? cy * APRON + c2 : -1;                      // cell of the small staging tiles,
-            const int mr = g.wrap_y && r2 >= 0 && r2 < APRON ? r2 * TBW + cx : -1;            // -1 for none
-            // without PIECES: per-thread targets (named registers, not an indexed array: an array would live
-            // in local memory and put a load in front of every duplicate store).  Grids narrower or shorter than
-            // twice the apron can wrap more than once and take the general loop.
-            size_t off_x = 0, off_y = 0, off_xy = 0;
-            bool dup_x = false, dup_y = false;
-            if (!PIECES && valid_ep && !tiny) {
-                const int xd = x_ep < APRON ? x_ep + g.W : (x_ep >= g.W - APRON ? x_ep - g.W : -100);
-                const int rd = !g.wrap_y ? -100 : (r_ep < APRON ? r_ep + g.H : (r_ep >= g.H - APRON ? r_ep - g.H : -100));
-                dup_x = xd != -100;
-                dup_y = rd != -100;
-                if (dup_x) off_x = ((size_t)(r_ep + APRON) * g.ev_w + xd + APRON) * HD;
-                if (dup_y) off_y = ((size_t)(rd + APRON) * g.ev_w + x_ep + APRON) * HD;
-                if (dup_x && dup_y) off_xy = ((size_t)(rd + APRON) * g.ev_w + xd + APRON) * HD;
-            }
-            const bool any_dup = !PIECES && valid_ep && (dup_x || dup_y || tiny);
+            // the last two columns and rows of the grid, where this tile has them and they are copied
+            const int c2 = t.tx0 + cx - (g.W - APRON), r2 = t.ty0 + cy - (g.H - APRON);
+            const int mc = g.copy_x && c2 >= 0 && c2 < APRON ? cy * APRON + c2 : -1;                      // cell of the small staging
+            const int mr = g.copy_y && r2 >= 0 && r2 < APRON ? r2 * TBW + cx : -1;            // tiles, -1 for none
             for (int i = first; i < end; ++i) {
                 const int h = h0 + i, tb = i & 1;
                 const float mus = __ldg(prm + ((size_t)set * NH + h) * PRM + 9);   // mu * s; Wp carries s and Wi carries log2(e)
@@ -592,58 +553,24 @@ k1_bf16(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ K1St
                     *reinterpret_cast<uint4*>(stg_e + swz(m_ep, qa + 1)) = e_hi;
                     *reinterpret_cast<uint4*>(stg_v + swz(m_ep, qa)) = v_lo;
                     *reinterpret_cast<uint4*>(stg_v + swz(m_ep, qa + 1)) = v_hi;
-                    if (PIECES) {
-                        if (mc >= 0) {
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COL_E + swz(mc, qa)) = e_lo;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COL_E + swz(mc, qa + 1)) = e_hi;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COL_V + swz(mc, qa)) = v_lo;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COL_V + swz(mc, qa + 1)) = v_hi;
-                        }
-                        if (mr >= 0) {
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_E + swz(mr, qa)) = e_lo;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_E + swz(mr, qa + 1)) = e_hi;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_V + swz(mr, qa)) = v_lo;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_V + swz(mr, qa + 1)) = v_hi;
-                        }
-                        if (mc >= 0 && mr >= 0) {
-                            const int mq = mr / TBW * APRON + mc % APRON;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COR_E + swz(mq, qa)) = e_lo;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COR_E + swz(mq, qa + 1)) = e_hi;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COR_V + swz(mq, qa)) = v_lo;
-                            *reinterpret_cast<uint4*>(sm + k1b::STG_COR_V + swz(mq, qa + 1)) = v_hi;
-                        }
+                    if (mc >= 0) {
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COL_E + swz(mc, qa)) = e_lo;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COL_E + swz(mc, qa + 1)) = e_hi;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COL_V + swz(mc, qa)) = v_lo;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COL_V + swz(mc, qa + 1)) = v_hi;
                     }
-                    if (any_dup) {
-                        __nv_bfloat16* Eh = E + ((size_t)t.b * NH + h) * eplane + half * 32 + sub * 16;
-                        __nv_bfloat16* Vh = V + ((size_t)t.b * NH + h) * eplane + half * 32 + sub * 16;
-                        if (!tiny) {
-                            if (dup_x) {
-                                uint4* pE = reinterpret_cast<uint4*>(Eh + off_x);
-                                uint4* pV = reinterpret_cast<uint4*>(Vh + off_x);
-                                pE[0] = e_lo; pE[1] = e_hi; pV[0] = v_lo; pV[1] = v_hi;
-                            }
-                            if (dup_y) {
-                                uint4* pE = reinterpret_cast<uint4*>(Eh + off_y);
-                                uint4* pV = reinterpret_cast<uint4*>(Vh + off_y);
-                                pE[0] = e_lo; pE[1] = e_hi; pV[0] = v_lo; pV[1] = v_hi;
-                            }
-                            if (dup_x && dup_y) {
-                                uint4* pE = reinterpret_cast<uint4*>(Eh + off_xy);
-                                uint4* pV = reinterpret_cast<uint4*>(Vh + off_xy);
-                                pE[0] = e_lo; pE[1] = e_hi; pV[0] = v_lo; pV[1] = v_hi;
-                            }
-                        } else {
-                            for (int ky = -2 * APRON; ky <= 2 * APRON; ++ky)
-                                for (int kx = -2 * APRON; kx <= 2 * APRON; ++kx) {
-                                    if ((ky != 0 && !g.wrap_y) || (ky == 0 && kx == 0)) continue;
-                                    const int rr = r_ep + ky * g.H, xx = x_ep + kx * g.W;
-                                    if (rr < -APRON || rr >= g.H + APRON || xx < -APRON || xx >= g.W + APRON) continue;
-                                    const size_t off = ((size_t)(rr + APRON) * g.ev_w + xx + APRON) * HD;
-                                    uint4* pE = reinterpret_cast<uint4*>(Eh + off);
-                                    uint4* pV = reinterpret_cast<uint4*>(Vh + off);
-                                    pE[0] = e_lo; pE[1] = e_hi; pV[0] = v_lo; pV[1] = v_hi;
-                                }
-                        }
+                    if (mr >= 0) {
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_E + swz(mr, qa)) = e_lo;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_E + swz(mr, qa + 1)) = e_hi;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_V + swz(mr, qa)) = v_lo;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_ROW_V + swz(mr, qa + 1)) = v_hi;
+                    }
+                    if (mc >= 0 && mr >= 0) {
+                        const int mq = mr / TBW * APRON + mc % APRON;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COR_E + swz(mq, qa)) = e_lo;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COR_E + swz(mq, qa + 1)) = e_hi;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COR_V + swz(mq, qa)) = v_lo;
+                        *reinterpret_cast<uint4*>(sm + k1b::STG_COR_V + swz(mq, qa + 1)) = v_hi;
                     }
                 }
                 ptx::fence_proxy_async();
@@ -1383,9 +1310,7 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
             return -1;
         }
     }
-    p.k1_pieces = g.W >= 2 * APRON && g.W % TBW != 1 && (!g.wrap_y || (g.H >= 2 * APRON && g.H % TBH != 1));
-    if (cudaFuncSetAttribute(k1_bf16<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, k1b::SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(k1_bf16<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, k1b::SMEM) != cudaSuccess ||
+    if (cudaFuncSetAttribute(k1_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, k1b::SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(k2_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, k2m::SMEM) != cudaSuccess) {
         bf16_error_ref() = "could not opt in to the kernels' dynamic shared memory";
         return -1;
@@ -1402,10 +1327,9 @@ inline int bf16_setup(Bf16Plan& p, const __nv_bfloat16* w1, const __nv_bfloat16*
     return 0;
 }
 
-inline int bf16_k1(Bf16Plan& p, const __nv_bfloat16* X, const float* scale, const float* prm, __nv_bfloat16* E,
-                   __nv_bfloat16* V, int* status, const Geom& g, cudaStream_t st) {
-    return launch_pdl(p.k1_pieces ? k1_bf16<true> : k1_bf16<false>, p.k1_grid, k1b::THREADS, k1b::SMEM, st, p.map_w1, p.st, X, scale, prm,
-                      E, V, status, p.k1_tiles * g.B, p.k1_tiles, g) == cudaSuccess ? 0 : -1;
+inline int bf16_k1(Bf16Plan& p, const __nv_bfloat16* X, const float* scale, const float* prm, int* status, const Geom& g, cudaStream_t st) {
+    return launch_pdl(k1_bf16, p.k1_grid, k1b::THREADS, k1b::SMEM, st, p.map_w1, p.st, X, scale, prm,
+                      status, p.k1_tiles * g.B, p.k1_tiles, g) == cudaSuccess ? 0 : -1;
 }
 
 inline int bf16_k2(Bf16Plan& p, __nv_bfloat16* X, const float* scale, const __nv_bfloat16*, const __nv_bfloat16*,

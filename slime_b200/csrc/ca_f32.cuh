@@ -208,7 +208,7 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
         uint32_t tiles = 0;
         for (int n = 0; n < items.count; ++n) {
             if (!items.first(n)) continue;
-            const CaTile t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
+            const CaTile t = ca_tile(items.tile(n), tiles_per_grid, g);
             ptx::mbar_wait(xh_empty, (tiles & 1) ^ 1, status, 330);
             if (lane == 0) ptx::mbar_expect_tx(xh_full, k1f::XH_BYTES);
             __syncwarp();
@@ -236,7 +236,7 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
             const int h = items.head(n), tb = n & 1;
             const bool first = items.first(n);
             if (first) {
-                t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
+                t = ca_tile(items.tile(n), tiles_per_grid, g);
                 const float4 s4 = __ldg(reinterpret_cast<const float4*>(scale + t.b * NC + c4 * 4));
                 sc[0] = ptx::make_f2(s4.x, s4.y);
                 sc[1] = ptx::make_f2(s4.z, s4.w);
@@ -324,7 +324,7 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
         for (int n = 0; n < items.count; ++n) {
             const int h = items.head(n), tb = n & 1;
             if (items.first(n)) {
-                t = ca_tile(items.tile(n), tiles_per_grid, g.tiles_x, -g.he);
+                t = ca_tile(items.tile(n), tiles_per_grid, g);
                 apron.tile(t, quad, lane, g);
             }
             const float mus = __ldg(prm + ((size_t)(t.b / g.per_set) * NH + h) * PRM + 9);   // mu * s; Wp carries s and Wi carries log2(e)
@@ -374,7 +374,7 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                     apron.staged(t, quad, g, [&](int px, int py) { ptx::tma_store_4d(is_e ? &map_es : &map_vs, tile, d0, px, py, t.b * NH + h); });
                     ptx::bulk_commit();
                 }
-                apron.own(t, quad, lane, g, [&](int cell) {
+                apron.own([&](int cell) {
                     float4* p = reinterpret_cast<float4*>((is_e ? E : V) + ((size_t)t.b * NH + h) * eplane + (size_t)cell * HD + d0);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) p[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);

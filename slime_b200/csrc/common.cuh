@@ -28,6 +28,10 @@ struct Geom {
     int ev_h, ev_w;  // rows and columns of one E/V plane.  fp32 path: H + 2*he rows of W cells.  bf16 path: the
                      // plane carries a 2-cell apron all around, (H + 4) x (W + 4), holding wrapped copies (or, in
                      // stripe mode, the computed halo rows), so the second kernel reads it without any wrap logic
+    // k1's tiles (see k1_origin): the first one's column and row; multiples of W and H that bring a negative position near the
+    // first tile to one that is not; whether the apron's columns and rows are copies
+    int col0, row0, add_x, add_y;
+    bool copy_x, copy_y;
     float dt;
 
     __host__ __device__ int state_rows() const { return H + 2 * hx; }
@@ -35,13 +39,13 @@ struct Geom {
     __device__ int wrap_x(int x) const { x %= W; return x < 0 ? x + W : x; }
     // the same for positions at most one tile outside the grid: no division (a handful of steps on grids smaller than that)
     __device__ int wrap_x_near(int x) const {
-        if (x < 0) x += W;
+        if (x < 0) x += add_x;
         while (x >= W) x -= W;
         return x;
     }
     __device__ int xrow_near(int r) const {
         if (!wrap_y) return xrow(r);
-        if (r < 0) r += H;
+        if (r < 0) r += add_y;
         while (r >= H) r -= H;
         return r;
     }
@@ -58,6 +62,20 @@ struct Geom {
         return r + he;
     }
 };
+
+// Where k1's tiles start.  With the two-cell apron they have H + 4 rows and W + 4 columns to fill, and where that takes no more
+// tiles than the grid itself they start in the apron and compute it whole, from the wrapped state: the same bits as a copy.
+// Otherwise they start at the grid, and the apron holds copies of its edge cells; the last two columns (rows) then lie within
+// one tile, and the grid is no smaller than twice the apron.
+inline void k1_origin(Geom& g, int tile_w, int tile_h, int apron) {
+    auto tiles = [](int n, int of) { return (n + of - 1) / of; };
+    g.copy_x = tiles(g.W + 2 * apron, tile_w) > tiles(g.W, tile_w);
+    g.copy_y = g.wrap_y && tiles(g.H + 2 * apron, tile_h) > tiles(g.H, tile_h);
+    g.col0 = g.copy_x ? 0 : -apron;
+    g.row0 = g.copy_y ? 0 : g.wrap_y ? -apron : -g.he;
+    g.add_x = tiles(apron + 1, g.W) * g.W;
+    g.add_y = tiles(apron + 1, g.H) * g.H;
+}
 
 // Launch with programmatic stream serialization: the kernel starts its set-up while the one before it drains (it waits
 // for that with ptx::pdl_wait before it reads or writes global memory).

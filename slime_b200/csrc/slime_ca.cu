@@ -181,8 +181,7 @@ int step_kernels(slime_ca* h, void* emit, cudaStream_t st, cudaEvent_t* ev = nul
     const K2Sums fin{h->partial, is_bf16(h) ? 0 : h->partial_lo, h->k2_tiles > FUSE_PARTIALS ? nullptr : h->tickets, out};
     if (ev) CK(h, cudaEventRecord(ev[0], st));
     if (is_bf16(h)) {
-        if (bf16_k1(h->bf, (const __nv_bfloat16*)h->X, h->scale, h->prm, (__nv_bfloat16*)h->E, (__nv_bfloat16*)h->V,
-                    h->dev_status, g, st) != 0)
+        if (bf16_k1(h->bf, (const __nv_bfloat16*)h->X, h->scale, h->prm, h->dev_status, g, st) != 0)
             return fail(h, SLIME_CA_ECUDA, std::string("bf16 k1 launch: ") + cudaGetErrorString(cudaGetLastError()));
         ++h->launches;
         if (ev) CK(h, cudaEventRecord(ev[1], st));
@@ -335,6 +334,7 @@ int slime_ca_create(const slime_ca_config* cfg, slime_ca** out) {
     g.B = cfg->batch; g.H = cfg->height; g.W = cfg->width;
     g.hx = cfg->stripe ? 3 : 0; g.he = cfg->stripe ? 2 : 0;
     g.wrap_y = cfg->stripe ? 0 : 1;
+    k1_origin(g, TBW, TBH, APRON);
     g.per_set = cfg->batch / cfg->n_weight_sets;
     g.dt = cfg->dt;
     h->esz = cfg->dtype == SLIME_CA_BF16 ? 2 : 4;
@@ -1166,8 +1166,7 @@ int slime_ca_occupancy(slime_ca* h, float* occupancy) {
     int b1 = 0, b2 = 0, t1, t2;
     if (is_bf16(h)) {
         t1 = k1b::THREADS; t2 = k2m::THREADS;
-        if (h->bf.k1_pieces) CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_bf16<true>, t1, k1b::SMEM));
-        else CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_bf16<false>, t1, k1b::SMEM));
+        CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k1_bf16, t1, k1b::SMEM));
         CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k2_bf16, t2, k2m::SMEM));
     } else {
         t1 = k1f::THREADS; t2 = k2f::THREADS;
