@@ -36,7 +36,7 @@ enum slime_ca_status {
 };
 
 enum slime_ca_dtype {
-    SLIME_CA_F32 = 0,  /* fp32 storage and arithmetic (SIMT)                                             */
+    SLIME_CA_F32 = 0,  /* fp32 storage and arithmetic (products in three bf16 parts on the tensor cores)  */
     SLIME_CA_BF16 = 1  /* bf16 storage of state/weights/intermediates, fp32 accumulate, tcgen05 projections */
 };
 
@@ -178,7 +178,7 @@ int slime_ca_buffer(slime_ca* h, int which, void** dev_ptr, size_t* bytes);
 /*
  * Fitness of every grid from V' of the last two steps (needs keep_vprime and at least two steps):
  * HOST fp32 arrays of `batch` elements, any of which may be NULL.  rank = mean over heads of the
- * exp-entropy rank of that head's 64x64 Gram spectrum (Jacobi), coherence = Pearson r between the two
+ * exp-entropy rank of that head's 64x64 Gram spectrum, coherence = Pearson r between the two
  * steps, fitness = rank * coherence, hunger = 1 - coherence.  Replaces fitness_fused_kernel and its
  * children (slime/kernels/warp_ca.cu:66-226) and the hunger kernel (:229-240).  Synchronises `stream`.
  */
