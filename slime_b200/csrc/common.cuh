@@ -25,9 +25,8 @@ struct Geom {
     int wrap_y;      // 1 = torus in y
     int per_set;     // grids per weight set
     int tiles_x;     // tiles per row of tiles
-    int ev_h, ev_w;  // rows and columns of one E/V plane.  fp32 path: H + 2*he rows of W cells.  bf16 path: the
-                     // plane carries a 2-cell apron all around, (H + 4) x (W + 4), holding wrapped copies (or, in
-                     // stripe mode, the computed halo rows), so the second kernel reads it without any wrap logic
+    int ev_h, ev_w;  // rows and columns of one E/V plane: (H + 4) x (W + 4), a 2-cell apron all around that holds what wraps onto
+                     // it (or, in stripe mode, the computed halo rows), so the second kernel reads it without any wrap logic
     // k1's tiles (see k1_origin): the first one's column and row; multiples of W and H that bring a negative position near the
     // first tile to one that is not; whether the apron's columns and rows are copies
     int col0, row0, add_x, add_y;
@@ -35,9 +34,7 @@ struct Geom {
     float dt;
 
     __host__ __device__ int state_rows() const { return H + 2 * hx; }
-    __host__ __device__ int ev_rows() const { return ev_h; }
-    __device__ int wrap_x(int x) const { x %= W; return x < 0 ? x + W : x; }
-    // the same for positions at most one tile outside the grid: no division (a handful of steps on grids smaller than that)
+    // column of the grid for a position at most one tile outside it: no division (a handful of steps on grids smaller than that)
     __device__ int wrap_x_near(int x) const {
         if (x < 0) x += add_x;
         while (x >= W) x -= W;
@@ -54,12 +51,6 @@ struct Geom {
         if (wrap_y) { r %= H; return r < 0 ? r + H : r; }
         r = r < -hx ? -hx : (r > H + hx - 1 ? H + hx - 1 : r);
         return r + hx;
-    }
-    // physical row in an E/V plane of own-coordinate row r
-    __device__ int erow(int r) const {
-        if (wrap_y) { r %= H; return r < 0 ? r + H : r; }
-        r = r < -he ? -he : (r > H + he - 1 ? H + he - 1 : r);
-        return r + he;
     }
 };
 
