@@ -660,7 +660,7 @@ __device__ __forceinline__ void k2_epilogue(const CaTile& t, uint32_t acc_taddr,
 // =============================================================================================================
 // k2.  The grid is cut into macro tiles of 32 columns x 32 rows; a macro tile is eight 4 x 32-cell tiles (UMMA
 // M = 128) stacked in y, one 64-column TMEM accumulator each (8 x 64 = all 512 columns; launches with too few macro
-// tiles to fill the GPU use 4, 2 or 1 tiles per macro tile instead).  For one head
+// tiles to fill the GPU use fewer tiles per macro tile instead, see k2_macro_tiles).  For one head
 // after the other the kernel marches down the macro tile four rows at a time, carrying the vertical running sums of
 // both box sums in registers from block to block, so every E and V row of the strip is loaded and summed once per
 // head (square tiles with a 2-cell ring all round re-read 1.9x the E rows and 1.4x the V rows at 8 x 16 cells).  A
@@ -797,8 +797,8 @@ k2_bf16(const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUte
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + k2m::BARS);
-    uint64_t* full = bars;                           // [5] block landed                              (waits: A)
-    uint64_t* empty = full + k2m::NSTAGE;            // [5] B is done with the stage (256 arrivals)   (waits: TMA producer)
+    uint64_t* full = bars;                           // [4] block landed                              (waits: A)
+    uint64_t* empty = full + k2m::NSTAGE;            // [4] B is done with the stage (256 arrivals)   (waits: TMA producer)
     uint64_t* vp_full = empty + k2m::NSTAGE;         // [2] operand tile written (256 arrivals)       (waits: UMMA issuer)
     uint64_t* vp_empty = vp_full + 2;                // [2] the UMMAs reading it are done             (waits: B)
     uint64_t* wo_full = vp_empty + 2;                // [2] Wo slice landed                           (waits: UMMA issuer)

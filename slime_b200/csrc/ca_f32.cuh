@@ -85,6 +85,9 @@ static_assert(SMEM <= 227 * 1024, "k1 (fp32) shared memory");
 //   warp 21     loads the tile's state halo, a bulk copy per row (two where the row wraps): with loads by the stencil group
 //               a change of tile cost 14 000 cycles, two to three items
 // (24 warps: one more and a thread has 72 registers instead of 80.)
+// At X[64,128,128,64] 1.68-1.75 ms (2.7 TB/s of the 4.35 KB a cell; the SIMT step it is half of took 14.1 ms, this one 3.2): no
+// unit is full (issue slots half, tensor pipe a third, DRAM a third of the time), timing-only variants without stores
+// take 1.37 ms, without the stencil 1.57, without the I | V products 1.63.  Runs of more than some 15 ms meet the power cap.
 __global__ void __launch_bounds__(k1f::THREADS, 1)
 k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_es,
        const __grid_constant__ CUtensorMap map_vs, const float* __restrict__ X, const float* __restrict__ scale,
@@ -401,6 +404,8 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
 //   warps 20-23  P: adds every working accumulator to the tile's running sum in TMEM, rounded to nearest (16 half-heads:
 //                on the tensor core that sum would be truncated 192 times); after the last half-head X+ = scale X + dt Y,
 //                written back through shared memory, and the tile's channel sums in fp64
+// At X[64,128,128,64] 1.45-1.55 ms (3.2 TB/s); without A's box sums it takes 1.29, without B's 1.17, without the products 1.40:
+// they share the issue slots (half used), the shared-memory pipe (over half) and its latency.
 namespace k2f {
 constexpr int SW = k2m::SW, BR = k2m::BR, NB = 6;       // strip width, rows per block, blocks per macro tile at most
 constexpr int NHH = 2 * NH;                             // half-heads
