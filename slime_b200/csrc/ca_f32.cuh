@@ -300,10 +300,23 @@ k1_f32(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUten
                 ptx::tc_fence_after();
                 uint32_t a[3][16];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const float4 v = *reinterpret_cast<const float4*>(src + q * 16), s4 = __ldg(ss + q);
-                    split3(ptx::mul2(ptx::make_f2(v.x, v.y), ptx::make_f2(s4.x, s4.y)), a[0][2 * q], a[1][2 * q], a[2][2 * q]);
-                    split3(ptx::mul2(ptx::make_f2(v.z, v.w), ptx::make_f2(s4.z, s4.w)), a[0][2 * q + 1], a[1][2 * q + 1], a[2][2 * q + 1]);
+                for (int q0 = 0; q0 < 8; q0 += 4) {
+                    // the lanes' cells lie 256 bytes apart: each lane reads its four chunks in an order of its own (16-byte
+                    // loads of eight lanes then meet two to a bank, not eight) and puts them right by swaps
+                    float4 v[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) v[k] = *reinterpret_cast<const float4*>(src + (q0 + (k ^ (lane & 3))) * 16);
+#pragma unroll
+                    for (int k = 0; k < 4; k += 2) { const float4 lo = v[k], hi = v[k + 1]; v[k] = lane & 1 ? hi : lo; v[k + 1] = lane & 1 ? lo : hi; }
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) { const float4 lo = v[k], hi = v[k + 2]; v[k] = lane & 2 ? hi : lo; v[k + 2] = lane & 2 ? lo : hi; }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int q = q0 + k;
+                        const float4 s4 = __ldg(ss + q);
+                        split3(ptx::mul2(ptx::make_f2(v[k].x, v[k].y), ptx::make_f2(s4.x, s4.y)), a[0][2 * q], a[1][2 * q], a[2][2 * q]);
+                        split3(ptx::mul2(ptx::make_f2(v[k].z, v[k].w), ptx::make_f2(s4.z, s4.w)), a[0][2 * q + 1], a[1][2 * q + 1], a[2][2 * q + 1]);
+                    }
                 }
 #pragma unroll
                 for (int pa = 0; pa < 3; ++pa) ptx::tmem_st16(dst + pa * 32, a[pa]);
